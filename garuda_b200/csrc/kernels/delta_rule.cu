@@ -17,11 +17,16 @@
 //   delta_out         per head: o / rms(o) * weight * sigmoid(gate)
 //   delta_decode      all of the above for steps of one token per request, one block per
 //                     (request, head)
-// A token's result depends on its request's earlier tokens only through the state, which is
-// carried bit for bit: cutting a prompt anywhere gives the same numbers.
+//   delta_chunk_factors, delta_chunk::walk
+//                     the same for long stretches of tokens in a bfloat16 run, 32 tokens at a time
+//                     (delta_chunk.cuh)
+// In the token-by-token kernels a token's result depends on its request's earlier tokens only through the
+// state, which is carried bit for bit: cutting a prompt anywhere gives the same numbers. The chunked ones add the same
+// terms in another order, so there a cut moves the last bits.
 #include <type_traits>
 
 #include "common.cuh"
+#include "delta_chunk.cuh"
 
 namespace {
 
@@ -50,12 +55,13 @@ delta_prepare_kernel(const float* __restrict__ proj, int P, const float* __restr
                      long long state_stride, const WT* __restrict__ a_log, const WT* __restrict__ dt_bias,
                      const int32_t* __restrict__ token_req, const int32_t* __restrict__ cu_q,
                      const int32_t* __restrict__ slots, float* __restrict__ prep, int W, int H, int G, int dim,
-                     int vdim, int per_head) {
+                     int vdim, int per_head, int below) {
   gb::pdl_launch_dependents();
   gb::pdl_wait();
   extern __shared__ float act[];        // [C]
   const int t = blockIdx.x;
   const int r = token_req[t];
+  if (below > 0 && cu_q[r + 1] - cu_q[r] >= below) return;      // the chunked kernels' request
   const int j = t - cu_q[r];
   const int slot = slots[r];
   const float* kept = slot >= 0 ? conv_state + (size_t)slot * state_stride : nullptr;
@@ -131,8 +137,9 @@ template <int MAXD, bool EXACT>
 __global__ void __launch_bounds__(REC_THREADS)
 delta_recurrence_kernel(const float* __restrict__ prep, int W, const int32_t* __restrict__ cu_q,
                         const int32_t* __restrict__ slots, float* __restrict__ state, long long state_stride, int H,
-                        int G, int dim, int vdim, float* __restrict__ out) {
+                        int G, int dim, int vdim, int below, float* __restrict__ out) {
   gb::pdl_wait();
+  if (below > 0 && cu_q[blockIdx.y + 1] - cu_q[blockIdx.y] >= below) return;      // the chunked kernels' request
   constexpr int MINE = MAXD / SPLIT;
   extern __shared__ __align__(16) float stage[];      // 2 x [CHUNK][3 SPLIT per + 32 + 4]
   // a thread's rows, rounded up to whole 16-byte pieces, and one piece more: the four slices start
@@ -242,6 +249,215 @@ delta_recurrence_kernel(const float* __restrict__ prep, int W, const int32_t* __
       const int d = i * SPLIT + sub;
       if (d < dim) S_g[(size_t)d * vdim] = S[i];
     }
+  }
+}
+
+// What the walk of delta_chunk.cuh needs of a chunk and a head: convolution, SiLU, unit vectors, decays and beta as in
+// delta_prepare, then, with D_i the product of the decays up to token i,
+//     L_ij = beta_i sum_d k_i k_j D_i / D_j (j < i),   B_ij = sum_d q_i k_j D_i / D_j (j <= i)
+//     W = (I + L)^-1 beta (D k),   VP = (I + L)^-1 beta v,   Q = D q - B W,   OP = B VP,   K1_j = k_j D_last / D_j
+// The quotients D_i / D_j are running products of decays from j on (never above one, so nothing overflows and what
+// underflows is nothing), and the triangular system is solved by substitution, a thread per column of W and VP. 32-bit multiply-adds.
+// grid (chunk numbers, H), 256 threads; taps of at most four (the older ones' weights are zero where there are fewer).
+template <int DIM, typename WT>
+__global__ void __launch_bounds__(256, 3)
+delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* __restrict__ second, int P2,
+                           const WT* __restrict__ conv_w, int taps, const float* __restrict__ conv_state, long long conv_stride,
+                           const WT* __restrict__ a_log, const WT* __restrict__ dt_bias, const int32_t* __restrict__ cu_q,
+                           const int32_t* __restrict__ slots, float* __restrict__ blocks, int R, int H, int G, int vdim, int per_head,
+                           int cut) {
+  using namespace delta_chunk;
+  using delta_chunk::C;
+  gb::pdl_launch_dependents();
+  gb::pdl_wait();
+  constexpr int LD = DIM + 4, VEC = DIM / 32;
+  extern __shared__ __align__(16) float sh[];
+  float* sk = sh;                        // [C][LD]: k, then D k
+  float* sq = sk + C * LD;               // [C][LD]: q, then D q
+  float* sg = sq + C * LD;               // [C][LD]: decays
+  float* sL = sg + C * LD;               // [C][LT], a row per j (transposed)
+  float* sB = sL + C * LT;               // [C][LT], likewise
+  float* beta = sB + C * LT;             // [C]
+  const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int r, first, n, at;
+  if (!find_chunk(blockIdx.x, cu_q, R, cut, r, first, n, at)) return;
+  const Layout lay{DIM, vdim, 0};
+  float* block = blocks + ((size_t)blockIdx.x * H + h) * lay.floats();
+  const int slot = slots[r], kvh = h / (H / G), CH = 2 * G * DIM + H * vdim;
+  const float* kept = slot >= 0 ? conv_state + (size_t)slot * conv_stride : nullptr;
+  // Convolution and SiLU of a channel's tokens, eight at a time: take(i, value) for i = 0 .. C - 1
+  auto convolve = [&](int ch, auto&& take) {
+    float w[4], x[3];                    // by lag; the inputs in front of the chunk
+#pragma unroll
+    for (int lag = 0; lag < 4; ++lag) w[lag] = lag < taps ? gb::to_float<WT>(conv_w[(size_t)ch * taps + taps - 1 - lag]) : 0.f;
+#pragma unroll
+    for (int lag = 1; lag < 4; ++lag) x[lag - 1] = lag < taps ? conv_input(proj, P, first, at, lag, ch, kept, CH, taps) : 0.f;
+#pragma unroll
+    for (int i0 = 0; i0 < C; i0 += 8) {
+      float in[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) in[e] = i0 + e < n ? proj[(size_t)(first + i0 + e) * P + ch] : 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        float acc = fmaf(w[3], x[2], 0.f);
+        acc = fmaf(w[2], x[1], acc);
+        acc = fmaf(w[1], x[0], acc);
+        acc = fmaf(w[0], in[e], acc);
+        x[2] = x[1], x[1] = x[0], x[0] = in[e];
+        take(i0 + e, i0 + e < n ? silu(acc) : 0.f);
+      }
+    }
+  };
+  for (int c = tid; c < 2 * DIM; c += 256) {
+    const bool query = c < DIM;
+    float* to = query ? sq + c : sk + c - DIM;
+    convolve(query ? kvh * DIM + c : (G + kvh) * DIM + c - DIM, [&](int i, float v) { to[i * LD] = v; });
+  }
+  const float rate = expf(gb::to_float<WT>(a_log[h]));
+  if (per_head) {
+    // one decay for all key channels: every thread's warp makes one token's at a time
+    for (int t = warp; t < C; t += 8) {
+      const float g = t < n ? expf(-rate * softplus(second[(size_t)(first + t) * P2 + h] + gb::to_float<WT>(dt_bias[h]))) : 1.f;
+      for (int d = lane; d < DIM; d += 32) sg[t * LD + d] = g;
+    }
+  } else {
+#pragma unroll 4
+    for (int i = tid; i < C * DIM; i += 256) {
+      const int t = i / DIM, d = i % DIM, c = h * DIM + d;
+      sg[t * LD + d] = t < n ? expf(-rate * softplus(second[(size_t)(first + t) * P2 + c] + gb::to_float<WT>(dt_bias[c]))) : 1.f;
+    }
+  }
+  for (int i = tid; i < 2 * C * LT; i += 256) sL[i] = 0.f;
+  if (tid < C) beta[tid] = tid < n ? sigmoid(proj[(size_t)(first + tid) * P + CH + h]) : 0.f;
+  __syncthreads();
+#pragma unroll
+  for (int row = warp; row < 2 * C; row += 8) {
+    float* v = row < C ? sq + row * LD : sk + (row - C) * LD;
+    float x[VEC], ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) x[e] = v[lane + 32 * e], ss = fmaf(x[e], x[e], ss);
+    ss = gb::warp_sum(ss);
+    float inv = 1.0f / sqrtf(ss + 1e-6f);
+    if (row < C) inv *= 1.0f / sqrtf((float)DIM);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) v[lane + 32 * e] = x[e] * inv;
+  }
+  __syncthreads();
+  {
+    // L and B: a warp has four keys j, each decayed on from token to token; early and late keys paired on a scheduler
+    const int j0 = (warp < 4 ? warp : 11 - warp) * 4, d0 = lane * VEC;
+    pair_t p[4][VEC / 2];
+    auto row = [&](const float* m, int i, pair_t (&x)[VEC / 2]) {
+      if (VEC == 4) {
+        const pair2_t f = *reinterpret_cast<const pair2_t*>(m + i * LD + d0);
+        x[0] = f.a, x[VEC / 2 - 1] = f.b;
+      } else {
+        x[0] = *reinterpret_cast<const pair_t*>(m + i * LD + d0);
+      }
+    };
+    auto dot = [](const pair_t (&a)[VEC / 2], const pair_t (&b)[VEC / 2]) {
+      pair_t s = mul2(a[0], b[0]);
+#pragma unroll
+      for (int e = 1; e < VEC / 2; ++e) s = fma2(a[e], b[e], s);
+      const float2 f = both(s);
+      return f.x + f.y;
+    };
+    auto keep = [&](int i, float (&v)[8]) {
+      const float sum = sum_of_eight(v, lane);
+      const int which = lane >> 2, j = j0 + (which & 3);
+      if ((lane & 3) == 0) {
+        if (which < 4) {
+          if (j < i) sL[j * LT + i] = beta[i] * sum;
+        } else if (j <= i) {
+          sB[j * LT + i] = sum;
+        }
+      }
+    };
+#pragma unroll
+    for (int ii = 0; ii < 4; ++ii) {       // the tokens of the four keys themselves
+      const int i = j0 + ii;
+      if (i >= n) break;
+      pair_t g[VEC / 2], k[VEC / 2], q[VEC / 2];
+      row(sg, i, g), row(sk, i, k), row(sq, i, q);
+      float v[8];
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+#pragma unroll
+        for (int e = 0; e < VEC / 2; ++e) p[jj][e] = jj < ii ? mul2(p[jj][e], g[e]) : k[e];
+        v[jj] = jj < ii ? dot(p[jj], k) : 0.f;
+        v[4 + jj] = jj <= ii ? dot(p[jj], q) : 0.f;
+      }
+      keep(i, v);
+    }
+#pragma unroll 2
+    for (int i = j0 + 4; i < n; ++i) {
+      pair_t g[VEC / 2], k[VEC / 2], q[VEC / 2];
+      row(sg, i, g), row(sk, i, k), row(sq, i, q);
+      float v[8];
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+#pragma unroll
+        for (int e = 0; e < VEC / 2; ++e) p[jj][e] = mul2(p[jj][e], g[e]);
+        v[jj] = dot(p[jj], k);
+        v[4 + jj] = dot(p[jj], q);
+      }
+      keep(i, v);
+    }
+  }
+  __syncthreads();
+  if (tid < DIM) {                       // a thread per channel
+    float run = 1.f;
+#pragma unroll
+    for (int j0 = C - 8; j0 >= 0; j0 -= 8) {
+      float x[8];
+#pragma unroll
+      for (int e = 7; e >= 0; --e) {
+        x[e] = sk[(j0 + e) * LD + tid] * run;
+        run *= sg[(j0 + e) * LD + tid];
+      }
+      float4* to = reinterpret_cast<float4*>(block + lay.k1(j0, tid));
+      to[0] = make_float4(x[0], x[1], x[2], x[3]), to[1] = make_float4(x[4], x[5], x[6], x[7]);
+    }
+    block[lay.last() + tid] = run;
+    run = 1.f;
+#pragma unroll 8
+    for (int i = 0; i < C; ++i) sk[i * LD + tid] *= run *= sg[i * LD + tid];
+  } else if (tid >= 128 && tid < 128 + DIM) {
+    float run = 1.f;
+#pragma unroll 8
+    for (int i = 0; i < C; ++i) sq[i * LD + tid - 128] *= run *= sg[i * LD + tid - 128];
+  }
+  __syncthreads();
+  for (int c = tid; c < DIM + vdim; c += 256) {
+    const bool key = c < DIM;            // the same for a warp
+    pair_t w[C / 2], o[C / 2];
+    if (key) {
+#pragma unroll
+      for (int i = 0; i < C; i += 2) w[i / 2] = make_pair(beta[i] * sk[i * LD + c], beta[i + 1] * sk[(i + 1) * LD + c]);
+    } else {
+      float even = 0.f;
+      convolve(2 * G * DIM + h * vdim + c - DIM, [&](int i, float v) {
+        if (i & 1) w[i / 2] = make_pair(even, beta[i] * v);
+        else even = beta[i] * v;
+      });
+    }
+#pragma unroll
+    for (int j = 0; j + 1 < C; ++j) {
+      add_row<true>(w, sL, j, -entry(w, j));
+      asm volatile("" ::: "memory");     // (else the rows are all fetched at once, and spilled)
+    }
+    if (key) store_rows(block, lay, 0, c, w);
+    else store_column(block + lay.vp() + (c - DIM) * C, w);
+#pragma unroll
+    for (int i = 0; i < C; i += 2) o[i / 2] = key ? make_pair(sq[i * LD + c], sq[(i + 1) * LD + c]) : 0ull;
+    const float sign = key ? -1.f : 1.f;
+#pragma unroll
+    for (int j = 0; j < C; ++j) {
+      add_row<false>(o, sB, j, sign * entry(w, j));
+      asm volatile("" ::: "memory");
+    }
+    if (key) store_rows(block, lay, C, c, o);
+    else store_column(block + lay.op() + (c - DIM) * C, o);
   }
 }
 
@@ -380,12 +596,13 @@ int check_sizes(const char* what, int H, int G, int dim, int vdim, int taps) {
 
 }  // namespace
 
-// state_stride, conv_stride: floats between two slots' states.
+// state_stride, conv_stride: floats between two slots' states. below (of delta_prepare and delta_recurrence): only requests
+// with fewer tokens in the step than this (0: all).
 GB_EXPORT int gb_delta_prepare(const float* proj, int P, const float* second, int P2, const void* conv_w, int w_dtype,
                                int taps, const float* conv_state, long long conv_stride, const void* a_log,
                                const void* dt_bias, const int32_t* token_req, const int32_t* cu_q, const int32_t* slots,
                                float* prep, int W, int T, int H, int G, int dim, int vdim, int per_head,
-                               cudaStream_t stream) {
+                               int below, cudaStream_t stream) {
   if (T <= 0) return GB_OK;
   int rc = check_sizes("delta_prepare", H, G, dim, vdim, taps);
   if (rc != GB_OK) return rc;
@@ -407,7 +624,7 @@ GB_EXPORT int gb_delta_prepare(const float* proj, int P, const float* second, in
     return gb::check_pdl_launch(
         gb::launch_pdl(delta_prepare_kernel<WT>, dim3(T), dim3(256), smem, stream, dim3(1, 1, 1), proj, P, second, P2,
                        (const WT*)conv_w, taps, conv_state, conv_stride, (const WT*)a_log, (const WT*)dt_bias, token_req,
-                       cu_q, slots, prep, W, H, G, dim, vdim, per_head),
+                       cu_q, slots, prep, W, H, G, dim, vdim, per_head, below),
         "delta_prepare");
   });
 }
@@ -421,7 +638,7 @@ GB_EXPORT int gb_delta_conv_state(const float* proj, int P, float* conv_state, l
 }
 
 GB_EXPORT int gb_delta_recurrence(const float* prep, int W, const int32_t* cu_q, const int32_t* slots, float* state,
-                                  long long state_stride, int R, int H, int G, int dim, int vdim, float* out,
+                                  long long state_stride, int R, int H, int G, int dim, int vdim, int below, float* out,
                                   cudaStream_t stream) {
   if (R <= 0) return GB_OK;
   int rc = check_sizes("delta_recurrence", H, G, dim, vdim, 1);
@@ -441,9 +658,46 @@ GB_EXPORT int gb_delta_recurrence(const float* prep, int W, const int32_t* cu_q,
     constexpr int MAXD = decltype(maxd)::value;
     auto kernel = dim == MAXD ? delta_recurrence_kernel<MAXD, true> : delta_recurrence_kernel<MAXD, false>;
     return gb::check_pdl_launch(gb::launch_after(kernel, grid, dim3(threads), smem, stream, dim3(1, 1, 1), prep, W, cu_q,
-                                               slots, state, state_stride, H, G, dim, vdim, out),
+                                               slots, state, state_stride, H, G, dim, vdim, below, out),
                                 "delta_recurrence");
   });
+}
+
+// Whether the chunked kernels take these sizes, and the floats of `blocks` for a step of T tokens of R requests (0: they do not).
+GB_EXPORT long long gb_delta_chunk_floats(int T, int R, int H, int G, int dim, int vdim, int taps) {
+  if (T <= 0 || R <= 0 || H < 1 || H > 65535 || R > 65535 || G < 1 || H % G || taps < 1 || taps > 4 || !delta_chunk::takes(dim, vdim)) return 0;
+  return (long long)delta_chunk::chunk_numbers(T, R) * H * delta_chunk::Layout{dim, vdim, 0}.floats();
+}
+
+// Requests of at least `cut` tokens: everything from the projected rows to the read-out o [T, H vdim] and the state. The rows
+// are those of delta_prepare; blocks starts on 16 bytes.
+GB_EXPORT int gb_delta_chunk(const float* proj, int P, const float* second, int P2, const void* conv_w, int w_dtype, int taps,
+                             const float* conv_state, long long conv_stride, const void* a_log, const void* dt_bias,
+                             const int32_t* cu_q, const int32_t* slots, float* state, long long state_stride, float* blocks, int T,
+                             int R, int H, int G, int dim, int vdim, int per_head, int cut, float* out, cudaStream_t stream) {
+  if (T <= 0 || R <= 0) return GB_OK;
+  if (gb_delta_chunk_floats(T, R, H, G, dim, vdim, taps) == 0)
+    return gb::fail(GB_UNSUPPORTED, "delta_chunk: %d heads of %d x %d, %d key heads, %d taps", H, dim, vdim, G, taps);
+  const int CH = 2 * G * dim + H * vdim;
+  if (P < CH + H || P2 < (per_head ? H : H * dim)) return gb::fail(GB_BAD_ARGUMENT, "delta_chunk: row widths");
+  if ((uintptr_t)blocks & 15) return gb::fail(GB_BAD_ARGUMENT, "delta_chunk: blocks start on 16 bytes");
+  const size_t smem = (size_t)(delta_chunk::C * (3 * (dim + 4) + 2 * delta_chunk::LT + 1)) * sizeof(float);
+  const int rc = GB_DISPATCH_DTYPE(w_dtype, WT, [&]() -> int {
+    auto kernel = dim == 128 ? delta_chunk_factors_kernel<128, WT> : delta_chunk_factors_kernel<64, WT>;
+    static gb::OncePerDevice configured[2];      // per weight type: this lambda is instantiated for each
+    if (configured[dim == 128].needed()) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return gb::fail(GB_CUDA_ERROR, "delta_chunk: %s", cudaGetErrorString(e));
+      configured[dim == 128].done();
+    }
+    return gb::check_pdl_launch(
+        gb::launch_pdl(kernel, dim3(delta_chunk::chunk_numbers(T, R), H), dim3(256), smem, stream, dim3(1, 1, 1), proj, P, second, P2,
+                       (const WT*)conv_w, taps, conv_state, conv_stride, (const WT*)a_log, (const WT*)dt_bias, cu_q, slots, blocks, R, H,
+                       G, vdim, per_head, cut),
+        "delta_chunk");
+  });
+  if (rc != GB_OK) return rc;
+  return delta_chunk::launch_walk<false>("delta_chunk", blocks, cu_q, slots, state, state_stride, R, H, dim, vdim, cut, out, stream);
 }
 
 GB_EXPORT int gb_delta_out(const float* o, const float* second, int P2, int gate_off, const void* w, int w_dtype,

@@ -14,11 +14,16 @@
 //                       through shared memory, eight (or four) tokens at a time in two buffers
 //   gdelta_decode       all of it, with the read-out's norm, weight and gate, for steps of one
 //                       token per request: a block per (request, head)
-// The read-out's norm for longer steps is delta_out (delta_rule.cu). A token's result depends on
-// its request's earlier tokens only through the state, which is carried bit for bit.
+//   gdelta_chunk_factors, delta_chunk::walk
+//                       the same for long stretches of tokens in a bfloat16 run, 32 tokens at a time
+//                       (delta_chunk.cuh)
+// The read-out's norm for longer steps is delta_out (delta_rule.cu). In the token-by-token kernels a token's
+// result depends on its request's earlier tokens only through the state, which is carried bit for bit; the
+// chunked ones add the same terms in another order, so there a cut moves the last bits.
 #include <type_traits>
 
 #include "common.cuh"
+#include "delta_chunk.cuh"
 
 namespace {
 
@@ -30,10 +35,12 @@ __device__ __forceinline__ float sigmoid(float z) { return 1.0f / (1.0f + expf(-
 __global__ void __launch_bounds__(256)
 gdelta_prepare_kernel(const float* __restrict__ proj, int P, int col_r, int col_k, int col_v, int col_a,
                       const float* __restrict__ zdec, int PZ, const float* __restrict__ w0, const float* __restrict__ a0,
-                      float decay_scale, float* __restrict__ prep, int W, int H, int dim, int vdim) {
+                      float decay_scale, float* __restrict__ prep, int W, int H, int dim, int vdim,
+                      const int32_t* __restrict__ token_req, const int32_t* __restrict__ cu_q, int below) {
   gb::pdl_launch_dependents();
   gb::pdl_wait();
   const size_t t = blockIdx.x;
+  if (below > 0 && cu_q[token_req[t] + 1] - cu_q[token_req[t]] >= below) return;      // the chunked kernels' request
   const float* row = proj + t * P;
   float* out = prep + t * W;
   const int HD = H * dim;
@@ -73,8 +80,9 @@ template <int MAXD, bool EXACT, int CHUNK>
 __global__ void __launch_bounds__(REC_THREADS)
 gdelta_recurrence_kernel(const float* __restrict__ prep, int W, const int32_t* __restrict__ cu_q,
                          const int32_t* __restrict__ slots, float* __restrict__ state, long long state_stride, int H,
-                         int dim, int vdim, float* __restrict__ out) {
+                         int dim, int vdim, int below, float* __restrict__ out) {
   gb::pdl_wait();
+  if (below > 0 && cu_q[blockIdx.y + 1] - cu_q[blockIdx.y] >= below) return;      // the chunked kernels' request
   constexpr int MINE = MAXD / SPLIT;
   extern __shared__ __align__(16) float stage[];      // 2 x [CHUNK][VECS SPLIT per + 16 + 4]
   const int per = ((dim + SPLIT - 1) / SPLIT + 3) / 4 * 4 + 4;
@@ -178,6 +186,204 @@ gdelta_recurrence_kernel(const float* __restrict__ prep, int W, const int32_t* _
   }
 }
 
+// What the walk of delta_chunk.cuh needs of a chunk and a head. With D_i the product of the decays up to token i and
+// alpha = a * u, the row x_i = u_i^T S of token i, taken from the state in front of it, is
+//     x_i = (D_i-1 u_i)^T S_0 + sum_{j<i} F_ij v_j - E_ij x_j,   E_ij = sum_d u_i alpha_j D_i-1 / D_j,   F_ij likewise with k_j
+//     o_i = (D_i r_i)^T S_0 + sum_{j<=i} H_ij v_j - G_ij x_j,    G_ij = sum_d r_i alpha_j D_i / D_j,     H_ij likewise with k_j
+// so  W = (I + E)^-1 (D u),   VP = -(I + E)^-1 F v,   Q = D r - G W,   OP = H v + G VP,   K1_j = alpha_j D_last / D_j,   K2_j = k_j
+// D_last / D_j, and the walk's Y is -x. Quotients of decays are running products and the system is solved by substitution, a
+// thread per column, in 32-bit multiply-adds, as for the gated rule (delta_rule.cu). grid (chunk numbers, H), 256 threads.
+template <int DIM>
+__global__ void __launch_bounds__(256, 2)
+gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, int col_k, int col_v, int col_a,
+                            const float* __restrict__ zdec, int PZ, const float* __restrict__ w0, const float* __restrict__ a0,
+                            float decay_scale, const int32_t* __restrict__ cu_q, float* __restrict__ blocks, int R, int H, int vdim,
+                            int cut) {
+  using namespace delta_chunk;
+  using delta_chunk::C;
+  gb::pdl_launch_dependents();
+  gb::pdl_wait();
+  constexpr int LD = DIM + 4, VEC = DIM / 32;
+  extern __shared__ __align__(16) float sh[];
+  float* su = sh;                        // [C][LD]: u, then D u
+  float* sr = su + C * LD;               // [C][LD]: r, then D r
+  float* sw = sr + C * LD;               // [C][LD]: decays
+  float* sa = sw + C * LD;               // [C][LD]: alpha
+  float* sE = sa + C * LD;               // [C][LT] each, a row per j (transposed)
+  float* sF = sE + C * LT;
+  float* sG = sF + C * LT;
+  float* sH = sG + C * LT;
+  const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int r, first, n, at;
+  if (!find_chunk(blockIdx.x, cu_q, R, cut, r, first, n, at)) return;
+  const Layout lay{DIM, vdim, 1};
+  float* block = blocks + ((size_t)blockIdx.x * H + h) * lay.floats();
+  const float* row0 = proj + (size_t)first * P;
+#pragma unroll 2
+  for (int t = warp; t < C; t += 8) {
+    const float* row = row0 + (size_t)t * P;
+    float k[VEC], x[VEC], y[VEC], z[VEC], ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+      const int c = h * DIM + lane + 32 * e;
+      k[e] = t < n ? row[col_k + c] : 0.f;
+      x[e] = t < n ? row[col_r + c] : 0.f;
+      y[e] = t < n ? row[col_a + c] : 0.f;
+      z[e] = t < n ? zdec[(size_t)(first + t) * PZ + c] : 0.f;
+      ss = fmaf(k[e], k[e], ss);
+    }
+    const float inv = 1.0f / sqrtf(gb::warp_sum(ss) + 1e-6f);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+      const int d = lane + 32 * e, c = h * DIM + d;
+      const float u = k[e] * inv;
+      su[t * LD + d] = u;
+      sr[t * LD + d] = x[e];
+      sw[t * LD + d] = t < n ? expf(-decay_scale * sigmoid(z[e] + w0[c])) : 1.f;
+      sa[t * LD + d] = t < n ? sigmoid(y[e] + a0[c]) * u : 0.f;
+    }
+  }
+  for (int i = tid; i < 4 * C * LT; i += 256) sE[i] = 0.f;
+  __syncthreads();
+  {
+    const int j0 = (warp < 4 ? warp : 11 - warp) * 4, d0 = lane * VEC;
+    pair_t pa[4][VEC / 2], pk[4][VEC / 2];                // alpha_j and k_j, decayed on
+    auto row = [&](const float* m, int i, pair_t (&x)[VEC / 2]) {
+      if (VEC == 4) {
+        const pair2_t f = *reinterpret_cast<const pair2_t*>(m + i * LD + d0);
+        x[0] = f.a, x[VEC / 2 - 1] = f.b;
+      } else {
+        x[0] = *reinterpret_cast<const pair_t*>(m + i * LD + d0);
+      }
+    };
+    auto dot = [](const pair_t (&a)[VEC / 2], const pair_t (&b)[VEC / 2]) {
+      pair_t s = mul2(a[0], b[0]);
+#pragma unroll
+      for (int e = 1; e < VEC / 2; ++e) s = fma2(a[e], b[e], s);
+      const float2 f = both(s);
+      return f.x + f.y;
+    };
+    auto keep = [&](int i, float (&before)[8], float (&after)[8]) {
+      const float b = sum_of_eight(before, lane), a = sum_of_eight(after, lane);
+      const int which = lane >> 2, j = j0 + (which & 3);
+      if ((lane & 3) == 0 && j <= i) {
+        if (j < i) (which < 4 ? sE : sF)[j * LT + i] = b;
+        (which < 4 ? sG : sH)[j * LT + i] = a;
+      }
+    };
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+      for (int e = 0; e < VEC / 2; ++e) {
+        const float* k = row0 + (size_t)(j0 + jj) * P + col_k + h * DIM + d0 + 2 * e;
+        pk[jj][e] = j0 + jj < n ? make_pair(k[0], k[1]) : 0ull;
+      }
+#pragma unroll
+    for (int ii = 0; ii < 4; ++ii) {       // the tokens of the four keys themselves
+      const int i = j0 + ii;
+      if (i >= n) break;
+      pair_t w[VEC / 2], u[VEC / 2], x[VEC / 2];
+      row(sw, i, w), row(su, i, u), row(sr, i, x);
+      row(sa, i, pa[ii]);
+      float before[8], after[8];
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        before[jj] = jj < ii ? dot(pa[jj], u) : 0.f, before[4 + jj] = jj < ii ? dot(pk[jj], u) : 0.f;
+        if (jj < ii) {
+#pragma unroll
+          for (int e = 0; e < VEC / 2; ++e) pa[jj][e] = mul2(pa[jj][e], w[e]), pk[jj][e] = mul2(pk[jj][e], w[e]);
+        }
+        after[jj] = jj <= ii ? dot(pa[jj], x) : 0.f, after[4 + jj] = jj <= ii ? dot(pk[jj], x) : 0.f;
+      }
+      keep(i, before, after);
+    }
+    for (int i = j0 + 4; i < n; ++i) {
+      pair_t w[VEC / 2], u[VEC / 2], x[VEC / 2];
+      row(sw, i, w), row(su, i, u), row(sr, i, x);
+      float before[8], after[8];
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        before[jj] = dot(pa[jj], u), before[4 + jj] = dot(pk[jj], u);
+#pragma unroll
+        for (int e = 0; e < VEC / 2; ++e) pa[jj][e] = mul2(pa[jj][e], w[e]), pk[jj][e] = mul2(pk[jj][e], w[e]);
+        after[jj] = dot(pa[jj], x), after[4 + jj] = dot(pk[jj], x);
+      }
+      keep(i, before, after);
+    }
+  }
+  __syncthreads();
+  if (tid < DIM) {                       // a thread per channel
+    float run = 1.f;
+#pragma unroll
+    for (int j0 = C - 8; j0 >= 0; j0 -= 8) {
+      float x[8], y[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) y[e] = j0 + e < n ? row0[(size_t)(j0 + e) * P + col_k + h * DIM + tid] : 0.f;
+#pragma unroll
+      for (int e = 7; e >= 0; --e) {
+        x[e] = sa[(j0 + e) * LD + tid] * run, y[e] *= run;
+        run *= sw[(j0 + e) * LD + tid];
+      }
+      float4* to = reinterpret_cast<float4*>(block + lay.k1(j0, tid));
+      to[0] = make_float4(x[0], x[1], x[2], x[3]), to[1] = make_float4(x[4], x[5], x[6], x[7]);
+      to = reinterpret_cast<float4*>(block + lay.k1(C + j0, tid));
+      to[0] = make_float4(y[0], y[1], y[2], y[3]), to[1] = make_float4(y[4], y[5], y[6], y[7]);
+    }
+    block[lay.last() + tid] = run;
+    run = 1.f;
+#pragma unroll 8
+    for (int i = 0; i < C; ++i) {
+      su[i * LD + tid] *= run;
+      run *= sw[i * LD + tid];
+    }
+  } else if (tid >= 128 && tid < 128 + DIM) {
+    float run = 1.f;
+#pragma unroll 8
+    for (int i = 0; i < C; ++i) sr[i * LD + tid - 128] *= run *= sw[i * LD + tid - 128];
+  }
+  __syncthreads();
+  for (int c = tid; c < DIM + vdim; c += 256) {
+    const bool key = c < DIM;                             // the same for a warp
+    const float* v = row0 + col_v + h * vdim + c - DIM;   // a value column's numbers
+    pair_t w[C / 2], o[C / 2];
+#pragma unroll
+    for (int i = 0; i < C; i += 2) {
+      w[i / 2] = key ? make_pair(su[i * LD + c], su[(i + 1) * LD + c]) : 0ull;
+      o[i / 2] = key ? make_pair(sr[i * LD + c], sr[(i + 1) * LD + c]) : 0ull;
+    }
+    if (!key) {
+#pragma unroll
+      for (int j4 = 0; j4 < C; j4 += 4) {
+        float x[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[e] = j4 + e < n ? v[(size_t)(j4 + e) * P] : 0.f;
+        *reinterpret_cast<float4*>(block + lay.v() + (c - DIM) * C + j4) = make_float4(x[0], x[1], x[2], x[3]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          add_row<true>(w, sF, j4 + e, -x[e]);
+          add_row<false>(o, sH, j4 + e, x[e]);
+          asm volatile("" ::: "memory");                  // (else the rows are all fetched at once, and spilled)
+        }
+      }
+    }
+    // (a value column's w is VP = -x from here on)
+    const float sign = key ? -1.f : 1.f;
+#pragma unroll
+    for (int j = 0; j < C; ++j) {
+      add_row<true>(w, sE, j, -entry(w, j));
+      add_row<false>(o, sG, j, sign * entry(w, j));
+      asm volatile("" ::: "memory");
+    }
+    if (key) {
+      store_rows(block, lay, 0, c, w);
+      store_rows(block, lay, C, c, o);
+    } else {
+      store_column(block + lay.vp() + (c - DIM) * C, w);
+      store_column(block + lay.op() + (c - DIM) * C, o);
+    }
+  }
+}
+
 // A step of one token per request: grid (H, R), vdim threads (a column of S each, rounded up to a
 // warp). The state column lives in registers for the one token: read, updated, written. The sums
 // are taken as the kernel for longer steps takes them, so a token's result is the same bits
@@ -266,19 +472,20 @@ int by_dim(int dim, const char* what, F&& f) {
 
 }  // namespace
 
+// below (here and in gdelta_recurrence): only requests with fewer tokens in the step than this (0: all).
 GB_EXPORT int gb_gdelta_prepare(const float* proj, int P, int col_r, int col_k, int col_v, int col_a, const float* zdec,
                                 int PZ, const float* w0, const float* a0, float decay_scale, float* prep, int W, int T, int H,
-                                int dim, int vdim, cudaStream_t stream) {
+                                int dim, int vdim, const int32_t* token_req, const int32_t* cu_q, int below, cudaStream_t stream) {
   if (T <= 0) return GB_OK;
   if (H < 1 || dim < 1 || vdim < 1) return gb::fail(GB_BAD_ARGUMENT, "gdelta_prepare: sizes");
   if (W != 5 * H * dim + H * vdim || PZ < H * dim) return gb::fail(GB_BAD_ARGUMENT, "gdelta_prepare: row widths");
   return gb::check_pdl_launch(gb::launch_pdl(gdelta_prepare_kernel, dim3(T), dim3(256), 0, stream, dim3(1, 1, 1), proj, P, col_r,
-                                             col_k, col_v, col_a, zdec, PZ, w0, a0, decay_scale, prep, W, H, dim, vdim),
+                                             col_k, col_v, col_a, zdec, PZ, w0, a0, decay_scale, prep, W, H, dim, vdim, token_req, cu_q, below),
                               "gdelta_prepare");
 }
 
 GB_EXPORT int gb_gdelta_recurrence(const float* prep, int W, const int32_t* cu_q, const int32_t* slots, float* state,
-                                   long long state_stride, int R, int H, int dim, int vdim, float* out, cudaStream_t stream) {
+                                   long long state_stride, int R, int H, int dim, int vdim, int below, float* out, cudaStream_t stream) {
   if (R <= 0) return GB_OK;
   if (H < 1 || dim < 1 || vdim < 1) return gb::fail(GB_BAD_ARGUMENT, "gdelta_recurrence: sizes");
   const dim3 grid(H, R, (vdim + REC_COLS - 1) / REC_COLS);
@@ -293,9 +500,42 @@ GB_EXPORT int gb_gdelta_recurrence(const float* prep, int W, const int32_t* cu_q
     auto kernel = eight ? (dim == MAXD ? gdelta_recurrence_kernel<MAXD, true, 8> : gdelta_recurrence_kernel<MAXD, false, 8>)
                         : (dim == MAXD ? gdelta_recurrence_kernel<MAXD, true, 4> : gdelta_recurrence_kernel<MAXD, false, 4>);
     return gb::check_pdl_launch(gb::launch_after(kernel, grid, dim3(REC_THREADS), smem, stream, dim3(1, 1, 1), prep, W, cu_q, slots,
-                                               state, state_stride, H, dim, vdim, out),
+                                               state, state_stride, H, dim, vdim, below, out),
                                 "gdelta_recurrence");
   });
+}
+
+// Whether the chunked kernels take these sizes, and the floats of `blocks` for a step of T tokens of R requests (0: they do not).
+GB_EXPORT long long gb_gdelta_chunk_floats(int T, int R, int H, int dim, int vdim) {
+  if (T <= 0 || R <= 0 || H < 1 || H > 65535 || R > 65535 || !delta_chunk::takes(dim, vdim)) return 0;
+  return (long long)delta_chunk::chunk_numbers(T, R) * H * delta_chunk::Layout{dim, vdim, 1}.floats();
+}
+
+// Requests of at least `cut` tokens: everything from the projected rows to the read-out o [T, H vdim] and the state. The rows
+// are those of gdelta_prepare; blocks starts on 16 bytes.
+GB_EXPORT int gb_gdelta_chunk(const float* proj, int P, int col_r, int col_k, int col_v, int col_a, const float* zdec, int PZ,
+                              const float* w0, const float* a0, float decay_scale, const int32_t* cu_q, const int32_t* slots,
+                              float* state, long long state_stride, float* blocks, int T, int R, int H, int dim, int vdim, int cut,
+                              float* out, cudaStream_t stream) {
+  if (T <= 0 || R <= 0) return GB_OK;
+  if (gb_gdelta_chunk_floats(T, R, H, dim, vdim) == 0)
+    return gb::fail(GB_UNSUPPORTED, "gdelta_chunk: %d heads of %d x %d", H, dim, vdim);
+  if (PZ < H * dim) return gb::fail(GB_BAD_ARGUMENT, "gdelta_chunk: row widths");
+  if ((uintptr_t)blocks & 15) return gb::fail(GB_BAD_ARGUMENT, "gdelta_chunk: blocks start on 16 bytes");
+  const size_t smem = (size_t)(delta_chunk::C * 4 * (dim + 4 + delta_chunk::LT)) * sizeof(float);
+  auto kernel = dim == 128 ? gdelta_chunk_factors_kernel<128> : gdelta_chunk_factors_kernel<64>;
+  static gb::OncePerDevice configured[2];
+  if (configured[dim == 128].needed()) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return gb::fail(GB_CUDA_ERROR, "gdelta_chunk: %s", cudaGetErrorString(e));
+    configured[dim == 128].done();
+  }
+  const int rc = gb::check_pdl_launch(
+      gb::launch_pdl(kernel, dim3(delta_chunk::chunk_numbers(T, R), H), dim3(256), smem, stream, dim3(1, 1, 1), proj, P, col_r, col_k,
+                     col_v, col_a, zdec, PZ, w0, a0, decay_scale, cu_q, blocks, R, H, vdim, cut),
+      "gdelta_chunk");
+  if (rc != GB_OK) return rc;
+  return delta_chunk::launch_walk<true>("gdelta_chunk", blocks, cu_q, slots, state, state_stride, R, H, dim, vdim, cut, out, stream);
 }
 
 // One token per request (row t of the batch is request t). Takes vdim <= 256.

@@ -192,6 +192,9 @@ class CudaOps:
                 fn = getattr(L, name)
                 fn.argtypes = argtypes
                 fn.restype = c_int
+            L.gb_delta_chunk_floats.argtypes = [c_int] * 7
+            L.gb_gdelta_chunk_floats.argtypes = [c_int] * 5
+            L.gb_delta_chunk_floats.restype = L.gb_gdelta_chunk_floats.restype = c_longlong
             self._state = L
         return self._state
 
@@ -287,19 +290,24 @@ class CudaOps:
                                c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "gb_delta_prepare": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_longlong, c_void_p,
                              c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
-                             c_int, c_void_p],
+                             c_int, c_int, c_void_p],
         "gb_delta_conv_state": [c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
         "gb_delta_recurrence": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int,
-                                c_int, c_void_p, c_void_p],
+                                c_int, c_int, c_void_p, c_void_p],
+        "gb_delta_chunk": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_longlong, c_void_p, c_void_p,
+                           c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                           c_int, c_void_p, c_void_p],
+        "gb_gdelta_chunk": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float, c_void_p,
+                            c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
         "gb_delta_out": [c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_float, c_void_p, c_int, c_int, c_int, c_int,
                          c_int, c_int, c_void_p],
         "gb_delta_decode": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_longlong, c_void_p,
                             c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int,
                             c_void_p, c_int, c_int, c_int, c_int, c_void_p],
         "gb_gdelta_prepare": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float,
-                              c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                              c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p],
         "gb_gdelta_recurrence": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int,
-                                 c_void_p, c_void_p],
+                                 c_int, c_void_p, c_void_p],
         "gb_gdelta_decode": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float,
                              c_void_p, c_float, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_int,
                              c_void_p],
@@ -1161,21 +1169,40 @@ class CudaOps:
                 state.data_ptr(), stride, T, H, G, dim, vdim, out.data_ptr(), _tag(out, "delta_rule out"),
                 int(decay_per_head), n_decay, silu_gate, self._stream()), "delta_decode")
         else:
-            W = C + H * dim + H
-            prep = ctx.ws.get("delta_prep", (T, W), torch.float32)
             o = ctx.ws.get("delta_o", (T, H * vdim), torch.float32)
-            self._check(L, L.gb_delta_prepare(
-                proj.data_ptr(), proj.stride(0), second.data_ptr(), second.stride(0), conv_w.data_ptr(), wt, taps, conv_state,
-                stride, a_log.data_ptr(), dt_bias.data_ptr(), b.token_req.data_ptr(), b.cu_q.data_ptr(), b.slots.data_ptr(),
-                prep.data_ptr(), W, T, H, G, dim, vdim, int(decay_per_head), self._stream()), "delta_prepare")
-            self._check(L, L.gb_delta_recurrence(
-                prep.data_ptr(), W, b.cu_q.data_ptr(), b.slots.data_ptr(), state.data_ptr(), stride, b.num_requests, H, G,
-                dim, vdim, o.data_ptr(), self._stream()), "delta_recurrence")
+            floats = L.gb_delta_chunk_floats(T, b.num_requests, H, G, dim, vdim, taps)
+            cut = self._delta_chunk_cut(b, out, floats)
+            if cut:
+                blocks = ctx.ws.get("delta_blocks", (floats,), torch.float32)
+                self._check(L, L.gb_delta_chunk(
+                    proj.data_ptr(), proj.stride(0), second.data_ptr(), second.stride(0), conv_w.data_ptr(), wt, taps, conv_state,
+                    stride, a_log.data_ptr(), dt_bias.data_ptr(), b.cu_q.data_ptr(), b.slots.data_ptr(), state.data_ptr(), stride,
+                    blocks.data_ptr(), T, b.num_requests, H, G, dim, vdim, int(decay_per_head), cut, o.data_ptr(), self._stream()),
+                    "delta_chunk", kernels=2)
+            if not cut or getattr(b, "min_q_len", 1) < cut:
+                W = C + H * dim + H
+                prep = ctx.ws.get("delta_prep", (T, W), torch.float32)
+                self._check(L, L.gb_delta_prepare(
+                    proj.data_ptr(), proj.stride(0), second.data_ptr(), second.stride(0), conv_w.data_ptr(), wt, taps, conv_state,
+                    stride, a_log.data_ptr(), dt_bias.data_ptr(), b.token_req.data_ptr(), b.cu_q.data_ptr(), b.slots.data_ptr(),
+                    prep.data_ptr(), W, T, H, G, dim, vdim, int(decay_per_head), cut, self._stream()), "delta_prepare")
+                self._check(L, L.gb_delta_recurrence(
+                    prep.data_ptr(), W, b.cu_q.data_ptr(), b.slots.data_ptr(), state.data_ptr(), stride, b.num_requests, H, G,
+                    dim, vdim, cut, o.data_ptr(), self._stream()), "delta_recurrence")
             self._check(L, L.gb_delta_out(
                 o.data_ptr(), second.data_ptr(), second.stride(0), n_decay, norm_w.data_ptr(), wt, float(eps), out.data_ptr(),
                 _tag(out, "delta_rule out"), T, H, vdim, silu_gate, 0, self._stream()), "delta_out")
         self._check(L, L.gb_delta_conv_state(proj.data_ptr(), proj.stride(0), conv_state, stride, b.cu_q.data_ptr(),
                                              b.slots.data_ptr(), b.num_requests, C, taps, self._stream()), "delta_conv_state")
+
+    #: Requests with at least this many tokens in a step run the chunked delta-rule kernels, whose fixed cost is that of
+    #: a whole chunk and a third launch.
+    DELTA_CHUNK_CUT = 48
+
+    def _delta_chunk_cut(self, b, out, floats: int) -> int:
+        """From how many tokens on a request of this step is walked by chunks (delta_chunk.cuh); 0: none is. In a 32-bit run
+        every request is walked token by token, so that its numbers do not depend on how its prompt was cut."""
+        return self.DELTA_CHUNK_CUT if floats and out.dtype == torch.bfloat16 and b.max_q_len >= self.DELTA_CHUNK_CUT else 0
 
     # ------------------------------------------------------------------ the generalized delta rule
     def general_delta(self, ctx, proj, cols, zdec, w0, a0, decay_scale, norm_w, eps, state, heads, dim, vdim, out):
@@ -1208,15 +1235,25 @@ class CudaOps:
                 state.data_ptr(), stride, T, H, dim, vdim, out.data_ptr(), _tag(out, "general_delta out"), self._stream()),
                 "gdelta_decode")
             return
-        W = 5 * HD + HV
-        prep = ctx.ws.get("gdelta_prep", (T, W), torch.float32)
         o = ctx.ws.get("gdelta_o", (T, HV), torch.float32)
-        self._check(L, L.gb_gdelta_prepare(
-            proj.data_ptr(), proj.stride(0), col_r, col_k, col_v, col_a, zdec.data_ptr(), zdec.stride(0), w0.data_ptr(),
-            a0.data_ptr(), float(decay_scale), prep.data_ptr(), W, T, H, dim, vdim, self._stream()), "gdelta_prepare")
-        self._check(L, L.gb_gdelta_recurrence(
-            prep.data_ptr(), W, b.cu_q.data_ptr(), b.slots.data_ptr(), state.data_ptr(), stride, b.num_requests, H, dim,
-            vdim, o.data_ptr(), self._stream()), "gdelta_recurrence")
+        floats = L.gb_gdelta_chunk_floats(T, b.num_requests, H, dim, vdim)
+        cut = self._delta_chunk_cut(b, out, floats)
+        if cut:
+            blocks = ctx.ws.get("delta_blocks", (floats,), torch.float32)
+            self._check(L, L.gb_gdelta_chunk(
+                proj.data_ptr(), proj.stride(0), col_r, col_k, col_v, col_a, zdec.data_ptr(), zdec.stride(0), w0.data_ptr(),
+                a0.data_ptr(), float(decay_scale), b.cu_q.data_ptr(), b.slots.data_ptr(), state.data_ptr(), stride,
+                blocks.data_ptr(), T, b.num_requests, H, dim, vdim, cut, o.data_ptr(), self._stream()), "gdelta_chunk", kernels=2)
+        if not cut or getattr(b, "min_q_len", 1) < cut:
+            W = 5 * HD + HV
+            prep = ctx.ws.get("gdelta_prep", (T, W), torch.float32)
+            self._check(L, L.gb_gdelta_prepare(
+                proj.data_ptr(), proj.stride(0), col_r, col_k, col_v, col_a, zdec.data_ptr(), zdec.stride(0), w0.data_ptr(),
+                a0.data_ptr(), float(decay_scale), prep.data_ptr(), W, T, H, dim, vdim, b.token_req.data_ptr(), b.cu_q.data_ptr(),
+                cut, self._stream()), "gdelta_prepare")
+            self._check(L, L.gb_gdelta_recurrence(
+                prep.data_ptr(), W, b.cu_q.data_ptr(), b.slots.data_ptr(), state.data_ptr(), stride, b.num_requests, H, dim,
+                vdim, cut, o.data_ptr(), self._stream()), "gdelta_recurrence")
         gate = proj[:, col_g:col_g + HV]
         self._check(L, L.gb_delta_out(
             o.data_ptr(), gate.data_ptr(), proj.stride(0), 0, norm_w.data_ptr(), GB_F32, float(eps), out.data_ptr(),

@@ -1,0 +1,123 @@
+"""The delta rules walked by chunks of 32 tokens (bfloat16 runs, requests of many tokens) against the
+plain references, which walk token by token: chunks that are full, one short and one over, requests
+below the line beside requests above it, a state that is carried over, padding rows, decays so strong
+that a chunk's product of them underflows, rows that are column ranges of wider ones."""
+import pytest
+import torch
+
+from tests.gpu_helpers import batches, close, rnd, step_batch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from garuda_b200.kernels.ops import CudaOps
+    from tests.plain.cpu_ops import CpuOps
+    return CudaOps("cuda:0"), CpuOps()
+
+
+CUT = 48
+STEPS = [(CUT - 1, CUT, 97), (1, 64, 5), (CUT, 1, 1), (65, 63, 50)]
+
+
+def step(lens, slots):
+    return step_batch(lens, [0] * len(lens), slots, 16)[0]
+
+
+@pytest.mark.parametrize("H,G,dim,vdim,taps,per_head,strong", [
+    (2, 2, 64, 64, 4, False, False), (4, 2, 128, 128, 4, True, False), (1, 1, 128, 32, 1, False, True), (3, 1, 64, 160, 3, True, True),
+    (40, 20, 64, 96, 2, False, False), (2, 1, 128, 256, 4, False, False)])
+def test_gated_rule(ops, H, G, dim, vdim, taps, per_head, strong):
+    cuda, cpu = ops
+    assert cuda.DELTA_CHUNK_CUT == CUT
+    C, n_decay = 2 * G * dim + H * vdim, H if per_head else H * dim
+    n_state = H * dim * vdim
+    conv_w, a_log = rnd(C, taps, scale=0.5), rnd(H, scale=0.5, seed=1) + (3.0 if strong else 0.0)
+    dt_bias, norm_w = rnd(n_decay, seed=2) - (0.0 if strong else 3.0), rnd(vdim, seed=3) + 1.0
+    state_g, state_r = torch.zeros(5, n_state + (taps - 1) * C, device="cuda"), torch.zeros(5, n_state + (taps - 1) * C)
+    state_g[4] = float("nan")                           # a slot nobody uses
+    for k, lens in enumerate(STEPS):
+        T = sum(lens)
+        ctx_g, ctx_r = batches(step(lens, [3, 0, 2]))
+        wide = rnd(T, 3 + C + H + n_decay + H * vdim + 5, scale=1.5, seed=10 + k)
+        first, second = 3 + C + H, 3 + C + H + n_decay + H * vdim
+        out, ref = torch.zeros(T, H * vdim, dtype=torch.bfloat16, device="cuda"), torch.zeros(T, H * vdim, dtype=torch.bfloat16)
+        before = cuda.launches
+        for o, c, row, st, to, y in ((cuda, ctx_g, wide.cuda(), state_g, lambda t: t.cuda(), out), (cpu, ctx_r, wide, state_r, lambda t: t, ref)):
+            o.delta_rule(c, row[:, 3:first], row[:, first:second], to(conv_w), to(a_log), to(dt_bias), to(norm_w), 1e-5, st, H, G, dim, vdim,
+                         taps, y, decay_per_head=per_head, gate="silu" if per_head else "sigmoid")
+        assert cuda.launches - before == 2 + 2 * (min(lens) < CUT) + 2, "the step's chunked kernels, and the others beside them"
+        close(out, ref, torch.bfloat16, f"step {k}: outputs")
+        # sums of at most 256 terms of 32-bit, a hundred tokens deep: the two orders differ by parts in a million
+        close(state_g[:4], state_r[:4], torch.float32, f"step {k}: state", tol=2e-5)
+
+
+@pytest.mark.parametrize("H,dim,vdim,strong", [(2, 64, 64, False), (3, 128, 128, False), (1, 64, 32, True), (50, 64, 96, False), (2, 128, 160, True)])
+def test_general_rule(ops, H, dim, vdim, strong):
+    cuda, cpu = ops
+    HD, HV = H * dim, H * vdim
+    cols = (3, 3 + HD, 3 + 2 * HD, 3 + 2 * HD + HV, 3 + 3 * HD + HV)
+    w0, a0, norm_w = rnd(HD, scale=1.5, seed=1) - 2.0, rnd(HD, seed=2), rnd(HV, seed=3) + 1.0
+    state_g, state_r = torch.zeros(5, HD * vdim, device="cuda"), torch.zeros(5, HD * vdim)
+    state_g[1] = float("nan")
+    for k, lens in enumerate(STEPS):
+        T = sum(lens)
+        ctx_g, ctx_r = batches(step(lens, [3, 0, 2]))
+        proj, zdec = rnd(T, cols[4] + HV + 6, scale=1.5, seed=10 + k), rnd(T, HD + 2, scale=2.0, seed=20 + k)
+        out, ref = torch.zeros(T, HV, dtype=torch.bfloat16, device="cuda"), torch.zeros(T, HV, dtype=torch.bfloat16)
+        for o, c, st, to, y in ((cuda, ctx_g, state_g, lambda t: t.cuda(), out), (cpu, ctx_r, state_r, lambda t: t, ref)):
+            o.general_delta(c, to(proj), cols, to(zdec)[:, :HD], to(w0), to(a0), 20.0 if strong else 0.6, to(norm_w), 1e-5, st, H, dim, vdim, y)
+        close(out, ref, torch.bfloat16, f"step {k}: outputs")
+        keep = [0, 2, 3, 4]
+        close(state_g[keep], state_r[keep], torch.float32, f"step {k}: state", tol=2e-5)
+
+
+def test_padding_rows_touch_no_state(ops):
+    cuda, _ = ops
+    H, dim, vdim, taps = 2, 64, 32, 4
+    C = 2 * H * dim + H * vdim
+    state = rnd(3, H * dim * vdim + (taps - 1) * C).cuda()
+    before = state.clone()
+    ctx, _ = batches(step([CUT + 5, 70], [-1, -1]))
+    out = torch.zeros(CUT + 75, H * vdim, dtype=torch.bfloat16, device="cuda")
+    cuda.delta_rule(ctx, rnd(CUT + 75, C + H).cuda(), rnd(CUT + 75, H + H * vdim).cuda(), rnd(C, taps).cuda(), rnd(H).cuda(), rnd(H).cuda(),
+                    rnd(vdim).cuda(), 1e-5, state, H, H, dim, vdim, taps, out, decay_per_head=True)
+    assert torch.equal(state, before) and torch.isfinite(out.float()).all()
+
+
+def test_a_value_that_is_not_a_number_leaves_the_tokens_in_front_of_it_alone(ops):
+    cuda, _ = ops
+    H, dim, vdim, taps, T, bad = 2, 64, 64, 4, 100, 45
+    C = 2 * H * dim + H * vdim
+    proj, second = rnd(T, C + H).cuda(), rnd(T, H + H * vdim, seed=1).cuda()
+    w = [t.cuda() for t in (rnd(C, taps, seed=2), rnd(H, seed=3), rnd(H, seed=4), rnd(vdim, seed=5))]
+    outs = []
+    for spoil in (False, True):
+        p = proj.clone()
+        if spoil:
+            p[bad] = float("nan")
+        ctx, _ = batches(step([T], [0]))
+        outs.append(torch.zeros(T, H * vdim, dtype=torch.bfloat16, device="cuda"))
+        state = torch.zeros(1, H * dim * vdim + (taps - 1) * C, device="cuda")
+        cuda.delta_rule(ctx, p, second, *w, 1e-5, state, H, H, dim, vdim, taps, outs[-1], decay_per_head=True)
+    assert torch.equal(outs[0][:bad], outs[1][:bad]) and torch.isnan(outs[1][bad:].float()).all()
+
+
+def test_a_32_bit_run_is_walked_token_by_token(ops):
+    """There the numbers do not depend on how a prompt was cut."""
+    cuda, _ = ops
+    H, dim, vdim, taps, T = 2, 64, 64, 3, 130
+    C = 2 * H * dim + H * vdim
+    proj, second = rnd(T, C + H).cuda(), rnd(T, H + H * vdim, seed=1).cuda()
+    w = [t.cuda() for t in (rnd(C, taps, seed=2), rnd(H, seed=3), rnd(H, seed=4), rnd(vdim, seed=5))]
+    got = []
+    for cuts in ([T], [61, 69]):
+        state, at, outs = torch.zeros(1, H * dim * vdim + (taps - 1) * C, device="cuda"), 0, []
+        for n in cuts:
+            ctx, _ = batches(step([n], [0]))
+            outs.append(torch.zeros(n, H * vdim, device="cuda"))
+            cuda.delta_rule(ctx, proj[at:at + n], second[at:at + n], *w, 1e-5, state, H, H, dim, vdim, taps, outs[-1], decay_per_head=True)
+            at += n
+        got.append((torch.cat(outs), state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
