@@ -123,7 +123,242 @@ attention_simple_kernel(const T* __restrict__ q, const T* __restrict__ k_pool, c
   }
 }
 
+// ---- 32-bit prompts: the same arithmetic in tiles ------------------------------------------------
+//
+// A warp per (token, head) reads every key for itself (500 tokens of 32 heads of 64: 0.9 ms). Here a CTA takes 64 consecutive
+// (token, head of a kv head's group) rows of a request against 32 keys at a time in shared memory, every number by
+// the same operations in the same order as above: the eight interleaved sums of a score and their tree, a block's maximum, its
+// exponentials' sum as the warp's tree, a block's values by themselves in the order of the keys. So a token's bits do not depend on
+// which of the two kernels ran. Plain attention without a window; heads of 64 or 128 channels.
+// What bounds it: shared memory (a thread's 4 x 2 scores read 6 numbers for 8 multiply-adds) and, with few
+// long rows, the chain of a block's barriers: prompts of 125 and 375 tokens, 32 heads over 4, take 95 us (a warp per row: 0.9 ms).
+constexpr int TR = 64, TK = 32;              // rows and keys of a tile
+constexpr int T32 = 256;                     // threads
+
+// two 32-bit multiply-adds in one instruction, on numbers that lie side by side
+using pair_t = unsigned long long;
+struct __align__(16) pair2_t { pair_t a, b; };
+__device__ __forceinline__ void fma2(pair_t& d, pair_t a, pair_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
+__device__ __forceinline__ pair_t make_pair(float lo, float hi) {
+  pair_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float2 both(pair_t p) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(p));
+  return f;
+}
+
+template <int HD>
+struct TileSmem {
+  float q[TR][HD + 4], k[2][TK][HD + 4], v[2][TK][HD + 4], p[TR][TK + 4], corr[TR];
+  int limit[TR];                             // the last key that a row reads
+};
+
+__device__ __forceinline__ void copy_16(float* smem, const float* gmem, bool valid) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  const int bytes = valid ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
+}
+
+// grid (tiles of the longest request's rows, Hkv, R)
+template <int HD>
+__global__ void __launch_bounds__(T32, 2)
+attention_tile32_kernel(const float* __restrict__ q, const float* __restrict__ k_pool, const float* __restrict__ v_pool,
+                        const int32_t* __restrict__ block_table, int table_width, const int32_t* __restrict__ cu_q,
+                        const int32_t* __restrict__ kv_lens, float* __restrict__ out, int Hq, int Hkv, float scale, int page_size) {
+  constexpr int WARPS_T = T32 / 32, RPW = TR / WARPS_T;          // rows of a warp in the softmax
+  constexpr int RV = TR * HD / 4 / T32;                          // rows of a thread's values (by four channels)
+  extern __shared__ __align__(16) unsigned char raw[];
+  TileSmem<HD>& sm = *reinterpret_cast<TileSmem<HD>*>(raw);
+  const int r = blockIdx.z, kvh = blockIdx.y, G = Hq / Hkv;
+  // (the last rows, which read the most keys, first)
+  const int t0 = cu_q[r], n = cu_q[r + 1] - t0, row0 = (gridDim.x - 1 - blockIdx.x) * TR, rows = min(TR, n * G - row0);
+  if (rows <= 0) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int pos0 = kv_lens[r] - n;                               // the position of the request's first token of the step
+  const int last = pos0 + (row0 + rows - 1) / G;                 // the last key that a row of the tile reads
+  const int blocks = last / TK + 1;
+  const int32_t* table = block_table + (size_t)r * table_width;
+  auto where = [&](int row) {                                    // (token, head) row of q and out
+    const int i = row0 + row;
+    return (size_t)(t0 + i / G) * Hq + kvh * G + i % G;
+  };
+  auto load = [&](int b) {
+    for (int i = tid; i < TK * (HD / 4); i += T32) {
+      const int key = i / (HD / 4), c = i % (HD / 4) * 4, j = b * TK + key;
+      const int page = j <= last ? table[j / page_size] : -1;
+      const size_t at = page >= 0 ? (((size_t)page * Hkv + kvh) * page_size + j % page_size) * HD + c : 0;
+      copy_16(&sm.k[b & 1][key][c], k_pool + at, page >= 0);
+      copy_16(&sm.v[b & 1][key][c], v_pool + at, page >= 0);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  load(0);
+  for (int row = warp; row < TR; row += WARPS_T) {
+    const float* from = q + (row < rows ? where(row) * HD : 0);
+    for (int c = lane; c < HD; c += 32) sm.q[row][c] = row < rows ? from[c] : 0.f;
+    if (lane == 0) sm.limit[row] = row < rows ? pos0 + (row0 + row) / G : -1;
+  }
+  // the softmax: a warp has RPW rows, a lane a key
+  float m[RPW], l[RPW];
+#pragma unroll
+  for (int i = 0; i < RPW; ++i) m[i] = -INFINITY, l[i] = 0.f;
+  // the values: a thread has RV rows and four channels
+  const int c4 = tid % (HD / 4) * 4, rv = tid / (HD / 4) * RV;
+  pair_t acc[RV][2];
+#pragma unroll
+  for (int i = 0; i < RV; ++i) acc[i][0] = acc[i][1] = 0ull;
+  // the scores: four rows (four apart), two keys (eight apart)
+  const int rs = (warp & 3) * 16 + (lane >> 3), ks = (warp >> 2) * 16 + (lane & 7);
+  for (int b = 0; b < blocks; ++b) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                       // the block has landed; everyone is done with the one in front
+    if (b + 1 < blocks) load(b + 1);
+    {
+      pair_t d8[4][2][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) d8[i][j][e] = 0ull;
+#pragma unroll 4
+      for (int c = 0; c < HD; c += 8) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          pair2_t x[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const pair2_t*>(&sm.q[rs + 4 * i][c + 4 * half]);
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const pair2_t y = *reinterpret_cast<const pair2_t*>(&sm.k[b & 1][ks + 8 * j][c + 4 * half]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) fma2(d8[i][j][2 * half], x[i].a, y.a), fma2(d8[i][j][2 * half + 1], x[i].b, y.b);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const float2 d01 = both(d8[i][j][0]), d23 = both(d8[i][j][1]), d45 = both(d8[i][j][2]), d67 = both(d8[i][j][3]);
+          sm.p[rs + 4 * i][ks + 8 * j] = (((d01.x + d01.y) + (d23.x + d23.y)) + ((d45.x + d45.y) + (d67.x + d67.y))) * scale;
+        }
+    }
+    __syncthreads();
+    const int key = b * TK + lane;
+    const bool stored = key <= last && table[key / page_size] >= 0;
+#pragma unroll
+    for (int i = 0; i < RPW; ++i) {
+      const int row = warp * RPW + i;
+      const bool seen = stored && key <= sm.limit[row];
+      const float s = seen ? sm.p[row][lane] : -INFINITY;
+      const float m_new = fmaxf(m[i], gb::warp_max(s));
+      float p = 0.f, corr = 1.f;           // (a block without a stored key that the row reads changes nothing)
+      if (m_new != -INFINITY) {
+        p = seen ? expf(s - m_new) : 0.f;
+        corr = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
+        l[i] = l[i] * corr + gb::warp_sum(p);
+        m[i] = m_new;
+      }
+      sm.p[row][lane] = p;
+      if (lane == 0) sm.corr[row] = corr;
+    }
+    __syncthreads();
+    pair_t part[RV][2];
+#pragma unroll
+    for (int i = 0; i < RV; ++i) part[i][0] = part[i][1] = 0ull;
+    // A row must not meet the values of keys behind its own, which may be anything: where the block holds such keys for some row
+    // the sums look at each. (A zero weight adds an exact zero otherwise.)
+    if (b * TK + TK - 1 <= pos0 + row0 / G) {
+#pragma unroll
+      for (int j = 0; j < TK; j += 4) {
+        pair2_t y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = *reinterpret_cast<const pair2_t*>(&sm.v[b & 1][j + e][c4]);
+#pragma unroll
+        for (int i = 0; i < RV; ++i) {
+          const float4 p4 = *reinterpret_cast<const float4*>(&sm.p[rv + i][j]);
+          const float p[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const pair_t pp = make_pair(p[e], p[e]);
+            fma2(part[i][0], pp, y[e].a), fma2(part[i][1], pp, y[e].b);
+          }
+        }
+      }
+    } else {
+      int seen[RV];                        // how many of the block's keys a row reads
+#pragma unroll
+      for (int i = 0; i < RV; ++i) seen[i] = sm.limit[rv + i] - b * TK + 1;
+#pragma unroll 4
+      for (int j = 0; j < TK; ++j) {
+        const pair2_t y = *reinterpret_cast<const pair2_t*>(&sm.v[b & 1][j][c4]);
+#pragma unroll
+        for (int i = 0; i < RV; ++i) {
+          const float p = sm.p[rv + i][j];
+          const pair_t pp = make_pair(p, p);
+          if (j < seen[i]) fma2(part[i][0], pp, y.a), fma2(part[i][1], pp, y.b);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < RV; ++i) {
+      const float corr = sm.corr[rv + i];
+      const pair_t cc = make_pair(corr, corr);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        fma2(part[i][e], acc[i][e], cc);
+        acc[i][e] = part[i][e];
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < RPW; ++i)
+    if (lane == 0) sm.corr[warp * RPW + i] = l[i] > 0.f ? 1.0f / l[i] : 0.f;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < RV; ++i) {
+    if (rv + i >= rows) continue;
+    const float inv = sm.corr[rv + i];
+    const float2 lo = both(acc[i][0]), hi = both(acc[i][1]);
+    *reinterpret_cast<float4*>(out + where(rv + i) * HD + c4) = make_float4(lo.x * inv, lo.y * inv, hi.x * inv, hi.y * inv);
+  }
+}
+
+template <int HD>
+int launch_tile32(const float* q, const float* k_pool, const float* v_pool, const int32_t* block_table, int table_width,
+                  const int32_t* cu_q, const int32_t* kv_lens, float* out, int R, int max_q, int Hq, int Hkv, float scale, int page_size,
+                  cudaStream_t stream) {
+  static gb::OncePerDevice configured;
+  if (configured.needed()) {
+    const cudaError_t e = cudaFuncSetAttribute(attention_tile32_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileSmem<HD>));
+    if (e != cudaSuccess) return gb::fail(GB_CUDA_ERROR, "attention_tile32: %s", cudaGetErrorString(e));
+    configured.done();
+  }
+  const long long tiles = ((long long)max_q * (Hq / Hkv) + TR - 1) / TR;
+  attention_tile32_kernel<HD><<<dim3((unsigned)tiles, Hkv, R), T32, sizeof(TileSmem<HD>), stream>>>(
+      q, k_pool, v_pool, block_table, table_width, cu_q, kv_lens, out, Hq, Hkv, scale, page_size);
+  return gb::check_launch("attention_tile32");
+}
+
 }  // namespace
+
+// Plain causal attention of a 32-bit prompt, bit for bit what gb_attention_simple gives. hd 64 or 128; q, out and the pools start on 16
+// bytes; max_q: the most tokens that a request of the step has.
+GB_EXPORT int gb_attention_tile32(const float* q, const float* k_pool, const float* v_pool, const int32_t* block_table, int table_width,
+                                  const int32_t* cu_q, const int32_t* kv_lens, float* out, int R, int max_q, int Hq, int Hkv, int hd,
+                                  float scale, int page_size, cudaStream_t stream) {
+  if (R <= 0 || max_q <= 0) return GB_OK;
+  if (Hkv < 1 || Hq % Hkv || Hkv > 65535 || R > 65535) return gb::fail(GB_BAD_ARGUMENT, "attention_tile32: %d query heads for %d kv heads, %d requests", Hq, Hkv, R);
+  if (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out) & 15) return gb::fail(GB_BAD_ARGUMENT, "attention_tile32: 16-byte addresses");
+  if (hd == 64) return launch_tile32<64>(q, k_pool, v_pool, block_table, table_width, cu_q, kv_lens, out, R, max_q, Hq, Hkv, scale, page_size, stream);
+  if (hd == 128) return launch_tile32<128>(q, k_pool, v_pool, block_table, table_width, cu_q, kv_lens, out, R, max_q, Hq, Hkv, scale, page_size, stream);
+  return gb::fail(GB_UNSUPPORTED, "attention_tile32: heads of %d channels", hd);
+}
 
 // v_hd: width of a value row in its pool; vd: how many of its first channels are the value
 // (out is [T, Hq, vd]). Ordinary attention passes hd for both.

@@ -152,6 +152,8 @@ class CudaOps:
             "gb_attention_simple": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p,
                                     c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int,
                                     c_int, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
+            "gb_attention_tile32": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                                    c_int, c_int, c_float, c_int, c_void_p],
             "gb_argmax": [c_void_p, c_void_p, c_int, c_int, c_void_p],
             "gb_sample": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                           c_void_p],
@@ -656,6 +658,14 @@ class CudaOps:
         if plain and vd == hd and self.tc is not None and q.dtype == torch.bfloat16 and self.tc.paged_attention(
                 q, k_pool, v_pool, block_table, cu_q, kv_lens, token_req, out, scale, window, page_size,
                 num_requests, max_q_len, max_kv_len, ws, min_q_len):
+            return
+        # a tile takes 64 (token, head of a group) rows of a request; with less than half of one a warp per row is faster
+        if (plain and vd == hd and not window and q.dtype == torch.float32 and hd in (64, 128) and max_q_len * (Hq // Hkv) >= 32
+                and num_requests <= 65535 and not any(t.data_ptr() & 15 for t in (q, k_pool, v_pool, out))):
+            self._check(self.core, self.core.gb_attention_tile32(
+                q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), block_table.data_ptr(), block_table.shape[1], cu_q.data_ptr(),
+                kv_lens.data_ptr(), out.data_ptr(), num_requests, max_q_len, Hq, Hkv, hd, float(scale), page_size, self._stream()),
+                "attention_tile32")
             return
         self._check(self.core, self.core.gb_attention_simple(
             q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), _tag(q, "attention q"),
