@@ -25,7 +25,7 @@
 // A group of four warps has 16 columns of S, a quarter of the channels each: S^T in the accumulators' layout is at once the first
 // operand of S^T [W; Q]^T, so nothing of S is ever exchanged, only the warps' shares of Y and o. One group a block while such
 // blocks are at most one an SM (16 heads x 8 groups are 128 blocks for 148 SMs); two (which share WQ, K1 and K2) where the
-// heads are more. 2,048 tokens of 16 heads of 128 x 128 take 101 us here and 143 us in the kernel in front (B200), where the
+// heads are more. 2,048 tokens of 16 heads of 128 x 128 take 98 us here and 119 us in the kernel in front (B200), where the
 // token-by-token walk took 0.89 ms; the tensor cores are 44% busy, the rest is the latency of a chunk's three barriers.
 #pragma once
 
