@@ -186,7 +186,7 @@ def _lib_recipe(name: str):
         return ["attention_capped_mma.cu"], [f"-DGB_KEY_DIM={int(kd)}", f"-DGB_VALUE_DIM={int(vd)}"]
     if name.startswith("garuda_latent_r"):
         rank, rot = name[len("garuda_latent_r"):].split("_t")
-        return ["latent_attention_mma.cu"], [f"-DGB_LATENT_RANK={int(rank)}", f"-DGB_LATENT_ROT={int(rot)}"]
+        return ["latent_attention_mma.cu", "latent_attention_tcgen05.cu"], [f"-DGB_LATENT_RANK={int(rank)}", f"-DGB_LATENT_ROT={int(rot)}"]
     if name.startswith("garuda_attn_hd"):
         return ["attention_mma.cu", "attention_tcgen05.cu", "attention_decode_tma.cu"], [f"-DGB_HEAD_DIM={int(name[len('garuda_attn_hd'):])}"]
     return KERNEL_LIBS[name], []

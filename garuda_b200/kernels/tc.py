@@ -71,6 +71,8 @@ class TensorCoreKernels:
         code = self.lib.gb_tc_error_check()
         for lib in self._attn.values():
             code = lib.gb_attention_error_check() or code
+        for lib in self._latent.values():
+            code = lib.gb_latent_attention_error_check() or code
         seen, self.ops.error_word[0] = int(self.ops.error_word[0]), 0
         code = code or seen
         if code:
@@ -412,6 +414,15 @@ class TensorCoreKernels:
             lib.gb_latent_attention.restype = c_int
             lib.gb_latent_attention_scratch_bytes.argtypes = [ctypes.c_longlong, c_int]
             lib.gb_latent_attention_scratch_bytes.restype = ctypes.c_longlong
+            lib.gb_latent_attention_tc_takes.argtypes = [c_void_p] * 3 + [c_int] * 2 + [ctypes.c_longlong]
+            lib.gb_latent_attention_tc_takes.restype = c_int
+            lib.gb_latent_attention_tc.argtypes = ([c_void_p] * 4 + [c_int] + [c_void_p] * 2 + [c_int] * 3 + [c_float]
+                                                   + [c_int] * 3 + [c_void_p] * 2)
+            lib.gb_latent_attention_tc.restype = c_int
+            lib.gb_latent_attention_error_check.restype = c_int
+            lib.gb_latent_attention_set_error_sink.argtypes = [c_void_p]
+            lib.gb_latent_attention_set_error_sink.restype = c_int
+            lib.gb_latent_attention_set_error_sink(self.ops.error_word.data_ptr())
             self._latent[(rank, rot)] = lib
         return lib
 
@@ -435,6 +446,15 @@ class TensorCoreKernels:
             return False
         lib = self._latent_lib(rank, rot)
         splits = self.latent_plan(num_requests, H, max_q_len, max_kv_len)
+        if splits == 1 and num_requests <= 65535 and lib.gb_latent_attention_tc_takes(q.data_ptr(), pool.data_ptr(), out.data_ptr(), int(page_size),
+                                                                                      pool.shape[0], T * H):
+            # enough query rows to fill the GPU without cutting the keys: 128 of them a CTA on the tcgen05 kernel
+            code = lib.gb_latent_attention_tc(
+                q.data_ptr(), pool.data_ptr(), out.data_ptr(), block_table.data_ptr(), block_table.shape[1], cu_q.data_ptr(),
+                kv_lens.data_ptr(), T, num_requests, H, float(scale), int(page_size), pool.shape[0], int(max_q_len),
+                None if sink_values is None else sink_values.data_ptr(), self.ops._stream())
+            self.ops._check(lib, code, "latent_attention_tc")
+            return True
         while splits > 1 and lib.gb_latent_attention_scratch_bytes(T * H, splits) > (256 << 20):
             splits //= 2
         need = int(lib.gb_latent_attention_scratch_bytes(T * H, splits))

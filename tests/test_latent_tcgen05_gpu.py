@@ -1,0 +1,56 @@
+"""Attention over cached latent rows for prompt portions on the tcgen05 kernel, against 64-bit attention over
+the same rows: every block count of a row (with and without a rotated part that fills its block), one tile of
+64 keys and its edges, portions behind cached positions, single tokens beside them, pages of every size, sinks, whatever
+lies behind a request's last position."""
+import pytest
+import torch
+
+from tests.gpu_helpers import close
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from garuda_b200.kernels.ops import CudaOps
+    return CudaOps("cuda:0")
+
+
+# (rank, rot, heads, page size, (cached length after the step, tokens of the step) of every request, sinks)
+@pytest.mark.parametrize("rank,rot,H,page,reqs,sinks", [
+    (256, 32, 32, 32, [(300, 300)], False), (256, 64, 16, 16, [(64, 64), (65, 65), (700, 350), (129, 1)], True),
+    (64, 32, 32, 8, [(333, 333), (63, 63)], False), (128, 0, 24, 64, [(1000, 340), (128, 128)], True), (192, 16, 40, 32, [(2111, 200)], False)])
+def test_prompt_portions(ops, rank, rot, H, page, reqs, sinks):
+    row, R = rank + rot, len(reqs)
+    g = torch.Generator(device="cuda").manual_seed(rank + rot)
+    T = sum(n for _, n in reqs)
+    each = [(kv + page - 1) // page for kv, _ in reqs]
+    pool = torch.full((sum(each) + 3, 1, page, row), float("nan"), dtype=torch.bfloat16, device="cuda")      # what nobody wrote
+    order = torch.randperm(sum(each) + 3, generator=g, device="cuda").int()
+    table = torch.full((R, max(each) + 1), -1, dtype=torch.int32, device="cuda")
+    q = torch.randn(T, H, row, generator=g, device="cuda").bfloat16()
+    sink = torch.randn(H, generator=g, device="cuda") + 2.0 if sinks else None
+    scale, at, t0, ref = row ** -0.5, 0, 0, torch.empty(T, H, rank, dtype=torch.float64, device="cuda")
+    for r, (kv, n) in enumerate(reqs):
+        table[r, :each[r]] = order[at:at + each[r]]
+        rows = torch.randn(kv, row, generator=g, device="cuda").bfloat16()
+        j = torch.arange(kv, device="cuda")
+        pool[table[r].long()[j // page], 0, j % page] = rows
+        s = torch.einsum("thc,jc->htj", q[t0:t0 + n].double(), rows.double()) * scale
+        s = s.masked_fill(j[None, None, :] > (kv - n + torch.arange(n, device="cuda"))[None, :, None], -float("inf"))
+        e = torch.exp(s - s.amax(-1, keepdim=True))
+        den = e.sum(-1, keepdim=True) + (torch.exp(sink.double()[:, None, None] - s.amax(-1, keepdim=True)) if sinks else 0.0)
+        ref[t0:t0 + n] = torch.einsum("htj,jc->thc", e / den, rows[:, :rank].double())
+        at, t0 = at + each[r], t0 + n
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    cu = i32([sum(n for _, n in reqs[:r]) for r in range(R + 1)])
+    out = torch.full((T, H * rank), float("nan"), dtype=torch.bfloat16, device="cuda")
+    lib = ops.tc._latent_lib(rank, rot)
+    assert lib.gb_latent_attention_tc_takes(q.data_ptr(), pool.data_ptr(), out.data_ptr(), page, pool.shape[0], T * H) == 1
+    assert ops.tc.latent_plan(R, H, max(n for _, n in reqs), max(kv for kv, _ in reqs)) == 1
+    req = torch.repeat_interleave(torch.arange(R, dtype=torch.int32), torch.tensor([n for _, n in reqs])).cuda()
+    more = {} if sink is None else dict(sink_values=sink)
+    ops.paged_attention(q, pool, pool, table, cu, i32([kv for kv, _ in reqs]), req, out, scale, 0, page, R, max(n for _, n in reqs),
+                        max(kv for kv, _ in reqs), value_dim=rank, **more)
+    ops.tc.check_errors()
+    close(out.view(T, H, rank), ref.cpu(), torch.bfloat16, "latent attention")
