@@ -183,7 +183,7 @@ def _lib_recipe(name: str):
         return ["ssd_chunk_mma.cu"], [f"-DGB_STATE_DIM={int(n)}", f"-DGB_HEAD_DIM={int(p)}"]
     if name.startswith("garuda_cattn_k"):
         kd, vd = name[len("garuda_cattn_k"):].split("_v")
-        return ["attention_capped_mma.cu"], [f"-DGB_KEY_DIM={int(kd)}", f"-DGB_VALUE_DIM={int(vd)}"]
+        return ["attention_capped_mma.cu", "attention_capped_tcgen05.cu"], [f"-DGB_KEY_DIM={int(kd)}", f"-DGB_VALUE_DIM={int(vd)}"]
     if name.startswith("garuda_latent_r"):
         rank, rot = name[len("garuda_latent_r"):].split("_t")
         return ["latent_attention_mma.cu", "latent_attention_tcgen05.cu"], [f"-DGB_LATENT_RANK={int(rank)}", f"-DGB_LATENT_ROT={int(rot)}"]

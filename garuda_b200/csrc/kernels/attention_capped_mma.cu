@@ -21,9 +21,11 @@
 //  * DECODE (a request with at most 16 rows): the four warps take a quarter of every tile's keys
 //    each for the same rows and merge in shared memory; `splits` CTAs share a request's tiles and
 //    leave partial results in the caller's scratch, which a second kernel merges in split order.
-// A request belongs to DECODE if q_len * g <= 16, else to TILE; each launch skips the other's.
+// A request belongs to DECODE if q_len * g <= 16, else to TILE; each launch skips the other's. Prompt portions run on tcgen05
+// instead where attention_capped_tcgen05.cu takes the shape.
 //
 // Compiled per (key width, value width): GB_KEY_DIM, GB_VALUE_DIM (multiples of 16, at most 128).
+#include "attention_capped.cuh"
 #include "attention_mma_core.cuh"
 #include "common.cuh"
 
@@ -37,40 +39,20 @@
 namespace {
 
 using namespace attn_mma;
+using capped::Params;
+using capped::first_seen;
+using capped::ROWS_DECODE;
 
 constexpr int HD = GB_KEY_DIM, VD = GB_VALUE_DIM;
 static_assert(HD % 16 == 0 && HD >= 16 && HD <= 128 && VD % 16 == 0 && VD >= 16 && VD <= 128, "widths are multiples of 16 up to 128");
 constexpr int PAD = 8;
 constexpr int LDK = HD + PAD, LDV = VD + PAD;
 constexpr int THREADS = 128;
-constexpr int ROWS_TILE = 64, ROWS_DECODE = 16;
+constexpr int ROWS_TILE = 64;
 constexpr int MAX_SPLITS = 32;
 constexpr int PR = VD + 2;                 // floats of a row's partial result: sums, maximum, denominator
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr size_t SMEM = (size_t)(ROWS_TILE * LDK + 2 * KT * (LDK + LDV)) * sizeof(__nv_bfloat16);
-
-struct Params {
-  const __nv_bfloat16* q;        // [T, Hq, HD]
-  const __nv_bfloat16* k_pool;   // [pages, Hkv, page_size, HD]
-  const __nv_bfloat16* v_pool;   // [pages, Hkv, page_size, VD]
-  __nv_bfloat16* out;            // [T, Hq * VD]
-  const int32_t* block_table;
-  const int32_t* cu_q;
-  const int32_t* kv_lens;
-  float* partials;               // [R, Hkv, splits, ROWS_DECODE, PR] (DECODE with splits > 1)
-  int table_width, Hq, Hkv, g, window, keep_first, page_size, sink, splits;
-  float scale, softcap;
-  const float* sink_v;           // [Hq] or null: a learned sink per query head
-  const float* r1;               // [Hq] or null: the distance term's two numbers per query head
-  const float* r2;
-  int chunk;                     // > 0: a query reads its own stretch of this many positions (no window then)
-};
-
-// First position that the query at `pos` reads (kept first positions aside).
-__device__ __forceinline__ int first_seen(const Params& p, int pos) {
-  if (p.chunk > 0) return pos / p.chunk * p.chunk;
-  return p.window > 0 ? max(0, pos + 1 - p.window) : 0;
-}
 
 // What the sink adds to a row's denominator, in units of exp(-m).
 __device__ __forceinline__ float sink_term(const Params& p, int head, float m) {
@@ -484,13 +466,13 @@ GB_EXPORT long long gb_capped_attention_scratch_bytes(int R, int kv_heads, int s
 }
 
 // q [T, Hq, HD], k_pool [pages, Hkv, page_size, HD], v_pool [pages, Hkv, page_size, VD], out [T, Hq * VD],
-// bfloat16. A split that holds no key of a request leaves a partial with maximum -inf, which the merge skips.
+// bfloat16. num_pages: pages in each pool. A split that holds no key of a request leaves a partial with maximum -inf, which the merge skips.
 GB_EXPORT int gb_capped_attention(const void* q, const void* k_pool, const void* v_pool, void* out,
                                   const int32_t* block_table, int table_width, const int32_t* cu_q,
                                   const int32_t* kv_lens, int T, int R, int Hq, int Hkv, float scale, float softcap,
                                   int window, int keep_first, int sink, int page_size, int max_q_len, int min_q_len,
                                   int splits, void* scratch, long long scratch_bytes, const float* sink_v, const float* r1,
-                                  const float* r2, int chunk, cudaStream_t stream) {
+                                  const float* r2, int chunk, long long num_pages, cudaStream_t stream) {
   if (T <= 0 || R <= 0) return GB_OK;
   if (Hkv < 1 || Hq % Hkv) return gb::fail(GB_BAD_ARGUMENT, "capped_attention: %d query heads for %d kv heads", Hq, Hkv);
   if ((r1 == nullptr) != (r2 == nullptr)) return gb::fail(GB_BAD_ARGUMENT, "capped_attention: the distance term takes both of its numbers");
@@ -533,6 +515,7 @@ GB_EXPORT int gb_capped_attention(const void* q, const void* k_pool, const void*
     }
   }
   if (max_q_len * g > ROWS_DECODE) {
+    if (capped::tc_takes(p, num_pages, R)) return capped::launch_tc(p, T, num_pages, R, max_q_len, stream);
     const int tokens_per_tile = ROWS_TILE / g;
     dim3 grid((max_q_len + tokens_per_tile - 1) / tokens_per_tile, Hkv, R);
     return gb::check_pdl_launch(gb::launch_pdl(tile_kernel, grid, dim3(THREADS), SMEM, stream,
@@ -540,3 +523,8 @@ GB_EXPORT int gb_capped_attention(const void* q, const void* k_pool, const void*
   }
   return GB_OK;
 }
+
+// Non-zero if a CTA gave up on a wait since the last call; clears it. And a word of pinned host memory that a failed wait
+// also writes its code to (null: none).
+GB_EXPORT int gb_capped_attention_error_check() { return capped::tc_error_check(); }
+GB_EXPORT int gb_capped_attention_set_error_sink(int* host_word) { return capped::tc_set_error_sink(host_word); }

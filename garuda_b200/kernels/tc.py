@@ -73,6 +73,8 @@ class TensorCoreKernels:
             code = lib.gb_attention_error_check() or code
         for lib in self._latent.values():
             code = lib.gb_latent_attention_error_check() or code
+        for lib in self._capped.values():
+            code = lib.gb_capped_attention_error_check() or code
         seen, self.ops.error_word[0] = int(self.ops.error_word[0]), 0
         code = code or seen
         if code:
@@ -311,8 +313,12 @@ class TensorCoreKernels:
             lib = load_kernel_lib(capped_attention_lib_name(hd, vd))
             lib.gb_last_error.restype = ctypes.c_char_p
             lib.gb_capped_attention.argtypes = ([c_void_p] * 5 + [c_int] + [c_void_p] * 2 + [c_int] * 4 + [c_float, c_float]
-                                                + [c_int] * 7 + [c_void_p, ctypes.c_longlong] + [c_void_p] * 3 + [c_int, c_void_p])
+                                                + [c_int] * 7 + [c_void_p, ctypes.c_longlong] + [c_void_p] * 3 + [c_int, ctypes.c_longlong, c_void_p])
             lib.gb_capped_attention.restype = c_int
+            lib.gb_capped_attention_error_check.restype = c_int
+            lib.gb_capped_attention_set_error_sink.argtypes = [c_void_p]
+            lib.gb_capped_attention_set_error_sink.restype = c_int
+            lib.gb_capped_attention_set_error_sink(self.ops.error_word.data_ptr())
             lib.gb_capped_attention_scratch_bytes.argtypes = [c_int, c_int, c_int]
             lib.gb_capped_attention_scratch_bytes.restype = ctypes.c_longlong
             self._capped[(hd, vd)] = lib
@@ -329,7 +335,7 @@ class TensorCoreKernels:
             float(softcap), int(window), int(keep_first), int(bool(sink)), int(page_size), int(max_q_len), int(min_q_len),
             int(splits), None if scratch is None else scratch.data_ptr(), need,
             None if sink_values is None else sink_values.data_ptr(), None if r1 is None else r1.data_ptr(),
-            None if r2 is None else r2.data_ptr(), int(chunk), self.ops._stream())
+            None if r2 is None else r2.data_ptr(), int(chunk), int(min(k_pool.shape[0], v_pool.shape[0])), self.ops._stream())
         self.ops._check(lib, code, "capped_attention",
                         ((2 if splits > 1 else 1) if has_decode else 0) + (1 if max_q_len * g > 16 else 0))
         return True
