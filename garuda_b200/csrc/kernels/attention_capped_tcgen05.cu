@@ -12,7 +12,7 @@
 //              memory, is rescaled), P in bfloat16 over the scores read. The sink joins the denominator at the end.
 // What bounds it: instruction issue of the softmax warps. The cap's polynomial is nine operations a score, taken two scores an
 // instruction (f32x2); a score's exponential and sum are four more. A prompt of 2,048 tokens, 32 heads over 4 of 64, window 1,024, cap 30 and
-// sink: 125 us with mma.sync, 87 here.
+// sink: 125 us with mma.sync, 70 here (87 with a branch a pair of scores for those beyond the cap, which the fetch of instructions waited for).
 // Every wait is bounded; a wait that runs out sets the error word and the CTA winds down.
 #include "attention_capped.cuh"
 #include "error_word.cuh"
@@ -295,31 +295,37 @@ capped_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
       auto sc = [&](int c) -> float& { return reinterpret_cast<float&>(sv[c >> 5][c & 31]); };
       if (CAP) {
         // tanh within [-1, 1] as an odd polynomial of degree 13, two scores an instruction; where a score of the warp lies beyond,
-        // those that do by way of the exponential (attention_capped_mma.cu gives the polynomial's error)
+        // by way of the exponential for those that do (attention_capped_mma.cu gives the polynomial's error)
         float largest = 0.f;
         const pair_t pre2 = make_pair(pre, pre);
 #pragma unroll
         for (int c = 0; c < KT; c += 2) largest = max3(largest, fabsf(sc(c)), fabsf(sc(c + 1)));
         const bool beyond = __any_sync(0xffffffffu, !(largest * pre <= 1.0f));
-        auto k2 = [](float k) { return make_pair(k, k); };
+        if (!beyond) {                                             // the usual case, in one piece: a branch a score is fetched late
+          auto k2 = [](float k) { return make_pair(k, k); };
 #pragma unroll
-        for (int c = 0; c < KT; c += 2) {
-          const pair_t x = mul2(make_pair(sc(c), sc(c + 1)), pre2), x2 = mul2(x, x);
-          pair_t q = fma2(k2(0.0009637729963287711f), x2, k2(-0.005951283033937216f));
-          q = fma2(q, x2, k2(0.019973287358880043f));
-          q = fma2(q, x2, k2(-0.05326583608984947f));
-          q = fma2(q, x2, k2(0.13319583237171173f));
-          q = fma2(q, x2, k2(-0.33332130312919617f));
-          q = fma2(q, x2, k2(0.9999997019767761f));
-          q = mul2(q, x);
-          float a, b;
-          unpack(q, a, b);
-          if (beyond) {                                            // the same for the warp
-            float xa, xb;
-            unpack(x, xa, xb);
-            a = xa * xa <= 1.0f ? a : tanh_exp2(xa), b = xb * xb <= 1.0f ? b : tanh_exp2(xb);
+          for (int c = 0; c < KT; c += 2) {
+            const pair_t x = mul2(make_pair(sc(c), sc(c + 1)), pre2), x2 = mul2(x, x);
+            pair_t q = fma2(k2(0.0009637729963287711f), x2, k2(-0.005951283033937216f));
+            q = fma2(q, x2, k2(0.019973287358880043f));
+            q = fma2(q, x2, k2(-0.05326583608984947f));
+            q = fma2(q, x2, k2(0.13319583237171173f));
+            q = fma2(q, x2, k2(-0.33332130312919617f));
+            q = fma2(q, x2, k2(0.9999997019767761f));
+            unpack(mul2(q, x), sc(c), sc(c + 1));
           }
-          sc(c) = a, sc(c + 1) = b;
+        } else {
+#pragma unroll
+          for (int c = 0; c < KT; ++c) {
+            const float x = sc(c) * pre, x2 = x * x;
+            float q = fmaf(0.0009637729963287711f, x2, -0.005951283033937216f);
+            q = fmaf(q, x2, 0.019973287358880043f);
+            q = fmaf(q, x2, -0.05326583608984947f);
+            q = fmaf(q, x2, 0.13319583237171173f);
+            q = fmaf(q, x2, -0.33332130312919617f);
+            q = fmaf(q, x2, 0.9999997019767761f);
+            sc(c) = x2 <= 1.0f ? q * x : tanh_exp2(x);
+          }
         }
       }
       if (FAR) {
