@@ -136,24 +136,39 @@ grouped_gemm_kernel(const __nv_bfloat16* __restrict__ a, int lda, long long a_gr
   __syncthreads();
   const __nv_bfloat16* ae = a + (size_t)e * a_group;
   const __nv_bfloat16* we = w + (size_t)e * w_group;
+  // Every step copies the same rows and chunks of a row, further along K: where each of a thread's copies starts is found once (found anew
+  // for every copy, the addresses were most of the instructions, which bound the product for few rows).
+  constexpr int NA = TM * CH / THREADS, NB = BROWS * CH / THREADS;
+  static_assert(NA * THREADS == TM * CH && NB * THREADS == BROWS * CH && THREADS % CH == 0, "whole copies a thread");
+  const int c8 = tid % CH * 8;                     // the thread's chunk of every row it copies
+  const __nv_bfloat16 *a_from[NA], *b_from[NB];    // null: a row of zeros
+#pragma unroll
+  for (int i = 0; i < NA; ++i) {
+    const int src = src_row[tid / CH + i * (THREADS / CH)];
+    a_from[i] = src >= 0 ? ae + (size_t)src * lda + c8 : nullptr;
+  }
+#pragma unroll
+  for (int i = 0; i < NB; ++i) {
+    const int r = tid / CH + i * (THREADS / CH), n = n0 + r % TN;
+    // gate row n and up row n of the group: N gate rows then N up rows, or (packed) gate and up rows
+    // interleaved in groups of 64, which is the layout of the tcgen05 product's gated epilogue
+    const size_t wrow = packed ? (size_t)((n >> 6) * 128 + (n & 63) + (r < TN ? 0 : 64)) : (size_t)(r < TN ? n : N + n);
+    b_from[i] = n < N ? we + wrow * K + c8 : nullptr;
+  }
+  const int to = tid / CH * GPITCH + c8 * 2;
   auto load = [&](int k0, int stage) {
-    unsigned char* as = a_tile(stage);
-    unsigned char* bs = b_tile(stage);
-    for (int idx = tid; idx < TM * CH; idx += THREADS) {
-      const int r = idx / CH, c = idx % CH;
-      const int k = k0 + c * 8;
-      const bool valid = src_row[r] >= 0 && k < K;
-      cp16(as + r * GPITCH + c * 16, ae + (valid ? (size_t)src_row[r] * lda + k : 0), valid);
+    unsigned char* as = a_tile(stage) + to;
+    unsigned char* bs = b_tile(stage) + to;
+    const bool in = k0 + c8 < K;
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+      const bool valid = in && a_from[i] != nullptr;
+      cp16(as + i * (THREADS / CH) * GPITCH, valid ? a_from[i] + k0 : ae, valid);
     }
-    for (int idx = tid; idx < BROWS * CH; idx += THREADS) {
-      const int r = idx / CH, c = idx % CH;
-      const int k = k0 + c * 8;
-      const int n = n0 + (r % TN);
-      const bool valid = n < N && k < K;
-      // gate row n and up row n of the group: N gate rows then N up rows, or (packed) gate and up rows
-      // interleaved in groups of 64, which is the layout of the tcgen05 product's gated epilogue
-      const size_t wrow = packed ? (size_t)((n >> 6) * 128 + (n & 63) + (r < TN ? 0 : 64)) : (size_t)(r < TN ? n : N + n);
-      cp16(bs + r * GPITCH + c * 16, we + (valid ? wrow * K + k : 0), valid);
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const bool valid = in && b_from[i] != nullptr;
+      cp16(bs + i * (THREADS / CH) * GPITCH, valid ? b_from[i] + k0 : we, valid);
     }
   };
   const int wm = warp / WN, wn = warp % WN;
