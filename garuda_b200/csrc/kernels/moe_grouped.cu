@@ -225,6 +225,36 @@ grouped_gemm_kernel(const __nv_bfloat16* __restrict__ a, int lda, long long a_gr
   }
   const int g = lane >> 2, tig = lane & 3;
   OT* oe = out + (size_t)e * out_group;
+  auto result = [&](int mi, int nt, int x, int r) {
+    float v = acc[mi][nt][x];
+    if (GATED) v = gate_act(kind, limit, v * row_scale[GATED ? r : 0], acc_u[GATED ? mi : 0][nt][x] * row_scale[GATED ? r : 0]);
+    if (MODE == ACT_UP) v = plain_act(kind, v * row_scale[SCALED ? r : 0]);
+    return v;
+  };
+  // bfloat16 rows that start on 16 bytes go out 16 bytes a store, by way of shared memory (2-byte stores took most of the time of
+  // the products of few channels: queries into a latent, 2,048 tokens of 32 heads, 32 channels to 256, 52 us against 20)
+  if (sizeof(OT) == 2 && N % 8 == 0 && ldo % 8 == 0 && ((uintptr_t)oe & 15) == 0) {
+    constexpr int OP = TN * 2 + 16;                // bytes between rows
+    static_assert((size_t)TM * OP <= (size_t)STAGES * (TM + BROWS) * GPITCH, "the finished tile takes the stages' place");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int mi = 0; mi < MI; ++mi)
+#pragma unroll
+      for (int nt = 0; nt < 2 * NP; ++nt)
+#pragma unroll
+        for (int up = 0; up < 2; ++up) {
+          const int r = (wm * MI + mi) * 16 + g + up * 8;
+          gb::store_pair(reinterpret_cast<__nv_bfloat16*>(tiles + r * OP) + wn * NP * 16 + nt * 8 + 2 * tig, result(mi, nt, up * 2, r),
+                         result(mi, nt, up * 2 + 1, r));
+        }
+    __syncthreads();
+    for (int idx = tid; idx < TM * (TN / 8); idx += THREADS) {
+      const int r = idx / (TN / 8), c = idx % (TN / 8) * 8;
+      if (r < rows && n0 + c < N) *reinterpret_cast<uint4*>(oe + (size_t)(row0 + r) * ldo + n0 + c) = *reinterpret_cast<const uint4*>(tiles + r * OP + c * 2);
+    }
+    return;
+  }
 #pragma unroll
   for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
@@ -233,11 +263,7 @@ grouped_gemm_kernel(const __nv_bfloat16* __restrict__ a, int lda, long long a_gr
       for (int x = 0; x < 4; ++x) {
         const int r = (wm * MI + mi) * 16 + g + (x >> 1) * 8;
         const int n = n0 + wn * NP * 16 + nt * 8 + 2 * tig + (x & 1);
-        if (r >= rows || n >= N) continue;
-        float v = acc[mi][nt][x];
-        if (GATED) v = gate_act(kind, limit, v * row_scale[GATED ? r : 0], acc_u[GATED ? mi : 0][nt][x] * row_scale[GATED ? r : 0]);
-        if (MODE == ACT_UP) v = plain_act(kind, v * row_scale[SCALED ? r : 0]);
-        oe[(size_t)(row0 + r) * ldo + n] = gb::from_float<OT>(v);
+        if (r < rows && n < N) oe[(size_t)(row0 + r) * ldo + n] = gb::from_float<OT>(result(mi, nt, x, r));
       }
 }
 
