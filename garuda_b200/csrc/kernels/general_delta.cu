@@ -192,9 +192,10 @@ gdelta_recurrence_kernel(const float* __restrict__ prep, int W, const int32_t* _
 //     o_i = (D_i r_i)^T S_0 + sum_{j<=i} H_ij v_j - G_ij x_j,    G_ij = sum_d r_i alpha_j D_i / D_j,     H_ij likewise with k_j
 // so  W = (I + E)^-1 (D u),   VP = -(I + E)^-1 F v,   Q = D r - G W,   OP = H v + G VP,   K1_j = alpha_j D_last / D_j,   K2_j = k_j
 // D_last / D_j, and the walk's Y is -x. Quotients of decays are running products and the system is solved by substitution, a
-// thread per column, in 32-bit multiply-adds, as for the gated rule (delta_rule.cu). grid (chunk numbers, H), 256 threads.
+// thread per column, in 32-bit multiply-adds, as for the gated rule (delta_rule.cu). grid (chunk numbers, H), 2 DIM threads: with 256 for
+// 64 channels half of them had no column (2,048 tokens of 32 heads of 64 x 64: 211 us, now 171).
 template <int DIM>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(2 * DIM, DIM == 64 ? 4 : 2)
 gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, int col_k, int col_v, int col_a,
                             const float* __restrict__ zdec, int PZ, const float* __restrict__ w0, const float* __restrict__ a0,
                             float decay_scale, const int32_t* __restrict__ cu_q, float* __restrict__ blocks, int R, int H, int vdim,
@@ -204,6 +205,7 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
   gb::pdl_launch_dependents();
   gb::pdl_wait();
   constexpr int LD = DIM + 4, VEC = DIM / 32;
+  constexpr int THREADS = 2 * DIM, WARPS = THREADS / 32;      // a thread a channel in two walks over the tokens, or a column of W and VP
   extern __shared__ __align__(16) float sh[];
   float* su = sh;                        // [C][LD]: u, then D u
   float* sr = su + C * LD;               // [C][LD]: r, then D r
@@ -220,7 +222,7 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
   float* block = blocks + ((size_t)blockIdx.x * H + h) * lay.floats();
   const float* row0 = proj + (size_t)first * P;
 #pragma unroll 2
-  for (int t = warp; t < C; t += 8) {
+  for (int t = warp; t < C; t += WARPS) {
     const float* row = row0 + (size_t)t * P;
     float k[VEC], x[VEC], y[VEC], z[VEC], ss = 0.f;
 #pragma unroll
@@ -243,10 +245,12 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
       sa[t * LD + d] = t < n ? sigmoid(y[e] + a0[c]) * u : 0.f;
     }
   }
-  for (int i = tid; i < 4 * C * LT; i += 256) sE[i] = 0.f;
+  for (int i = tid; i < 4 * C * LT; i += THREADS) sE[i] = 0.f;
   __syncthreads();
-  {
-    const int j0 = (warp < 4 ? warp : 11 - warp) * 4, d0 = lane * VEC;
+  // four keys a warp at a time; early and late ones, which meet more and fewer tokens, in turn on a scheduler
+#pragma unroll 1
+  for (int turn = 0; turn < 8 / WARPS; ++turn) {
+    const int j0 = (WARPS == 8 ? (warp < 4 ? warp : 11 - warp) : (turn == 0 ? warp : 7 - warp)) * 4, d0 = lane * VEC;
     pair_t pa[4][VEC / 2], pk[4][VEC / 2];                // alpha_j and k_j, decayed on
     auto row = [&](const float* m, int i, pair_t (&x)[VEC / 2]) {
       if (VEC == 4) {
@@ -336,13 +340,13 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
       su[i * LD + tid] *= run;
       run *= sw[i * LD + tid];
     }
-  } else if (tid >= 128 && tid < 128 + DIM) {
+  } else {
     float run = 1.f;
 #pragma unroll 8
-    for (int i = 0; i < C; ++i) sr[i * LD + tid - 128] *= run *= sw[i * LD + tid - 128];
+    for (int i = 0; i < C; ++i) sr[i * LD + tid - DIM] *= run *= sw[i * LD + tid - DIM];
   }
   __syncthreads();
-  for (int c = tid; c < DIM + vdim; c += 256) {
+  for (int c = tid; c < DIM + vdim; c += THREADS) {
     const bool key = c < DIM;                             // the same for a warp
     const float* v = row0 + col_v + h * vdim + c - DIM;   // a value column's numbers
     pair_t w[C / 2], o[C / 2];
@@ -531,7 +535,7 @@ GB_EXPORT int gb_gdelta_chunk(const float* proj, int P, int col_r, int col_k, in
     configured[dim == 128].done();
   }
   const int rc = gb::check_pdl_launch(
-      gb::launch_pdl(kernel, dim3(delta_chunk::chunk_numbers(T, R), H), dim3(256), smem, stream, dim3(1, 1, 1), proj, P, col_r, col_k,
+      gb::launch_pdl(kernel, dim3(delta_chunk::chunk_numbers(T, R), H), dim3(2 * dim), smem, stream, dim3(1, 1, 1), proj, P, col_r, col_k,
                      col_v, col_a, zdec, PZ, w0, a0, decay_scale, cu_q, blocks, R, H, vdim, cut),
       "gdelta_chunk");
   if (rc != GB_OK) return rc;
