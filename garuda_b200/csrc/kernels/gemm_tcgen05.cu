@@ -1385,6 +1385,205 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_cons
   if (warp == 1) tmem_dealloc_pair(tmem_base, TMEM_COLS);
 }
 
+// The gated product of some hundreds of tokens: the weights are the products' rows (256 a pair of CTAs: a group of 128 packed rows, 64
+// features' gate and up rows, each CTA), up to 512 tokens their columns, so that every weight is fetched once and a step's
+// operands, which L2 delivers at about 75 GB/s and SM and which bound the 256 x 256 tiles, serve up to 256 x 512 products. The
+// tokens are padded to two equal parts of a multiple of 32 (333 to 384), where token tiles of 256 rows pad them to 512; both
+// parts' accumulators lie side by side in tensor memory (512 columns, one stage). The result is on its side: a lane holds a
+// feature, and the weights' boxes bring 16 gate rows and the up
+// rows of the same features to the lanes of one warp, which exchange them by shuffles.
+// 333 tokens, 4,096 channels, 2 x 14,336 rows: 112 us with 256 x 256 tiles (224 tiles are four rounds of 74 pairs, the last
+// nearly empty), 102 here.
+constexpr int W_STAGES = 5;                           // at the narrowest; 48 KB stages: four
+constexpr int W_TOKENS = 512;
+constexpr int W_PIPE_BYTES = 192 * 1024;
+__host__ __device__ constexpr int wide_part(int tokens) { return ((tokens + 1) / 2 + 31) / 32 * 32; }     // a part's tokens: 32 to 256
+__host__ __device__ constexpr int wide_stage_bytes(int part) { return BM * BK * 2 + part * BK * 2; }      // a CTA's half of both parts
+
+// A group of 128 packed rows (64 gate, 64 up) with 16 gate and their 16 up rows in turn, as the boxes of gated_map lie.
+__device__ __forceinline__ void load_gated_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int k, int group) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %4, %4, %5}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(k), "r"(0), "r"(group)
+      : "memory");
+}
+
+// silu_gate_fast with the reciprocal to a last place instead of rounded, without a branch: nothing hides this epilogue, and the
+// branches of 32 rounded reciprocals kept one value's latencies from covering the next one's (2.8 us every 32 tokens).
+__device__ __forceinline__ float silu_gate_approx(float g, float u) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.0f + __expf(-g)));
+  return g * r * u;
+}
+
+template <int EPI>
+__global__ void __launch_bounds__(p_threads(EPI_SWIGLU), 1)
+gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, __nv_bfloat16* __restrict__ out,
+                    int ldo, int tokens, int features, int K, int total_tiles, int part, int stages, const EpilogueArgs ra) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[W_STAGES];
+  __shared__ __align__(8) uint64_t empty_bar[W_STAGES];
+  __shared__ __align__(8) uint64_t acc_full, acc_empty;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int abort_s;
+  __shared__ __align__(16) __nv_bfloat16 out_s[8][33 * 16];      // per epilogue warp: 32 tokens' rows of 16 features on their way out
+  __shared__ float inv_s[W_TOKENS];                              // the folded norm's factor per token
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int num_kb = (K + BK - 1) / BK, stage_bytes = wide_stage_bytes(part);
+  const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(smem_u32(&full_bar[s]), 1);
+      mbar_init(smem_u32(&empty_bar[s]), 1);
+    }
+    mbar_init(smem_u32(&acc_full), 1);
+    mbar_init(smem_u32(&acc_empty), 2 * epilogue_warps(EPI_SWIGLU));
+    abort_s = 0;
+    fence_barrier_init();
+    fence_proxy_async();
+    prefetch_tensormap(&map_w);
+    prefetch_tensormap(&map_x);
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(smem_u32(&tmem_base_s), 512);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_arrive_wait();        // both CTAs' barriers exist before either signals the other's
+  tc_fence_after_sync();
+  const uint32_t tmem_base = tmem_base_s;
+  volatile int* aborted = &abort_s;
+  gb::pdl_launch_dependents();
+  gb::pdl_wait();
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // ------------------------------------------------------------ producer (both CTAs)
+      int s = 0, par = 1, issued = 0;
+      for (int tile = pair; tile < total_tiles && !*aborted; tile += pairs) {
+        for (int kb = 0; kb < num_kb; ++kb) {
+          if (!mbar_wait(smem_u32(&empty_bar[s]), par)) {
+            gb_err::report(ERR_WAIT_EMPTY);
+            *aborted = 1;
+          }
+          if (*aborted) break;
+          const uint32_t bar = map_to_rank(smem_u32(&full_bar[s]), 0);     // the even CTA's barrier
+          const uint32_t base = tiles + s * stage_bytes;
+          if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[s]), 2 * stage_bytes);
+          load_gated_pair(base, &map_w, bar, kb * BK, tile * 2 + (int)rank);
+          // this CTA's half of either part's tokens
+          tma_load_2d_pair(base + BM * BK * 2, &map_x, bar, kb * BK, (int)rank * (part / 2));
+          tma_load_2d_pair(base + BM * BK * 2 + part * BK, &map_x, bar, kb * BK, part + (int)rank * (part / 2));
+          ++issued;
+          if (++s == stages) s = 0, par ^= 1;
+        }
+      }
+      if (*aborted && issued > 0) {
+        // wind down, as in the pair kernel
+        const unsigned long long t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 2000000ull) {}
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {
+      // ------------------------------------------------------------ MMA issuer (even CTA)
+      const uint32_t idesc = instr_desc_bf16(2 * BM, part);
+      int s = 0, par = 0, t = 0;
+      for (int tile = pair; tile < total_tiles && !*aborted; tile += pairs, ++t) {
+        if (!mbar_wait(smem_u32(&acc_empty), (t & 1) ^ 1)) {
+          gb_err::report(ERR_WAIT_ACCUM);
+          *aborted = 1;
+          break;
+        }
+        tc_fence_after_sync();
+        for (int kb = 0; kb < num_kb; ++kb) {
+          if (!mbar_wait(smem_u32(&full_bar[s]), par)) {
+            gb_err::report(ERR_WAIT_FULL);
+            *aborted = 1;
+          }
+          if (*aborted) break;
+          tc_fence_after_sync();
+          const uint64_t da = smem_desc_sw128(tiles + s * stage_bytes), db0 = smem_desc_sw128(tiles + s * stage_bytes + BM * BK * 2),
+                         db1 = smem_desc_sw128(tiles + s * stage_bytes + BM * BK * 2 + part * BK);
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k) {
+            mma_bf16_pair(tmem_base, da + 2 * k, db0 + 2 * k, idesc, kb > 0 || k > 0);
+            mma_bf16_pair(tmem_base + part, da + 2 * k, db1 + 2 * k, idesc, kb > 0 || k > 0);
+          }
+          mma_commit_pair(smem_u32(&empty_bar[s]), 3);
+          if (++s == stages) s = 0, par ^= 1;
+        }
+        mma_commit_pair(smem_u32(&acc_full), 3);
+      }
+    }
+  } else {
+    // -------------------------------------------------------------- epilogue: two sets of four warps, 32 tokens at a time in turn
+    const int quarter = warp & 3, set = (warp - 2) >> 2;
+    for (int r = threadIdx.x - 64; r < W_TOKENS; r += 256) inv_s[r] = epilogue_row_scale(ra, r, tokens);
+    asm volatile("barrier.cta.sync 1, 256;" ::: "memory");
+    const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    const bool gate = lane < 16;                          // lanes 0 to 15: gate rows of 16 features, the others their up rows
+    __nv_bfloat16* rows_s = out_s[warp - 2];
+    int t = 0;
+    for (int tile = pair; tile < total_tiles; tile += pairs, ++t) {
+      const bool have = mbar_wait(smem_u32(&acc_full), t & 1);
+      if (!have && lane == 0) {
+        gb_err::report(ERR_WAIT_ACCUM);
+        *aborted = 1;
+      }
+      if (!have || *aborted) break;
+      tc_fence_after_sync();
+      const int f0 = (tile * 2 + (int)rank) * 64 + quarter * 16;
+      const bool vec = f0 + 16 <= features && ldo % 8 == 0 && (((uintptr_t)out) & 15) == 0;
+      for (int t0 = set * 32; t0 < tokens; t0 += 64) {
+        __syncwarp();
+        uint32_t r[32];
+        tmem_ld_32(taddr + t0, r);
+        tmem_ld_wait();
+        // a gate lane keeps the first 16 tokens and sends the others, an up lane the other way round
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const int token = gate ? j : j + 16;
+          const float inv = inv_s[t0 + token], mine = __uint_as_float(gate ? r[j] : r[j + 16]) * inv;
+          const float theirs = __uint_as_float(__shfl_xor_sync(0xffffffffu, gate ? r[j + 16] : r[j], 16)) * inv;
+          const float g = gate ? mine : theirs, u = gate ? theirs : mine;
+          rows_s[(token + (gate ? 0 : 1)) * 16 + (lane & 15)] = __float2bfloat16_rn((EPI & EPI_GENERAL) ? gate_fast(ra, g, u) : silu_gate_approx(g, u));
+        }
+        __syncwarp();
+        if (vec) {
+#pragma unroll
+          for (int i = lane; i < 64; i += 32) {
+            const int row = i >> 1, c = (i & 1) * 8;
+            if (t0 + row < tokens)
+              *reinterpret_cast<uint4*>(out + (size_t)(t0 + row) * ldo + f0 + c) = *reinterpret_cast<const uint4*>(rows_s + (row + (row >> 4)) * 16 + c);
+          }
+        } else {
+          for (int i = lane; i < 32 * 16; i += 32) {
+            const int row = i >> 4, c = i & 15;
+            if (t0 + row < tokens && f0 + c < features) out[(size_t)(t0 + row) * ldo + f0 + c] = rows_s[(row + (row >> 4)) * 16 + c];
+          }
+        }
+      }
+      // every read of the accumulators has completed: hand them back to the issuer
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        if (rank == 0) mbar_arrive(smem_u32(&acc_empty));
+        else mbar_arrive_cluster(map_to_rank(smem_u32(&acc_empty), 0));
+      }
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_arrive_wait();
+  if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
+}
+
 // ------------------------------------------------------------------ host side
 // How many CTAs of a cluster share K. Measured on B200 (2048- to 5632-wide layers, 8 tokens): a CTA
 // costs about 3.5 us before and after its stream of K blocks and streams one 16 KB block in about
@@ -1534,6 +1733,37 @@ int launch_pair(const CUtensorMap& mm, const CUtensorMap& mn, OT* out, int ldo, 
                               "gemm_tc (pairs)");
 }
 
+// Packed gate and up rows [groups of 64 + 64, K] as boxes of one group and 64 channels: (channel, row of 16, gate or up, 16 rows of 64, group).
+int gated_map(const void* w, int groups, int K, CUtensorMap* out) {
+  auto encode = tc_host::encode_fn();
+  if (!encode) return gb::fail(GB_CUDA_ERROR, "cuTensorMapEncodeTiled is not available from this driver");
+  const cuuint64_t row = (cuuint64_t)K * 2;
+  const cuuint64_t dims[5] = {(cuuint64_t)K, 16, 2, 4, (cuuint64_t)groups}, strides[4] = {row, 64 * row, 16 * row, 128 * row};
+  const cuuint32_t box[5] = {BK, 16, 2, 4, 1}, step[5] = {1, 1, 1, 1, 1};
+  const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(w), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? GB_OK : gb::fail(GB_CUDA_ERROR, "cuTensorMapEncodeTiled failed with code %d for %d groups of %d channels", (int)r, groups, K);
+}
+
+// Up to 512 tokens on the wide tiles.
+template <int EPI>
+int launch_wide(const CUtensorMap& mw, const CUtensorMap& mx, __nv_bfloat16* out, int ldo, int tokens, int weight_rows, int features, int K,
+                cudaStream_t stream, const EpilogueArgs& ra) {
+  auto kernel = gemm_tc_wide_kernel<EPI>;
+  static gb::OncePerDevice configured;
+  if (configured.needed()) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, W_PIPE_BYTES + 1024);
+    if (e != cudaSuccess) return gb::fail(GB_CUDA_ERROR, "gemm_tc: %s", cudaGetErrorString(e));
+    configured.done();
+  }
+  const int part = wide_part(tokens), fit = W_PIPE_BYTES / wide_stage_bytes(part), stages = fit < W_STAGES ? fit : W_STAGES;
+  const int total = (weight_rows + 2 * BM - 1) / (2 * BM), most = sm_count() / 2;
+  return gb::check_pdl_launch(gb::launch_pdl(kernel, dim3(2 * (total < most ? total : most)), dim3(p_threads(EPI_SWIGLU)),
+                                             (size_t)stages * wide_stage_bytes(part) + 1024, stream, dim3(2, 1, 1), mw, mx, out, ldo, tokens,
+                                             features, K, total, part, stages, ra),
+                              "gemm_tc (wide)");
+}
+
 // Tile width for many tokens: the one that needs fewer rounds over the SMs (a 256-wide tile costs
 // two 128-wide ones but reads each operand half as often); ties go to the wide tile.
 int pick_tile_width(int rows_m, int rows_n) {
@@ -1572,6 +1802,26 @@ bool many_token_pairs(int tokens, int weight_rows, int epi = -1) {
 }
 int many_token_width(int tokens, int weight_rows, int epi = -1) {
   return many_token_pairs(tokens, weight_rows, epi) ? 256 : pick_tile_width(tokens, weight_rows);
+}
+
+// Whether a gated product takes the wide tiles: where their rounds over the pairs fetch fewer bytes a CTA than the other tiles' rounds
+// do (KB a step of 64 channels: a wide tile 16 of weights and an eighth of a part's tokens, the others 32 or, one CTA's 256 columns,
+// 48), a wide tile's epilogue, which its one accumulator stage leaves bare, counted at the 14 us in which a CTA fetches 1,050 KB.
+// In us, other tiles against wide ones, for 257 / 333 / 448 / 512 tokens: 2 x 14,336 rows of 4,096 channels, four rounds against
+// two, 115 / 117 / 118 / 118 against 96 / 102 / 109 / 119; 2 x 9,472 rows of 4,096, two against one, 68 / 68 / 70 / 70 against 56 /
+// 60 / 64 / -; 2 x 28,672 rows of 8,192, 370 / 377 / 387 / 413 against 319 / 344 / 375 / 399; where the line says no: 2 x 11,008 rows
+// of 4,096, three against two, 91 / 91 / 92 / 92 against 94 / 101 / 106 / -; 2 x 8,192 rows of 2,048, 41 / 41 / 42 / 43 against 37 /
+// 40 / 43 / 45.
+bool wide_gated(int tokens, int weight_rows, int K) {
+  if (tokens <= few_token_limit() || tokens > W_TOKENS || weight_rows < 2 * BM) return false;
+  const int sms = sm_count(), pairs = sms / 2;
+  const long long steps = (K + BK - 1) / BK;
+  auto rounds = [](int tiles, int places) { return (tiles + places - 1) / places; };
+  const long long wide = rounds((weight_rows + 2 * BM - 1) / (2 * BM), pairs) * (steps * (16 + wide_part(tokens) / 8) + 1050);
+  const int tiles_m = (tokens + BM - 1) / BM;
+  const int pair_cost = rounds(((tokens + 2 * BM - 1) / (2 * BM)) * ((weight_rows + 255) / 256), pairs) * 32;
+  const int one128 = rounds(tiles_m * ((weight_rows + 127) / 128), sms) * 32, one256 = rounds(tiles_m * ((weight_rows + 255) / 256), sms) * 48;
+  return wide < steps * pair_cost && wide < steps * one128 && wide < steps * one256;
 }
 
 }  // namespace
@@ -1699,6 +1949,12 @@ GB_EXPORT int gb_gemm_tc(const void* x, const void* w, void* out, int Mx, int Nw
     if (bn == 16) return dispatch_cluster<16>(epi, out_dtype, mm, mn, out, Nw, weight_rows, Nw, Mx, K, stream, ra);
     if (bn == 32) return dispatch_cluster<32>(epi, out_dtype, mm, mn, out, Nw, weight_rows, Nw, Mx, K, stream, ra);
     return dispatch_cluster<64>(epi, out_dtype, mm, mn, out, Nw, weight_rows, Nw, Mx, K, stream, ra);
+  }
+  if ((epi & 7) == EPI_SWIGLU && wide_gated(Mx, weight_rows, K)) {
+    if ((rc = gated_map(w, weight_rows / 128, K, &mm))) return rc;
+    if ((rc = tensor_map_2d(x, Mx, K, wide_part(Mx) / 2, &mn))) return rc;
+    if (ra.gate_act != GATE_SILU) return launch_wide<EPI_SWIGLU | EPI_GENERAL>(mm, mn, (__nv_bfloat16*)out, Nw, Mx, weight_rows, Nw, K, stream, ra);
+    return launch_wide<EPI_SWIGLU>(mm, mn, (__nv_bfloat16*)out, Nw, Mx, weight_rows, Nw, K, stream, ra);
   }
   if ((rc = tensor_map_2d(x, Mx, K, BM, &mm))) return rc;
   const bool pairs = many_token_pairs(Mx, weight_rows, epi);
