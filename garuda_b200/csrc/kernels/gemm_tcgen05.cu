@@ -1390,9 +1390,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_cons
 // operands, which L2 delivers at about 75 GB/s and SM and which bound the 256 x 256 tiles, serve up to 256 x 512 products. The
 // tokens are padded to two equal parts of a multiple of 32 (333 to 384), where token tiles of 256 rows pad them to 512; both
 // parts' accumulators lie side by side in tensor memory (512 columns, one stage). The result is on its side: a lane holds a
-// feature, and the weights' boxes bring 16 gate rows and the up
-// rows of the same features to the lanes of one warp, which exchange them by shuffles.
-// 333 tokens, 4,096 channels, 2 x 14,336 rows: 112 us with 256 x 256 tiles (224 tiles are four rounds of 74 pairs, the last
+// feature, and the weights' boxes bring 16 gate rows and the up rows of the same features to the lanes of one warp, which
+// exchange them by shuffles.
+// 333 tokens, 4,096 channels, 2 x 14,336 rows: 115 us with 256 x 256 tiles (224 tiles are four rounds of 74 pairs, the last
 // nearly empty), 102 here.
 constexpr int W_STAGES = 5;                           // at the narrowest; 48 KB stages: four
 constexpr int W_TOKENS = 512;
