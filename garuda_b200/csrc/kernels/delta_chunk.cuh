@@ -54,23 +54,43 @@ struct Layout {
   __host__ __device__ int k1(int j, int c) const { return k1() + ((j >> 3) * (dim / 8) + (c >> 3)) * 64 + (c & 7) * 8 + (j & 7); }
 };
 
-// Chunks are numbered so that no two of a step share a number: the k-th chunk of request r, which starts at token
-// t0 = cu_q[r], has the number t0 / C + r + k. All numbers are below chunk_numbers(T, R).
-__host__ __device__ __forceinline__ int chunk_numbers(int T, int R) { return T / C + R; }
+// Chunks are numbered over the requests that are walked (of `cut` tokens or more in the step), so that no two share a number and a
+// step's many short requests take no room: the chunks of the w-th of them (from 0), which starts at token t0, have the numbers from
+// t0 / C + w on. All numbers of `walked` such requests are below chunk_numbers(T, walked).
+__host__ __device__ __forceinline__ int chunk_numbers(int T, int walked) { return T / C + walked; }
 
-// The request and chunk of a number (all threads of a warp call this): false where there is none, or where the
-// request has fewer than `cut` tokens.
+// How many of the requests below r are walked (all threads of a warp call this).
+__device__ __forceinline__ int walked_before(const int32_t* __restrict__ cu_q, int r, int cut) {
+  const int lane = threadIdx.x & 31;
+  int count = 0;
+  for (int r0 = 0; r0 < r; r0 += 32) {
+    const int i = r0 + lane;
+    count += __popc(__ballot_sync(0xffffffffu, i < r && cu_q[min(i, r - 1) + 1] - cu_q[min(i, r - 1)] >= cut));
+  }
+  return count;
+}
+
+// The request and chunk of a number (all threads of a warp call this): false where there is none.
 __device__ __forceinline__ bool find_chunk(int number, const int32_t* __restrict__ cu_q, int R, int cut, int& request, int& first,
                                            int& tokens, int& in_request) {
-  int best = -1;
-  for (int r = threadIdx.x & 31; r < R; r += 32)
-    if (cu_q[r] / C + r <= number) best = r;
+  const int lane = threadIdx.x & 31;
+  int count = 0, best = -1, start = 0;       // the last walked request whose first number is not above this one, and that first number
+  for (int r0 = 0; r0 < R; r0 += 32) {
+    const int r = min(r0 + lane, R - 1), t0 = cu_q[r];
+    const uint32_t walked = __ballot_sync(0xffffffffu, r0 + lane < R && cu_q[r + 1] - t0 >= cut);
+    const int at = t0 / C + count + __popc(walked & ((1u << lane) - 1));
+    if ((walked >> lane & 1) && at <= number) best = r, start = at;
+    count += __popc(walked);
+  }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+  for (int o = 16; o > 0; o >>= 1) {         // both grow with the request
+    best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+    start = max(start, __shfl_xor_sync(0xffffffffu, start, o));
+  }
   if (best < 0) return false;
   const int t0 = cu_q[best], n = cu_q[best + 1] - t0;
-  in_request = (number - (t0 / C + best)) * C;
-  if (n < cut || in_request >= n) return false;
+  in_request = (number - start) * C;
+  if (in_request >= n) return false;
   request = best, first = t0 + in_request, tokens = min(C, n - in_request);
   return true;
 }
@@ -183,18 +203,19 @@ struct WalkSmem {
   float y[GROUPS][TWO ? 2 : 1][COLS][LDY]; // Y^T (and V^T)
 };
 
-// grid (H, vdim / (16 GROUPS), R). blocks [chunk numbers, H, Layout::floats()]. out [T, H vdim].
+// grid (H, vdim / (16 GROUPS), R). blocks [numbers, H, Layout::floats()]. out [T, H vdim].
 template <int DIM, int GROUPS, bool TWO>
 __global__ void __launch_bounds__(GROUP * GROUPS, 1)
 walk_kernel(const float* __restrict__ blocks, const int32_t* __restrict__ cu_q, const int32_t* __restrict__ slots,
-            float* __restrict__ state, long long state_stride, int H, int vdim, int cut, float* __restrict__ out) {
+            float* __restrict__ state, long long state_stride, int H, int vdim, int cut, int numbers, float* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char raw[];
   using Smem = WalkSmem<DIM, GROUPS, TWO>;
   Smem& sm = *reinterpret_cast<Smem*>(raw);
   gb::pdl_wait();
   const int h = blockIdx.x, r = blockIdx.z;
   const int t0 = cu_q[r], n = cu_q[r + 1] - t0;
-  if (n < cut || n <= 0) return;
+  if (n < cut) return;
+  const int number = t0 / C + walked_before(cu_q, r, cut);
   const Layout lay{DIM, vdim, TWO ? 1 : 0};
   constexpr int THREADS = GROUP * GROUPS;
   constexpr int KS = DIM / 32;                       // tiles of 8 channels of a warp
@@ -204,8 +225,9 @@ walk_kernel(const float* __restrict__ blocks, const int32_t* __restrict__ cu_q, 
   const int mycol = (tid >> 1) & 15, tok4 = ((tid & 1) | (warp << 1)) * 4;      // where Y and o are formed: a column, four tokens
   const int slot = slots[r];
   const int chunks = (n + C - 1) / C;
+  if (number + chunks > numbers) return;             // more requests than the caller counted: nothing beyond blocks is read
   const size_t per = (size_t)H * lay.floats();
-  const float* base = blocks + ((size_t)(t0 / C + r) * H + h) * lay.floats();
+  const float* base = blocks + ((size_t)number * H + h) * lay.floats();
 
   auto load = [&](int k) {
     const float* src = base + k * per;
@@ -346,7 +368,7 @@ walk_kernel(const float* __restrict__ blocks, const int32_t* __restrict__ cu_q, 
 
 template <int DIM, int GROUPS, bool TWO>
 int launch_walk_as(const char* what, const float* blocks, const int32_t* cu_q, const int32_t* slots, float* state, long long state_stride,
-                   int R, int H, int vdim, int cut, float* out, cudaStream_t stream) {
+                   int R, int H, int vdim, int cut, int numbers, float* out, cudaStream_t stream) {
   auto kernel = walk_kernel<DIM, GROUPS, TWO>;
   constexpr size_t smem = sizeof(WalkSmem<DIM, GROUPS, TWO>);
   static_assert(smem <= 227 * 1024, "a block's shared memory");
@@ -357,20 +379,20 @@ int launch_walk_as(const char* what, const float* blocks, const int32_t* cu_q, c
     configured.done();
   }
   return gb::check_pdl_launch(gb::launch_after(kernel, dim3(H, vdim / (COLS * GROUPS), R), dim3(GROUP * GROUPS), smem, stream,
-                                               dim3(1, 1, 1), blocks, cu_q, slots, state, state_stride, H, vdim, cut, out),
+                                               dim3(1, 1, 1), blocks, cu_q, slots, state, state_stride, H, vdim, cut, numbers, out),
                               what);
 }
 
-// dim 64 or 128, vdim a multiple of 32.
+// dim 64 or 128, vdim a multiple of 32. numbers: what blocks has room for, chunk_numbers(T, walked).
 template <bool TWO>
 int launch_walk(const char* what, const float* blocks, const int32_t* cu_q, const int32_t* slots, float* state, long long state_stride,
-                int R, int H, int dim, int vdim, int cut, float* out, cudaStream_t stream) {
+                int R, int H, int dim, int vdim, int cut, int numbers, float* out, cudaStream_t stream) {
   const bool one = (long long)R * H * (vdim / COLS) <= 148;
   if (dim == 128)
-    return one ? launch_walk_as<128, 1, TWO>(what, blocks, cu_q, slots, state, state_stride, R, H, vdim, cut, out, stream)
-               : launch_walk_as<128, 2, TWO>(what, blocks, cu_q, slots, state, state_stride, R, H, vdim, cut, out, stream);
-  return one ? launch_walk_as<64, 1, TWO>(what, blocks, cu_q, slots, state, state_stride, R, H, vdim, cut, out, stream)
-             : launch_walk_as<64, 2, TWO>(what, blocks, cu_q, slots, state, state_stride, R, H, vdim, cut, out, stream);
+    return one ? launch_walk_as<128, 1, TWO>(what, blocks, cu_q, slots, state, state_stride, R, H, vdim, cut, numbers, out, stream)
+               : launch_walk_as<128, 2, TWO>(what, blocks, cu_q, slots, state, state_stride, R, H, vdim, cut, numbers, out, stream);
+  return one ? launch_walk_as<64, 1, TWO>(what, blocks, cu_q, slots, state, state_stride, R, H, vdim, cut, numbers, out, stream)
+             : launch_walk_as<64, 2, TWO>(what, blocks, cu_q, slots, state, state_stride, R, H, vdim, cut, numbers, out, stream);
 }
 
 inline bool takes(int dim, int vdim) { return (dim == 64 || dim == 128) && vdim >= 32 && vdim % 32 == 0 && vdim <= 256; }

@@ -258,7 +258,7 @@ delta_recurrence_kernel(const float* __restrict__ prep, int W, const int32_t* __
 //     W = (I + L)^-1 beta (D k),   VP = (I + L)^-1 beta v,   Q = D q - B W,   OP = B VP,   K1_j = k_j D_last / D_j
 // The quotients D_i / D_j are running products of decays from j on (never above one, so nothing overflows and what
 // underflows is nothing), and the triangular system is solved by substitution, a thread per column of W and VP. 32-bit multiply-adds.
-// grid (chunk numbers, H), 256 threads; taps of at most four (the older ones' weights are zero where there are fewer).
+// grid (numbers, H), 256 threads; taps of at most four (the older ones' weights are zero where there are fewer).
 template <int DIM, typename WT>
 __global__ void __launch_bounds__(256, 3)
 delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* __restrict__ second, int P2,
@@ -723,22 +723,23 @@ GB_EXPORT int gb_delta_recurrence(const float* prep, int W, const int32_t* cu_q,
   });
 }
 
-// Whether the chunked kernels take these sizes, and the floats of `blocks` for a step of T tokens of R requests (0: they do not).
-GB_EXPORT long long gb_delta_chunk_floats(int T, int R, int H, int G, int dim, int vdim, int taps) {
-  if (T <= 0 || R <= 0 || H < 1 || H > 65535 || R > 65535 || G < 1 || H % G || taps < 1 || taps > 4 || !delta_chunk::takes(dim, vdim)) return 0;
-  return (long long)delta_chunk::chunk_numbers(T, R) * H * delta_chunk::Layout{dim, vdim, 0}.floats();
+// Whether the chunked kernels take these sizes, and the floats of `blocks` for a step of T tokens, `walked` requests of which have at
+// least `cut` (0: they do not).
+GB_EXPORT long long gb_delta_chunk_floats(int T, int walked, int H, int G, int dim, int vdim, int taps) {
+  if (T <= 0 || walked <= 0 || H < 1 || H > 65535 || walked > 65535 || G < 1 || H % G || taps < 1 || taps > 4 || !delta_chunk::takes(dim, vdim)) return 0;
+  return (long long)delta_chunk::chunk_numbers(T, walked) * H * delta_chunk::Layout{dim, vdim, 0}.floats();
 }
 
 // Requests of at least `cut` tokens: everything from the projected rows to the read-out o [T, H vdim] and the state. The rows
-// are those of delta_prepare; blocks starts on 16 bytes.
+// are those of delta_prepare; walked: how many such requests the step has; blocks starts on 16 bytes.
 GB_EXPORT int gb_delta_chunk(const float* proj, int P, const float* second, int P2, const void* conv_w, int w_dtype, int taps,
                              const float* conv_state, long long conv_stride, const void* a_log, const void* dt_bias,
                              const int32_t* cu_q, const int32_t* slots, float* state, long long state_stride, float* blocks, int T,
-                             int R, int H, int G, int dim, int vdim, int per_head, int cut, float* out, cudaStream_t stream) {
-  if (T <= 0 || R <= 0) return GB_OK;
-  if (gb_delta_chunk_floats(T, R, H, G, dim, vdim, taps) == 0)
+                             int R, int walked, int H, int G, int dim, int vdim, int per_head, int cut, float* out, cudaStream_t stream) {
+  if (T <= 0 || R <= 0 || walked <= 0) return GB_OK;
+  if (R > 65535 || gb_delta_chunk_floats(T, walked, H, G, dim, vdim, taps) == 0)
     return gb::fail(GB_UNSUPPORTED, "delta_chunk: %d heads of %d x %d, %d key heads, %d taps", H, dim, vdim, G, taps);
-  const int CH = 2 * G * dim + H * vdim;
+  const int CH = 2 * G * dim + H * vdim, numbers = delta_chunk::chunk_numbers(T, walked);
   if (P < CH + H || P2 < (per_head ? H : H * dim)) return gb::fail(GB_BAD_ARGUMENT, "delta_chunk: row widths");
   if ((uintptr_t)blocks & 15) return gb::fail(GB_BAD_ARGUMENT, "delta_chunk: blocks start on 16 bytes");
   const size_t smem = (size_t)(delta_chunk::C * (3 * (dim + 4) + 2 * delta_chunk::LT + 1)) * sizeof(float);
@@ -751,13 +752,13 @@ GB_EXPORT int gb_delta_chunk(const float* proj, int P, const float* second, int 
       configured[dim == 128].done();
     }
     return gb::check_pdl_launch(
-        gb::launch_pdl(kernel, dim3(delta_chunk::chunk_numbers(T, R), H), dim3(256), smem, stream, dim3(1, 1, 1), proj, P, second, P2,
+        gb::launch_pdl(kernel, dim3(numbers, H), dim3(256), smem, stream, dim3(1, 1, 1), proj, P, second, P2,
                        (const WT*)conv_w, taps, conv_state, conv_stride, (const WT*)a_log, (const WT*)dt_bias, cu_q, slots, blocks, R, H,
                        G, vdim, per_head, cut),
         "delta_chunk");
   });
   if (rc != GB_OK) return rc;
-  return delta_chunk::launch_walk<false>("delta_chunk", blocks, cu_q, slots, state, state_stride, R, H, dim, vdim, cut, out, stream);
+  return delta_chunk::launch_walk<false>("delta_chunk", blocks, cu_q, slots, state, state_stride, R, H, dim, vdim, cut, numbers, out, stream);
 }
 
 GB_EXPORT int gb_delta_out(const float* o, const float* second, int P2, int gate_off, const void* w, int w_dtype,

@@ -192,7 +192,7 @@ gdelta_recurrence_kernel(const float* __restrict__ prep, int W, const int32_t* _
 //     o_i = (D_i r_i)^T S_0 + sum_{j<=i} H_ij v_j - G_ij x_j,    G_ij = sum_d r_i alpha_j D_i / D_j,     H_ij likewise with k_j
 // so  W = (I + E)^-1 (D u),   VP = -(I + E)^-1 F v,   Q = D r - G W,   OP = H v + G VP,   K1_j = alpha_j D_last / D_j,   K2_j = k_j
 // D_last / D_j, and the walk's Y is -x. Quotients of decays are running products and the system is solved by substitution, a
-// thread per column, in 32-bit multiply-adds, as for the gated rule (delta_rule.cu). grid (chunk numbers, H), 2 DIM threads: with 256 for
+// thread per column, in 32-bit multiply-adds, as for the gated rule (delta_rule.cu). grid (numbers, H), 2 DIM threads: with 256 for
 // 64 channels half of them had no column (2,048 tokens of 32 heads of 64 x 64: 211 us, now 171).
 template <int DIM>
 __global__ void __launch_bounds__(2 * DIM, DIM == 64 ? 4 : 2)
@@ -509,23 +509,25 @@ GB_EXPORT int gb_gdelta_recurrence(const float* prep, int W, const int32_t* cu_q
   });
 }
 
-// Whether the chunked kernels take these sizes, and the floats of `blocks` for a step of T tokens of R requests (0: they do not).
-GB_EXPORT long long gb_gdelta_chunk_floats(int T, int R, int H, int dim, int vdim) {
-  if (T <= 0 || R <= 0 || H < 1 || H > 65535 || R > 65535 || !delta_chunk::takes(dim, vdim)) return 0;
-  return (long long)delta_chunk::chunk_numbers(T, R) * H * delta_chunk::Layout{dim, vdim, 1}.floats();
+// Whether the chunked kernels take these sizes, and the floats of `blocks` for a step of T tokens, `walked` requests of which have at
+// least `cut` (0: they do not).
+GB_EXPORT long long gb_gdelta_chunk_floats(int T, int walked, int H, int dim, int vdim) {
+  if (T <= 0 || walked <= 0 || H < 1 || H > 65535 || walked > 65535 || !delta_chunk::takes(dim, vdim)) return 0;
+  return (long long)delta_chunk::chunk_numbers(T, walked) * H * delta_chunk::Layout{dim, vdim, 1}.floats();
 }
 
 // Requests of at least `cut` tokens: everything from the projected rows to the read-out o [T, H vdim] and the state. The rows
-// are those of gdelta_prepare; blocks starts on 16 bytes.
+// are those of gdelta_prepare; walked: how many such requests the step has; blocks starts on 16 bytes.
 GB_EXPORT int gb_gdelta_chunk(const float* proj, int P, int col_r, int col_k, int col_v, int col_a, const float* zdec, int PZ,
                               const float* w0, const float* a0, float decay_scale, const int32_t* cu_q, const int32_t* slots,
-                              float* state, long long state_stride, float* blocks, int T, int R, int H, int dim, int vdim, int cut,
+                              float* state, long long state_stride, float* blocks, int T, int R, int walked, int H, int dim, int vdim, int cut,
                               float* out, cudaStream_t stream) {
-  if (T <= 0 || R <= 0) return GB_OK;
-  if (gb_gdelta_chunk_floats(T, R, H, dim, vdim) == 0)
+  if (T <= 0 || R <= 0 || walked <= 0) return GB_OK;
+  if (R > 65535 || gb_gdelta_chunk_floats(T, walked, H, dim, vdim) == 0)
     return gb::fail(GB_UNSUPPORTED, "gdelta_chunk: %d heads of %d x %d", H, dim, vdim);
   if (PZ < H * dim) return gb::fail(GB_BAD_ARGUMENT, "gdelta_chunk: row widths");
   if ((uintptr_t)blocks & 15) return gb::fail(GB_BAD_ARGUMENT, "gdelta_chunk: blocks start on 16 bytes");
+  const int numbers = delta_chunk::chunk_numbers(T, walked);
   const size_t smem = (size_t)(delta_chunk::C * 4 * (dim + 4 + delta_chunk::LT)) * sizeof(float);
   auto kernel = dim == 128 ? gdelta_chunk_factors_kernel<128> : gdelta_chunk_factors_kernel<64>;
   static gb::OncePerDevice configured[2];
@@ -535,11 +537,11 @@ GB_EXPORT int gb_gdelta_chunk(const float* proj, int P, int col_r, int col_k, in
     configured[dim == 128].done();
   }
   const int rc = gb::check_pdl_launch(
-      gb::launch_pdl(kernel, dim3(delta_chunk::chunk_numbers(T, R), H), dim3(2 * dim), smem, stream, dim3(1, 1, 1), proj, P, col_r, col_k,
+      gb::launch_pdl(kernel, dim3(numbers, H), dim3(2 * dim), smem, stream, dim3(1, 1, 1), proj, P, col_r, col_k,
                      col_v, col_a, zdec, PZ, w0, a0, decay_scale, cu_q, blocks, R, H, vdim, cut),
       "gdelta_chunk");
   if (rc != GB_OK) return rc;
-  return delta_chunk::launch_walk<true>("gdelta_chunk", blocks, cu_q, slots, state, state_stride, R, H, dim, vdim, cut, out, stream);
+  return delta_chunk::launch_walk<true>("gdelta_chunk", blocks, cu_q, slots, state, state_stride, R, H, dim, vdim, cut, numbers, out, stream);
 }
 
 // One token per request (row t of the batch is request t). Takes vdim <= 256.

@@ -298,9 +298,10 @@ class CudaOps:
                                 c_int, c_int, c_void_p, c_void_p],
         "gb_delta_chunk": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_longlong, c_void_p, c_void_p,
                            c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                           c_int, c_void_p, c_void_p],
+                           c_int, c_int, c_void_p, c_void_p],
         "gb_gdelta_chunk": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float, c_void_p,
-                            c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+                            c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                            c_void_p],
         "gb_delta_out": [c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_float, c_void_p, c_int, c_int, c_int, c_int,
                          c_int, c_int, c_void_p],
         "gb_delta_decode": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_longlong, c_void_p,
@@ -1180,14 +1181,15 @@ class CudaOps:
                 int(decay_per_head), n_decay, silu_gate, self._stream()), "delta_decode")
         else:
             o = ctx.ws.get("delta_o", (T, H * vdim), torch.float32)
-            floats = L.gb_delta_chunk_floats(T, b.num_requests, H, G, dim, vdim, taps)
-            cut = self._delta_chunk_cut(b, out, floats)
+            walked = self._delta_walked(b, out)
+            floats = L.gb_delta_chunk_floats(T, walked, H, G, dim, vdim, taps)
+            cut = self.DELTA_CHUNK_CUT if floats else 0
             if cut:
                 blocks = ctx.ws.get("delta_blocks", (floats,), torch.float32)
                 self._check(L, L.gb_delta_chunk(
                     proj.data_ptr(), proj.stride(0), second.data_ptr(), second.stride(0), conv_w.data_ptr(), wt, taps, conv_state,
                     stride, a_log.data_ptr(), dt_bias.data_ptr(), b.cu_q.data_ptr(), b.slots.data_ptr(), state.data_ptr(), stride,
-                    blocks.data_ptr(), T, b.num_requests, H, G, dim, vdim, int(decay_per_head), cut, o.data_ptr(), self._stream()),
+                    blocks.data_ptr(), T, b.num_requests, walked, H, G, dim, vdim, int(decay_per_head), cut, o.data_ptr(), self._stream()),
                     "delta_chunk", kernels=2)
             if not cut or getattr(b, "min_q_len", 1) < cut:
                 W = C + H * dim + H
@@ -1209,10 +1211,16 @@ class CudaOps:
     #: a whole chunk and a third launch.
     DELTA_CHUNK_CUT = 48
 
-    def _delta_chunk_cut(self, b, out, floats: int) -> int:
-        """From how many tokens on a request of this step is walked by chunks (delta_chunk.cuh); 0: none is. In a 32-bit run
-        every request is walked token by token, so that its numbers do not depend on how its prompt was cut."""
-        return self.DELTA_CHUNK_CUT if floats and out.dtype == torch.bfloat16 and b.max_q_len >= self.DELTA_CHUNK_CUT else 0
+    def _delta_walked(self, b, out) -> int:
+        """How many requests of this step are walked by chunks (delta_chunk.cuh): those of ``DELTA_CHUNK_CUT`` tokens and more, counted
+        where the batch has its lengths on the host, else as many as can be. Only they take room in the chunks' scratch. In a 32-bit run every
+        request is walked token by token, so that its numbers do not depend on how its prompt was cut."""
+        if out.dtype != torch.bfloat16 or b.max_q_len < self.DELTA_CHUNK_CUT:
+            return 0
+        cu = getattr(b, "host", {}).get("cu_q")
+        if cu is None:
+            return min(b.num_requests, out.shape[0] // self.DELTA_CHUNK_CUT)
+        return int((np.diff(cu) >= self.DELTA_CHUNK_CUT).sum())
 
     # ------------------------------------------------------------------ the generalized delta rule
     def general_delta(self, ctx, proj, cols, zdec, w0, a0, decay_scale, norm_w, eps, state, heads, dim, vdim, out):
@@ -1246,14 +1254,15 @@ class CudaOps:
                 "gdelta_decode")
             return
         o = ctx.ws.get("gdelta_o", (T, HV), torch.float32)
-        floats = L.gb_gdelta_chunk_floats(T, b.num_requests, H, dim, vdim)
-        cut = self._delta_chunk_cut(b, out, floats)
+        walked = self._delta_walked(b, out)
+        floats = L.gb_gdelta_chunk_floats(T, walked, H, dim, vdim)
+        cut = self.DELTA_CHUNK_CUT if floats else 0
         if cut:
             blocks = ctx.ws.get("delta_blocks", (floats,), torch.float32)
             self._check(L, L.gb_gdelta_chunk(
                 proj.data_ptr(), proj.stride(0), col_r, col_k, col_v, col_a, zdec.data_ptr(), zdec.stride(0), w0.data_ptr(),
                 a0.data_ptr(), float(decay_scale), b.cu_q.data_ptr(), b.slots.data_ptr(), state.data_ptr(), stride,
-                blocks.data_ptr(), T, b.num_requests, H, dim, vdim, cut, o.data_ptr(), self._stream()), "gdelta_chunk", kernels=2)
+                blocks.data_ptr(), T, b.num_requests, walked, H, dim, vdim, cut, o.data_ptr(), self._stream()), "gdelta_chunk", kernels=2)
         if not cut or getattr(b, "min_q_len", 1) < cut:
             W = 5 * HD + HV
             prep = ctx.ws.get("gdelta_prep", (T, W), torch.float32)

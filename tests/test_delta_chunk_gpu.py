@@ -73,6 +73,43 @@ def test_general_rule(ops, H, dim, vdim, strong):
         close(state_g[keep], state_r[keep], torch.float32, f"step {k}: state", tol=2e-5)
 
 
+@pytest.mark.parametrize("counted", [True, False])
+@pytest.mark.parametrize("lens", [(CUT + 16,) + (1,) * 40, (3, 0, 97, 1, 0, 64) + (2,) * 40 + (CUT, 1), (0, CUT, 0)])
+def test_scratch_is_for_the_requests_that_are_walked(ops, lens, counted):
+    """Single tokens (and requests without any) beside a few long stretches: no room for those that are not walked, whether the batch
+    brings its lengths on the host or not; more than a warp's requests in front of one that is walked."""
+    cuda, cpu = ops
+    H, dim, vdim, taps, R, T = 2, 64, 32, 2, len(lens), sum(lens)
+    C, long = 2 * H * dim + H * vdim, sum(n >= CUT for n in lens)
+    b = step(list(lens), list(range(R))[::-1])
+    if counted:
+        b.host = {"cu_q": b.cu_q.numpy()}
+    ctx_g, ctx_r = batches(b)
+    room = T // 32 + (long if counted else min(R, T // CUT))
+    args = [rnd(T, C + H, scale=1.5), rnd(T, H + H * vdim, seed=1), rnd(C, taps, seed=2), rnd(H, seed=3), rnd(H, seed=4), rnd(vdim, seed=5)]
+    state = rnd(R, H * dim * vdim + (taps - 1) * C, seed=6)
+    got, want = state.cuda(), state.clone()
+    out, ref = torch.zeros(T, H * vdim, dtype=torch.bfloat16, device="cuda"), torch.zeros(T, H * vdim, dtype=torch.bfloat16)
+    cuda.delta_rule(ctx_g, *(t.cuda() for t in args), 1e-5, got, H, H, dim, vdim, taps, out, decay_per_head=True)
+    cpu.delta_rule(ctx_r, *args, 1e-5, want, H, H, dim, vdim, taps, ref, decay_per_head=True)
+    close(out, ref, torch.bfloat16, "gated rule: outputs")
+    close(got, want, torch.float32, "gated rule: state", tol=2e-5)
+    chunk = 96 * dim + dim + 64 * vdim               # W, Q and K1; the chunk's decay; VP and OP
+    assert ctx_g.ws._bufs["delta_blocks"].numel() <= room * H * chunk * 4 + 256
+    ctx_g, ctx_r = batches(b)
+    HD, HV = H * dim, H * vdim
+    cols = (0, HD, 2 * HD, 2 * HD + HV, 3 * HD + HV)
+    args = [rnd(T, cols[4] + HV, scale=1.5, seed=7), cols, rnd(T, HD, seed=8), rnd(HD, seed=9), rnd(HD, seed=10), 0.6, rnd(HV, seed=11)]
+    to = lambda v: v.cuda() if torch.is_tensor(v) else v
+    got, want = state[:, :HD * vdim].cuda(), state[:, :HD * vdim].clone()
+    cuda.general_delta(ctx_g, *map(to, args), 1e-5, got, H, dim, vdim, out)
+    cpu.general_delta(ctx_r, *args, 1e-5, want, H, dim, vdim, ref)
+    close(out, ref, torch.bfloat16, "general rule: outputs")
+    close(got, want, torch.float32, "general rule: state", tol=2e-5)
+    chunk = 128 * dim + dim + 96 * vdim              # K2 and V beside them
+    assert ctx_g.ws._bufs["delta_blocks"].numel() <= room * H * chunk * 4 + 256
+
+
 def test_padding_rows_touch_no_state(ops):
     cuda, _ = ops
     H, dim, vdim, taps = 2, 64, 32, 4
