@@ -324,7 +324,7 @@ capped_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
             q = fmaf(q, x2, 0.13319583237171173f);
             q = fmaf(q, x2, -0.33332130312919617f);
             q = fmaf(q, x2, 0.9999997019767761f);
-            sc(c) = x2 <= 1.0f ? q * x : tanh_exp2(x);
+            sc(c) = x2 > 1.0f ? tanh_exp2(x) : q * x;              // (its clamps would turn what is not a number into a score)
           }
         }
       }

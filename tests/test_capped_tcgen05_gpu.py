@@ -79,3 +79,23 @@ def test_prompt_portions(ops, kd, vd, Hq, Hkv, page, cap, window, keep, sink, fa
     ops.tc.check_errors()
     assert (kd, vd) in ops.tc._capped, "the tensor-core kernel did not take these sizes"
     close(out.view(T, Hq, vd), ref.cpu(), torch.bfloat16, "capped attention")
+
+
+def test_a_score_that_is_not_a_number(ops):
+    """Beside scores within the cap and beside one beyond it: the rows that read it are not numbers, the others as if it were not there."""
+    Hq, Hkv, hd, page, n, bad, large = 8, 2, 64, 16, 128, 50, 40
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, kp, vp = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((n, Hq, hd), (n // page, Hkv, page, hd), (n // page, Hkv, page, hd)))
+    table = torch.arange(n // page, dtype=torch.int32, device="cuda")[None]
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    for beyond in (False, True):
+        if beyond:
+            kp[large // page, :, large % page] *= 100.0
+        outs = []
+        for k in (kp, kp.clone()):
+            if outs:
+                k[bad // page, :, bad % page] = float("nan")
+            outs.append(torch.zeros(n, Hq * hd, dtype=torch.bfloat16, device="cuda"))
+            ops.paged_attention(q, k, vp, table, i32(0, n), i32(n), torch.zeros(n, dtype=torch.int32, device="cuda"), outs[-1], hd ** -0.5, 0, page, 1, n, n,
+                                softcap=5.0)
+        assert torch.isfinite(outs[0]).all() and torch.equal(outs[0][:bad], outs[1][:bad]) and torch.isnan(outs[1][bad:]).all()
