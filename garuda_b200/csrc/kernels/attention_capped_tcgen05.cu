@@ -8,11 +8,13 @@
 //              Pages that are not there or that no row reads are asked for beyond the pool's end, which fills their rows with zeros.
 //   warp 1     one lane: S = Q K^T a tile ahead into one of two S buffers in tensor memory, O += P V of the tile whose softmax just ended.
 //   warps 2-5  a thread owns a query row: its 64 scores, the cap, the distance term, the mask on tiles that some row does not see whole,
-//              exp2 against a reference maximum that follows the running one only when outgrown by 2^8 (then O, which stays in tensor
-//              memory, is rescaled), P in bfloat16 over the scores read. The sink joins the denominator at the end.
+//              exp2 against the running maximum (where it grows for some row of a warp, that warp rescales O, which stays in tensor
+//              memory: a reference that lags behind would round the largest weights, as latent_attention_tcgen05.cu tells), P in
+//              bfloat16 over the scores read. The sink joins the denominator at the end.
 // What bounds it: instruction issue of the softmax warps. The cap's polynomial is nine operations a score, taken two scores an
 // instruction (f32x2); a score's exponential and sum are four more. A prompt of 2,048 tokens, 32 heads over 4 of 64, window 1,024, cap 30 and
-// sink: 125 us with mma.sync, 70 here (87 with a branch a pair of scores for those beyond the cap, which the fetch of instructions waited for).
+// sink: 126 us with mma.sync, 79 here (a branch a pair of scores for those beyond the cap, which the fetch of instructions waited for, cost 17
+// more).
 // Every wait is bounded; a wait that runs out sets the error word and the CTA winds down.
 #include "attention_capped.cuh"
 #include "error_word.cuh"
@@ -48,7 +50,6 @@ static_assert(STAGES >= 2 && TILE_BYTES >= 77824, "two CTAs an SM");
 constexpr int S_BUFS = 2, O_COL0 = S_BUFS * KT, TMEM_COLS = 256;
 static_assert(O_COL0 + VD <= TMEM_COLS, "tensor memory layout");
 constexpr int THREADS = 64 + QROWS;
-constexpr float RESCALE_ABOVE = 8.f;                            // in powers of two
 constexpr float LOG2E = 1.4426950408889634f;
 
 struct Misc {
@@ -254,7 +255,7 @@ capped_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
     const float unit = CAP ? p.softcap * LOG2E : p.scale * LOG2E;
     const float pre = CAP ? p.scale / p.softcap : 1.f;
     const float far1 = FAR ? p.r1[head] / unit : 0.f, far2 = FAR ? p.r2[head] : 0.f;      // r1 ln x = r1 log2 x / log2 e
-    float m = -INFINITY, l = 0.f;                                  // m: the reference maximum, in units
+    float m = -INFINITY, l = 0.f;                                  // m: the largest score so far, in units
     bool ok = true;
     auto wait_o = [&](int t) {                                     // until the P V product of tile t has ended
       if (!mbar_wait(smem_u32(&mc.o_ready), t & 1)) {
@@ -350,7 +351,7 @@ capped_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
 #pragma unroll
         for (int e = 0; e < 4; ++e) mx[e] = max3(mx[e], sc(c + e), sc(c + 4 + e));
       const float m_new = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      const bool grown = m != -INFINITY && (m_new - m) * unit > RESCALE_ABOVE;
+      const bool grown = m != -INFINITY && m_new > m;
       bool waited = false;
       if (t > 0 && __any_sync(0xffffffffu, grown)) {
         wait_o(t - 1);

@@ -11,12 +11,14 @@
 //   warp 1     one lane: S = Q K^T for two tiles ahead, into one of two S buffers; O += P V of the tile whose softmax just ended,
 //              P read from the S buffer in tensor memory. O stays in tensor memory to the end.
 //   warps 2-5  a thread owns a query row: its 64 scores, the mask on tiles that reach beyond the tile's first position, exp2 with the
-//              scale folded in against a reference maximum that follows the running one only when outgrown by 2^8 (then O is
-//              rescaled), P in bfloat16 over the scores read.
+//              scale folded in against the running maximum (where it grows for some row of a warp, that warp rescales O), P in
+//              bfloat16 over the scores read. A reference that lags behind the maximum would save most of the rescaling (97 us for the
+//              prompt below) but round the largest weights, which are powers of two otherwise: for scores that spread over four powers of e
+//              the results would be three times as far off before they are rounded themselves.
 // What bounds it: the products (18 of 128 x 64 x 16 for the scores, each as long as one of 128 columns, and 4 of 128 x 256 x 16 a tile,
 // about 1,800 cycles), which the softmax of one group of 128 threads fits under; tiles of 128 keys would halve the scores' products but
 // not leave room for two of them. A prompt of 2,048 tokens,
-// 32 heads over rows of 256 + 32 channels: 360 us with mma.sync, 97 here.
+// 32 heads over rows of 256 + 32 channels: 354 us with mma.sync, 108 here.
 // Every wait is bounded; a wait that runs out sets the error word and the CTA winds down.
 #include "error_word.cuh"
 #include "tc_common.cuh"
@@ -43,7 +45,6 @@ constexpr int STAGES = 3, S_BUFS = 2;
 constexpr int TILE_BYTES = Q_BYTES + STAGES * K_BYTES;
 constexpr int S_COL0 = RANK, TMEM_COLS = 512;
 constexpr int THREADS = 64 + QROWS;
-constexpr float RESCALE_ABOVE = 8.f;                             // in powers of two
 static_assert(S_COL0 + S_BUFS * KT <= TMEM_COLS, "tensor memory layout");
 
 struct Misc {
@@ -206,7 +207,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const int row_pos = row < rows ? pos0 + (row0 + row) / H : -1; // no key is valid for a padding row
     const int first_pos = pos0 + row0 / H;
-    float m = -INFINITY, l = 0.f;                                  // m: the reference maximum of the raw dot products
+    float m = -INFINITY, l = 0.f;                                  // m: the largest raw dot product so far
     bool ok = true;
     auto wait_o = [&](int t) {                                     // until the P V product of tile t has ended
       if (!mbar_wait(smem_u32(&mc.o_ready), t & 1)) {
@@ -255,7 +256,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
 #pragma unroll
         for (int e = 0; e < 4; ++e) mx[e] = fmaxf(mx[e], sc(c + e));
       const float m_new = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      const bool grown = m != -INFINITY && (m_new - m) * scale_log2 > RESCALE_ABOVE;
+      const bool grown = m != -INFINITY && m_new > m;
       bool waited = false;
       if (t > 0 && __any_sync(0xffffffffu, grown)) {
         wait_o(t - 1);
@@ -263,13 +264,15 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
         if (!ok) break;
         const float corr = m == -INFINITY ? 1.f : fast_exp2((m - m_new) * scale_log2);
 #pragma unroll 1
-        for (int h = 0; h < RANK / 32; ++h) {
-          uint32_t v[32];
-          tmem_ld_32(lane_addr + h * 32, v);
+        for (int h = 0; h < RANK; h += 64) {
+          uint32_t v[2][32];
+          tmem_ld_32(lane_addr + h, v[0]);
+          tmem_ld_32(lane_addr + h + 32, v[1]);
           tmem_ld_wait();
 #pragma unroll
-          for (int c = 0; c < 32; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) * corr);
-          tmem_st_32(lane_addr + h * 32, v);
+          for (int c = 0; c < 64; ++c) v[c >> 5][c & 31] = __float_as_uint(__uint_as_float(v[c >> 5][c & 31]) * corr);
+          tmem_st_32(lane_addr + h, v[0]);
+          tmem_st_32(lane_addr + h + 32, v[1]);
         }
         l *= corr;
         m = m_new;

@@ -99,3 +99,21 @@ def test_a_score_that_is_not_a_number(ops):
             ops.paged_attention(q, k, vp, table, i32(0, n), i32(n), torch.zeros(n, dtype=torch.int32, device="cuda"), outs[-1], hd ** -0.5, 0, page, 1, n, n,
                                 softcap=5.0)
         assert torch.isfinite(outs[0]).all() and torch.equal(outs[0][:bad], outs[1][:bad]) and torch.isnan(outs[1][bad:]).all()
+
+
+@pytest.mark.parametrize("hd,cap,chunk", [(64, 0.0, 512), (128, 30.0, 0)])
+def test_the_largest_weight_is_not_rounded(ops, hd, cap, chunk):
+    """Every value is one and two keys have a weight: the result is one, whatever the later key's score is above the earlier one's. Its
+    weight, taken against any other score than the largest, would be rounded to bfloat16 and be off by up to a 256th."""
+    Hq, Hkv, page, n, late = 16, 2, 32, 300, 70
+    kp = torch.zeros(n // page + 1, Hkv, page, hd, dtype=torch.bfloat16, device="cuda")
+    vp = torch.ones_like(kp)
+    kp[..., 0], kp[0, :, 0, 0], kp[late // page, :, late % page, 0] = -1000.0, 0.0, 1.0
+    q = torch.zeros(n, Hq, hd, dtype=torch.bfloat16, device="cuda")
+    q[:, :, 0] = torch.linspace(0.1, 5.5, n * Hq, device="cuda").view(n, Hq).bfloat16()
+    table = torch.arange(n // page + 1, dtype=torch.int32, device="cuda")[None]
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    out = torch.full((n, Hq * hd), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.paged_attention(q, kp, vp, table, i32(0, n), i32(n), torch.zeros(n, dtype=torch.int32, device="cuda"), out, 1.0, 0, page, 1, n, n, softcap=cap, chunk=chunk)
+    ops.tc.check_errors()
+    assert torch.equal(out, torch.ones_like(out))

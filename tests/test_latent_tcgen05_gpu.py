@@ -54,3 +54,21 @@ def test_prompt_portions(ops, rank, rot, H, page, reqs, sinks):
                         max(kv for kv, _ in reqs), value_dim=rank, **more)
     ops.tc.check_errors()
     close(out.view(T, H, rank), ref.cpu(), torch.bfloat16, "latent attention")
+
+
+def test_the_largest_weight_is_not_rounded(ops):
+    """Every value is one and two keys have a weight: the result is one, whatever the later key's score is above the earlier one's. Its
+    weight, taken against any other score than the largest, would be rounded to bfloat16 and be off by up to a 256th."""
+    rank, rot, H, page, n, late = 256, 32, 32, 32, 600, 70
+    pool = torch.zeros(n // page + 1, 1, page, rank + rot, dtype=torch.bfloat16, device="cuda")
+    flat = pool.view(-1, rank + rot)
+    flat[:, :rank], flat[:, rank], flat[0, rank], flat[late, rank] = 1.0, -1000.0, 0.0, 1.0
+    q = torch.zeros(n, H, rank + rot, dtype=torch.bfloat16, device="cuda")
+    q[:, :, rank] = torch.linspace(0.1, 5.5, n * H, device="cuda").view(n, H).bfloat16()      # 0.14 to 7.9 powers of two
+    table = torch.arange(n // page + 1, dtype=torch.int32, device="cuda")[None]
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    out = torch.full((n, H * rank), float("nan"), dtype=torch.bfloat16, device="cuda")
+    assert ops.tc._latent_lib(rank, rot).gb_latent_attention_tc_takes(q.data_ptr(), pool.data_ptr(), out.data_ptr(), page, pool.shape[0], n * H) == 1
+    ops.paged_attention(q, pool, pool, table, i32(0, n), i32(n), torch.zeros(n, dtype=torch.int32, device="cuda"), out, 1.0, 0, page, 1, n, n, value_dim=rank)
+    ops.tc.check_errors()
+    assert torch.equal(out, torch.ones_like(out))
