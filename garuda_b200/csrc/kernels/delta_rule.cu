@@ -258,7 +258,7 @@ delta_recurrence_kernel(const float* __restrict__ prep, int W, const int32_t* __
 //     W = (I + L)^-1 beta (D k),   VP = (I + L)^-1 beta v,   Q = D q - B W,   OP = B VP,   K1_j = k_j D_last / D_j
 // The quotients D_i / D_j are running products of decays from j on (never above one, so nothing overflows and what
 // underflows is nothing), and the triangular system is solved by substitution, a thread per column of W and VP. 32-bit multiply-adds.
-// grid (numbers, H), 256 threads; taps of at most four (the older ones' weights are zero where there are fewer).
+// grid (numbers, H), 256 threads; at most four taps.
 template <int DIM, typename WT>
 __global__ void __launch_bounds__(256, 3)
 delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* __restrict__ second, int P2,
@@ -316,9 +316,10 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
       for (int e = 0; e < 16; ++e) in[e] = i0 + e < n ? input(i0 + e) : 0.f;
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
-        float acc = fmaf(w[3], x[2], 0.f);
-        acc = fmaf(w[2], x[1], acc);
-        acc = fmaf(w[1], x[0], acc);
+        // (an input further back than the taps reach must not count: with a weight of zero an infinity would)
+        float acc = taps > 3 ? fmaf(w[3], x[2], 0.f) : 0.f;
+        if (taps > 2) acc = fmaf(w[2], x[1], acc);
+        if (taps > 1) acc = fmaf(w[1], x[0], acc);
         acc = fmaf(w[0], in[e], acc);
         x[2] = x[1], x[1] = x[0], x[0] = in[e];
         take(i0 + e, i0 + e < n ? silu(acc) : 0.f);

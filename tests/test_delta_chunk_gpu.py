@@ -141,6 +141,27 @@ def test_a_value_that_is_not_a_number_leaves_the_tokens_in_front_of_it_alone(ops
     assert torch.equal(outs[0][:bad], outs[1][:bad]) and torch.isnan(outs[1][bad:].float()).all()
 
 
+@pytest.mark.parametrize("taps", [1, 2, 3, 4])
+def test_a_query_that_is_not_a_number_reaches_as_far_as_the_taps(ops, taps):
+    cuda, _ = ops
+    H, dim, vdim, T, bad = 2, 64, 64, 100, 45
+    C = 2 * H * dim + H * vdim
+    proj, second = rnd(T, C + H).cuda(), rnd(T, H + H * vdim, seed=1).cuda()
+    w = [t.cuda() for t in (rnd(C, taps, seed=2), rnd(H, seed=3), rnd(H, seed=4), rnd(vdim, seed=5))]
+    outs, states = [], []
+    for spoil in (0.0, float("inf"), float("nan")):
+        p = proj.clone()
+        p[bad, :H * dim] += spoil                       # the queries' inputs alone: nothing of it may stay in the state
+        ctx, _ = batches(step([T], [0]))
+        outs.append(torch.zeros(T, H * vdim, dtype=torch.bfloat16, device="cuda"))
+        states.append(torch.zeros(1, H * dim * vdim + (taps - 1) * C, device="cuda"))
+        cuda.delta_rule(ctx, p, second, *w, 1e-5, states[-1], H, H, dim, vdim, taps, outs[-1], decay_per_head=True)
+    for out, state in zip(outs[1:], states[1:]):
+        hit = torch.isnan(out.float()).any(1)
+        assert hit[bad:bad + taps].all() and hit.sum() == taps and torch.equal(out[~hit], outs[0][~hit])
+        assert torch.equal(state[:, :H * dim * vdim], states[0][:, :H * dim * vdim])
+
+
 def test_a_32_bit_run_is_walked_token_by_token(ops):
     """There the numbers do not depend on how a prompt was cut."""
     cuda, _ = ops
