@@ -257,7 +257,8 @@ delta_recurrence_kernel(const float* __restrict__ prep, int W, const int32_t* __
 //     L_ij = beta_i sum_d k_i k_j D_i / D_j (j < i),   B_ij = sum_d q_i k_j D_i / D_j (j <= i)
 //     W = (I + L)^-1 beta (D k),   VP = (I + L)^-1 beta v,   Q = D q - B W,   OP = B VP,   K1_j = k_j D_last / D_j
 // The quotients D_i / D_j are running products of decays from j on (never above one, so nothing overflows and what
-// underflows is nothing), and the triangular system is solved by substitution, a thread per column of W and VP. 32-bit multiply-adds.
+// underflows is nothing), and the triangular system is solved by substitution, a thread per column of W and VP. 32-bit multiply-adds; what a row
+// loses to those in front of it is summed before it is taken off, which halves the error of taking it off term by term.
 // grid (numbers, H), 256 threads; at most four taps.
 template <int DIM, typename WT>
 __global__ void __launch_bounds__(256, 3)
@@ -278,6 +279,9 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
   float* sL = sg + C * LD;               // [C][LT], a row per j (transposed)
   float* sB = sL + C * LT;               // [C][LT], likewise
   float* beta = sB + C * LT;             // [C]
+  // [C][LX]: the value columns of the block's first turn, in the decays' place where they fit
+  constexpr int LX = DIM == 128 ? LD : 256 - DIM;
+  float* sx = DIM == 128 ? sg : beta + C;
   const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int r, first, n, at;
   if (!find_chunk(blockIdx.x, cu_q, R, cut, r, first, n, at)) return;
@@ -453,35 +457,42 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
   __syncthreads();
   for (int c = tid; c < DIM + vdim; c += 256) {
     const bool key = c < DIM;            // the same for a warp
-    pair_t w[C / 2], o[C / 2];
-    if (key) {
-#pragma unroll
-      for (int i = 0; i < C; i += 2) w[i / 2] = make_pair(beta[i] * sk[i * LD + c], beta[i + 1] * sk[(i + 1) * LD + c]);
-    } else {
-      float even = 0.f;
+    // a thread's column: of keys; of values; of values in a second turn, where the thread's keys were
+    const bool in_sx = !key && c < 256;
+    const int ld = in_sx ? LX : LD;
+    float* x = in_sx ? sx + c - DIM : sk + tid;
+    if (!key) {
       const int ch = 2 * G * DIM + h * vdim + c - DIM;
-      convolve(ch, [&](int i) { return proj[(size_t)(first + i) * P + ch]; }, [&](int i, float v) {
-        if (i & 1) w[i / 2] = make_pair(even, beta[i] * v);
-        else even = beta[i] * v;
-      });
+      convolve(ch, [&](int i) { return proj[(size_t)(first + i) * P + ch]; }, [&](int i, float v) { x[i * ld] = v; });
     }
+    pair_t w[C / 2], o[C / 2];           // what the rows in front take off a row, summed by itself: it is small beside the row
 #pragma unroll
-    for (int j = 0; j + 1 < C; ++j) {
-      add_row<true>(w, sL, j, -entry(w, j));
-      asm volatile("" ::: "memory");     // (else the rows are all fetched at once, and spilled)
+    for (int i = 0; i < C / 2; ++i) w[i] = o[i] = 0ull;
+    float next = x[0];
+#pragma unroll
+    for (int j = 0; j < C; ++j) {
+      const float y = fmaf(beta[j], next, entry(w, j));
+      set_entry(w, j, y);
+      if (j + 1 == C) break;
+      next = x[(j + 1) * ld];
+      add_row<true>(w, sL, j, -y);
+      asm volatile("" ::: "memory");     // (else all rows are fetched at once, and more is spilled)
     }
     if (key) store_rows(block, lay, 0, c, w);
     else store_column(block + lay.vp() + (c - DIM) * C, w);
-#pragma unroll
-    for (int i = 0; i < C; i += 2) o[i / 2] = key ? make_pair(sq[i * LD + c], sq[(i + 1) * LD + c]) : 0ull;
     const float sign = key ? -1.f : 1.f;
 #pragma unroll
     for (int j = 0; j < C; ++j) {
       add_row<false>(o, sB, j, sign * entry(w, j));
       asm volatile("" ::: "memory");
     }
-    if (key) store_rows(block, lay, C, c, o);
-    else store_column(block + lay.op() + (c - DIM) * C, o);
+    if (key) {
+#pragma unroll
+      for (int i = 0; i < C; ++i) set_entry(o, i, sq[i * LD + c] + entry(o, i));
+      store_rows(block, lay, C, c, o);
+    } else {
+      store_column(block + lay.op() + (c - DIM) * C, o);
+    }
   }
 }
 
@@ -743,7 +754,7 @@ GB_EXPORT int gb_delta_chunk(const float* proj, int P, const float* second, int 
   const int CH = 2 * G * dim + H * vdim, numbers = delta_chunk::chunk_numbers(T, walked);
   if (P < CH + H || P2 < (per_head ? H : H * dim)) return gb::fail(GB_BAD_ARGUMENT, "delta_chunk: row widths");
   if ((uintptr_t)blocks & 15) return gb::fail(GB_BAD_ARGUMENT, "delta_chunk: blocks start on 16 bytes");
-  const size_t smem = (size_t)(delta_chunk::C * (3 * (dim + 4) + 2 * delta_chunk::LT + 1)) * sizeof(float);
+  const size_t smem = (size_t)(delta_chunk::C * (3 * (dim + 4) + 2 * delta_chunk::LT + 1 + (dim == 128 ? 0 : 256 - dim))) * sizeof(float);
   const int rc = GB_DISPATCH_DTYPE(w_dtype, WT, [&]() -> int {
     auto kernel = dim == 128 ? delta_chunk_factors_kernel<128, WT> : delta_chunk_factors_kernel<64, WT>;
     static gb::OncePerDevice configured[2];      // per weight type: this lambda is instantiated for each

@@ -349,12 +349,9 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
   for (int c = tid; c < DIM + vdim; c += THREADS) {
     const bool key = c < DIM;                             // the same for a warp
     const float* v = row0 + col_v + h * vdim + c - DIM;   // a value column's numbers
-    pair_t w[C / 2], o[C / 2];
+    pair_t w[C / 2], o[C / 2];                            // what is added to D u and D r, summed by itself: it is small beside them
 #pragma unroll
-    for (int i = 0; i < C; i += 2) {
-      w[i / 2] = key ? make_pair(su[i * LD + c], su[(i + 1) * LD + c]) : 0ull;
-      o[i / 2] = key ? make_pair(sr[i * LD + c], sr[(i + 1) * LD + c]) : 0ull;
-    }
+    for (int i = 0; i < C / 2; ++i) w[i] = o[i] = 0ull;
     if (!key) {
 #pragma unroll
       for (int j4 = 0; j4 < C; j4 += 4) {
@@ -366,19 +363,25 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
         for (int e = 0; e < 4; ++e) {
           add_row<true>(w, sF, j4 + e, -x[e]);
           add_row<false>(o, sH, j4 + e, x[e]);
-          asm volatile("" ::: "memory");                  // (else the rows are all fetched at once, and spilled)
+          asm volatile("" ::: "memory");                  // (else all rows are fetched at once, and more is spilled)
         }
       }
     }
     // (a value column's w is VP = -x from here on)
     const float sign = key ? -1.f : 1.f;
+    float next = key ? su[c] : 0.f;
 #pragma unroll
     for (int j = 0; j < C; ++j) {
-      add_row<true>(w, sE, j, -entry(w, j));
-      add_row<false>(o, sG, j, sign * entry(w, j));
+      const float y = next + entry(w, j);
+      set_entry(w, j, y);
+      if (j + 1 < C) next = key ? su[(j + 1) * LD + c] : 0.f;
+      add_row<true>(w, sE, j, -y);
+      add_row<false>(o, sG, j, sign * y);
       asm volatile("" ::: "memory");
     }
     if (key) {
+#pragma unroll
+      for (int i = 0; i < C; ++i) set_entry(o, i, sr[i * LD + c] + entry(o, i));
       store_rows(block, lay, 0, c, w);
       store_rows(block, lay, C, c, o);
     } else {

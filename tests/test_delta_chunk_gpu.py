@@ -179,3 +179,65 @@ def test_a_32_bit_run_is_walked_token_by_token(ops):
             at += n
         got.append((torch.cat(outs), state))
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+def _gated64(proj, second, conv_w, a_log, dt_bias, H, G, dim, vdim, taps, per_head):
+    T, C, dev = proj.shape[0], 2 * G * dim + H * vdim, proj.device
+    x = torch.cat([torch.zeros(taps - 1, C, device=dev, dtype=torch.float64), proj[:, :C].double()])
+    a = torch.nn.functional.silu(sum(x[i:i + T] * conv_w.double()[:, i] for i in range(taps)))
+    q, k, v = (t.view(T, -1, n) for t, n in zip(a.split([G * dim, G * dim, H * vdim], 1), (dim, dim, vdim)))
+    q, k = ((t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)).repeat_interleave(H // G, 1) for t in (q, k))
+    beta, rate = torch.sigmoid(proj[:, C:].double()), torch.exp(a_log.double())
+    step = torch.nn.functional.softplus(second[:, :dt_bias.numel()].double() + dt_bias.double()).view(T, H, -1)
+    g = torch.exp(-rate[:, None] * step)
+    S, o = torch.zeros(H, dim, vdim, dtype=torch.float64, device=dev), torch.empty(T, H, vdim, dtype=torch.float64, device=dev)
+    for t in range(T):
+        S *= g[t][:, :, None]
+        S += k[t][:, :, None] * (beta[t][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t])))[:, None, :]
+        o[t] = torch.einsum("hdv,hd->hv", S, q[t]) * dim ** -0.5
+    return o, S
+
+
+def _general64(proj, cols, zdec, w0, a0, scale, H, dim, vdim):
+    T, dev = proj.shape[0], proj.device
+    r, k, v, a = (proj[:, c:c + n].double() for c, n in zip(cols, (H * dim, H * dim, H * vdim, H * dim)))
+    a, w = torch.sigmoid(a + a0.double()).view(T, H, dim), torch.exp(-scale * torch.sigmoid(zdec.double() + w0.double())).view(T, H, dim)
+    r, k, v = r.view(T, H, dim), k.view(T, H, dim), v.view(T, H, vdim)
+    u = k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+    S, o = torch.zeros(H, dim, vdim, dtype=torch.float64, device=dev), torch.empty(T, H, vdim, dtype=torch.float64, device=dev)
+    for t in range(T):
+        S = w[t][:, :, None] * S - (a[t] * u[t])[:, :, None] * torch.einsum("hdv,hd->hv", S, u[t])[:, None, :] + k[t][:, :, None] * v[t][:, None, :]
+        o[t] = torch.einsum("hdv,hd->hv", S, r[t])
+    return o, S
+
+
+@pytest.mark.parametrize("rule,dim,decay", [("channel", 128, -3.0), ("channel", 128, -8.0), ("head", 128, -3.0), ("head", 128, -8.0), ("head", 64, -5.0),
+                                            ("general", 64, -3.0), ("general", 64, -8.0), ("general", 128, -3.0), ("general", 128, -8.0)])
+def test_as_near_64_bits_as_the_walk_token_by_token(ops, rule, dim, decay):
+    """2,048 tokens, decays that forget in a few tokens to some thousand: the read-outs and the state may be no further off than those of the
+    32-bit walk (what a 32-bit run takes). The two round at different places, so their errors are two draws of one size: 1.2 of it."""
+    cuda, _ = ops
+    H, G, T, taps, vdim = 4, 2, 2048, 4, dim
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    draw = lambda *s, std=1.0, mean=0.0: torch.randn(*s, generator=g, device="cuda") * std + mean
+    if rule == "general":
+        HD = H * dim
+        cols = (0, HD, 2 * HD, 3 * HD, 4 * HD)
+        args = [draw(T, 5 * HD), cols, draw(T, HD), draw(HD, mean=decay), draw(HD), 0.6]
+        ref, width = _general64(*args, H, dim, vdim), HD * vdim
+    else:
+        C, n_decay = 2 * G * dim + H * vdim, H if rule == "head" else H * dim
+        args = [draw(T, C + H), draw(T, n_decay + H * vdim), draw(C, taps, std=0.5), draw(H, std=0.3), draw(n_decay, std=0.3, mean=decay)]
+        ref, width = _gated64(*args, H, G, dim, vdim, taps, rule == "head"), H * dim * vdim + (taps - 1) * C
+    off = []
+    for dt in (torch.float32, torch.bfloat16):
+        ctx, _ = batches(step([T], [0]))
+        state, out = torch.zeros(1, width, device="cuda"), torch.zeros(T, H * vdim, dtype=dt, device="cuda")
+        if rule == "general":
+            cuda.general_delta(ctx, *args, torch.ones(H * vdim, device="cuda"), 1e-5, state, H, dim, vdim, out)
+        else:
+            cuda.delta_rule(ctx, *args, torch.ones(vdim, device="cuda"), 1e-5, state, H, G, dim, vdim, taps, out, decay_per_head=rule == "head")
+        assert ("delta_blocks" in ctx.ws._bufs) == (dt == torch.bfloat16)
+        o = ctx.ws._views["gdelta_o" if rule == "general" else "delta_o"][2]
+        off.append([((x.double().flatten() - y.flatten()).norm() / y.norm()).item() for x, y in zip((o, state[:, :H * dim * vdim]), ref)])
+    assert all(chunk <= 1.2 * token for token, chunk in zip(*off)), f"read-outs, state: token by token {off[0]}, by chunks {off[1]}"
