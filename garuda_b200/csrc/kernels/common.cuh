@@ -93,6 +93,17 @@ struct OncePerDevice {
   }
 };
 
+// SMs of the device that was current at the first call.
+inline int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v;
+  }();
+  return n;
+}
+
 // ---- programmatic dependent launch ----------------------------------------
 // A kernel launched with launch_pdl may start while the kernel before it in the
 // stream is still running. It must call pdl_wait() before it reads anything that

@@ -25,8 +25,8 @@
 // token of 16 heads of 128 x 128, whatever the tokens do); a chunk's three products have no chain. On multiply-adds instead of the
 // tensor cores the walk was bound by shared memory, whose bandwidth serves four multiply-adds a number only (162 us for 2,048 tokens).
 // A group of four warps has 16 columns of S, a quarter of the channels each: S^T in the accumulators' layout is at once the first
-// operand of S^T [W; Q]^T, so nothing of S is ever exchanged, only the warps' shares of Y and o. One group a block while such
-// blocks are at most one an SM (16 heads x 8 groups are 128 blocks for 148 SMs); two (which share WQ, K1 and K2) where the
+// operand of S^T [W; Q]^T, so nothing of S is ever exchanged, only the warps' shares of Y and o. One group a block while the
+// walked requests' blocks are at most one an SM (16 heads x 8 groups are 128 blocks for 148 SMs); two (which share WQ, K1 and K2) where the
 // heads are more. 2,048 tokens of 16 heads of 128 x 128 take 98 us here and 119 us in the kernel in front (B200), where the
 // token-by-token walk took 0.89 ms; the tensor cores are 44% busy, the rest is the latency of a chunk's three barriers.
 #pragma once
@@ -61,15 +61,17 @@ struct Layout {
 // t0 / C + w on. All numbers of `walked` such requests are below chunk_numbers(T, walked).
 __host__ __device__ __forceinline__ int chunk_numbers(int T, int walked) { return T / C + walked; }
 
-// How many of the requests below r are walked (all threads of a warp call this).
-__device__ __forceinline__ int walked_before(const int32_t* __restrict__ cu_q, int r, int cut) {
+// The w-th request that is walked (all threads of a warp call this); -1: there are no more.
+__device__ __forceinline__ int nth_walked(const int32_t* __restrict__ cu_q, int R, int cut, int w) {
   const int lane = threadIdx.x & 31;
-  int count = 0;
-  for (int r0 = 0; r0 < r; r0 += 32) {
-    const int i = r0 + lane;
-    count += __popc(__ballot_sync(0xffffffffu, i < r && cu_q[min(i, r - 1) + 1] - cu_q[min(i, r - 1)] >= cut));
+  for (int r0 = 0; r0 < R; r0 += 32) {
+    const int r = min(r0 + lane, R - 1);
+    const uint32_t walked = __ballot_sync(0xffffffffu, r0 + lane < R && cu_q[r + 1] - cu_q[r] >= cut);
+    const uint32_t it = __ballot_sync(0xffffffffu, (walked >> lane & 1) && __popc(walked & ((1u << lane) - 1)) == w);
+    if (it != 0) return r0 + __ffs(it) - 1;
+    w -= __popc(walked);
   }
-  return count;
+  return -1;
 }
 
 // The request and chunk of a number (all threads of a warp call this): false where there is none.
@@ -217,19 +219,19 @@ struct WalkSmem {
   float y[GROUPS][TWO ? 2 : 1][COLS][LDY]; // Y^T (and V^T)
 };
 
-// grid (H, vdim / (16 GROUPS), R). blocks [numbers, H, Layout::floats()]. out [T, H vdim].
+// grid (H, vdim / (16 GROUPS), walked): a block for a request that is not walked would hold an SM's shared memory only to return (64 single
+// tokens beside a prompt of 48, 16 heads: 152 us, with blocks for all 167). blocks [numbers, H, Layout::floats()]. out [T, H vdim].
 template <int DIM, int GROUPS, bool TWO>
 __global__ void __launch_bounds__(GROUP * GROUPS, 1)
 walk_kernel(const float* __restrict__ blocks, const int32_t* __restrict__ cu_q, const int32_t* __restrict__ slots,
-            float* __restrict__ state, long long state_stride, int H, int vdim, int cut, int numbers, float* __restrict__ out) {
+            float* __restrict__ state, long long state_stride, int R, int H, int vdim, int cut, int numbers, float* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char raw[];
   using Smem = WalkSmem<DIM, GROUPS, TWO>;
   Smem& sm = *reinterpret_cast<Smem*>(raw);
   gb::pdl_wait();
-  const int h = blockIdx.x, r = blockIdx.z;
-  const int t0 = cu_q[r], n = cu_q[r + 1] - t0;
-  if (n < cut) return;
-  const int number = t0 / C + walked_before(cu_q, r, cut);
+  const int h = blockIdx.x, r = nth_walked(cu_q, R, cut, blockIdx.z);
+  if (r < 0) return;
+  const int t0 = cu_q[r], n = cu_q[r + 1] - t0, number = t0 / C + blockIdx.z;
   const Layout lay{DIM, vdim, TWO ? 1 : 0};
   constexpr int THREADS = GROUP * GROUPS;
   constexpr int KS = DIM / 32;                       // tiles of 8 channels of a warp
@@ -392,7 +394,7 @@ walk_kernel(const float* __restrict__ blocks, const int32_t* __restrict__ cu_q, 
 
 template <int DIM, int GROUPS, bool TWO>
 int launch_walk_as(const char* what, const float* blocks, const int32_t* cu_q, const int32_t* slots, float* state, long long state_stride,
-                   int R, int H, int vdim, int cut, int numbers, float* out, cudaStream_t stream) {
+                   int R, int walked, int H, int vdim, int cut, int numbers, float* out, cudaStream_t stream) {
   auto kernel = walk_kernel<DIM, GROUPS, TWO>;
   constexpr size_t smem = sizeof(WalkSmem<DIM, GROUPS, TWO>);
   static_assert(smem <= 227 * 1024, "a block's shared memory");
@@ -402,21 +404,22 @@ int launch_walk_as(const char* what, const float* blocks, const int32_t* cu_q, c
     if (e != cudaSuccess) return gb::fail(GB_CUDA_ERROR, "%s: %s", what, cudaGetErrorString(e));
     configured.done();
   }
-  return gb::check_pdl_launch(gb::launch_after(kernel, dim3(H, vdim / (COLS * GROUPS), R), dim3(GROUP * GROUPS), smem, stream,
-                                               dim3(1, 1, 1), blocks, cu_q, slots, state, state_stride, H, vdim, cut, numbers, out),
+  return gb::check_pdl_launch(gb::launch_after(kernel, dim3(H, vdim / (COLS * GROUPS), walked), dim3(GROUP * GROUPS), smem, stream,
+                                               dim3(1, 1, 1), blocks, cu_q, slots, state, state_stride, R, H, vdim, cut, numbers, out),
                               what);
 }
 
 // dim 64 or 128, vdim a multiple of 32. numbers: what blocks has room for, chunk_numbers(T, walked).
 template <bool TWO>
 int launch_walk(const char* what, const float* blocks, const int32_t* cu_q, const int32_t* slots, float* state, long long state_stride,
-                int R, int H, int dim, int vdim, int cut, int numbers, float* out, cudaStream_t stream) {
-  const bool one = (long long)R * H * (vdim / COLS) <= 148;
+                int R, int walked, int H, int dim, int vdim, int cut, int numbers, float* out, cudaStream_t stream) {
+  // requests that are not walked have no blocks to speak of: a prompt of 2,048 tokens beside eight single ones, 379 us, now 294
+  const bool one = (long long)walked * H * (vdim / COLS) <= gb::sm_count();
   if (dim == 128)
-    return one ? launch_walk_as<128, 1, TWO>(what, blocks, cu_q, slots, state, state_stride, R, H, vdim, cut, numbers, out, stream)
-               : launch_walk_as<128, 2, TWO>(what, blocks, cu_q, slots, state, state_stride, R, H, vdim, cut, numbers, out, stream);
-  return one ? launch_walk_as<64, 1, TWO>(what, blocks, cu_q, slots, state, state_stride, R, H, vdim, cut, numbers, out, stream)
-             : launch_walk_as<64, 2, TWO>(what, blocks, cu_q, slots, state, state_stride, R, H, vdim, cut, numbers, out, stream);
+    return one ? launch_walk_as<128, 1, TWO>(what, blocks, cu_q, slots, state, state_stride, R, walked, H, vdim, cut, numbers, out, stream)
+               : launch_walk_as<128, 2, TWO>(what, blocks, cu_q, slots, state, state_stride, R, walked, H, vdim, cut, numbers, out, stream);
+  return one ? launch_walk_as<64, 1, TWO>(what, blocks, cu_q, slots, state, state_stride, R, walked, H, vdim, cut, numbers, out, stream)
+             : launch_walk_as<64, 2, TWO>(what, blocks, cu_q, slots, state, state_stride, R, walked, H, vdim, cut, numbers, out, stream);
 }
 
 inline bool takes(int dim, int vdim) { return (dim == 64 || dim == 128) && vdim >= 32 && vdim % 32 == 0 && vdim <= 256; }

@@ -770,7 +770,8 @@ GB_EXPORT int gb_delta_chunk(const float* proj, int P, const float* second, int 
         "delta_chunk");
   });
   if (rc != GB_OK) return rc;
-  return delta_chunk::launch_walk<false>("delta_chunk", blocks, cu_q, slots, state, state_stride, R, H, dim, vdim, cut, numbers, out, stream);
+  return delta_chunk::launch_walk<false>("delta_chunk", blocks, cu_q, slots, state, state_stride, R, walked, H, dim, vdim, cut, numbers, out,
+                                         stream);
 }
 
 GB_EXPORT int gb_delta_out(const float* o, const float* second, int P2, int gate_off, const void* w, int w_dtype,

@@ -544,7 +544,8 @@ GB_EXPORT int gb_gdelta_chunk(const float* proj, int P, int col_r, int col_k, in
                      col_v, col_a, zdec, PZ, w0, a0, decay_scale, cu_q, blocks, R, H, vdim, cut),
       "gdelta_chunk");
   if (rc != GB_OK) return rc;
-  return delta_chunk::launch_walk<true>("gdelta_chunk", blocks, cu_q, slots, state, state_stride, R, H, dim, vdim, cut, numbers, out, stream);
+  return delta_chunk::launch_walk<true>("gdelta_chunk", blocks, cu_q, slots, state, state_stride, R, walked, H, dim, vdim, cut, numbers, out,
+                                         stream);
 }
 
 // One token per request (row t of the batch is request t). Takes vdim <= 256.

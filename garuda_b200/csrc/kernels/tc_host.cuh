@@ -73,15 +73,6 @@ inline int tensor_map_2d(const void* ptr, long long rows, long long cols, int bo
   return GB_OK;
 }
 
-inline int sm_count() {
-  static int n = [] {
-    int dev = 0, v = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    return v;
-  }();
-  return n;
-}
-
+using gb::sm_count;
 
 }  // namespace tc_host
