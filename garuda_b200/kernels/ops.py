@@ -1181,9 +1181,10 @@ class CudaOps:
                 int(decay_per_head), n_decay, silu_gate, self._stream()), "delta_decode")
         else:
             o = ctx.ws.get("delta_o", (T, H * vdim), torch.float32)
-            walked = self._delta_walked(b, out)
+            cut = self.DELTA_CHUNK_CUT
+            walked = self._delta_walked(b, out, cut)
             floats = L.gb_delta_chunk_floats(T, walked, H, G, dim, vdim, taps)
-            cut = self.DELTA_CHUNK_CUT if floats else 0
+            cut = cut if floats else 0
             if cut:
                 blocks = ctx.ws.get("delta_blocks", (floats,), torch.float32)
                 self._check(L, L.gb_delta_chunk(
@@ -1210,17 +1211,25 @@ class CudaOps:
     #: Requests with at least this many tokens in a step run the chunked delta-rule kernels, whose fixed cost is that of
     #: a whole chunk and a third launch.
     DELTA_CHUNK_CUT = 48
+    #: The same for the generalized rule of up to 64 channels and of more, whose tokens walked one by one cost less: (from how many tokens on,
+    #: from how many the step's longest request must have where there are shorter ones beside it, in a step of fewer than 256 tokens). us
+    #: token by token / by chunks, 32 heads, one request: 64 channels, 48 tokens 29 / 47, 100 43 / 50, 128 52 / 51, 200 72 / 56; 128 channels, 48 50 /
+    #: 50, 64 60 / 51. Beside a single token: 64 channels, 128 tokens 60 / 65, 200 86 / 70; 128 channels, 64 tokens 69 / 72, 100 96 / 80;
+    #: beside 40 tokens: 64 channels, 200 tokens 88 / 84; 128 channels, 64 tokens 76 / 103, 100 103 / 110.
+    GENERAL_CHUNK_CUTS = ((128, 160), (48, 100))
 
-    def _delta_walked(self, b, out) -> int:
-        """How many requests of this step are walked by chunks (delta_chunk.cuh): those of ``DELTA_CHUNK_CUT`` tokens and more, counted
-        where the batch has its lengths on the host, else as many as can be. Only they take room in the chunks' scratch. In a 32-bit run every
+    def _delta_walked(self, b, out, cut: int, mixed: int = 0) -> int:
+        """How many requests of this step are walked by chunks (delta_chunk.cuh): those of ``cut`` tokens and more, counted
+        where the batch has its lengths on the host, else as many as can be; none in a step of fewer than 256 tokens that has shorter
+        requests too and none of ``mixed``. Only they take room in the chunks' scratch. In a 32-bit run every
         request is walked token by token, so that its numbers do not depend on how its prompt was cut."""
-        if out.dtype != torch.bfloat16 or b.max_q_len < self.DELTA_CHUNK_CUT:
+        T = out.shape[0]
+        if out.dtype != torch.bfloat16 or b.max_q_len < cut or (T < 256 and b.max_q_len < mixed and getattr(b, "min_q_len", 1) < cut):
             return 0
         cu = getattr(b, "host", {}).get("cu_q")
         if cu is None:
-            return min(b.num_requests, out.shape[0] // self.DELTA_CHUNK_CUT)
-        return int((np.diff(cu) >= self.DELTA_CHUNK_CUT).sum())
+            return min(b.num_requests, T // cut)
+        return int((np.diff(cu) >= cut).sum())
 
     # ------------------------------------------------------------------ the generalized delta rule
     def general_delta(self, ctx, proj, cols, zdec, w0, a0, decay_scale, norm_w, eps, state, heads, dim, vdim, out):
@@ -1254,9 +1263,10 @@ class CudaOps:
                 "gdelta_decode")
             return
         o = ctx.ws.get("gdelta_o", (T, HV), torch.float32)
-        walked = self._delta_walked(b, out)
+        cut, mixed = self.GENERAL_CHUNK_CUTS[dim > 64]
+        walked = self._delta_walked(b, out, cut, mixed)
         floats = L.gb_gdelta_chunk_floats(T, walked, H, dim, vdim)
-        cut = self.DELTA_CHUNK_CUT if floats else 0
+        cut = cut if floats else 0
         if cut:
             blocks = ctx.ws.get("delta_blocks", (floats,), torch.float32)
             self._check(L, L.gb_gdelta_chunk(

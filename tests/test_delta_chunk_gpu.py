@@ -61,20 +61,25 @@ def test_general_rule(ops, H, dim, vdim, strong):
     w0, a0, norm_w = rnd(HD, scale=1.5, seed=1) - 2.0, rnd(HD, seed=2), rnd(HV, seed=3) + 1.0
     state_g, state_r = torch.zeros(5, HD * vdim, device="cuda"), torch.zeros(5, HD * vdim)
     state_g[1] = float("nan")
-    for k, lens in enumerate(STEPS):
+    # from how many tokens on a request is walked by chunks, and where there are shorter ones beside it
+    cut, mixed = (128, 160) if dim == 64 else (CUT, 100)
+    assert cuda.GENERAL_CHUNK_CUTS[dim > 64] == (cut, mixed)
+    for k, lens in enumerate(STEPS + [(cut - 1, 1, mixed - 1), (mixed, 1, cut - 1), (1, cut, 256)] + [(cut + 1, 10, cut - 3)] * (dim == 128)):
         T = sum(lens)
         ctx_g, ctx_r = batches(step(lens, [3, 0, 2]))
         proj, zdec = rnd(T, cols[4] + HV + 6, scale=1.5, seed=10 + k), rnd(T, HD + 2, scale=2.0, seed=20 + k)
         out, ref = torch.zeros(T, HV, dtype=torch.bfloat16, device="cuda"), torch.zeros(T, HV, dtype=torch.bfloat16)
         for o, c, st, to, y in ((cuda, ctx_g, state_g, lambda t: t.cuda(), out), (cpu, ctx_r, state_r, lambda t: t, ref)):
             o.general_delta(c, to(proj), cols, to(zdec)[:, :HD], to(w0), to(a0), 20.0 if strong else 0.6, to(norm_w), 1e-5, st, H, dim, vdim, y)
+        walks = max(lens) >= cut and (min(lens) >= cut or max(lens) >= mixed or T >= 256)
+        assert ("delta_blocks" in ctx_g.ws._bufs) == walks, lens
         close(out, ref, torch.bfloat16, f"step {k}: outputs")
         keep = [0, 2, 3, 4]
         close(state_g[keep], state_r[keep], torch.float32, f"step {k}: state", tol=2e-5)
 
 
 @pytest.mark.parametrize("counted", [True, False])
-@pytest.mark.parametrize("lens", [(CUT + 16,) + (1,) * 40, (3, 0, 97, 1, 0, 64) + (2,) * 40 + (CUT, 1), (0, CUT, 0)])
+@pytest.mark.parametrize("lens", [(CUT + 52,) + (1,) * 40, (3, 0, 107, 1, 0, 64) + (2,) * 40 + (CUT, 1), (0, CUT, 0)])
 def test_scratch_is_for_the_requests_that_are_walked(ops, lens, counted):
     """Single tokens (and requests without any) beside a few long stretches: no room for those that are not walked, whether the batch
     brings its lengths on the host or not; more than a warp's requests in front of one that is walked."""
@@ -97,17 +102,20 @@ def test_scratch_is_for_the_requests_that_are_walked(ops, lens, counted):
     chunk = 96 * dim + dim + 64 * vdim               # W, Q and K1; the chunk's decay; VP and OP
     assert ctx_g.ws._bufs["delta_blocks"].numel() <= room * H * chunk * 4 + 256
     ctx_g, ctx_r = batches(b)
+    dim = 128                                        # (the generalized rule of 64 channels walks longer stretches only)
     HD, HV = H * dim, H * vdim
     cols = (0, HD, 2 * HD, 2 * HD + HV, 3 * HD + HV)
     args = [rnd(T, cols[4] + HV, scale=1.5, seed=7), cols, rnd(T, HD, seed=8), rnd(HD, seed=9), rnd(HD, seed=10), 0.6, rnd(HV, seed=11)]
     to = lambda v: v.cuda() if torch.is_tensor(v) else v
-    got, want = state[:, :HD * vdim].cuda(), state[:, :HD * vdim].clone()
+    state = rnd(R, HD * vdim, seed=6)
+    got, want = state.cuda(), state.clone()
     cuda.general_delta(ctx_g, *map(to, args), 1e-5, got, H, dim, vdim, out)
     cpu.general_delta(ctx_r, *args, 1e-5, want, H, dim, vdim, ref)
     close(out, ref, torch.bfloat16, "general rule: outputs")
     close(got, want, torch.float32, "general rule: state", tol=2e-5)
     chunk = 128 * dim + dim + 96 * vdim              # K2 and V beside them
-    assert ctx_g.ws._bufs["delta_blocks"].numel() <= room * H * chunk * 4 + 256
+    walks = T >= 256 or max(lens) >= 100 or min(lens) >= CUT
+    assert ctx_g.ws._bufs["delta_blocks"].numel() <= room * H * chunk * 4 + 256 if walks else "delta_blocks" not in ctx_g.ws._bufs
 
 
 def test_padding_rows_touch_no_state(ops):
