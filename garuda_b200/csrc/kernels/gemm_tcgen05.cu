@@ -211,24 +211,38 @@ __device__ __forceinline__ void store_value<float>(float* p, float v) { *p = v; 
 template <>
 __device__ __forceinline__ void store_value<__nv_bfloat16>(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 
+// 1 / x, rounded, of an x from 1 to infinity. STRAIGHT: without a branch, as one step of Newton's iteration from the hardware's
+// approximation (x a quarter of what it was meanwhile, so that no reciprocal of a finite number is subnormal): the bits of __frcp_rn for
+// every x up to 2^126 (all compared); beyond, where reciprocals are subnormal, one in five is a last place off.
+template <bool STRAIGHT>
+__device__ __forceinline__ float rounded_reciprocal(float x) {
+  if (!STRAIGHT) return __frcp_rn(x);
+  const float y = 0.25f * x;
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return 0.25f * (x < INFINITY ? fmaf(r, fmaf(-y, r, 1.0f), r) : r);
+}
+
 // The SiLU-gate of the fused epilogues. The exponential is the hardware's fast one: its error
 // (about 2 ulp of a float) is far below the rounding of the bfloat16 result.
+template <bool STRAIGHT = false>
 __device__ __forceinline__ float silu_gate_fast(float g, float u) {
-  return g * __frcp_rn(1.0f + __expf(-g)) * u;
+  return g * rounded_reciprocal<STRAIGHT>(1.0f + __expf(-g)) * u;
 }
 
 // The gated epilogues' activation, chosen at run time (uniform over the launch). tanh through the
 // fast exponential: tanh(z) = 1 - 2 / (exp(2 z) + 1), which is exact at both ends.
+template <bool STRAIGHT = false>
 __device__ __forceinline__ float gate_fast(const EpilogueArgs& ra, float g, float u) {
-  if (ra.gate_act == GATE_SILU) return silu_gate_fast(g, u);
+  if (ra.gate_act == GATE_SILU) return silu_gate_fast<STRAIGHT>(g, u);
   if (ra.gate_act == GATE_GELU_TANH) {
     const float z = 0.7978845608028654f * (g + 0.044715f * g * g * g);
-    const float th = 1.0f - 2.0f * __frcp_rn(__expf(2.0f * z) + 1.0f);
+    const float th = 1.0f - 2.0f * rounded_reciprocal<STRAIGHT>(__expf(2.0f * z) + 1.0f);
     return 0.5f * g * (1.0f + th) * u;
   }
   g = fminf(g, ra.gate_limit);
   u = fminf(fmaxf(u, -ra.gate_limit), ra.gate_limit);
-  return g * __frcp_rn(1.0f + __expf(-1.702f * g)) * (u + 1.0f);
+  return g * rounded_reciprocal<STRAIGHT>(1.0f + __expf(-1.702f * g)) * (u + 1.0f);
 }
 
 // The exact gelu, z Phi(z). The complementary error function by formula 7.1.26 of Abramowitz and Stegun's "Handbook of
@@ -1408,26 +1422,6 @@ __device__ __forceinline__ void load_gated_pair(uint32_t dst, const CUtensorMap*
       : "memory");
 }
 
-// silu_gate_fast and gate_fast with the reciprocal to a last place instead of rounded, without a branch: nothing hides this
-// epilogue, and the branches of 32 rounded reciprocals kept one value's latencies from covering the next one's (2.8 us every 32 tokens).
-// 2 x 14,336 rows of 4,096 channels, 333 tokens, other tiles against these: gelu 121 / 107 us, clamped swish 121 / 106.
-__device__ __forceinline__ float reciprocal(float x) {
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-template <bool GENERAL>
-__device__ __forceinline__ float gate_approx(const EpilogueArgs& ra, float g, float u) {
-  if (!GENERAL) return g * reciprocal(1.0f + __expf(-g)) * u;
-  if (ra.gate_act == GATE_GELU_TANH) {
-    const float z = 0.7978845608028654f * (g + 0.044715f * g * g * g);
-    return g * reciprocal(1.0f + __expf(-2.0f * z)) * u;        // (1 + tanh z) / 2 = 1 / (1 + exp(-2 z))
-  }
-  g = fminf(g, ra.gate_limit);
-  u = fminf(fmaxf(u, -ra.gate_limit), ra.gate_limit);
-  return g * reciprocal(1.0f + __expf(-1.702f * g)) * (u + 1.0f);
-}
-
 template <int EPI>
 __global__ void __launch_bounds__(p_threads(EPI_SWIGLU), 1)
 gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, __nv_bfloat16* __restrict__ out,
@@ -1564,7 +1558,7 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
           const float inv = inv_s[t0 + token], mine = __uint_as_float(gate ? r[j] : r[j + 16]) * inv;
           const float theirs = __uint_as_float(__shfl_xor_sync(0xffffffffu, gate ? r[j + 16] : r[j], 16)) * inv;
           const float g = gate ? mine : theirs, u = gate ? theirs : mine;
-          rows_s[(token + (gate ? 0 : 1)) * 16 + (lane & 15)] = __float2bfloat16_rn(gate_approx<(EPI & EPI_GENERAL) != 0>(ra, g, u));
+          rows_s[(token + (gate ? 0 : 1)) * 16 + (lane & 15)] = __float2bfloat16_rn((EPI & EPI_GENERAL) ? gate_fast<true>(ra, g, u) : silu_gate_fast<true>(g, u));
         }
         __syncwarp();
         if (vec) {
@@ -1823,7 +1817,8 @@ int many_token_width(int tokens, int weight_rows, int epi = -1) {
 // two, 115 / 117 / 118 / 118 against 96 / 102 / 109 / 119; 2 x 9,472 rows of 4,096, two against one, 68 / 68 / 70 / 70 against 56 /
 // 60 / 64 / -; 2 x 28,672 rows of 8,192, 370 / 377 / 387 / 413 against 319 / 344 / 375 / 399; where the line says no: 2 x 11,008 rows
 // of 4,096, three against two, 91 / 91 / 92 / 92 against 94 / 101 / 106 / -; 2 x 8,192 rows of 2,048, 41 / 41 / 42 / 43 against 37 /
-// 40 / 43 / 45.
+// 40 / 43 / 45. (Taken one call at a time behind a flushed L2. The activation's reciprocals have been rounded since: of calls that follow one another, 333
+// tokens of the first shape, SiLU 94 us then and 96 now, gelu 98 and 103.)
 bool wide_gated(int tokens, int weight_rows, int K) {
   if (tokens <= few_token_limit() || tokens > W_TOKENS || weight_rows < 2 * BM) return false;
   const int sms = sm_count(), pairs = sms / 2;

@@ -56,3 +56,19 @@ def test_behind_a_folded_norm(ops, T):
     ops.linear_swiglu(ctx, pending, ops.pack_gate_up(gate, up), out)
     ops.tc.check_errors()
     close(out, (torch.nn.functional.silu(h @ gate.double().T) * (h @ up.double().T)).cpu(), torch.bfloat16, "behind a norm", tol=2 ** -8)
+
+
+@pytest.mark.parametrize("kind", ["silu", "gelu_tanh", "clamped_swish"])
+def test_the_tiles_do_not_show(ops, kind):
+    """A token's result is the same bits in a step of 400 tokens (wide tiles) as in one of 600 (the other tiles), gates up to
+    70 on both sides among them (below -87 the two may differ in a last place of results below 1e-35)."""
+    F, K, T = 14336, 4096, 400
+    g = torch.Generator(device="cuda").manual_seed(7)
+    h = (torch.randn(600, K, generator=g, device="cuda") * 0.5).bfloat16()
+    h[::7] *= 8.0
+    w = ops.pack_gate_up(*((torch.randn(F, K, generator=g, device="cuda") * 0.05).bfloat16() for _ in range(2)))
+    outs = [torch.zeros(n, F, dtype=torch.bfloat16, device="cuda") for n in (T, 600)]
+    for n, out in zip((T, 600), outs):
+        assert ops.tc.linear_swiglu(h[:n], w, out, kind=ops.GATE_ACTS[kind], limit=50.0)
+    ops.tc.check_errors()
+    assert torch.equal(outs[0], outs[1][:T])
