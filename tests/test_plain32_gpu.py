@@ -15,8 +15,10 @@ def plain():
     return CudaOps("cuda:0", tensor_cores=False)
 
 
-# (N, K): one tile, K in one part; a tail of both; eight parts; parts of unequal length; two parts; many tiles; K % 4 != 0 (the older kernel)
-@pytest.mark.parametrize("N,K", [(128, 16), (130, 20), (256, 1024), (2000, 1284), (11264, 256), (24000, 64), (96, 70)])
+# (N, K): K of one block at most and K % 4 != 0 (the older kernel); one tile, K in one part; a tail of both; eight parts; parts of unequal length; two
+# parts; many tiles; tiles of 16, 32 and 64 rows for the most rows
+@pytest.mark.parametrize("N,K", [(128, 16), (130, 20), (96, 32), (96, 70), (128, 36), (130, 44), (256, 1024), (2000, 1284), (11264, 256), (24000, 64),
+                                 (16, 192), (6000, 40), (8192, 100)])
 def test_product_over_row_counts(plain, N, K):
     g = torch.Generator(device="cuda").manual_seed(N + K)
     a, w = torch.randn(200, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda") * 0.1
