@@ -660,9 +660,10 @@ class CudaOps:
                 q, k_pool, v_pool, block_table, cu_q, kv_lens, token_req, out, scale, window, page_size,
                 num_requests, max_q_len, max_kv_len, ws, min_q_len):
             return
-        # a tile takes 64 (token, head of a group) rows of a request; with less than half of one a warp per row is faster
+        # a tile takes 64 (token, head of a group) rows of a request and 32 keys at a time; with less than half the rows, or a single block of
+        # keys, a warp per row is faster (4 tokens, 32 heads on one of 64: 8 us against 15; the two give the same bits)
         if (plain and vd == hd and not window and q.dtype == torch.float32 and hd in (64, 128) and max_q_len * (Hq // Hkv) >= 32
-                and num_requests <= 65535 and not any(t.data_ptr() & 15 for t in (q, k_pool, v_pool, out))):
+                and max_kv_len > 32 and num_requests <= 65535 and not any(t.data_ptr() & 15 for t in (q, k_pool, v_pool, out))):
             self._check(self.core, self.core.gb_attention_tile32(
                 q.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), block_table.data_ptr(), block_table.shape[1], cu_q.data_ptr(),
                 kv_lens.data_ptr(), out.data_ptr(), num_requests, max_q_len, Hq, Hkv, hd, float(scale), page_size, self._stream()),
