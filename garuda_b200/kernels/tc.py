@@ -54,6 +54,7 @@ class TensorCoreKernels:
         L.gb_gemm_tc_qkv.restype = c_int
         L.gb_tc_hint_next_stream.argtypes = [c_void_p, ctypes.c_longlong]
         L.gb_tc_hint_next_stream.restype = c_int
+        self.sms = torch.cuda.get_device_properties(ops.device).multi_processor_count
         self._attn = {}
         self._latent = {}
         self._capped = {}
@@ -442,6 +443,23 @@ class TensorCoreKernels:
             return 1
         return max(1, min(296 // tiles, -(-max_kv_len // 128), 16))
 
+    @staticmethod
+    def latent_on_tcgen05(rank: int, tokens: int, num_requests: int, heads: int, max_q_len: int, max_kv_len: int, sms: int) -> bool:
+        """Whether a step that is not cut along its keys (``latent_plan``) takes the tcgen05 kernel, 128 query rows a CTA and one CTA
+        an SM, or the ``mma.sync`` one, 64 rows a CTA and several an SM. One round of CTAs: tcgen05 for every size (0.3 to 1.0 of the other's time,
+        latents of 64 and 256, 8 to 64 heads, 1 to 2,048 tokens a request behind 0 to 8,192). More rounds of full tiles: likewise, but for
+        narrow latents over less than two tiles of keys (64 channels, 16 prompts of 60 tokens, 64 heads: 13.7 us against 12.4). More rounds of
+        tiles that are mostly empty, as of single tokens: only wide latents behind so many keys that the tiles' fixed cost does not count (us,
+        tcgen05 against mma.sync: latent of 256, 32 heads, 256 requests behind 64 / 512 / 2,048 positions 15 / 35 / 113 against 13 / 44 / 152; 8
+        heads, 512 requests 30 / 84 / 211 against 19 / 74 / 248; latent of 64, 16 heads, 512 requests 16 / 40 / 137 against 8 / 23 / 80)."""
+        tiles = min(num_requests * -(-max_q_len * heads // 128), tokens * heads // 128 + num_requests)
+        if tiles <= sms:
+            return True
+        full = tokens * heads / (128 * tiles)
+        if full >= 0.75:
+            return rank > 128 or max_kv_len > 96
+        return rank > 128 and max_kv_len >= (256 if full >= 0.25 else 1024)
+
     def latent_attention(self, q, pool, out, block_table, cu_q, kv_lens, rank, scale, page_size, num_requests,
                          max_q_len, max_kv_len, ws=None, sink_values=None) -> bool:
         """``q [T, H, rank + rot]``, ``pool [pages, 1, page_size, rank + rot]``, ``out [T, H * rank]``.
@@ -452,9 +470,8 @@ class TensorCoreKernels:
             return False
         lib = self._latent_lib(rank, rot)
         splits = self.latent_plan(num_requests, H, max_q_len, max_kv_len)
-        if splits == 1 and num_requests <= 65535 and lib.gb_latent_attention_tc_takes(q.data_ptr(), pool.data_ptr(), out.data_ptr(), int(page_size),
-                                                                                      pool.shape[0], T * H):
-            # enough query rows to fill the GPU without cutting the keys: 128 of them a CTA on the tcgen05 kernel
+        if (splits == 1 and num_requests <= 65535 and self.latent_on_tcgen05(rank, T, num_requests, H, max_q_len, max_kv_len, self.sms)
+                and lib.gb_latent_attention_tc_takes(q.data_ptr(), pool.data_ptr(), out.data_ptr(), int(page_size), pool.shape[0], T * H)):
             code = lib.gb_latent_attention_tc(
                 q.data_ptr(), pool.data_ptr(), out.data_ptr(), block_table.data_ptr(), block_table.shape[1], cu_q.data_ptr(),
                 kv_lens.data_ptr(), T, num_requests, H, float(scale), int(page_size), pool.shape[0], int(max_q_len),

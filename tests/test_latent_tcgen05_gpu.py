@@ -19,7 +19,11 @@ def ops():
 # (rank, rot, heads, page size, (cached length after the step, tokens of the step) of every request, sinks)
 @pytest.mark.parametrize("rank,rot,H,page,reqs,sinks", [
     (256, 32, 32, 32, [(300, 300)], False), (256, 64, 16, 16, [(64, 64), (65, 65), (700, 350), (129, 1)], True),
-    (64, 32, 32, 8, [(333, 333), (63, 63)], False), (128, 0, 24, 64, [(1000, 340), (128, 128)], True), (192, 16, 40, 32, [(2111, 200)], False)])
+    (64, 32, 32, 8, [(333, 333), (63, 63)], False), (128, 0, 24, 64, [(1000, 340), (128, 128)], True), (192, 16, 40, 32, [(2111, 200)], False),
+    # decoded tokens, on either side of the line between the two kernels
+    (64, 32, 16, 8, [(40 + i % 100, 1) for i in range(130)], True), (64, 32, 16, 8, [(40 + i % 100, 1) for i in range(200)], True),
+    (256, 32, 32, 32, [(400 - i % 90, 1) for i in range(170)], False), (256, 32, 32, 32, [(200 - i % 90, 1) for i in range(170)], True),
+    (256, 32, 8, 16, [(1024 + i % 70, 1) for i in range(150)], False)])
 def test_prompt_portions(ops, rank, rot, H, page, reqs, sinks):
     row, R = rank + rot, len(reqs)
     g = torch.Generator(device="cuda").manual_seed(rank + rot)
@@ -72,3 +76,31 @@ def test_the_largest_weight_is_not_rounded(ops):
     ops.paged_attention(q, pool, pool, table, i32(0, n), i32(n), torch.zeros(n, dtype=torch.int32, device="cuda"), out, 1.0, 0, page, 1, n, n, value_dim=rank)
     ops.tc.check_errors()
     assert torch.equal(out, torch.ones_like(out))
+
+
+@pytest.mark.parametrize("what", ["nan", "inf"])
+def test_a_cached_row_that_is_not_finite(ops, what):
+    """Every row that reads it is not a number; those in front of its tile of 128 query rows are as if it were not there."""
+    rank, rot, H, page, n, bad = 64, 32, 32, 16, 300, 150
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, pool = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((n, H, rank + rot), (n // page + 1, 1, page, rank + rot)))
+    q[..., 0] = q[..., 0].abs() + 0.5                     # a score of plus infinity, not minus
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    table, outs = torch.arange(n // page + 1, dtype=torch.int32, device="cuda")[None], []
+    for value in (None, float(what)):
+        if value is not None:
+            pool[bad // page, 0, bad % page, 0] = value
+        outs.append(torch.zeros(n, H * rank, dtype=torch.bfloat16, device="cuda"))
+        ops.paged_attention(q, pool, pool, table, i32(0, n), i32(n), torch.zeros(n, dtype=torch.int32, device="cuda"), outs[-1], 0.1, 0, page, 1, n, n,
+                            value_dim=rank)
+    first = bad * H // 128 * 128 // H                     # the tile's first token
+    assert torch.isfinite(outs[0]).all() and torch.equal(outs[0][:first], outs[1][:first])
+    assert torch.isnan(outs[1][bad:].view(-1, H, rank)).all()
+
+
+@pytest.mark.parametrize("rank,H,lens,kv,tcgen05", [
+    (256, 32, [300], 300, True), (256, 8, [1] * 148, 70, True), (256, 8, [1] * 149, 1023, False), (256, 8, [1] * 149, 1024, True),
+    (256, 32, [1] * 149, 255, False), (256, 32, [1] * 149, 256, True), (64, 64, [1] * 149, 4000, False), (64, 16, [60, 1, 1, 1], 4000, True),
+    (64, 16, [200] + [1] * 200, 1200, False), (64, 32, [90] * 16, 90, False), (64, 32, [97] * 16, 97, True), (256, 64, [45] * 16, 45, True)])
+def test_which_kernel(ops, rank, H, lens, kv, tcgen05):
+    assert ops.tc.latent_on_tcgen05(rank, sum(lens), len(lens), H, max(lens), kv, 148) == tcgen05
