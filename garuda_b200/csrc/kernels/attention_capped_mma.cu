@@ -524,6 +524,15 @@ GB_EXPORT int gb_capped_attention(const void* q, const void* k_pool, const void*
   return GB_OK;
 }
 
+// Whether prompt portions of these sizes run on tcgen05.
+GB_EXPORT int gb_capped_attention_tc_takes(const void* q, const void* k_pool, const void* v_pool, const void* out, int R, int Hq, int Hkv, float scale,
+                                           int page_size, long long num_pages) {
+  Params p = {};
+  p.q = (const __nv_bfloat16*)q; p.k_pool = (const __nv_bfloat16*)k_pool; p.v_pool = (const __nv_bfloat16*)v_pool; p.out = (__nv_bfloat16*)out;
+  p.Hq = Hq; p.Hkv = Hkv; p.g = Hkv > 0 ? Hq / Hkv : 0; p.page_size = page_size; p.scale = scale;
+  return p.g > 0 && capped::tc_takes(p, num_pages, R);
+}
+
 // Non-zero if a CTA gave up on a wait since the last call; clears it. And a word of pinned host memory that a failed wait
 // also writes its code to (null: none).
 GB_EXPORT int gb_capped_attention_error_check() { return capped::tc_error_check(); }

@@ -1924,6 +1924,9 @@ GB_EXPORT int gb_gemm_tc_supported(const void* x, const void* w, int Mx, int Nw,
 // alpha: the accumulating epilogue adds alpha * product. gate_act, gate_limit: the gated epilogue's
 // activation (GateAct), or with epi 0 and a bfloat16 output STORE_RELU2 / STORE_TANH / STORE_XIELU / STORE_GELU: out =
 // act(x w^T); act_second: the second number of an activation that has two (STORE_XIELU).
+// Whether a gated product of `tokens` rows takes the wide tiles.
+GB_EXPORT int gb_gemm_tc_wide(int tokens, int weight_rows, int K) { return wide_gated(tokens, weight_rows, K); }
+
 GB_EXPORT int gb_gemm_tc(const void* x, const void* w, void* out, int Mx, int Nw, int K, int out_dtype, int epi,
                          const GbNormFold* norm, float alpha, int gate_act, float gate_limit, float act_second,
                          cudaStream_t stream) {

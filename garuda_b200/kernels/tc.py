@@ -37,6 +37,8 @@ class TensorCoreKernels:
         L.gb_gemm_tc_grouped.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int,
                                          c_float, c_int, c_float, c_void_p]
         L.gb_gemm_tc_grouped.restype = c_int
+        L.gb_gemm_tc_wide.argtypes = [c_int] * 3
+        L.gb_gemm_tc_wide.restype = c_int
         L.gb_gemm_tc_norm_tiles.argtypes = [c_int, c_int]
         L.gb_gemm_tc_norm_tiles.restype = c_int
         L.gb_gemm_tc_supported.argtypes = [c_void_p, c_void_p, c_int, c_int, c_int]
@@ -316,6 +318,8 @@ class TensorCoreKernels:
             lib.gb_capped_attention.argtypes = ([c_void_p] * 5 + [c_int] + [c_void_p] * 2 + [c_int] * 4 + [c_float, c_float]
                                                 + [c_int] * 7 + [c_void_p, ctypes.c_longlong] + [c_void_p] * 3 + [c_int, ctypes.c_longlong, c_void_p])
             lib.gb_capped_attention.restype = c_int
+            lib.gb_capped_attention_tc_takes.argtypes = [c_void_p] * 4 + [c_int] * 3 + [c_float, c_int, ctypes.c_longlong]
+            lib.gb_capped_attention_tc_takes.restype = c_int
             lib.gb_capped_attention_error_check.restype = c_int
             lib.gb_capped_attention_set_error_sink.argtypes = [c_void_p]
             lib.gb_capped_attention_set_error_sink.restype = c_int

@@ -77,7 +77,7 @@ def test_prompt_portions(ops, kd, vd, Hq, Hkv, page, cap, window, keep, sink, fa
                         max(kv for kv, _ in REQS), softcap=cap, keep_first=keep, sink=sink == "one", sink_values=sinks,
                         distance=(r1, r2) if far else None, chunk=chunk)
     ops.tc.check_errors()
-    assert (kd, vd) in ops.tc._capped, "the tensor-core kernel did not take these sizes"
+    assert ops.tc._capped[kd, vd].gb_capped_attention_tc_takes(*(t.data_ptr() for t in (q, kp, vp, out)), R, Hq, Hkv, scale, page, total) == 1
     close(out.view(T, Hq, vd), ref.cpu(), torch.bfloat16, "capped attention")
 
 
@@ -117,3 +117,20 @@ def test_the_largest_weight_is_not_rounded(ops, hd, cap, chunk):
     ops.paged_attention(q, kp, vp, table, i32(0, n), i32(n), torch.zeros(n, dtype=torch.int32, device="cuda"), out, 1.0, 0, page, 1, n, n, softcap=cap, chunk=chunk)
     ops.tc.check_errors()
     assert torch.equal(out, torch.ones_like(out))
+
+
+def test_what_is_not_for_tcgen05(ops):
+    """Refused by the kernel's own rule, and taken by the other kernel: pages of four and of 128 keys, a group that is no power of two."""
+    for Hq, Hkv, page in ((8, 2, 4), (8, 2, 128), (6, 2, 16)):
+        n, hd = 100, 64
+        g = torch.Generator(device="cuda").manual_seed(page)
+        q, kp, vp = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((n, Hq, hd), (n // page + 1, Hkv, page, hd), (n // page + 1, Hkv, page, hd)))
+        i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+        out = torch.zeros(n, Hq * hd, dtype=torch.bfloat16, device="cuda")
+        ops.paged_attention(q, kp, vp, torch.arange(n // page + 1, dtype=torch.int32, device="cuda")[None], i32(0, n), i32(n),
+                            torch.zeros(n, dtype=torch.int32, device="cuda"), out, hd ** -0.5, 0, page, 1, n, n, softcap=20.0)
+        assert ops.tc._capped[hd, hd].gb_capped_attention_tc_takes(*(t.data_ptr() for t in (q, kp, vp, out)), 1, Hq, Hkv, hd ** -0.5, page, len(kp)) == 0
+        flat = lambda t: t.transpose(1, 2).reshape(-1, Hkv, hd)[:n].double().repeat_interleave(Hq // Hkv, 1)
+        s = 20.0 * torch.tanh(torch.einsum("ihd,jhd->hij", q.double(), flat(kp)) * hd ** -0.5 / 20.0)
+        p = torch.softmax(s.masked_fill(~torch.ones(n, n, dtype=torch.bool, device="cuda").tril(), -float("inf")), -1)
+        close(out.view(n, Hq, hd), torch.einsum("hij,jhd->ihd", p, flat(vp)).cpu(), torch.bfloat16, "capped attention")

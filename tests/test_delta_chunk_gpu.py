@@ -189,6 +189,24 @@ def test_a_32_bit_run_is_walked_token_by_token(ops):
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
+def test_a_cut_where_a_chunk_ends_moves_no_bit(ops):
+    cuda, _ = ops
+    H, dim, vdim, taps, T = 2, 128, 64, 4, 192
+    C = 2 * H * dim + H * vdim
+    proj, second = rnd(T, C + H).cuda(), rnd(T, H * dim + H * vdim, seed=1).cuda()
+    w = [t.cuda() for t in (rnd(C, taps, seed=2), rnd(H, seed=3), rnd(H * dim, seed=4), rnd(vdim, seed=5))]
+    got = []
+    for cuts in ([T], [96, 96], [128, 64]):
+        state, at, outs = torch.zeros(1, H * dim * vdim + (taps - 1) * C, device="cuda"), 0, []
+        for n in cuts:
+            ctx, _ = batches(step([n], [0]))
+            outs.append(torch.zeros(n, H * vdim, dtype=torch.bfloat16, device="cuda"))
+            cuda.delta_rule(ctx, proj[at:at + n], second[at:at + n], *w, 1e-5, state, H, H, dim, vdim, taps, outs[-1])
+            at += n
+        got.append((torch.cat(outs), state))
+    assert all(torch.equal(a, b) for other in got[1:] for a, b in zip(got[0], other))
+
+
 def _gated64(proj, second, conv_w, a_log, dt_bias, H, G, dim, vdim, taps, per_head):
     T, C, dev = proj.shape[0], 2 * G * dim + H * vdim, proj.device
     x = torch.cat([torch.zeros(taps - 1, C, device=dev, dtype=torch.float64), proj[:, :C].double()])

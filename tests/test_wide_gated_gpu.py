@@ -24,7 +24,9 @@ def test_gated_product(ops, T, F, K, kind):
     gate, up = ((torch.randn(F, K, generator=g, device="cuda") * 0.05).bfloat16() for _ in range(2))
     room = torch.full((T + 1, F), float("nan"), dtype=torch.bfloat16, device="cuda")
     room[T] = 9.0
-    assert ops.tc.linear_swiglu(h, ops.pack_gate_up(gate, up), room[:T], kind=ops.GATE_ACTS[kind], limit=3.0)
+    packed = ops.pack_gate_up(gate, up)
+    assert ops.tc.lib.gb_gemm_tc_wide(T, packed.shape[0], K) == 1, "the sizes are for the wide tiles"
+    assert ops.tc.linear_swiglu(h, packed, room[:T], kind=ops.GATE_ACTS[kind], limit=3.0)
     ops.tc.check_errors()
     a, u = h.double() @ gate.double().T, h.double() @ up.double().T
     if kind == "clamped_swish":
