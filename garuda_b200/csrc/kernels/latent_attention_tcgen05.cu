@@ -12,13 +12,13 @@
 //              P read from the S buffer in tensor memory. O stays in tensor memory to the end.
 //   warps 2-5  a thread owns a query row: its 64 scores, the mask on tiles that reach beyond the tile's first position, exp2 with the
 //              scale folded in against the running maximum (where it grows for some row of a warp, that warp rescales O), P in
-//              bfloat16 over the scores read. A reference that lags behind the maximum would save most of the rescaling (97 us for the
+//              bfloat16 over the scores read. A reference that lags behind the maximum would save most of the rescaling (8 us of the
 //              prompt below) but round the largest weights, which are powers of two otherwise: for scores that spread over four powers of e
 //              the results would be three times as far off before they are rounded themselves.
 // What bounds it: the products (18 of 128 x 64 x 16 for the scores, each as long as one of 128 columns, and 4 of 128 x 256 x 16 a tile,
 // about 1,800 cycles), which the softmax of one group of 128 threads fits under; tiles of 128 keys would halve the scores' products but
 // not leave room for two of them. A prompt of 2,048 tokens,
-// 32 heads over rows of 256 + 32 channels: 354 us with mma.sync, 108 here.
+// 32 heads over rows of 256 + 32 channels: 350 us with mma.sync, 103 here (calls in a row).
 // Every wait is bounded; a wait that runs out sets the error word and the CTA winds down.
 #include "error_word.cuh"
 #include "tc_common.cuh"
@@ -286,8 +286,9 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
       uint32_t pk[KT / 2];
 #pragma unroll
       for (int c = 0; c < KT; c += 2) {
-        ls[(c >> 1) & 3] += sc(c) + sc(c + 1);
+        // (the denominator counts the weights as they are multiplied: their rounding then cancels in part)
         pk[c >> 1] = pack_bf16(sc(c), sc(c + 1));
+        ls[(c >> 1) & 3] += __uint_as_float(pk[c >> 1] << 16) + __uint_as_float(pk[c >> 1] & 0xffff0000u);
       }
       l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
       tmem_st(s_addr, pk);                                         // over the first half of the scores just read
