@@ -6,7 +6,7 @@
 // while the other waits for tensor memory.
 //   warp 0     TMA: the query tile (3-D boxes [tokens][group][64]), then keys and values, one 4-D box per page and block of 64 channels.
 //              Pages that are not there or that no row reads are asked for beyond the pool's end, which fills their rows with zeros.
-//   warp 1     one lane: S = Q K^T a tile ahead into one of two S buffers in tensor memory, O += P V of the tile whose softmax just ended.
+//   warp 1     one elected lane: S = Q K^T a tile ahead into one of two S buffers in tensor memory, O += P V of the tile whose softmax just ended.
 //   warps 2-5  a thread owns a query row: its 64 scores, the cap, the distance term, the mask on tiles that some row does not see whole,
 //              exp2 against the running maximum (where it grows for some row of a warp, that warp rescales O, which stays in tensor
 //              memory: a reference that lags behind would round the largest weights, as latent_attention_tcgen05.cu tells), P in
@@ -200,6 +200,7 @@ capped_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------------- MMA issuer
+    const bool leader = elect_one();
     constexpr uint32_t idesc_s = instr_desc_bf16(QROWS, KT);
     constexpr uint32_t idesc_o = instr_desc_bf16(QROWS, VD) | INSTR_B_MN_MAJOR;
     const uint64_t dq0 = smem_desc_sw128(q_s), dk0 = smem_desc_sw128(kv_s), dv0 = smem_desc_sw128_mn(kv_s + K_BYTES, K_BLOCK);
@@ -213,7 +214,7 @@ capped_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
         return;
       }
       tc_fence_after_sync();
-      if (lane == 0) {
+      if (leader) {
 #pragma unroll
         for (int b = 0; b < KBLOCKS; ++b)
           mma_bf16_x4(tmem_base + buf * KT, dq0 + (uint64_t)(b * (Q_BLOCK >> 4)), dk0 + (uint64_t)(st * (STAGE_BYTES >> 4) + b * (K_BLOCK >> 4)),
@@ -235,7 +236,7 @@ capped_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
         break;
       }
       tc_fence_after_sync();
-      if (lane == 0) {
+      if (leader) {
         mma_bf16_ts<KT / 16>(tmem_base + O_COL0, tmem_base + buf * KT, dv0 + (uint64_t)(st * (STAGE_BYTES >> 4)), idesc_o, 16 * ROW_BYTES >> 4, t > 0);
         mma_commit(smem_u32(&mc.empty[st]));
         mma_commit(smem_u32(&mc.o_ready));

@@ -18,7 +18,7 @@
 //            4-D box per page and block of 64 channels, keys and values in rings of their own
 //            (keys are needed two tiles before their values). The lanes look up the pages of
 //            several tiles in one round trip and issue one page's copies each.
-//   warp 1   one lane: O += P V of the tile whose softmax just ended (P from tensor memory, V as
+//   warp 1   one elected lane: O += P V of the tile whose softmax just ended (P from tensor memory, V as
 //            it lies in the cache, keys along the rows: an MN-major operand), one accumulator per
 //            group for the whole piece; then S = Q K^T for the tile two ahead into the S buffer
 //            that this tile's P has just been read from. This warp is the one the tensor cores
@@ -403,6 +403,7 @@ attention_tile_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid
     // lie side by side). After a tile's softmax its P V goes first: it reads the probabilities
     // from the S buffer that the S product two tiles ahead then overwrites (products run in the
     // order of their issue).
+    const bool leader = elect_one();
     constexpr uint32_t idesc_s = instr_desc_bf16(QROWS, KT);
     constexpr uint32_t idesc_o = instr_desc_bf16(QROWS, HD) | INSTR_B_MN_MAJOR;
     const uint64_t dq0 = smem_desc_sw128(q_s), dk0 = smem_desc_sw128(k_s),
@@ -424,7 +425,7 @@ attention_tile_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid
         return;
       }
       tc_fence_after_sync();
-      if (lane == 0) {
+      if (leader) {
 #pragma unroll
         for (int h = 0; h < BLOCKS; ++h)
           mma_bf16_x4(tmem_base + s_buf * KT, dq0 + (uint64_t)(qb * (Q_BYTES >> 4) + h * (BLOCK_BYTES >> 4)),
@@ -452,7 +453,7 @@ attention_tile_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid
       }
       if (!ok) break;
       tc_fence_after_sync();
-      if (lane == 0) {
+      if (leader) {
 #pragma unroll
         for (int g = 0; g < GROUPS; ++g)
           mma_bf16_ts<GK / 16>(tmem_base + O_COL0 + g * HD, tmem_base + p_buf * KT + g * GK,

@@ -451,18 +451,21 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // -------------------------------------------------------------- MMA issuer
-      constexpr uint32_t idesc = instr_desc_bf16(BM, BN);
-      int s = 0, par = 0;
-      for (int it = 0; it < num_kb; ++it, s = (s + 1 == stages ? 0 : s + 1), par ^= (s == 0)) {
-        if (!mbar_wait(smem_u32(&full_bar[s]), par)) {
+    // ---------------------------------------------------------------- MMA issuer (elect_one's lane)
+    constexpr uint32_t idesc = instr_desc_bf16(BM, BN);
+    const bool leader = elect_one();
+    int s = 0, par = 0;
+    for (int it = 0; it < num_kb; ++it, s = (s + 1 == stages ? 0 : s + 1), par ^= (s == 0)) {
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&full_bar[s]), par))) {
+        if (leader) {
           gb_err::report(ERR_WAIT_FULL);
           abort_s = 1;
-          break;
         }
-        tc_fence_after_sync();
-        const uint32_t base = tiles + s * G::STAGE_BYTES;
+        break;
+      }
+      tc_fence_after_sync();
+      const uint32_t base = tiles + s * G::STAGE_BYTES;
+      if (leader) {
 #pragma unroll
         for (int k = 0; k < BK / UMMA_K; ++k) {
           const uint32_t koff = k * UMMA_K * 2;  // bytes along the swizzled row
@@ -473,8 +476,10 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_c
         }
         mma_commit(smem_u32(&empty_bar[s]));  // the stage is free once these MMAs have read it
       }
-      mma_commit(smem_u32(&accum_bar));       // fires when every MMA above has retired
+      __syncwarp();
     }
+    if (leader) mma_commit(smem_u32(&accum_bar));       // fires when every MMA above has retired
+    __syncwarp();
   } else {
     // ---------------------------------------------------------------- epilogue warps
     const int quarter = warp & 3;                         // the TMEM lanes this warp may read
@@ -1132,39 +1137,37 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_m, const __gri
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------------------ MMA issuer
-      constexpr uint32_t idesc = instr_desc_bf16(BM, BN);
-      int it = 0, t = 0;
-      for (int tile = blockIdx.x; tile < total_tiles && !*aborted; tile += gridDim.x, ++t) {
-        const int as = t & 1;
-        if (!mbar_wait(smem_u32(&acc_empty[as]), ((t >> 1) & 1) ^ 1)) {   // the epilogue has drained this stage
-          gb_err::report(ERR_WAIT_ACCUM);
-          *aborted = 1;
+    // -------------------------------------------------------------- MMA issuer (elect_one's lane)
+    constexpr uint32_t idesc = instr_desc_bf16(BM, BN);
+    const uint64_t da0 = smem_desc_sw128(tiles), db0 = smem_desc_sw128(tiles + G::A_BYTES);
+    const bool leader = elect_one();
+    bool go = true, ran_out;
+    int s = 0, par = 0, t = 0;
+    for (int tile = blockIdx.x; tile < total_tiles && go; tile += gridDim.x, ++t) {
+      const int as = t & 1;
+      if (!(go = mbar_wait_warp(smem_u32(&acc_empty[as]), ((t >> 1) & 1) ^ 1, aborted, ran_out))) {   // the epilogue has drained this stage
+        if (ran_out) gb_err::report(ERR_WAIT_ACCUM), *aborted = 1;
+        break;
+      }
+      tc_fence_after_sync();
+      const uint32_t acc = tmem_base + as * ACC_COLS;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!(go = mbar_wait_warp(smem_u32(&full_bar[s]), par, aborted, ran_out))) {
+          if (ran_out) gb_err::report(ERR_WAIT_FULL), *aborted = 1;
           break;
         }
         tc_fence_after_sync();
-        const uint32_t acc = tmem_base + as * ACC_COLS;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % STAGES;
-          if (!mbar_wait(smem_u32(&full_bar[s]), (it / STAGES) & 1)) {
-            gb_err::report(ERR_WAIT_FULL);
-            *aborted = 1;
-          }
-          if (*aborted) break;
-          tc_fence_after_sync();
-          const uint32_t base = tiles + s * G::STAGE_BYTES;
+        const uint64_t at = (uint64_t)(s * (G::STAGE_BYTES >> 4));
+        if (leader) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint32_t koff = k * UMMA_K * 2;
-            const bool accumulate = kb > 0 || k > 0;
-            const uint64_t da = smem_desc_sw128(base + koff);
-            mma_bf16(acc, da, smem_desc_sw128(base + G::A_BYTES + koff), idesc, accumulate);
-          }
+          for (int k = 0; k < BK / UMMA_K; ++k) mma_bf16(acc, da0 + at + 2 * k, db0 + at + 2 * k, idesc, kb > 0 || k > 0);
           mma_commit(smem_u32(&empty_bar[s]));
         }
-        mma_commit(smem_u32(&acc_full[as]));
+        __syncwarp();
+        if (++s == STAGES) s = 0, par ^= 1;
       }
+      if (leader) mma_commit(smem_u32(&acc_full[as]));
+      __syncwarp();
     }
   } else {
     // -------------------------------------------------------------- epilogue warps
@@ -1287,20 +1290,21 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_cons
   gb::pdl_wait();     // the activations, and for an accumulating epilogue the output, come from earlier kernels
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ------------------------------------------------------------ producer (both CTAs)
-      int s = 0, par = 1, issued = 0;
-      for (int tile = pair; tile < total_tiles && !*aborted; tile += pairs) {
-        const int m0 = (tile % tiles_m) * (2 * BM) + (int)rank * BM;
-        const int nt0 = (tile / tiles_m) * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(smem_u32(&empty_bar[s]), par)) {
-            gb_err::report(ERR_WAIT_EMPTY);
-            *aborted = 1;
-          }
-          if (*aborted) break;
-          const uint32_t bar = map_to_rank(smem_u32(&full_bar[s]), 0);     // the even CTA's barrier
-          const uint32_t base = tiles + s * PAIR_STAGE_BYTES;
+    // -------------------------------------------------------------- producer (both CTAs, elect_one's lane)
+    const bool leader = elect_one();
+    bool go = true, ran_out;
+    int s = 0, par = 1, issued = 0;
+    for (int tile = pair; tile < total_tiles && go; tile += pairs) {
+      const int m0 = (tile % tiles_m) * (2 * BM) + (int)rank * BM;
+      const int nt0 = (tile / tiles_m) * BN;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!(go = mbar_wait_warp(smem_u32(&empty_bar[s]), par, aborted, ran_out))) {
+          if (ran_out) gb_err::report(ERR_WAIT_EMPTY), *aborted = 1;
+          break;
+        }
+        const uint32_t bar = map_to_rank(smem_u32(&full_bar[s]), 0);     // the even CTA's barrier
+        const uint32_t base = tiles + s * PAIR_STAGE_BYTES;
+        if (leader) {
           if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[s]), 2 * PAIR_STAGE_BYTES);
           tma_load_2d_pair(base, &map_m, bar, kb * BK, m0);
           // this CTA's half of the first product's weight rows, then of the second's, box by box
@@ -1311,52 +1315,58 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_cons
                                                    : PG::COLS0 + (int)rank * (PG::COLS1 / 2) + (r0 - PG::COLS0 / 2);
             tma_load_2d_pair(base + BM * BK * 2 + r0 * BK * 2, &map_n, bar, kb * BK, nt0 + feature);
           }
-          ++issued;
-          if (++s == STAGES) s = 0, par ^= 1;
         }
-      }
-      if (*aborted && issued > 0) {
-        // wind down: the copies in flight (counted on the even CTA's barriers) need microseconds
-        // to land; give them two milliseconds before the CTA's shared memory is given up
-        const unsigned long long t0 = globaltimer_ns();
-        while (globaltimer_ns() - t0 < 2000000ull) {}
+        __syncwarp();
+        ++issued;
+        if (++s == STAGES) s = 0, par ^= 1;
       }
     }
+    if (leader && *aborted && issued > 0) {
+      // wind down: the copies in flight (counted on the even CTA's barriers) need microseconds
+      // to land; give them two milliseconds before the CTA's shared memory is given up
+      const unsigned long long t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 2000000ull) {}
+    }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
-      // ------------------------------------------------------------ MMA issuer (even CTA)
+    if (rank == 0) {
+      // ------------------------------------------------------------ MMA issuer (even CTA, elect_one's lane)
       constexpr uint32_t idesc = instr_desc_bf16(2 * BM, PG::COLS0);
       constexpr uint32_t idesc1 = instr_desc_bf16(2 * BM, PG::COLS1 > 0 ? PG::COLS1 : 16);
       const uint64_t da0 = smem_desc_sw128(tiles), db0 = smem_desc_sw128(tiles + BM * BK * 2);
+      const bool leader = elect_one();
+      bool go = true, ran_out;
       int s = 0, par = 0, t = 0;
-      for (int tile = pair; tile < total_tiles && !*aborted; tile += pairs, ++t) {
+      for (int tile = pair; tile < total_tiles && go; tile += pairs, ++t) {
         const int as = ACC == 2 ? (t & 1) : 0;
-        if (!mbar_wait(smem_u32(&acc_empty[as]), ((ACC == 2 ? (t >> 1) : t) & 1) ^ 1)) {   // both epilogues have drained this stage
-          gb_err::report(ERR_WAIT_ACCUM);
-          *aborted = 1;
+        // both epilogues have drained this stage
+        if (!(go = mbar_wait_warp(smem_u32(&acc_empty[as]), ((ACC == 2 ? (t >> 1) : t) & 1) ^ 1, aborted, ran_out))) {
+          if (ran_out) gb_err::report(ERR_WAIT_ACCUM), *aborted = 1;
           break;
         }
         tc_fence_after_sync();
         const uint32_t acc = tmem_base + as * BN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(smem_u32(&full_bar[s]), par)) {
-            gb_err::report(ERR_WAIT_FULL);
-            *aborted = 1;
+          if (!(go = mbar_wait_warp(smem_u32(&full_bar[s]), par, aborted, ran_out))) {
+            if (ran_out) gb_err::report(ERR_WAIT_FULL), *aborted = 1;
+            break;
           }
-          if (*aborted) break;
           tc_fence_after_sync();
           const uint64_t da = da0 + (uint64_t)(s * (PAIR_STAGE_BYTES >> 4)), db = db0 + (uint64_t)(s * (PAIR_STAGE_BYTES >> 4));
+          if (leader) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            mma_bf16_pair(acc, da + 2 * k, db + 2 * k, idesc, kb > 0 || k > 0);
-            if (PG::PARTS == 2)
-              mma_bf16_pair(acc + PG::COLS0, da + 2 * k, db + (uint64_t)((PG::COLS0 / 2) * BK * 2 >> 4) + 2 * k, idesc1,
-                            kb > 0 || k > 0);
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+              mma_bf16_pair(acc, da + 2 * k, db + 2 * k, idesc, kb > 0 || k > 0);
+              if (PG::PARTS == 2)
+                mma_bf16_pair(acc + PG::COLS0, da + 2 * k, db + (uint64_t)((PG::COLS0 / 2) * BK * 2 >> 4) + 2 * k, idesc1,
+                              kb > 0 || k > 0);
+            }
+            mma_commit_pair(smem_u32(&empty_bar[s]), 3);      // the stage is free in both CTAs
           }
-          mma_commit_pair(smem_u32(&empty_bar[s]), 3);      // the stage is free in both CTAs
+          __syncwarp();
           if (++s == STAGES) s = 0, par ^= 1;
         }
-        mma_commit_pair(smem_u32(&acc_full[as]), 3);
+        if (leader) mma_commit_pair(smem_u32(&acc_full[as]), 3);
+        __syncwarp();
       }
     }
   } else {
@@ -1496,35 +1506,39 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
-      // ------------------------------------------------------------ MMA issuer (even CTA)
+    if (rank == 0) {
+      // ------------------------------------------------------------ MMA issuer (even CTA, elect_one's lane)
       const uint32_t idesc = instr_desc_bf16(2 * BM, part);
+      const uint64_t da0 = smem_desc_sw128(tiles), db0 = smem_desc_sw128(tiles + BM * BK * 2), db1 = smem_desc_sw128(tiles + BM * BK * 2 + part * BK);
+      const bool leader = elect_one();
+      bool go = true, ran_out;
       int s = 0, par = 0, t = 0;
-      for (int tile = pair; tile < total_tiles && !*aborted; tile += pairs, ++t) {
-        if (!mbar_wait(smem_u32(&acc_empty), (t & 1) ^ 1)) {
-          gb_err::report(ERR_WAIT_ACCUM);
-          *aborted = 1;
+      for (int tile = pair; tile < total_tiles && go; tile += pairs, ++t) {
+        if (!(go = mbar_wait_warp(smem_u32(&acc_empty), (t & 1) ^ 1, aborted, ran_out))) {
+          if (ran_out) gb_err::report(ERR_WAIT_ACCUM), *aborted = 1;
           break;
         }
         tc_fence_after_sync();
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(smem_u32(&full_bar[s]), par)) {
-            gb_err::report(ERR_WAIT_FULL);
-            *aborted = 1;
+          if (!(go = mbar_wait_warp(smem_u32(&full_bar[s]), par, aborted, ran_out))) {
+            if (ran_out) gb_err::report(ERR_WAIT_FULL), *aborted = 1;
+            break;
           }
-          if (*aborted) break;
           tc_fence_after_sync();
-          const uint64_t da = smem_desc_sw128(tiles + s * stage_bytes), db0 = smem_desc_sw128(tiles + s * stage_bytes + BM * BK * 2),
-                         db1 = smem_desc_sw128(tiles + s * stage_bytes + BM * BK * 2 + part * BK);
+          const uint64_t at = (uint64_t)(s * (stage_bytes >> 4));
+          if (leader) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            mma_bf16_pair(tmem_base, da + 2 * k, db0 + 2 * k, idesc, kb > 0 || k > 0);
-            mma_bf16_pair(tmem_base + part, da + 2 * k, db1 + 2 * k, idesc, kb > 0 || k > 0);
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+              mma_bf16_pair(tmem_base, da0 + at + 2 * k, db0 + at + 2 * k, idesc, kb > 0 || k > 0);
+              mma_bf16_pair(tmem_base + part, da0 + at + 2 * k, db1 + at + 2 * k, idesc, kb > 0 || k > 0);
+            }
+            mma_commit_pair(smem_u32(&empty_bar[s]), 3);
           }
-          mma_commit_pair(smem_u32(&empty_bar[s]), 3);
+          __syncwarp();
           if (++s == stages) s = 0, par ^= 1;
         }
-        mma_commit_pair(smem_u32(&acc_full), 3);
+        if (leader) mma_commit_pair(smem_u32(&acc_full), 3);
+        __syncwarp();
       }
     }
   } else {

@@ -8,7 +8,7 @@
 // the queries' 80 KB.
 //   warp 0     TMA: the query tile, then the tiles, one box per page and block of 64 channels. Pages that are not there or that
 //              lie behind the last key are asked for beyond the pool's end, which fills their rows with zeros.
-//   warp 1     one lane: S = Q K^T for two tiles ahead, into one of two S buffers; O += P V of the tile whose softmax just ended,
+//   warp 1     one elected lane: S = Q K^T for two tiles ahead, into one of two S buffers; O += P V of the tile whose softmax just ended,
 //              P read from the S buffer in tensor memory. O stays in tensor memory to the end.
 //   warps 2-5  a thread owns a query row: its 64 scores, the mask on tiles that reach beyond the tile's first position, exp2 with the
 //              scale folded in against the running maximum (where it grows for some row of a warp, that warp rescales O), P in
@@ -158,6 +158,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------------- MMA issuer
+    const bool leader = elect_one();
     constexpr uint32_t idesc_s = instr_desc_bf16(QROWS, KT);
     constexpr uint32_t idesc_o = instr_desc_bf16(QROWS, RANK) | INSTR_B_MN_MAJOR;
     const uint64_t dq0 = smem_desc_sw128(q_s), dk0 = smem_desc_sw128(k_s), dv0 = smem_desc_sw128_mn(k_s, K_BLOCK);
@@ -171,7 +172,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
         return;
       }
       tc_fence_after_sync();
-      if (lane == 0) {
+      if (leader) {
 #pragma unroll
         for (int k = 0; k < ROW / 16; ++k)                         // 16 channels a product, 32 bytes on within a block's rows
           mma_bf16(tmem_base + S_COL0 + buf * KT, dq0 + (uint64_t)((k / 4) * (Q_BLOCK >> 4) + (k % 4) * 2),
@@ -190,7 +191,7 @@ latent_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constan
         break;
       }
       tc_fence_after_sync();
-      if (lane == 0) {
+      if (leader) {
         mma_bf16_ts<KT / 16>(tmem_base, tmem_base + S_COL0 + buf * KT, dv0 + (uint64_t)(st * (K_BYTES >> 4)), idesc_o, 16 * ROW_BYTES >> 4, t > 0);
         mma_commit(smem_u32(&mc.k_empty[st]));
         mma_commit(smem_u32(&mc.o_ready));

@@ -75,6 +75,26 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
   return true;
 }
 
+// One lane of a converged warp, chosen by the hardware. The loops that issue tcgen05.mma, commits and TMA copies are walked by
+// a whole warp whose elected lane issues: operands of these instructions live in uniform registers, which the compiler
+// can only fill directly where control flow is a warp's. Issued by one thread of a warp that had parted (`if (lane == 0)` around the
+// loop), a step of four products of 256 x 256 x 16 a pair of CTAs took 610 cycles; elected, 535 (the products themselves 512).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t yes;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(yes));
+  return yes != 0;
+}
+// mbar_wait by a whole warp. False for all lanes if the wait ran out for one of them (then ran_out is set there) or if *aborted
+// is set: the warp leaves its loop together.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const volatile int* aborted, bool& ran_out) {
+  ran_out = !mbar_wait(bar, parity);
+  return __all_sync(0xffffffffu, !ran_out && !*aborted);
+}
+
 // ------------------------------------------------------------------ TMA
 // One box of a 2-D tensor map into shared memory; completion is counted in
 // bytes on `bar`. c0 is the coordinate along the contiguous dimension (its
