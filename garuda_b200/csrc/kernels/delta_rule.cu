@@ -32,8 +32,8 @@ namespace {
 
 constexpr int MAX_TAPS = 8;
 
-__device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
-__device__ __forceinline__ float sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
+__device__ __forceinline__ float silu(float z) { return gb::divide(z, 1.0f + expf(-z)); }
+__device__ __forceinline__ float sigmoid(float z) { return gb::over(1.0f + expf(-z)); }
 __device__ __forceinline__ float softplus(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 // Input of channel c at `lag` tokens before token t (index j within its request's rows of this step):

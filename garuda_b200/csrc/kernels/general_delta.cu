@@ -27,7 +27,7 @@
 
 namespace {
 
-__device__ __forceinline__ float sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
+__device__ __forceinline__ float sigmoid(float z) { return gb::over(1.0f + expf(-z)); }
 
 // proj [T, P]: columns r | k | v | removal logits | ...; each block H dim wide (v: H vdim).
 // zdec [T, PZ]: the decay's pre-activation, H dim wide.

@@ -25,7 +25,7 @@ namespace {
 
 constexpr int MAX_TAPS = 16;
 
-__device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
+__device__ __forceinline__ float silu(float z) { return gb::divide(z, 1.0f + expf(-z)); }
 __device__ __forceinline__ float softplus(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 // A decay a = exp(log_a) as the two numbers that a state is moved on with, S <- keep S + (change S + input). A slow
