@@ -27,7 +27,7 @@
 // A group of four warps has 16 columns of S, a quarter of the channels each: S^T in the accumulators' layout is at once the first
 // operand of S^T [W; Q]^T, so nothing of S is ever exchanged, only the warps' shares of Y and o. One group a block while the
 // walked requests' blocks are at most one an SM (16 heads x 8 groups are 128 blocks for 148 SMs); two (which share WQ, K1 and K2) where the
-// heads are more. 2,048 tokens of 16 heads of 128 x 128 take 98 us here and 119 us in the kernel in front (B200), where the
+// heads are more. 2,048 tokens of 16 heads of 128 x 128 take 98 us here and 118 us in the kernel in front (B200), where the
 // token-by-token walk took 0.89 ms; the tensor cores are 44% busy, the rest is the latency of a chunk's three barriers.
 #pragma once
 
@@ -138,56 +138,17 @@ __device__ __forceinline__ float sum_of_eight(float (&v)[8], int lane) {
   return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-// ---- the substitution's building blocks: a column of C numbers in registers, in pairs -----------
-constexpr int LT = C + 4;            // floats between the rows of the small matrices
-
-// x_i += sign * m[j][i] * y for the i > j (STRICT) or i >= j; m is held transposed, a row per j. Numbers of the other
-// side of the diagonal are not touched: an infinity at token j must not reach the tokens in front of it.
-template <bool STRICT>
-__device__ __forceinline__ void add_row(pair_t (&x)[C / 2], const float* m, int j, float y) {
-  const int from = STRICT ? j + 1 : j;
-  const pair_t yy = make_pair(y, y);
-#pragma unroll
-  for (int i4 = 0; i4 < C; i4 += 4) {
-    if (i4 + 3 < from) continue;
-    const pair2_t f = *reinterpret_cast<const pair2_t*>(m + j * LT + i4);
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      const int i = i4 + 2 * p;
-      const pair_t c = p ? f.b : f.a;
-      if (i >= from) {
-        x[i / 2] = fma2(c, yy, x[i / 2]);
-      } else if (i + 1 >= from) {
-        const float2 old = both(x[i / 2]);
-        x[i / 2] = make_pair(old.x, fmaf(both(c).y, y, old.y));
-      }
-    }
-  }
-}
-__device__ __forceinline__ float entry(const pair_t (&x)[C / 2], int i) { return i & 1 ? both(x[i / 2]).y : both(x[i / 2]).x; }
-__device__ __forceinline__ void set_entry(pair_t (&x)[C / 2], int i, float v) {
-  const float2 old = both(x[i / 2]);
-  x[i / 2] = i & 1 ? make_pair(old.x, v) : make_pair(v, old.y);
-}
-
-__device__ __forceinline__ void store_rows(float* block, const Layout& lay, int first_row, int c, const pair_t (&x)[C / 2]) {
-#pragma unroll
-  for (int i = 0; i < C; ++i) block[lay.wq(first_row + i, c)] = entry(x, i);
-}
-__device__ __forceinline__ void store_column(float* to, const pair_t (&x)[C / 2]) {
-#pragma unroll
-  for (int i = 0; i < C / 4; ++i) {
-    const float2 a = both(x[2 * i]), b = both(x[2 * i + 1]);
-    reinterpret_cast<float4*>(to)[i] = make_float4(a.x, a.y, b.x, b.y);
-  }
-}
-
-// ---- the walk ------------------------------------------------------------------------------------
+// 16 and 4 bytes into shared memory, asynchronously
 __device__ __forceinline__ void copy_16(float* smem, const float* gmem) {
   const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void copy_4(float* smem, const float* gmem) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s), "l"(gmem) : "memory");
+}
 
+// ---- 32-bit products on the tensor cores ----------------------------------------------------------
 // A 32-bit number as two tf32 ones: the nearest (ties away from zero), and the rest, whose low bits the tensor cores do
 // not read (the rest has either sign, so cutting it off leans to neither side). A number that is not finite makes the rest not a
 // number, whatever the rounding makes of its own bits.
@@ -210,6 +171,124 @@ __device__ __forceinline__ void mma_1688_first(float (&d)[4], const uint32_t (&a
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
 
+// a b of eight channels or tokens, b given in its parts: the sum of the three products, in the tensor cores
+__device__ __forceinline__ void piece_of(float (&d)[4], const uint32_t (&hi)[4], const uint32_t (&lo)[4], uint32_t bh0, uint32_t bh1, uint32_t bl0,
+                                         uint32_t bl1) {
+  mma_1688_first(d, lo, bh0, bh1);
+  mma_1688(d, hi, bl0, bl1);
+  mma_1688(d, hi, bh0, bh1);
+}
+
+// ---- what the kernels in front of the walk share ----------------------------------------------------
+// A chunk's small matrices are lower triangular, [token i][token j], and are made and used in blocks of 8 x 8 tokens. Those below the
+// diagonal are sums over channels of products of a row of token i, decayed on from its block's start, and a row of token j, decayed on to its
+// block's end (and through the blocks between): no factor is above one, so nothing overflows and what underflows is nothing. They
+// come off the tensor cores in the layout in which the substitution's products read them as their second operand, and are kept there
+// split in two. Those on the diagonal are sums of running products, token by token, and are used so: a number that is not
+// finite at token j must not meet the zeros of the tokens in front of it.
+constexpr int NB = C / 8, BELOW = NB * (NB - 1) / 2;      // blocks; those below the diagonal
+__host__ __device__ constexpr int below(int bi, int bj) { return bi * (bi - 1) / 2 + bj; }
+struct Lower {
+  float4 off[BELOW][32];               // a lane's two numbers (token i = lane / 4, tokens j = 2 (lane % 4) and the next): high parts, low parts
+  float on[NB][64];                    // [token j][token i]
+};
+__device__ __forceinline__ float4 split_pair(float a, float b) {
+  uint32_t ah, al, bh, bl;
+  split(a, ah, al), split(b, bh, bl);
+  return make_float4(__uint_as_float(ah), __uint_as_float(bh), __uint_as_float(al), __uint_as_float(bl));
+}
+
+// A running product of decays in two numbers, so that it is rounded once however long it is: a head's one decay for all channels makes
+// its rounding the whole row's (with single numbers the gated rule's read-outs were up to 1.1 times as far from 64 bits).
+struct Product {
+  float hi = 1.f, lo = 0.f;
+  __device__ __forceinline__ void by(float g) {
+    const float p = hi * g;
+    lo = fmaf(lo, g, fmaf(hi, g, -p)), hi = p;
+  }
+  __device__ __forceinline__ void by(float2 g) {
+    const float p = hi * g.x;
+    lo = fmaf(hi, g.y, fmaf(lo, g.x, fmaf(hi, g.x, -p))), hi = p;
+  }
+  __device__ __forceinline__ float of(float x) const { return fmaf(x, hi, x * lo); }
+  __device__ __forceinline__ float2 both() const { return make_float2(hi, lo); }
+  __device__ __forceinline__ float value() const { return hi + lo; }
+};
+
+// The block (bi, bj) below the diagonal of two matrices at once: rows 0 to 7 of the product's 16 belong to `first`, the others to
+// `second` [tokens of bi][LD], the second operand is `with` [tokens of bj][LD]; through [NB][DIM]: whole blocks' decays.
+template <int DIM, int LD>
+__device__ __forceinline__ void block_below(float (&acc)[4], const float* first, const float* second, const float* with, const float2* through, int bi,
+                                            int bj, int lane) {
+  const int at = (lane >> 2) * LD + 2 * (lane & 3);
+  const float *a = first + bi * 8 * LD + at, *b = second + bi * 8 * LD + at, *c = with + bj * 8 * LD + at;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) acc[e] = 0.f;
+#pragma unroll 4
+  for (int s = 0; s < DIM; s += 8) {
+    const float2 x = *reinterpret_cast<const float2*>(a + s), y = *reinterpret_cast<const float2*>(b + s);
+    float2 z = *reinterpret_cast<const float2*>(c + s);
+    for (int between = bj + 1; between < bi; ++between) {
+      const float4 g = *reinterpret_cast<const float4*>(through + between * DIM + s + 2 * (lane & 3));
+      z.x = fmaf(z.x, g.x, z.x * g.y), z.y = fmaf(z.y, g.z, z.y * g.w);
+    }
+    uint32_t hi[4], lo[4], h0, l0, h1, l1;
+    split(x.x, hi[0], lo[0]), split(y.x, hi[1], lo[1]), split(x.y, hi[2], lo[2]), split(y.y, hi[3], lo[3]);
+    split(z.x, h0, l0), split(z.y, h1, l1);
+    float piece[4];
+    piece_of(piece, hi, lo, h0, h1, l0, l1);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[e] += piece[e];
+  }
+}
+
+// The substitution, a warp per 16 columns in the accumulators' layout: [e] is column lane / 4 + 8 (e / 2), token 2 (lane % 4) + (e & 1) of
+// a block. take holds what the tokens in front take off (or, for a second matrix, add to) a row, summed by itself: it is small beside
+// the row, and what is added last is rounded last. This: the block's own tokens, one after another. now(e): token e & 1's number as it stands;
+// where a lane's token is behind token j it loses m1_ij times it, and from j on `more` gains m2_ij times it.
+template <class Now>
+__device__ __forceinline__ void on_diagonal(const float* m1, const float* m2, int lane, float (&take)[4], float (&more)[4], Now&& now) {
+  const int tig = lane & 3;
+  const float *a = m1 + 2 * tig, *b = m2 + 2 * tig;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float2 x = *reinterpret_cast<const float2*>(a + j * 8), z = *reinterpret_cast<const float2*>(b + j * 8);
+    const float y0 = __shfl_sync(0xffffffffu, now(j & 1), (lane & 28) | (j >> 1));
+    const float y1 = __shfl_sync(0xffffffffu, now(2 + (j & 1)), (lane & 28) | (j >> 1));
+    if (2 * tig > j) take[0] = fmaf(-x.x, y0, take[0]), take[2] = fmaf(-x.x, y1, take[2]);
+    if (2 * tig + 1 > j) take[1] = fmaf(-x.y, y0, take[1]), take[3] = fmaf(-x.y, y1, take[3]);
+    if (2 * tig >= j) more[0] = fmaf(z.x, y0, more[0]), more[2] = fmaf(z.x, y1, more[2]);
+    if (2 * tig + 1 >= j) more[1] = fmaf(z.y, y0, more[1]), more[3] = fmaf(z.y, y1, more[3]);
+  }
+}
+// The later blocks' share of a finished block bj: y its numbers.
+__device__ __forceinline__ void below_diagonal(const Lower& m1, const Lower& m2, int bj, int lane, const float (&y)[4], float (&take)[NB][4],
+                                               float (&more)[NB][4]) {
+  uint32_t hi[4], lo[4];
+  split(y[0], hi[0], lo[0]), split(y[2], hi[1], lo[1]), split(y[1], hi[2], lo[2]), split(y[3], hi[3], lo[3]);
+#pragma unroll
+  for (int bi = 1; bi < NB; ++bi) {
+    if (bi <= bj) continue;
+    const float4 f = m1.off[below(bi, bj)][lane], k = m2.off[below(bi, bj)][lane];
+    float p[4], q[4];
+    piece_of(p, hi, lo, __float_as_uint(f.x), __float_as_uint(f.y), __float_as_uint(f.z), __float_as_uint(f.w));
+    piece_of(q, hi, lo, __float_as_uint(k.x), __float_as_uint(k.y), __float_as_uint(k.z), __float_as_uint(k.w));
+#pragma unroll
+    for (int e = 0; e < 4; ++e) take[bi][e] -= p[e], more[bi][e] += q[e];
+  }
+}
+// A block's numbers into rows row0 .. of W or Q, or into columns of tokens from 8 bi on (VP, OP, V).
+__device__ __forceinline__ void store_tile_rows(float* block, const Layout& lay, int row0, int col0, int lane, const float (&x)[4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) block[lay.wq(row0 + 2 * (lane & 3) + (e & 1), col0 + (lane >> 2) + 8 * (e >> 1))] = x[e];
+}
+__device__ __forceinline__ void store_tile_columns(float* to, int col0, int bi, int lane, const float (&x)[4]) {
+  float* p = to + (col0 + (lane >> 2)) * C + bi * 8 + 2 * (lane & 3);
+  *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
+  *reinterpret_cast<float2*>(p + 8 * C) = make_float2(x[2], x[3]);
+}
+
+// ---- the walk ------------------------------------------------------------------------------------
 constexpr int LDR = 2 * C + 8, LDY = C + 8;        // floats between columns in shared memory: eight columns' reads fall into different banks
 
 template <int DIM, int GROUPS, bool TWO>

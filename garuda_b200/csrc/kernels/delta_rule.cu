@@ -256,10 +256,20 @@ delta_recurrence_kernel(const float* __restrict__ prep, int W, const int32_t* __
 // delta_prepare, then, with D_i the product of the decays up to token i,
 //     L_ij = beta_i sum_d k_i k_j D_i / D_j (j < i),   B_ij = sum_d q_i k_j D_i / D_j (j <= i)
 //     W = (I + L)^-1 beta (D k),   VP = (I + L)^-1 beta v,   Q = D q - B W,   OP = B VP,   K1_j = k_j D_last / D_j
-// The quotients D_i / D_j are running products of decays from j on (never above one, so nothing overflows and what
-// underflows is nothing), and the triangular system is solved by substitution, a thread per column of W and VP. 32-bit multiply-adds; what a row
-// loses to those in front of it is summed before it is taken off, which halves the error of taking it off term by term.
+// The quotients D_i / D_j are products of decays between j and i, and the triangular system is solved by substitution: both in blocks
+// of 8 tokens (delta_chunk.cuh), on the tensor cores off the diagonal and in 32-bit multiply-adds on it.
+// What bounds it: the chunk's rows and results (2,048 tokens of 16 heads of 128 x 128 read 68 MB and write 84, 23 us), and the latency of
+// its six phases, three blocks an SM. With dots of all pairs by running products and a thread per column in the substitution
+// (33,000 of a block's 84,000 cycles, for the rows of L and B, which every warp read from shared memory for itself) 124 us, now 118.
 // grid (numbers, H), 256 threads; at most four taps.
+template <int DIM>
+struct FactorsSmem {
+  delta_chunk::Lower L, B;
+  // [tokens][DIM + 8] each. k and q: then decayed on from their block's start; g: decays, keys decayed on to their block's end, values
+  float k[delta_chunk::C * (DIM + 8)], q[delta_chunk::C * (DIM + 8)], g[delta_chunk::C * (DIM + 8)];
+  float2 through[delta_chunk::NB * DIM];         // whole blocks' decays (delta_chunk::Product)
+  float beta[delta_chunk::C];
+};
 template <int DIM, typename WT>
 __global__ void __launch_bounds__(256, 3)
 delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* __restrict__ second, int P2,
@@ -271,17 +281,11 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
   using delta_chunk::C;
   gb::pdl_launch_dependents();
   gb::pdl_wait();
-  constexpr int LD = DIM + 4, VEC = DIM / 32;
-  extern __shared__ __align__(16) float sh[];
-  float* sk = sh;                        // [C][LD]: k, then D k
-  float* sq = sk + C * LD;               // [C][LD]: q, then D q
-  float* sg = sq + C * LD;               // [C][LD]: decays
-  float* sL = sg + C * LD;               // [C][LT], a row per j (transposed)
-  float* sB = sL + C * LT;               // [C][LT], likewise
-  float* beta = sB + C * LT;             // [C]
-  // [C][LX]: the value columns of the block's first turn, in the decays' place where they fit
-  constexpr int LX = DIM == 128 ? LD : 256 - DIM;
-  float* sx = DIM == 128 ? sg : beta + C;
+  constexpr int LD = DIM + 8, VEC = DIM / 32;
+  extern __shared__ __align__(16) unsigned char raw[];
+  FactorsSmem<DIM>& sm = *reinterpret_cast<FactorsSmem<DIM>*>(raw);
+  float *sk = sm.k, *sq = sm.q, *sg = sm.g, *beta = sm.beta;
+  Lower &L = sm.L, &B = sm.B;
   const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int r, first, n, at;
   if (!find_chunk(blockIdx.x, cu_q, R, cut, r, first, n, at)) return;
@@ -306,32 +310,29 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
     if (!per_head) rows(sg, second + (size_t)first * P2 + h * DIM, P2);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  // Convolution and SiLU of a channel's tokens, 16 at a time: take(i, value) for i = 0 .. C - 1 from input(i)
-  auto convolve = [&](int ch, auto&& input, auto&& take) {
-    float w[4], x[3];                    // by lag; the inputs in front of the chunk
+  // Convolution and SiLU of a channel's tokens from i1 on, TURN of them: `in` their inputs, x those in front, the last first
+  auto weights = [&](int ch, float (&w)[4]) {              // by lag
 #pragma unroll
     for (int lag = 0; lag < 4; ++lag) w[lag] = lag < taps ? gb::to_float<WT>(conv_w[(size_t)ch * taps + taps - 1 - lag]) : 0.f;
+  };
+  auto in_front = [&](int ch, int i1, float (&x)[3]) {
 #pragma unroll
-    for (int lag = 1; lag < 4; ++lag) x[lag - 1] = lag < taps ? conv_input(proj, P, first, at, lag, ch, kept, CH, taps) : 0.f;
+    for (int lag = 1; lag < 4; ++lag) x[lag - 1] = lag < taps && i1 < n ? conv_input(proj, P, first + i1, at + i1, lag, ch, kept, CH, taps) : 0.f;
+  };
+  auto convolve = [&](const float (&w)[4], float (&x)[3], int i1, const auto& in, auto&& take) {
+    constexpr int TURN = sizeof(in) / sizeof(float);
 #pragma unroll
-    for (int i0 = 0; i0 < C; i0 += 16) {
-      float in[16];
-#pragma unroll
-      for (int e = 0; e < 16; ++e) in[e] = i0 + e < n ? input(i0 + e) : 0.f;
-#pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        // (an input further back than the taps reach must not count: with a weight of zero an infinity would)
-        float acc = taps > 3 ? fmaf(w[3], x[2], 0.f) : 0.f;
-        if (taps > 2) acc = fmaf(w[2], x[1], acc);
-        if (taps > 1) acc = fmaf(w[1], x[0], acc);
-        acc = fmaf(w[0], in[e], acc);
-        x[2] = x[1], x[1] = x[0], x[0] = in[e];
-        take(i0 + e, i0 + e < n ? silu(acc) : 0.f);
-      }
+    for (int e = 0; e < TURN; ++e) {
+      // (an input further back than the taps reach must not count: with a weight of zero an infinity would)
+      float acc = taps > 3 ? fmaf(w[3], x[2], 0.f) : 0.f;
+      if (taps > 2) acc = fmaf(w[2], x[1], acc);
+      if (taps > 1) acc = fmaf(w[1], x[0], acc);
+      acc = fmaf(w[0], in[e], acc);
+      x[2] = x[1], x[1] = x[0], x[0] = in[e];
+      take(i1 + e, i1 + e < n ? silu(acc) : 0.f);
     }
   };
   const float rate = expf(gb::to_float<WT>(a_log[h]));
-  for (int i = tid; i < 2 * C * LT; i += 256) sL[i] = 0.f;
   if (tid < C) beta[tid] = tid < n ? sigmoid(proj[(size_t)(first + tid) * P + CH + h]) : 0.f;
   if (per_head) {
     // one decay for all key channels: every thread's warp makes one token's at a time
@@ -354,7 +355,15 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
   for (int c = tid; c < 2 * DIM; c += 256) {               // in place: a thread owns its channels' columns
     const bool query = c < DIM;
     float* col = query ? sq + c : sk + c - DIM;
-    convolve(query ? kvh * DIM + c : (G + kvh) * DIM + c - DIM, [&](int i) { return col[i * LD]; }, [&](int i, float v) { col[i * LD] = v; });
+    const int ch = query ? kvh * DIM + c : (G + kvh) * DIM + c - DIM;
+    float w[4], x[3], in[16];
+    weights(ch, w), in_front(ch, 0, x);
+#pragma unroll
+    for (int i0 = 0; i0 < C; i0 += 16) {
+#pragma unroll
+      for (int e = 0; e < 16; ++e) in[e] = i0 + e < n ? col[(i0 + e) * LD] : 0.f;
+      convolve(w, x, i0, in, [&](int i, float v) { col[i * LD] = v; });
+    }
   }
   __syncthreads();
 #pragma unroll
@@ -371,8 +380,8 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
   }
   __syncthreads();
   {
-    // L and B: a warp has four keys j, each decayed on from token to token; early and late keys paired on a scheduler
-    const int j0 = (warp < 4 ? warp : 11 - warp) * 4, d0 = lane * VEC;
+    // L and B on the diagonal: a warp has four keys j, each decayed on from token to token up to its block's end
+    const int j0 = warp * 4, j1 = (warp | 1) * 4 + 4, d0 = lane * VEC;
     pair_t p[4][VEC / 2];
     auto row = [&](const float* m, int i, pair_t (&x)[VEC / 2]) {
       if (VEC == 4) {
@@ -394,16 +403,15 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
       const int which = lane >> 2, j = j0 + (which & 3);
       if ((lane & 3) == 0) {
         if (which < 4) {
-          if (j < i) sL[j * LT + i] = beta[i] * sum;
+          if (j < i) L.on[j >> 3][(j & 7) * 8 + (i & 7)] = beta[i] * sum;
         } else if (j <= i) {
-          sB[j * LT + i] = sum;
+          B.on[j >> 3][(j & 7) * 8 + (i & 7)] = sum;
         }
       }
     };
 #pragma unroll
     for (int ii = 0; ii < 4; ++ii) {       // the tokens of the four keys themselves
       const int i = j0 + ii;
-      if (i >= n) break;
       pair_t g[VEC / 2], k[VEC / 2], q[VEC / 2];
       row(sg, i, g), row(sk, i, k), row(sq, i, q);
       float v[8];
@@ -417,7 +425,7 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
       keep(i, v);
     }
 #pragma unroll 2
-    for (int i = j0 + 4; i < n; ++i) {
+    for (int i = j0 + 4; i < j1; ++i) {
       pair_t g[VEC / 2], k[VEC / 2], q[VEC / 2];
       row(sg, i, g), row(sk, i, k), row(sq, i, q);
       float v[8];
@@ -432,67 +440,101 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
     }
   }
   __syncthreads();
-  if (tid < DIM) {                       // a thread per channel
-    float run = 1.f;
+  // decayed on within a block of tokens: queries and keys from its start, and keys, in the decays' place, to its end
+  for (int i = tid; i < NB * DIM; i += 256) {
+    const int c = i % DIM, at0 = i / DIM * 8 * LD + c;
+    float g[8], k[8];
 #pragma unroll
-    for (int j0 = C - 8; j0 >= 0; j0 -= 8) {
-      float x[8];
+    for (int t = 0; t < 8; ++t) g[t] = sg[at0 + t * LD], k[t] = sk[at0 + t * LD];
+    Product on, behind;
 #pragma unroll
-      for (int e = 7; e >= 0; --e) {
-        x[e] = sk[(j0 + e) * LD + tid] * run;
-        run *= sg[(j0 + e) * LD + tid];
-      }
-      float4* to = reinterpret_cast<float4*>(block + lay.k1(j0, tid));
-      to[0] = make_float4(x[0], x[1], x[2], x[3]), to[1] = make_float4(x[4], x[5], x[6], x[7]);
+    for (int t = 0; t < 8; ++t) {
+      on.by(g[t]);
+      sq[at0 + t * LD] = on.of(sq[at0 + t * LD]);
+      sk[at0 + t * LD] = on.of(k[t]);
     }
-    block[lay.last() + tid] = run;
-    run = 1.f;
-#pragma unroll 8
-    for (int i = 0; i < C; ++i) sk[i * LD + tid] *= run *= sg[i * LD + tid];
-  } else if (tid >= 128 && tid < 128 + DIM) {
-    float run = 1.f;
-#pragma unroll 8
-    for (int i = 0; i < C; ++i) sq[i * LD + tid - 128] *= run *= sg[i * LD + tid - 128];
+    sm.through[i] = on.both();
+#pragma unroll
+    for (int t = 7; t >= 0; --t) {
+      sg[at0 + t * LD] = behind.of(k[t]);
+      behind.by(g[t]);
+    }
   }
   __syncthreads();
-  for (int c = tid; c < DIM + vdim; c += 256) {
-    const bool key = c < DIM;            // the same for a warp
-    // a thread's column: of keys; of values; of values in a second turn, where the thread's keys were
-    const bool in_sx = !key && c < 256;
-    const int ld = in_sx ? LX : LD;
-    float* x = in_sx ? sx + c - DIM : sk + tid;
-    if (!key) {
-      const int ch = 2 * G * DIM + h * vdim + c - DIM;
-      convolve(ch, [&](int i) { return proj[(size_t)(first + i) * P + ch]; }, [&](int i, float v) { x[i * ld] = v; });
-    }
-    pair_t w[C / 2], o[C / 2];           // what the rows in front take off a row, summed by itself: it is small beside the row
+  for (int task = warp; task < BELOW; task += 8) {
+    const int bi = task < 1 ? 1 : task < 3 ? 2 : 3, bj = task - below(bi, 0);
+    float acc[4];
+    block_below<DIM, LD>(acc, sq, sk, sg, sm.through, bi, bj, lane);
+    const float b = beta[bi * 8 + (lane >> 2)];
+    B.off[task][lane] = split_pair(acc[0], acc[1]);
+    L.off[task][lane] = split_pair(b * acc[2], b * acc[3]);
+  }
+  for (int i = tid; i < NB * DIM; i += 256) {              // K1, and the chunk's whole decay
+    const int c = i % DIM, bj = i / DIM;
+    Product behind;
+    float x[8];
 #pragma unroll
-    for (int i = 0; i < C / 2; ++i) w[i] = o[i] = 0ull;
-    float next = x[0];
+    for (int b = NB - 1; b > 0; --b)
+      if (b > bj) behind.by(sm.through[b * DIM + c]);
 #pragma unroll
-    for (int j = 0; j < C; ++j) {
-      const float y = fmaf(beta[j], next, entry(w, j));
-      set_entry(w, j, y);
-      if (j + 1 == C) break;
-      next = x[(j + 1) * ld];
-      add_row<true>(w, sL, j, -y);
-      asm volatile("" ::: "memory");     // (else all rows are fetched at once, and more is spilled)
+    for (int t = 0; t < 8; ++t) x[t] = behind.of(sg[(bj * 8 + t) * LD + c]);
+    float4* to = reinterpret_cast<float4*>(block + lay.k1(bj * 8, c));
+    to[0] = make_float4(x[0], x[1], x[2], x[3]), to[1] = make_float4(x[4], x[5], x[6], x[7]);
+    if (bj == 0) {
+      behind.by(sm.through[c]);
+      block[lay.last() + c] = behind.value();
     }
-    if (key) store_rows(block, lay, 0, c, w);
-    else store_column(block + lay.vp() + (c - DIM) * C, w);
-    const float sign = key ? -1.f : 1.f;
+  }
+  __syncthreads();
+  // The substitution: the keys' columns, and the values' up to DIM at a time, which are convolved into the decays' place
+  const int g = lane >> 2, tig = lane & 3;
+  auto columns = [&](auto keys, int col0, const float* from, float* vp, float* op) {
+    float take[NB][4], more[NB][4];
 #pragma unroll
-    for (int j = 0; j < C; ++j) {
-      add_row<false>(o, sB, j, sign * entry(w, j));
-      asm volatile("" ::: "memory");
-    }
-    if (key) {
+    for (int b = 0; b < NB; ++b)
 #pragma unroll
-      for (int i = 0; i < C; ++i) set_entry(o, i, sq[i * LD + c] + entry(o, i));
-      store_rows(block, lay, C, c, o);
-    } else {
-      store_column(block + lay.op() + (c - DIM) * C, o);
+      for (int e = 0; e < 4; ++e) take[b][e] = more[b][e] = 0.f;
+    Product front[2];         // keys: D, as the blocks in front make it
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const float beta2[2] = {beta[b * 8 + 2 * tig], beta[b * 8 + 2 * tig + 1]};
+      float x[4], y[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        x[e] = from[(b * 8 + 2 * tig + (e & 1)) * LD + g + 8 * (e >> 1)];
+        if (keys) x[e] = front[e >> 1].of(x[e]);
+      }
+      on_diagonal(L.on[b], B.on[b], lane, take[b], more[b], [&](int e) { return fmaf(beta2[e & 1], x[e], take[b][e]); });
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[e] = fmaf(beta2[e & 1], x[e], take[b][e]);
+      if (b + 1 < NB) below_diagonal(L, B, b, lane, y, take, more);
+      if (keys) {
+        store_tile_rows(block, lay, b * 8, col0, lane, y);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[e] = front[e >> 1].of(sq[(b * 8 + 2 * tig + (e & 1)) * LD + col0 + g + 8 * (e >> 1)]) - more[b][e];
+        store_tile_rows(block, lay, C + b * 8, col0, lane, x);
+        front[0].by(sm.through[b * DIM + col0 + g]), front[1].by(sm.through[b * DIM + col0 + g + 8]);
+      } else {
+        store_tile_columns(vp, col0, b, lane, y);
+        store_tile_columns(op, col0, b, lane, more[b]);
+      }
     }
+  };
+  for (int v0 = 0; v0 < vdim; v0 += DIM) {
+    constexpr int EACH = C * DIM / 256;            // a thread's tokens of a channel
+    const int vc = tid % DIM, v1 = tid / DIM * EACH, ch = 2 * G * DIM + h * vdim + v0 + vc;
+    if (v0 > 0) __syncthreads();
+    if (v0 + vc < vdim) {
+      float w[4], x[3], in[EACH];
+      weights(ch, w), in_front(ch, v1, x);
+#pragma unroll
+      for (int e = 0; e < EACH; ++e) in[e] = v1 + e < n ? proj[(size_t)(first + v1 + e) * P + ch] : 0.f;
+      convolve(w, x, v1, in, [&](int i, float v) { sg[i * LD + vc] = v; });
+    }
+    if (v0 == 0 && warp * 16 < DIM) columns(std::true_type{}, warp * 16, sk + warp * 16, nullptr, nullptr);
+    __syncthreads();
+    if (v0 + warp * 16 < vdim && warp * 16 < DIM)
+      columns(std::false_type{}, v0 + warp * 16, sg + warp * 16, block + lay.vp(), block + lay.op());
   }
 }
 
@@ -754,7 +796,7 @@ GB_EXPORT int gb_delta_chunk(const float* proj, int P, const float* second, int 
   const int CH = 2 * G * dim + H * vdim, numbers = delta_chunk::chunk_numbers(T, walked);
   if (P < CH + H || P2 < (per_head ? H : H * dim)) return gb::fail(GB_BAD_ARGUMENT, "delta_chunk: row widths");
   if ((uintptr_t)blocks & 15) return gb::fail(GB_BAD_ARGUMENT, "delta_chunk: blocks start on 16 bytes");
-  const size_t smem = (size_t)(delta_chunk::C * (3 * (dim + 4) + 2 * delta_chunk::LT + 1 + (dim == 128 ? 0 : 256 - dim))) * sizeof(float);
+  const size_t smem = dim == 128 ? sizeof(FactorsSmem<128>) : sizeof(FactorsSmem<64>);
   const int rc = GB_DISPATCH_DTYPE(w_dtype, WT, [&]() -> int {
     auto kernel = dim == 128 ? delta_chunk_factors_kernel<128, WT> : delta_chunk_factors_kernel<64, WT>;
     static gb::OncePerDevice configured[2];      // per weight type: this lambda is instantiated for each

@@ -191,11 +191,22 @@ gdelta_recurrence_kernel(const float* __restrict__ prep, int W, const int32_t* _
 //     x_i = (D_i-1 u_i)^T S_0 + sum_{j<i} F_ij v_j - E_ij x_j,   E_ij = sum_d u_i alpha_j D_i-1 / D_j,   F_ij likewise with k_j
 //     o_i = (D_i r_i)^T S_0 + sum_{j<=i} H_ij v_j - G_ij x_j,    G_ij = sum_d r_i alpha_j D_i / D_j,     H_ij likewise with k_j
 // so  W = (I + E)^-1 (D u),   VP = -(I + E)^-1 F v,   Q = D r - G W,   OP = H v + G VP,   K1_j = alpha_j D_last / D_j,   K2_j = k_j
-// D_last / D_j, and the walk's Y is -x. Quotients of decays are running products and the system is solved by substitution, a
-// thread per column, in 32-bit multiply-adds, as for the gated rule (delta_rule.cu). grid (numbers, H), 2 DIM threads: with 256 for
-// 64 channels half of them had no column (2,048 tokens of 32 heads of 64 x 64: 211 us, now 171).
+// D_last / D_j, and the walk's Y is -x. As for the gated rule (delta_rule.cu), in blocks of 8 tokens: on the tensor cores off the
+// diagonal, in 32-bit multiply-adds on it. Bound as that kernel is. With running products for all pairs, a thread per column in the
+// substitution and rows fetched by the warps that use them 170 us for 2,048 tokens of 32 heads of 64 x 64, now 115.
+// grid (numbers, H), 256 threads.
 template <int DIM>
-__global__ void __launch_bounds__(2 * DIM, DIM == 64 ? 4 : 2)
+struct FactorsSmem {
+  delta_chunk::Lower E, F, G, H;
+  // [tokens][DIM + 8] each: u and r, then decayed on from their block's start (u up to the token in front of it); alpha and k, then decayed on
+  // to their block's end; decays
+  float u[delta_chunk::C * (DIM + 8)], r[delta_chunk::C * (DIM + 8)], a[delta_chunk::C * (DIM + 8)], k[delta_chunk::C * (DIM + 8)],
+      w[delta_chunk::C * (DIM + 8)];
+  float2 through[delta_chunk::NB * DIM];         // whole blocks' decays (delta_chunk::Product)
+};
+
+template <int DIM>
+__global__ void __launch_bounds__(256, DIM == 64 ? 3 : 2)
 gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, int col_k, int col_v, int col_a,
                             const float* __restrict__ zdec, int PZ, const float* __restrict__ w0, const float* __restrict__ a0,
                             float decay_scale, const int32_t* __restrict__ cu_q, float* __restrict__ blocks, int R, int H, int vdim,
@@ -204,54 +215,55 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
   using delta_chunk::C;
   gb::pdl_launch_dependents();
   gb::pdl_wait();
-  constexpr int LD = DIM + 4, VEC = DIM / 32;
-  constexpr int THREADS = 2 * DIM, WARPS = THREADS / 32;      // a thread a channel in two walks over the tokens, or a column of W and VP
-  extern __shared__ __align__(16) float sh[];
-  float* su = sh;                        // [C][LD]: u, then D u
-  float* sr = su + C * LD;               // [C][LD]: r, then D r
-  float* sw = sr + C * LD;               // [C][LD]: decays
-  float* sa = sw + C * LD;               // [C][LD]: alpha
-  float* sE = sa + C * LD;               // [C][LT] each, a row per j (transposed)
-  float* sF = sE + C * LT;
-  float* sG = sF + C * LT;
-  float* sH = sG + C * LT;
+  constexpr int LD = DIM + 8, VEC = DIM / 32;
+  extern __shared__ __align__(16) unsigned char raw[];
+  FactorsSmem<DIM>& sm = *reinterpret_cast<FactorsSmem<DIM>*>(raw);
+  float *su = sm.u, *sr = sm.r, *sa = sm.a, *sk = sm.k, *sw = sm.w;
   const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int r, first, n, at;
   if (!find_chunk(blockIdx.x, cu_q, R, cut, r, first, n, at)) return;
   const Layout lay{DIM, vdim, 1};
   float* block = blocks + ((size_t)blockIdx.x * H + h) * lay.floats();
   const float* row0 = proj + (size_t)first * P;
-#pragma unroll 2
-  for (int t = warp; t < C; t += WARPS) {
-    const float* row = row0 + (size_t)t * P;
-    float k[VEC], x[VEC], y[VEC], z[VEC], ss = 0.f;
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) {
-      const int c = h * DIM + lane + 32 * e;
-      k[e] = t < n ? row[col_k + c] : 0.f;
-      x[e] = t < n ? row[col_r + c] : 0.f;
-      y[e] = t < n ? row[col_a + c] : 0.f;
-      z[e] = t < n ? zdec[(size_t)(first + t) * PZ + c] : 0.f;
-      ss = fmaf(k[e], k[e], ss);
+  auto rows = [&](float* to, const float* from, int pitch) {      // all at once; 16 bytes a copy where rows start on 16 bytes
+    if (pitch % 4 == 0 && ((uintptr_t)from & 15) == 0) {
+      for (int i = tid; i < n * (DIM / 4); i += 256)
+        copy_16(to + i / (DIM / 4) * LD + i % (DIM / 4) * 4, from + (size_t)(i / (DIM / 4)) * pitch + i % (DIM / 4) * 4);
+    } else {
+      for (int i = tid; i < n * DIM; i += 256) copy_4(to + i / DIM * LD + i % DIM, from + (size_t)(i / DIM) * pitch + i % DIM);
     }
+  };
+  rows(sk, row0 + col_k + h * DIM, P);
+  rows(sa, row0 + col_a + h * DIM, P);
+  rows(sw, zdec + (size_t)first * PZ + h * DIM, PZ);
+  rows(sr, row0 + col_r + h * DIM, P);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  float rate[VEC], decay[VEC];
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) rate[e] = a0[h * DIM + lane + 32 * e], decay[e] = w0[h * DIM + lane + 32 * e];
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+#pragma unroll
+  for (int t = warp; t < C; t += 8) {
+    float k[VEC], ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) k[e] = t < n ? sk[t * LD + lane + 32 * e] : 0.f, ss = fmaf(k[e], k[e], ss);
     const float inv = 1.0f / sqrtf(gb::warp_sum(ss) + 1e-6f);
 #pragma unroll
     for (int e = 0; e < VEC; ++e) {
-      const int d = lane + 32 * e, c = h * DIM + d;
+      const int d = t * LD + lane + 32 * e;
       const float u = k[e] * inv;
-      su[t * LD + d] = u;
-      sr[t * LD + d] = x[e];
-      sw[t * LD + d] = t < n ? expf(-decay_scale * sigmoid(z[e] + w0[c])) : 1.f;
-      sa[t * LD + d] = t < n ? sigmoid(y[e] + a0[c]) * u : 0.f;
+      su[d] = u;
+      sa[d] = t < n ? sigmoid(sa[d] + rate[e]) * u : 0.f;
+      sw[d] = t < n ? expf(-decay_scale * sigmoid(sw[d] + decay[e])) : 1.f;
+      if (t >= n) sk[d] = sr[d] = 0.f;
     }
   }
-  for (int i = tid; i < 4 * C * LT; i += THREADS) sE[i] = 0.f;
   __syncthreads();
-  // four keys a warp at a time; early and late ones, which meet more and fewer tokens, in turn on a scheduler
-#pragma unroll 1
-  for (int turn = 0; turn < 8 / WARPS; ++turn) {
-    const int j0 = (WARPS == 8 ? (warp < 4 ? warp : 11 - warp) : (turn == 0 ? warp : 7 - warp)) * 4, d0 = lane * VEC;
-    pair_t pa[4][VEC / 2], pk[4][VEC / 2];                // alpha_j and k_j, decayed on
+  {
+    // the matrices on the diagonal: a warp has four keys j, decayed on from token to token up to their block's end
+    const int j0 = warp * 4, j1 = (warp | 1) * 4 + 4, d0 = lane * VEC;
+    pair_t pa[4][VEC / 2], pk[4][VEC / 2];                // alpha_j and k_j
     auto row = [&](const float* m, int i, pair_t (&x)[VEC / 2]) {
       if (VEC == 4) {
         const pair2_t f = *reinterpret_cast<const pair2_t*>(m + i * LD + d0);
@@ -269,26 +281,18 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
     };
     auto keep = [&](int i, float (&before)[8], float (&after)[8]) {
       const float b = sum_of_eight(before, lane), a = sum_of_eight(after, lane);
-      const int which = lane >> 2, j = j0 + (which & 3);
+      const int which = lane >> 2, j = j0 + (which & 3), place = (j & 7) * 8 + (i & 7);
       if ((lane & 3) == 0 && j <= i) {
-        if (j < i) (which < 4 ? sE : sF)[j * LT + i] = b;
-        (which < 4 ? sG : sH)[j * LT + i] = a;
+        if (j < i) (which < 4 ? sm.E : sm.F).on[j >> 3][place] = b;
+        (which < 4 ? sm.G : sm.H).on[j >> 3][place] = a;
       }
     };
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj)
-#pragma unroll
-      for (int e = 0; e < VEC / 2; ++e) {
-        const float* k = row0 + (size_t)(j0 + jj) * P + col_k + h * DIM + d0 + 2 * e;
-        pk[jj][e] = j0 + jj < n ? make_pair(k[0], k[1]) : 0ull;
-      }
-#pragma unroll
     for (int ii = 0; ii < 4; ++ii) {       // the tokens of the four keys themselves
       const int i = j0 + ii;
-      if (i >= n) break;
       pair_t w[VEC / 2], u[VEC / 2], x[VEC / 2];
       row(sw, i, w), row(su, i, u), row(sr, i, x);
-      row(sa, i, pa[ii]);
+      row(sa, i, pa[ii]), row(sk, i, pk[ii]);
       float before[8], after[8];
 #pragma unroll
       for (int jj = 0; jj < 4; ++jj) {
@@ -301,7 +305,7 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
       }
       keep(i, before, after);
     }
-    for (int i = j0 + 4; i < n; ++i) {
+    for (int i = j0 + 4; i < j1; ++i) {
       pair_t w[VEC / 2], u[VEC / 2], x[VEC / 2];
       row(sw, i, w), row(su, i, u), row(sr, i, x);
       float before[8], after[8];
@@ -316,77 +320,101 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
     }
   }
   __syncthreads();
-  if (tid < DIM) {                       // a thread per channel
-    float run = 1.f;
+  // decayed on within a block of tokens
+  for (int i = tid; i < NB * DIM; i += 256) {
+    const int c = i % DIM, at0 = i / DIM * 8 * LD + c;
+    float w[8];
 #pragma unroll
-    for (int j0 = C - 8; j0 >= 0; j0 -= 8) {
-      float x[8], y[8];
+    for (int t = 0; t < 8; ++t) w[t] = sw[at0 + t * LD];
+    Product on, behind;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) y[e] = j0 + e < n ? row0[(size_t)(j0 + e) * P + col_k + h * DIM + tid] : 0.f;
-#pragma unroll
-      for (int e = 7; e >= 0; --e) {
-        x[e] = sa[(j0 + e) * LD + tid] * run, y[e] *= run;
-        run *= sw[(j0 + e) * LD + tid];
-      }
-      float4* to = reinterpret_cast<float4*>(block + lay.k1(j0, tid));
-      to[0] = make_float4(x[0], x[1], x[2], x[3]), to[1] = make_float4(x[4], x[5], x[6], x[7]);
-      to = reinterpret_cast<float4*>(block + lay.k1(C + j0, tid));
-      to[0] = make_float4(y[0], y[1], y[2], y[3]), to[1] = make_float4(y[4], y[5], y[6], y[7]);
+    for (int t = 0; t < 8; ++t) {
+      su[at0 + t * LD] = on.of(su[at0 + t * LD]);
+      on.by(w[t]);
+      sr[at0 + t * LD] = on.of(sr[at0 + t * LD]);
     }
-    block[lay.last() + tid] = run;
-    run = 1.f;
-#pragma unroll 8
-    for (int i = 0; i < C; ++i) {
-      su[i * LD + tid] *= run;
-      run *= sw[i * LD + tid];
+    sm.through[i] = on.both();
+#pragma unroll
+    for (int t = 7; t >= 0; --t) {
+      sa[at0 + t * LD] = behind.of(sa[at0 + t * LD]), sk[at0 + t * LD] = behind.of(sk[at0 + t * LD]);
+      behind.by(w[t]);
     }
-  } else {
-    float run = 1.f;
-#pragma unroll 8
-    for (int i = 0; i < C; ++i) sr[i * LD + tid - DIM] *= run *= sw[i * LD + tid - DIM];
   }
   __syncthreads();
-  for (int c = tid; c < DIM + vdim; c += THREADS) {
-    const bool key = c < DIM;                             // the same for a warp
-    const float* v = row0 + col_v + h * vdim + c - DIM;   // a value column's numbers
-    pair_t w[C / 2], o[C / 2];                            // what is added to D u and D r, summed by itself: it is small beside them
+  for (int task = warp; task < 2 * BELOW; task += 8) {
+    const int which = task >> 1, bi = which < 1 ? 1 : which < 3 ? 2 : 3, bj = which - below(bi, 0);
+    float acc[4];
+    block_below<DIM, LD>(acc, su, sr, task & 1 ? sk : sa, sm.through, bi, bj, lane);
+    (task & 1 ? sm.F : sm.E).off[which][lane] = split_pair(acc[0], acc[1]);
+    (task & 1 ? sm.H : sm.G).off[which][lane] = split_pair(acc[2], acc[3]);
+  }
+  for (int i = tid; i < NB * DIM; i += 256) {              // K1, K2 and the chunk's whole decay
+    const int c = i % DIM, bj = i / DIM;
+    Product behind;
+    float x[8], y[8];
 #pragma unroll
-    for (int i = 0; i < C / 2; ++i) w[i] = o[i] = 0ull;
-    if (!key) {
+    for (int b = NB - 1; b > 0; --b)
+      if (b > bj) behind.by(sm.through[b * DIM + c]);
 #pragma unroll
-      for (int j4 = 0; j4 < C; j4 += 4) {
-        float x[4];
+    for (int t = 0; t < 8; ++t) x[t] = behind.of(sa[(bj * 8 + t) * LD + c]), y[t] = behind.of(sk[(bj * 8 + t) * LD + c]);
+    float4* to = reinterpret_cast<float4*>(block + lay.k1(bj * 8, c));
+    to[0] = make_float4(x[0], x[1], x[2], x[3]), to[1] = make_float4(x[4], x[5], x[6], x[7]);
+    to = reinterpret_cast<float4*>(block + lay.k1(C + bj * 8, c));
+    to[0] = make_float4(y[0], y[1], y[2], y[3]), to[1] = make_float4(y[4], y[5], y[6], y[7]);
+    if (bj == 0) {
+      behind.by(sm.through[c]);
+      block[lay.last() + c] = behind.value();
+    }
+  }
+  __syncthreads();
+  const int g = lane >> 2, tig = lane & 3;
+  for (int col0 = warp * 16; col0 < DIM + vdim; col0 += 128) {
+    float take[NB][4], more[NB][4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) x[e] = j4 + e < n ? v[(size_t)(j4 + e) * P] : 0.f;
-        *reinterpret_cast<float4*>(block + lay.v() + (c - DIM) * C + j4) = make_float4(x[0], x[1], x[2], x[3]);
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) take[b][e] = more[b][e] = 0.f;
+    if (col0 < DIM) {                    // D u, and what D r loses
+      Product front[2];       // the blocks in front
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        float x[4], y[4], q[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[e] = front[e >> 1].of(su[(b * 8 + 2 * tig + (e & 1)) * LD + col0 + g + 8 * (e >> 1)]);
+        on_diagonal(sm.E.on[b], sm.G.on[b], lane, take[b], more[b], [&](int e) { return x[e] + take[b][e]; });
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          add_row<true>(w, sF, j4 + e, -x[e]);
-          add_row<false>(o, sH, j4 + e, x[e]);
-          asm volatile("" ::: "memory");                  // (else all rows are fetched at once, and more is spilled)
+          y[e] = x[e] + take[b][e];
+          q[e] = front[e >> 1].of(sr[(b * 8 + 2 * tig + (e & 1)) * LD + col0 + g + 8 * (e >> 1)]) - more[b][e];
+        }
+        store_tile_rows(block, lay, b * 8, col0, lane, y);
+        store_tile_rows(block, lay, C + b * 8, col0, lane, q);
+        if (b + 1 < NB) below_diagonal(sm.E, sm.G, b, lane, y, take, more);
+        front[0].by(sm.through[b * DIM + col0 + g]), front[1].by(sm.through[b * DIM + col0 + g + 8]);
+      }
+    } else {                             // -F v, then VP; H v and what it gains
+      const int v0 = col0 - DIM;
+      const float* from = row0 + col_v + h * vdim + v0 + g;
+      float v[NB][4];
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int t = b * 8 + 2 * tig + (e & 1);
+          v[b][e] = t < n ? from[(size_t)t * P + 8 * (e >> 1)] : 0.f;
+        }
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        store_tile_columns(block + lay.v(), v0, b, lane, v[b]);
+        on_diagonal(sm.F.on[b], sm.H.on[b], lane, take[b], more[b], [&](int e) { return v[b][e]; });
+        on_diagonal(sm.E.on[b], sm.G.on[b], lane, take[b], more[b], [&](int e) { return take[b][e]; });
+        store_tile_columns(block + lay.vp(), v0, b, lane, take[b]);
+        store_tile_columns(block + lay.op(), v0, b, lane, more[b]);
+        if (b + 1 < NB) {
+          below_diagonal(sm.F, sm.H, b, lane, v[b], take, more);
+          below_diagonal(sm.E, sm.G, b, lane, take[b], take, more);
         }
       }
-    }
-    // (a value column's w is VP = -x from here on)
-    const float sign = key ? -1.f : 1.f;
-    float next = key ? su[c] : 0.f;
-#pragma unroll
-    for (int j = 0; j < C; ++j) {
-      const float y = next + entry(w, j);
-      set_entry(w, j, y);
-      if (j + 1 < C) next = key ? su[(j + 1) * LD + c] : 0.f;
-      add_row<true>(w, sE, j, -y);
-      add_row<false>(o, sG, j, sign * y);
-      asm volatile("" ::: "memory");
-    }
-    if (key) {
-#pragma unroll
-      for (int i = 0; i < C; ++i) set_entry(o, i, sr[i * LD + c] + entry(o, i));
-      store_rows(block, lay, 0, c, w);
-      store_rows(block, lay, C, c, o);
-    } else {
-      store_column(block + lay.vp() + (c - DIM) * C, w);
-      store_column(block + lay.op() + (c - DIM) * C, o);
     }
   }
 }
@@ -531,7 +559,7 @@ GB_EXPORT int gb_gdelta_chunk(const float* proj, int P, int col_r, int col_k, in
   if (PZ < H * dim) return gb::fail(GB_BAD_ARGUMENT, "gdelta_chunk: row widths");
   if ((uintptr_t)blocks & 15) return gb::fail(GB_BAD_ARGUMENT, "gdelta_chunk: blocks start on 16 bytes");
   const int numbers = delta_chunk::chunk_numbers(T, walked);
-  const size_t smem = (size_t)(delta_chunk::C * 4 * (dim + 4 + delta_chunk::LT)) * sizeof(float);
+  const size_t smem = dim == 128 ? sizeof(FactorsSmem<128>) : sizeof(FactorsSmem<64>);
   auto kernel = dim == 128 ? gdelta_chunk_factors_kernel<128> : gdelta_chunk_factors_kernel<64>;
   static gb::OncePerDevice configured[2];
   if (configured[dim == 128].needed()) {
@@ -540,7 +568,7 @@ GB_EXPORT int gb_gdelta_chunk(const float* proj, int P, int col_r, int col_k, in
     configured[dim == 128].done();
   }
   const int rc = gb::check_pdl_launch(
-      gb::launch_pdl(kernel, dim3(numbers, H), dim3(2 * dim), smem, stream, dim3(1, 1, 1), proj, P, col_r, col_k,
+      gb::launch_pdl(kernel, dim3(numbers, H), dim3(256), smem, stream, dim3(1, 1, 1), proj, P, col_r, col_k,
                      col_v, col_a, zdec, PZ, w0, a0, decay_scale, cu_q, blocks, R, H, vdim, cut),
       "gdelta_chunk");
   if (rc != GB_OK) return rc;
