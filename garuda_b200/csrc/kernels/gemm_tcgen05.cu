@@ -36,6 +36,8 @@
 // Rows outside a matrix are zero-filled by TMA and masked in the epilogue; K
 // need not be a multiple of 64 (the tail is zero-filled) but must be a multiple
 // of 8, because a TMA row pitch is a multiple of 16 bytes.
+#include <type_traits>
+
 #include "error_word.cuh"
 #include "tc_common.cuh"
 #include "tc_host.cuh"
@@ -825,54 +827,64 @@ __device__ __forceinline__ void epilogue_tile(uint32_t taddr, int row, int n0, O
     constexpr bool ACC = (EPI & 7) == EPI_ACCUMULATE || EMIT;
     float ssq = 0.f;                                           // EMIT: of the token row0 + lane
     __nv_bfloat16* hbase = EMIT ? ra.h_out + (size_t)row0 * ldo + n0 + lane : nullptr;
-    // the residual of a block is asked for one block ahead; the first block's before the tile's
-    // products have finished (first: the caller's prefetch)
-    float old_cur[ACC ? 32 : 1];
-    auto fetch = [&](float (&dst)[ACC ? 32 : 1], int c) {
+    // WHOLE: all 32 rows are the matrix's. Asking of every row whether it is, and 64-bit products for its address, are most of what
+    // is executed otherwise, and two warps a scheduler hide none of it: 2,048 x 2,048 x 5,632, added to the output, took 39.2 us, now 37.1.
+    auto blocks = [&](auto whole) {
+      constexpr bool WHOLE = decltype(whole)::value;
+      const uint32_t pitch = (uint32_t)ldo * sizeof(OT), hpitch = (uint32_t)ldo * 2;
+      auto at = [&](OT* p, int rr) { return reinterpret_cast<OT*>(reinterpret_cast<char*>(p) + (size_t)rr * pitch); };
+      // the residual of a block is asked for one block ahead; the first block's before the tile's
+      // products have finished (first: the caller's prefetch)
+      float old_cur[ACC ? 32 : 1];
+      auto fetch = [&](float (&dst)[ACC ? 32 : 1], int c) {
+        if (ACC) {
+#pragma unroll
+          for (int rr = 0; rr < 32; ++rr)
+            dst[ACC ? rr : 0] = WHOLE || rr < rows_valid ? gb::to_float<OT>(*at(gbase + c, rr)) : 0.f;
+        }
+      };
       if (ACC) {
 #pragma unroll
-        for (int rr = 0; rr < 32; ++rr)
-          dst[ACC ? rr : 0] = rr < rows_valid ? gb::to_float<OT>(gbase[(size_t)rr * ldo + c]) : 0.f;
+        for (int rr = 0; rr < 32; ++rr) old_cur[ACC ? rr : 0] = first[ACC ? rr : 0];
+      }
+      constexpr int BLOCKS = BN / 32 / (epilogue_warps(EPI) / 4);     // blocks of 32 columns per warp
+      constexpr bool ACT = (EPI & 7) == EPI_STORE && (EPI & EPI_GENERAL) != 0;
+      constexpr int UNROLL = ACC || ACT || !WHOLE ? 1 : BLOCKS;       // the folded norm's work needs the registers, an activation the instruction cache
+#pragma unroll UNROLL
+      for (int k = 0; k < BLOCKS; ++k) {
+        const int c = c_begin + 32 * k;
+        if (c >= c_end) break;
+        uint32_t r[32];
+        tmem_ld_32(taddr + c, r);
+        if (ACC && k > 0) fetch(old_cur, c);
+        tmem_ld_wait();
+        if (ACT) store_act_32(ra, r);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) turn[lane * 33 + j] = __uint_as_float(r[j]);
+        __syncwarp();
+        const float wv = EMIT ? ra.weight[n0 + c + lane] : 0.f;
+#pragma unroll
+        for (int rr = 0; rr < 32; ++rr) {
+          const bool mine = WHOLE || rr < rows_valid;
+          float v = turn[rr * 33 + lane];
+          if (ACC) v = (EPI & EPI_GENERAL) ? fmaf(ra.alpha, v, old_cur[ACC ? rr : 0]) : v + old_cur[ACC ? rr : 0];
+          if (mine) store_value<OT>(at(gbase + c, rr), v);
+          if (EMIT) {
+            // the squares go back the way the values came: each lane then adds up its own token's
+            if (mine) *reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<char*>(hbase + c) + (size_t)rr * hpitch) = __float2bfloat16_rn(v * wv);
+            turn[rr * 33 + lane] = mine ? v * v : 0.f;
+          }
+        }
+        if (EMIT) {
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) ssq += turn[lane * 33 + j];
+        }
+        __syncwarp();
       }
     };
-    if (ACC) {
-#pragma unroll
-      for (int rr = 0; rr < 32; ++rr) old_cur[ACC ? rr : 0] = first[ACC ? rr : 0];
-    }
-    constexpr int BLOCKS = BN / 32 / (epilogue_warps(EPI) / 4);     // blocks of 32 columns per warp
-    constexpr bool ACT = (EPI & 7) == EPI_STORE && (EPI & EPI_GENERAL) != 0;
-    constexpr int UNROLL = ACC || ACT ? 1 : BLOCKS;                // the folded norm's work needs the registers, an activation the instruction cache
-#pragma unroll UNROLL
-    for (int k = 0; k < BLOCKS; ++k) {
-      const int c = c_begin + 32 * k;
-      if (c >= c_end) break;
-      uint32_t r[32];
-      tmem_ld_32(taddr + c, r);
-      if (ACC && k > 0) fetch(old_cur, c);
-      tmem_ld_wait();
-      if (ACT) store_act_32(ra, r);
-#pragma unroll
-      for (int j = 0; j < 32; ++j) turn[lane * 33 + j] = __uint_as_float(r[j]);
-      __syncwarp();
-      const float wv = EMIT ? ra.weight[n0 + c + lane] : 0.f;
-#pragma unroll
-      for (int rr = 0; rr < 32; ++rr) {
-        float v = turn[rr * 33 + lane];
-        if (ACC) v = (EPI & EPI_GENERAL) ? fmaf(ra.alpha, v, old_cur[ACC ? rr : 0]) : v + old_cur[ACC ? rr : 0];
-        if (rr < rows_valid) store_value<OT>(gbase + (size_t)rr * ldo + c, v);
-        if (EMIT) {
-          // the squares go back the way the values came: each lane then adds up its own token's
-          if (rr < rows_valid) hbase[(size_t)rr * ldo + c] = __float2bfloat16_rn(v * wv);
-          turn[rr * 33 + lane] = rr < rows_valid ? v * v : 0.f;
-        }
-      }
-      if (EMIT) {
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < 32; ++j) ssq += turn[lane * 33 + j];
-      }
-      __syncwarp();
-    }
+    if (rows_valid >= 32) blocks(std::true_type{});
+    else blocks(std::false_type{});
     if (EMIT && row < rows_m) ra.sums_out[(size_t)sums_row * ra.sums_ld + row] = ssq;
     return;
   }
@@ -1601,6 +1613,344 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
 }
 
+// --------------------------------------------------------------------------
+// Some hundreds of tokens: too few 128- and 256-row tiles of tokens for the SMs. As in the gated kernel above the weights are the
+// products' rows, 256 a pair of CTAs, and a block of up to 512 tokens their columns; where that makes few pairs, the K range is split
+// over the pairs of a cluster. A lane holds an output feature, so a warp's stores and the residual it adds to are whole 128-byte lines. With
+// a split every pair sends the columns (chunks of 16 tokens, dealt out in turn) that are not its own to their owner, four tokens of a
+// feature at a time, into the pipeline's memory, which is idle once all pairs have passed the cluster's barrier; the owner adds the pairs'
+// sums in their order. No scratch in global memory, no atomics, the same sums every time.
+// What bounds it: the products (a step of 64 channels takes 2 cycles a token and pair) until a token block is narrower than about 300,
+// then what an SM takes in; in front of and behind them 5 to 9 us.
+// 333 tokens, 4,096 features of 14,336 channels: 68 us in 128 x 128 tiles (96 CTAs), 46 here.
+constexpr int T_STAGES = 6, T_TOKENS = 512, T_MAX_SPLIT = 4, T_CHUNK = 16;
+constexpr int T_CHUNK_BYTES = T_CHUNK * BM * 4;
+constexpr int T_PIPE_BYTES = 192 * 1024;
+static_assert((T_MAX_SPLIT - 1) * (T_TOKENS / T_CHUNK / T_MAX_SPLIT) * T_CHUNK_BYTES <= T_PIPE_BYTES, "what an owner receives");
+// A stage: 128 rows of weights, and a CTA's half of every part's tokens.
+__host__ __device__ constexpr int tall_stage_bytes(int part, int parts) { return BM * BK * 2 + parts * part * BK; }
+
+// A block of tokens: `parts` (one or two) products of `part` columns, a multiple of 32; K over `split` pairs.
+struct TallShape {
+  int block, part, parts, split;
+};
+
+__device__ __forceinline__ void st_async_v4(uint32_t remote_addr, uint32_t remote_bar, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2, %3, %4, %5}, [%1];"
+               ::"r"(remote_addr), "r"(remote_bar), "r"(a), "r"(b), "r"(c), "r"(d)
+               : "memory");
+}
+
+// grid (2 split x feature tiles of 256, token blocks), clusters of 2 split CTAs.
+template <int EPI, typename OT>
+__global__ void __launch_bounds__(320, 1)
+gemm_tc_tall_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, OT* __restrict__ out, int ldo, int tokens,
+                    int features, int K, const TallShape sh, int stages, const EpilogueArgs ra) {
+  constexpr bool ROPE = (EPI & 7) == EPI_ROPE, EMIT = (EPI & 7) == EPI_ACCUMULATE_NORM, ADD = (EPI & 7) == EPI_ACCUMULATE || EMIT;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[T_STAGES];
+  __shared__ __align__(8) uint64_t empty_bar[T_STAGES];
+  __shared__ __align__(8) uint64_t acc_full, partial_bar;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int abort_s;
+  __shared__ float inv_s[T_TOKENS];                               // the folded norm's factor per token
+  __shared__ __align__(16) float turn_s[ROPE ? 2 : 1][ROPE ? T_CHUNK * (BM + 4) : 4];      // per set of epilogue warps: a chunk, a row per token
+  __shared__ float red_s[EMIT ? 2 : 1][4][T_CHUNK];
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_ctarank(), pr = rank >> 1, even = rank & ~1;
+  const uint16_t both = (uint16_t)(3u << even);
+  const int m0 = (int)(blockIdx.x / (2 * sh.split)) * (2 * BM) + (rank & 1) * BM;
+  const int tok0 = blockIdx.y * sh.block, ntok = min(sh.block, tokens - tok0);
+  const int total_kb = (K + BK - 1) / BK, per = (total_kb + sh.split - 1) / sh.split;
+  const int kb0 = pr * per, num_kb = min(total_kb, kb0 + per) - kb0;
+  const int stage_bytes = tall_stage_bytes(sh.part, sh.parts);
+  const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const int chunks = (ntok + T_CHUNK - 1) / T_CHUNK, owned_most = (chunks + sh.split - 1) / sh.split;
+  const int owned = pr < chunks ? (chunks - pr + sh.split - 1) / sh.split : 0;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(smem_u32(&full_bar[s]), 1);
+      mbar_init(smem_u32(&empty_bar[s]), 1);
+    }
+    mbar_init(smem_u32(&acc_full), 1);
+    mbar_init(smem_u32(&partial_bar), 1);
+    abort_s = 0;
+    fence_barrier_init();
+    if (sh.split > 1 && owned > 0) mbar_arrive_expect_tx(smem_u32(&partial_bar), (uint32_t)((sh.split - 1) * owned * T_CHUNK_BYTES));
+    fence_proxy_async();
+    prefetch_tensormap(&map_w);
+    prefetch_tensormap(&map_x);
+  }
+  const uint32_t columns = sh.part * sh.parts <= 256 ? 256 : 512;
+  if (warp == 1) {
+    tmem_alloc_pair(smem_u32(&tmem_base_s), columns);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_arrive_wait();        // every CTA's barriers exist before another signals them
+  tc_fence_after_sync();
+  const uint32_t tmem_base = tmem_base_s;
+  volatile int* aborted = &abort_s;
+  gb::pdl_launch_dependents();
+
+  bool have = true;
+  // the epilogue's two sets of four warps take this pair's chunks of 16 tokens in turn; what a chunk is added to is asked for a chunk ahead
+  const int quarter = warp & 3, set = (warp - 2) >> 2, row_in_tile = quarter * 32 + lane, f = m0 + row_in_tile;
+  const uint32_t pitch = (uint32_t)ldo * sizeof(OT);
+  auto at_row = [&](OT* p, int j) { return reinterpret_cast<OT*>(reinterpret_cast<char*>(p) + (size_t)j * pitch); };
+  float old[ADD ? 16 : 1];
+  auto ask = [&](int k) {
+    if (!ADD || k >= owned || f >= features) return;
+    const int j0 = (pr + k * sh.split) * T_CHUNK;
+    OT* from = out + (size_t)(tok0 + j0) * ldo + f;
+    if (j0 + T_CHUNK <= ntok) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) old[ADD ? j : 0] = gb::to_float<OT>(*at_row(from, j));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) old[ADD ? j : 0] = j0 + j < ntok ? gb::to_float<OT>(*at_row(from, j)) : 0.f;
+    }
+  };
+  if (warp == 0) {
+    // -------------------------------------------------------------- producer (every CTA, elect_one's lane)
+    const bool leader = elect_one();
+    gb::pdl_wait();
+    bool ran_out;
+    int s = 0, par = 1, issued = 0;
+    for (int kb = kb0; kb < kb0 + num_kb; ++kb) {
+      if (!mbar_wait_warp(smem_u32(&empty_bar[s]), par, aborted, ran_out)) {
+        if (ran_out) gb_err::report(ERR_WAIT_EMPTY), *aborted = 1;
+        break;
+      }
+      const uint32_t bar = map_to_rank(smem_u32(&full_bar[s]), even);      // the pair's even CTA's barrier
+      const uint32_t base = tiles + s * stage_bytes;
+      if (leader) {
+        if (rank == even) mbar_arrive_expect_tx(smem_u32(&full_bar[s]), 2 * stage_bytes);
+        tma_load_2d_pair(base, &map_w, bar, kb * BK, m0);
+        // this CTA's half of either part's tokens
+        for (int i = 0; i < sh.parts; ++i)
+          tma_load_2d_pair(base + BM * BK * 2 + i * sh.part * BK, &map_x, bar, kb * BK, tok0 + i * sh.part + (rank & 1) * (sh.part / 2));
+      }
+      __syncwarp();
+      ++issued;
+      if (++s == stages) s = 0, par ^= 1;
+    }
+    if (leader && *aborted && issued > 0) {
+      // wind down, as in the pair kernel
+      const unsigned long long t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 2000000ull) {}
+    }
+  } else if (warp == 1) {
+    if (rank == even) {
+      // ------------------------------------------------------------ MMA issuer (even CTAs, elect_one's lane)
+      const uint32_t idesc = instr_desc_bf16(2 * BM, sh.part);
+      const uint64_t da0 = smem_desc_sw128(tiles), db0 = smem_desc_sw128(tiles + BM * BK * 2);
+      const bool leader = elect_one();
+      bool ran_out;
+      int s = 0, par = 0;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait_warp(smem_u32(&full_bar[s]), par, aborted, ran_out)) {
+          if (ran_out) gb_err::report(ERR_WAIT_FULL), *aborted = 1;
+          break;
+        }
+        tc_fence_after_sync();
+        const uint64_t at = (uint64_t)(s * (stage_bytes >> 4));
+        if (leader) {
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k) {
+            mma_bf16_pair(tmem_base, da0 + at + 2 * k, db0 + at + 2 * k, idesc, kb > 0 || k > 0);
+            if (sh.parts == 2) mma_bf16_pair(tmem_base + sh.part, da0 + at + 2 * k, db0 + at + (sh.part * BK >> 4) + 2 * k, idesc, kb > 0 || k > 0);
+          }
+          mma_commit_pair(smem_u32(&empty_bar[s]), both);
+        }
+        __syncwarp();
+        if (++s == stages) s = 0, par ^= 1;
+      }
+      if (leader) mma_commit_pair(smem_u32(&acc_full), both);
+      __syncwarp();
+    }
+  } else {
+    gb::pdl_wait();
+    if (ra.sums_in != nullptr)
+      for (int r = threadIdx.x - 64; r < ntok; r += 256) inv_s[r] = epilogue_row_scale(ra, tok0 + r, tokens);
+    ask(set);
+    have = mbar_wait(smem_u32(&acc_full), 0);
+    if (!have && lane == 0) {
+      gb_err::report(ERR_WAIT_ACCUM);
+      *aborted = 1;
+    }
+  }
+  // all products of the cluster have ended: nothing reads the pipelines' memory any more
+  tc_fence_before_sync();
+  __syncthreads();
+  if (sh.split > 1) cluster_arrive_wait();
+  tc_fence_after_sync();
+  if (warp >= 2) {
+    // -------------------------------------------------------------- epilogue
+    const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    have = have && !*aborted;
+    for (int o = 0; o < sh.split; ++o) {
+      if (o == pr) continue;
+      const uint32_t there = tiles + (uint32_t)((pr < o ? pr : pr - 1) * owned_most * T_CHUNK_BYTES + row_in_tile * 16);
+      const uint32_t remote = map_to_rank(there, 2 * o + (rank & 1)), bar = map_to_rank(smem_u32(&partial_bar), 2 * o + (rank & 1));
+      for (int k = set, c = o + set * sh.split; c < chunks; k += 2, c += 2 * sh.split) {
+        uint32_t r[16];
+        tmem_ld_16(taddr + c * T_CHUNK, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          st_async_v4(remote + k * T_CHUNK_BYTES + q * (BM * 16), bar, r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+      }
+    }
+    float weight = 0.f;
+    if (EMIT && f < features) weight = ra.weight[f];
+    bool waited = sh.split == 1;
+    for (int k = set; k < owned; k += 2) {
+      const int c = pr + k * sh.split, j0 = c * T_CHUNK, t0 = tok0 + j0;
+      const int valid = f < features ? min(T_CHUNK, ntok - j0) : 0;
+      OT* to = out + (size_t)t0 * ldo + f;
+      if (!waited) {
+        const bool got = mbar_wait(smem_u32(&partial_bar), 0);
+        if (!got && lane == 0) gb_err::report(ERR_WAIT_ACCUM);
+        have = have && got;
+        waited = true;
+      }
+      __syncwarp();
+      uint32_t r[16];
+      tmem_ld_16(taddr + j0, r);
+      tmem_ld_wait();
+      float v[16];
+      if (sh.split == 1) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = 0.f;
+        for (int p = 0; p < sh.split; ++p) {
+          if (p == pr) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(r[j]);
+          } else {
+            const float4* src = reinterpret_cast<const float4*>(smem_raw + (tiles - smem_u32(smem_raw)) +
+                                                                ((p < pr ? p : p - 1) * owned_most + k) * T_CHUNK_BYTES) + row_in_tile;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const float4 x = src[q * BM];
+              v[4 * q] += x.x, v[4 * q + 1] += x.y, v[4 * q + 2] += x.z, v[4 * q + 3] += x.w;
+            }
+          }
+        }
+      }
+      if (ra.sums_in != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] *= j0 + j < ntok ? inv_s[j0 + j] : 0.f;
+      }
+      if (ROPE) {
+        // A rotation pairs two features: the chunk goes through shared memory, and a thread takes eight pairs of a token
+        float* rows = turn_s[ROPE ? set : 0];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) rows[j * (BM + 4) + row_in_tile] = v[j];
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + set) : "memory");
+        const int t = row_in_tile >> 3, part = row_in_tile & 7;
+        const int hd = ra.head_dim, half = hd >> 1, dd = part * 8 % half, at = part * 8 / half * hd;
+        const int head = (m0 + at) / hd;
+        if (have && t < ntok - j0 && m0 + at < features) {
+          const int token = t0 + t;
+          const float* row = rows + t * (BM + 4) + at;
+          const bool rotate = ra.cs != nullptr && head < ra.heads + ra.kv_heads;
+          const int first = ra.interleaved ? 2 * dd : dd, second = ra.interleaved ? 2 * dd + 8 : half + dd;
+          float a[8], b[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) a[j] = row[first + j], b[j] = row[second + j];
+          if (rotate) {
+            const float2* cs = ra.cs + (size_t)token * half + dd;
+            if (ra.interleaved) {          // pairs (2i, 2i + 1): four in either piece
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float2 u = cs[i], w = cs[4 + i];
+                const float x = a[2 * i], y = a[2 * i + 1], z = b[2 * i], q = b[2 * i + 1];
+                a[2 * i] = x * u.x - y * u.y, a[2 * i + 1] = x * u.y + y * u.x;
+                b[2 * i] = z * w.x - q * w.y, b[2 * i + 1] = z * w.y + q * w.x;
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const float2 u = cs[j];
+                const float x = a[j], y = b[j];
+                a[j] = x * u.x - y * u.y, b[j] = x * u.y + y * u.x;
+              }
+            }
+          }
+          __nv_bfloat16* dst = rope_destination(ra, token, ra.token_req[token], ra.positions[token], head, 0);
+          if (dst != nullptr) {
+            auto eight = [](__nv_bfloat16* p, const float (&x)[8]) {
+              __nv_bfloat162 h[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
+              uint4 u;
+              u.x = *reinterpret_cast<uint32_t*>(&h[0]), u.y = *reinterpret_cast<uint32_t*>(&h[1]);
+              u.z = *reinterpret_cast<uint32_t*>(&h[2]), u.w = *reinterpret_cast<uint32_t*>(&h[3]);
+              *reinterpret_cast<uint4*>(p) = u;
+            };
+            eight(dst + first, a), eight(dst + second, b);
+          }
+        }
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + set) : "memory");      // before the next chunk reuses the rows
+        continue;
+      }
+      if (ADD) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = (EPI & EPI_GENERAL) ? fmaf(ra.alpha, v[j], old[ADD ? j : 0]) : v[j] + old[ADD ? j : 0];
+        ask(k + 2);
+      } else if (EPI & EPI_GENERAL) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = store_act_fast(ra, v[j]);
+      }
+      // whole chunks without a question a number: two warps a scheduler hide nothing, and what they execute is what the tail takes (512
+      // tokens a CTA: 27,000 cycles with the questions, 8,500 without)
+      if (have && valid == T_CHUNK) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          store_value<OT>(at_row(to, j), v[j]);
+          if (EMIT) ra.h_out[(size_t)(t0 + j) * ldo + f] = __float2bfloat16_rn(v[j] * weight);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (j < valid && have) {
+            store_value<OT>(at_row(to, j), v[j]);
+            if (EMIT) ra.h_out[(size_t)(t0 + j) * ldo + f] = __float2bfloat16_rn(v[j] * weight);
+          } else {
+            v[j] = 0.f;
+          }
+        }
+      }
+      if (EMIT) {
+        // the tile's sum of squares of every token: the four warps' parts in a fixed order
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] *= v[j];
+        const float total = warp_sum16(v, lane);
+        if ((lane & 1) == 0) red_s[EMIT ? set : 0][quarter][warp_sum16_index(lane)] = total;
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + set) : "memory");
+        if (have && row_in_tile < min(T_CHUNK, ntok - j0) && m0 < features) {
+          const float(*red)[T_CHUNK] = red_s[EMIT ? set : 0];
+          ra.sums_out[(size_t)(m0 / BM) * ra.sums_ld + t0 + row_in_tile] =
+              red[0][row_in_tile] + red[1][row_in_tile] + red[2][row_in_tile] + red[3][row_in_tile];
+        }
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + set) : "memory");
+      }
+    }
+  }
+  // No CTA leaves while another's products, copies or partial sums may still touch it.
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_arrive_wait();
+  if (warp == 1) tmem_dealloc_pair(tmem_base, columns);
+}
+
 // ------------------------------------------------------------------ host side
 // How many CTAs of a cluster share K. Measured on B200 (2048- to 5632-wide layers, 8 tokens): a CTA
 // costs about 3.5 us before and after its stream of K blocks and streams one 16 KB block in about
@@ -1781,6 +2131,49 @@ int launch_wide(const CUtensorMap& mw, const CUtensorMap& mx, __nv_bfloat16* out
                               "gemm_tc (wide)");
 }
 
+// Token blocks by 256 features, K over `split` pairs.
+template <int EPI, typename OT>
+int launch_tall(const CUtensorMap& mw, const CUtensorMap& mx, OT* out, int ldo, int tokens, int features, int K, const TallShape& sh,
+                cudaStream_t stream, const EpilogueArgs& ra) {
+  auto kernel = gemm_tc_tall_kernel<EPI, OT>;
+  static gb::OncePerDevice configured;
+  if (configured.needed()) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T_PIPE_BYTES + 1024);
+    if (e != cudaSuccess) return gb::fail(GB_CUDA_ERROR, "gemm_tc: %s", cudaGetErrorString(e));
+    configured.done();
+  }
+  const int fit = T_PIPE_BYTES / tall_stage_bytes(sh.part, sh.parts), stages = fit < T_STAGES ? fit : T_STAGES;
+  const int tiles = (features + 2 * BM - 1) / (2 * BM), blocks = (tokens + sh.block - 1) / sh.block;
+  return gb::check_pdl_launch(gb::launch_pdl(kernel, dim3(2 * sh.split * tiles, blocks), dim3(320), (size_t)T_PIPE_BYTES + 1024, stream,
+                                             dim3(2 * sh.split, 1, 1), mw, mx, out, ldo, tokens, features, K, sh, stages, ra),
+                              "gemm_tc (tall)");
+}
+
+// How many clusters of 2 s CTAs of the kernel above are resident at once (0: they cannot be). Asked once a size.
+int tall_clusters(int s) {
+  static int most[T_MAX_SPLIT + 1] = {};
+  if (most[s] == 0) {
+    auto kernel = gemm_tc_tall_kernel<EPI_STORE, float>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T_PIPE_BYTES + 1024);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * s, 148);
+    cfg.blockDim = dim3(320);
+    cfg.dynamicSmemBytes = T_PIPE_BYTES + 1024;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2 * s; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = -1;
+    }
+    most[s] = n;
+  }
+  return most[s] > 0 ? most[s] : 0;
+}
+
 // Tile width for many tokens: the one that needs fewer rounds over the SMs (a 256-wide tile costs
 // two 128-wide ones but reads each operand half as often); ties go to the wide tile.
 int pick_tile_width(int rows_m, int rows_n) {
@@ -1840,6 +2233,42 @@ bool wide_gated(int tokens, int weight_rows, int K) {
   const int pair_cost = rounds(((tokens + 2 * BM - 1) / (2 * BM)) * ((weight_rows + 255) / 256), pairs) * 32;
   const int one128 = rounds(tiles_m * ((weight_rows + 127) / 128), sms) * 32, one256 = rounds(tiles_m * ((weight_rows + 255) / 256), sms) * 48;
   return wide < steps * pair_cost && wide < steps * one128 && wide < steps * one256;
+}
+
+// Whether a product of some hundreds of tokens takes token blocks by 256 features, and how: cycles of a step of 64 channels times steps, and
+// what comes in front of and behind them, against those of the tiles that it would take otherwise; where it wins by less than a
+// tenth it stays with those. The numbers are fitted to back-to-back products of 257 to 2,048 tokens and 17 shapes (features x channels, us, other
+// tiles against these, 257 / 333 / 512 / 768 / 1,221 / 1,511 tokens): 4,096 x 14,336, 73 / 68 / 66 / 93 / 148 / 156 against 42 / 46 / 54 / 67 /
+// 100 / 118; 2,048 x 5,632, 28 / 28 / 28 / 29 / 34 / 35 against 17 / 18 / 22 / 23 / 27 / 31; where it says no: 6,160 x 2,048, 13.5 / 13.8 / 18.7 /
+// 23.3 against 14.9 / 16.3 / 19.6 / 22.9; 2,304 x 2,048, 13.3 at 768 and 17.2 at 1,221 against 15.0 and 19.4.
+bool tall_plan(int tokens, int features, int K, TallShape* best) {
+  if (tokens <= few_token_limit() || features < 2 * BM) return false;
+  const int sms = sm_count(), pairs = sms / 2, kb = (K + BK - 1) / BK;
+  auto rounds = [](int tiles, int places) { return (long long)((tiles + places - 1) / places); };
+  const int tiles_m = (tokens + BM - 1) / BM;
+  long long cost;
+  if (many_token_pairs(tokens, features)) cost = rounds((tokens + 255) / 256 * ((features + 255) / 256), pairs) * kb * 670 + 12500;
+  else if (pick_tile_width(tokens, features) == 128)
+    cost = rounds(tiles_m * ((features + 127) / 128), sms) * kb * (350 + 600 / tiles_m) + 7700;      // more rows of tiles share what L2 holds
+  else cost = rounds(tiles_m * ((features + 255) / 256), sms) * kb * 900 + 9000;
+  cost = cost * 10 / 11;
+  bool found = false;
+  for (int blocks = (tokens + T_TOKENS - 1) / T_TOKENS, last = blocks + 2; blocks <= last; ++blocks) {
+    TallShape sh;
+    sh.block = (tokens + blocks - 1) / blocks;
+    sh.parts = sh.block > 256 ? 2 : 1;
+    sh.part = ((sh.block + sh.parts - 1) / sh.parts + 31) / 32 * 32;
+    const int cols = sh.part * sh.parts, tiles = (features + 2 * BM - 1) / (2 * BM) * blocks;
+    if (tiles > pairs) break;
+    const int step = sh.parts == 2 ? 115 + cols * 19 / 10 : cols < 184 ? 610 : 260 + cols * 19 / 10;
+    for (sh.split = 1; sh.split <= T_MAX_SPLIT; ++sh.split) {
+      const int per = (kb + sh.split - 1) / sh.split;
+      if ((sh.split - 1) * per >= kb || (sh.split > 1 && tiles > tall_clusters(sh.split))) break;
+      const long long c = (long long)per * step + 12 * cols + (sh.split > 1 ? 11000 + 40 * cols * (sh.split - 1) / sh.split : 12500);
+      if (c < cost) cost = c, *best = sh, found = true;
+    }
+  }
+  return found;
 }
 
 }  // namespace
@@ -1916,8 +2345,9 @@ GB_EXPORT int gb_tc_hint_next_stream(const void* weights, long long bytes) {
 
 // Rows of sums_out that a product of Mx tokens and Nw output features writes when a norm is folded
 // in behind it; 0: this shape does not fold norms.
-GB_EXPORT int gb_gemm_tc_norm_tiles(int Mx, int Nw) {
-  if (Mx <= few_token_limit()) return (Nw + BM - 1) / BM;                   // a row per tile of 128 features
+GB_EXPORT int gb_gemm_tc_norm_tiles(int Mx, int Nw, int K) {
+  TallShape tall;
+  if (Mx <= few_token_limit() || tall_plan(Mx, Nw, K, &tall)) return (Nw + BM - 1) / BM;      // a row per tile of 128 features
   const int width = many_token_width(Mx, Nw);
   return 2 * ((Nw + width - 1) / width);                      // a row per epilogue warp of a lane quarter
 }
@@ -1937,6 +2367,12 @@ GB_EXPORT int gb_gemm_tc_supported(const void* x, const void* w, int Mx, int Nw,
 // act(x w^T); act_second: the second number of an activation that has two (STORE_XIELU).
 // Whether a gated product of `tokens` rows takes the wide tiles.
 GB_EXPORT int gb_gemm_tc_wide(int tokens, int weight_rows, int K) { return wide_gated(tokens, weight_rows, K); }
+
+// Whether another product of `tokens` rows takes token blocks by 256 features, and over how many pairs it splits K (0: it does not).
+GB_EXPORT int gb_gemm_tc_tall(int tokens, int features, int K) {
+  TallShape sh;
+  return tall_plan(tokens, features, K, &sh) ? sh.split : 0;
+}
 
 GB_EXPORT int gb_gemm_tc(const void* x, const void* w, void* out, int Mx, int Nw, int K, int out_dtype, int epi,
                          const GbNormFold* norm, float alpha, int gate_act, float gate_limit, float act_second,
@@ -1976,6 +2412,20 @@ GB_EXPORT int gb_gemm_tc(const void* x, const void* w, void* out, int Mx, int Nw
     if ((rc = tensor_map_2d(x, Mx, K, wide_part(Mx) / 2, &mn))) return rc;
     if (ra.gate_act != GATE_SILU) return launch_wide<EPI_SWIGLU | EPI_GENERAL>(mm, mn, (__nv_bfloat16*)out, Nw, Mx, weight_rows, Nw, K, stream, ra);
     return launch_wide<EPI_SWIGLU>(mm, mn, (__nv_bfloat16*)out, Nw, Mx, weight_rows, Nw, K, stream, ra);
+  }
+  TallShape tall;
+  if ((epi & 7) != EPI_SWIGLU && tall_plan(Mx, Nw, K, &tall)) {
+    if ((rc = tensor_map_2d(w, Nw, K, BM, &mm))) return rc;
+    if ((rc = tensor_map_2d(x, Mx, K, tall.part / 2, &mn))) return rc;
+    if ((epi & 7) == EPI_ACCUMULATE && ra.h_out != nullptr)
+      return launch_tall<EPI_ACCUMULATE_NORM>(mm, mn, (float*)out, Nw, Mx, Nw, K, tall, stream, ra);
+    if ((epi & 7) == EPI_ACCUMULATE && ra.alpha != 1.0f)
+      return launch_tall<EPI_ACCUMULATE | EPI_GENERAL>(mm, mn, (float*)out, Nw, Mx, Nw, K, tall, stream, ra);
+    if ((epi & 7) == EPI_ACCUMULATE) return launch_tall<EPI_ACCUMULATE>(mm, mn, (float*)out, Nw, Mx, Nw, K, tall, stream, ra);
+    if (ra.gate_act >= STORE_RELU2)
+      return launch_tall<EPI_STORE | EPI_GENERAL>(mm, mn, (__nv_bfloat16*)out, Nw, Mx, Nw, K, tall, stream, ra);
+    if (out_dtype == GB_F32) return launch_tall<EPI_STORE>(mm, mn, (float*)out, Nw, Mx, Nw, K, tall, stream, ra);
+    return launch_tall<EPI_STORE>(mm, mn, (__nv_bfloat16*)out, Nw, Mx, Nw, K, tall, stream, ra);
   }
   if ((rc = tensor_map_2d(x, Mx, K, BM, &mm))) return rc;
   const bool pairs = many_token_pairs(Mx, weight_rows, epi);
@@ -2089,6 +2539,12 @@ GB_EXPORT int gb_gemm_tc_qkv(const void* x, const void* w, int Mx, int K, void* 
     if (bn == 16) return launch_cluster<16, EPI_ROPE, __nv_bfloat16>(mm, mn, none, 0, Nw, Nw, Mx, K, stream, ra);
     if (bn == 32) return launch_cluster<32, EPI_ROPE, __nv_bfloat16>(mm, mn, none, 0, Nw, Nw, Mx, K, stream, ra);
     return launch_cluster<64, EPI_ROPE, __nv_bfloat16>(mm, mn, none, 0, Nw, Nw, Mx, K, stream, ra);
+  }
+  TallShape tall;
+  if (tall_plan(Mx, Nw, K, &tall)) {
+    if ((rc = tensor_map_2d(w, Nw, K, BM, &mm))) return rc;
+    if ((rc = tensor_map_2d(x, Mx, K, tall.part / 2, &mn))) return rc;
+    return launch_tall<EPI_ROPE>(mm, mn, none, 0, Mx, Nw, K, tall, stream, ra);
   }
   if ((rc = tensor_map_2d(x, Mx, K, BM, &mm))) return rc;
   if (many_token_pairs(Mx, Nw)) {

@@ -439,20 +439,20 @@ class CudaOps:
         _need(a.is_contiguous() and w.is_contiguous() and out.is_contiguous(), "linear: operands must be contiguous")
         _need(accumulate or alpha == 1.0, "linear: a multiplier goes with accumulation only")
         if self.tc is not None and a.dtype == torch.bfloat16:
-            pending = self._pending_for(ctx, emit_norm, out, accumulate) if alpha == 1.0 else None
+            pending = self._pending_for(ctx, emit_norm, out, K, accumulate) if alpha == 1.0 else None
             if self.tc.linear(a, w, out, accumulate, emit=pending, alpha=alpha):
                 return pending
         self._check(self.core, self.core.gb_gemm_simple(
             a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, _tag(a, "linear input"),
             _tag(out, "linear output"), int(accumulate), float(alpha), self._stream()), "linear")
 
-    def _pending_for(self, ctx, norm, x, accumulate):
+    def _pending_for(self, ctx, norm, x, inner, accumulate):
         """A ``PendingNorm`` with buffers for the product that adds into ``x``, or None."""
         if norm is None or ctx is None or not accumulate or x.dtype != torch.float32:
             return None
         fold = norm.fold() if hasattr(norm, "fold") else None
         T, d = x.shape
-        tiles = self.tc.norm_tiles(T, d)
+        tiles = self.tc.norm_tiles(T, d, inner)
         if fold is None or not tiles:
             return None
         weight, eps = fold

@@ -39,7 +39,9 @@ class TensorCoreKernels:
         L.gb_gemm_tc_grouped.restype = c_int
         L.gb_gemm_tc_wide.argtypes = [c_int] * 3
         L.gb_gemm_tc_wide.restype = c_int
-        L.gb_gemm_tc_norm_tiles.argtypes = [c_int, c_int]
+        L.gb_gemm_tc_tall.argtypes = [c_int] * 3
+        L.gb_gemm_tc_tall.restype = c_int
+        L.gb_gemm_tc_norm_tiles.argtypes = [c_int] * 3
         L.gb_gemm_tc_norm_tiles.restype = c_int
         L.gb_gemm_tc_supported.argtypes = [c_void_p, c_void_p, c_int, c_int, c_int]
         L.gb_gemm_tc_supported.restype = c_int
@@ -91,10 +93,10 @@ class TensorCoreKernels:
                         "selftest_wait_runs_out")
 
     # ------------------------------------------------------------------ folded norms
-    def norm_tiles(self, tokens: int, features: int) -> int:
+    def norm_tiles(self, tokens: int, features: int, inner: int) -> int:
         """Rows of partial sums that an accumulating product of this shape writes when the norm
         behind it is folded in; 0: it folds none."""
-        return int(self.lib.gb_gemm_tc_norm_tiles(tokens, features))
+        return int(self.lib.gb_gemm_tc_norm_tiles(tokens, features, inner))
 
     @staticmethod
     def _consume(pending):

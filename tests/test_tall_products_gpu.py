@@ -1,0 +1,115 @@
+"""Products of some hundreds of tokens in token blocks by 256 features with K split over a cluster's pairs, against plain 32-bit
+products: one and two parts a block, one and several blocks, every split, features that fill no pair of CTAs, a K that is no multiple of
+a step, and each epilogue (stored, added, added with the next norm folded in, rotated into pages)."""
+import pytest
+import torch
+
+from tests.gpu_helpers import close, rnd
+
+pytestmark = pytest.mark.gpu
+
+# tokens, features, K
+SHAPES = [(257, 264, 2048), (333, 4096, 4104), (384, 1000, 2048), (511, 2048, 5632), (512, 18560, 4096), (513, 2048, 5632), (1030, 4096, 2048),
+          (1221, 4096, 2048), (300, 288, 2040)]
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from garuda_b200.kernels.ops import CudaOps
+    torch.backends.cuda.matmul.allow_tf32 = False
+    return CudaOps("cuda:0", tensor_cores=True)
+
+
+def operands(M, N, K, seed=0):
+    a = rnd(M, K, scale=0.5, seed=seed).cuda().bfloat16()
+    w = rnd(N, K, scale=K ** -0.5, seed=seed + 1).cuda().bfloat16()
+    return a, w, a.float() @ w.float().T
+
+
+def test_the_shapes_take_the_kernel(ops):
+    splits = [ops.tc.lib.gb_gemm_tc_tall(*s) for s in SHAPES]
+    assert min(splits) > 0 and len(set(splits)) >= 3, splits
+    assert ops.tc.lib.gb_gemm_tc_tall(256, 4096, 4096) == 0 and ops.tc.lib.gb_gemm_tc_tall(4096, 4096, 4096) == 0
+
+
+# 32-bit sums of K products of either sign: the order moves them by some units of 2^-24 times sqrt(K)
+@pytest.mark.parametrize("M,N,K", SHAPES)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_stored(ops, M, N, K, dtype):
+    a, w, want = operands(M, N, K)
+    out = torch.full((M, N), float("nan"), dtype=dtype, device="cuda")
+    ops.linear(a, w, out=out)
+    close(out, want.cpu(), dtype, "stored", tol=3e-5 if dtype == torch.float32 else None)
+
+
+@pytest.mark.parametrize("M,N,K", SHAPES)
+@pytest.mark.parametrize("alpha", [1.0, 0.37])
+def test_added(ops, M, N, K, alpha):
+    a, w, want = operands(M, N, K, seed=3)
+    out = rnd(M, N, seed=9).cuda()
+    want = out + alpha * want
+    ops.linear(a, w, out=out, accumulate=True, alpha=alpha)
+    close(out, want.cpu(), torch.float32, "added", tol=3e-5)
+
+
+def test_the_same_bits_every_time(ops):
+    a, w, _ = operands(333, 4096, 14336, seed=5)
+    assert ops.tc.lib.gb_gemm_tc_tall(333, 4096, 14336) > 1
+    outs = [torch.empty(333, 4096, device="cuda") for _ in range(3)]
+    for o in outs:
+        ops.linear(a, w, out=o)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("T,Hq,Hkv,hd,d", [(448, 32, 8, 128, 4096), (300, 4, 2, 64, 2048), (513, 6, 1, 32, 2048), (1030, 12, 2, 16, 2048)])
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_rotated_into_pages(ops, T, Hq, Hkv, hd, d, interleaved):
+    from garuda_b200.engine.batch import Workspace
+    from garuda_b200.parts.rotary import RotaryParams
+    from tests.plain.cpu_ops import CpuOps
+    N, page = (Hq + 2 * Hkv) * hd, 8
+    assert ops.tc.lib.gb_gemm_tc_tall(T, N, d) > 0
+
+    class Ctx:
+        ws = Workspace("cuda:0")
+
+    h, w, _ = operands(T, N, d, seed=7)
+    h, w = h.cpu(), w.cpu()
+    req = torch.tensor([i % 3 for i in range(T)], dtype=torch.int32).sort().values
+    positions = torch.cat([s + torch.arange(int((req == r).sum())) for r, s in enumerate((0, 37, 100))]).to(torch.int32)
+    width = int(positions.max()) // page + 2
+    pages = torch.randperm(3 * width, generator=torch.Generator().manual_seed(T)).int().view(3, width)
+    for rotary in (RotaryParams(10000.0, hd, interleaved), None):
+        want = [torch.zeros(T, Hq, hd), torch.zeros(3 * width, Hkv, page, hd), torch.zeros(3 * width, Hkv, page, hd)]
+        CpuOps().qkv_rope_append(None, h, w, *want, positions, req, pages, Hq, Hkv, hd, rotary, page)
+        got = [torch.zeros_like(t, dtype=torch.bfloat16, device="cuda") for t in want]
+        ops.qkv_rope_append(Ctx, h.cuda(), w.cuda(), *got, positions.cuda(), req.cuda(), pages.cuda(), Hq, Hkv, hd, rotary, page)
+        for a, b, what in zip(got, want, "qkv"):
+            close(a, b, torch.bfloat16, what)
+
+
+@pytest.mark.parametrize("M,d,K", [(300, 2048, 5632), (1221, 4096, 2048), (333, 1000, 2048)])
+def test_norm_folded_in(ops, M, d, K):
+    from garuda_b200.engine.batch import StepContext, Workspace
+    from garuda_b200.parts.norm import RMSNorm
+    assert ops.tc.lib.gb_gemm_tc_tall(M, d, K) > 0
+    a, w, want = operands(M, d, K, seed=11)
+    x = (rnd(M, d, seed=12) * (1 + torch.arange(M) % 5).float()[:, None]).cuda()      # a token's sums are not another's
+    gamma = (1 + 0.3 * rnd(d, seed=13)).bfloat16().cuda()
+    norm = RMSNorm(d, 1e-3)
+    norm.load({"weight": gamma}, ops, torch.bfloat16)
+    ctx = StepContext(batch=None, ws=Workspace("cuda:0"), ops=ops, dtype=torch.bfloat16)
+    res = x.clone()
+    pending = ops.linear(a, w, res, accumulate=True, ctx=ctx, emit_norm=norm)
+    want = x + want
+    close(res, want.cpu(), torch.float32, "residual", tol=3e-5)
+    close(pending.values, (want * gamma.float()).cpu(), torch.bfloat16, "x * weight")
+    torch.testing.assert_close(pending.sums.sum(0), (want ** 2).sum(1), rtol=1e-4, atol=1e-6)
+    # and products behind it, which scale their results by 1/rms
+    v = (rnd(4096, d, seed=14) * d ** -0.5).bfloat16().cuda()
+    out = torch.empty(M, 4096 // 2, dtype=torch.bfloat16, device="cuda")
+    ops.linear_swiglu(ctx, pending, ops.pack_gate_up(v[:2048], v[2048:]), out)
+    h = want * torch.rsqrt((want ** 2).mean(1, keepdim=True) + 1e-3) * gamma.float()
+    g, u = h @ v[:2048].float().T, h @ v[2048:].float().T
+    close(out, (torch.nn.functional.silu(g) * u).cpu(), torch.bfloat16, "gate/up behind it")
+    ops.tc.check_errors()
