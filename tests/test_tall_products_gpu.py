@@ -61,7 +61,7 @@ def test_the_same_bits_every_time(ops):
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
 
 
-@pytest.mark.parametrize("T,Hq,Hkv,hd,d", [(448, 32, 8, 128, 4096), (300, 4, 2, 64, 2048), (513, 6, 1, 32, 2048), (1030, 12, 2, 16, 2048)])
+@pytest.mark.parametrize("T,Hq,Hkv,hd,d", [(448, 32, 8, 128, 4096), (300, 4, 2, 64, 4096), (513, 6, 1, 32, 4096), (1030, 12, 2, 16, 4096)])
 @pytest.mark.parametrize("interleaved", [False, True])
 def test_rotated_into_pages(ops, T, Hq, Hkv, hd, d, interleaved):
     from garuda_b200.engine.batch import Workspace
