@@ -62,22 +62,23 @@ __device__ __forceinline__ void store_pair(__nv_bfloat16* to, float a, float b) 
 
 // 1 / d and z / d, rounded, of a d from 1 to infinity (the denominators of sigmoid and SiLU), without a branch, so that a thread's many
 // stand beside one another: Newton's step from the hardware's approximation, then Markstein's correction of the quotient ("Computation of
-// elementary functions on the IBM RISC System/6000 processor", 1990). Operands are a quarter of what they were meanwhile, so that no
-// reciprocal of a finite number is subnormal. The rounded quotient's bits wherever z, d and the result are normal and d is at most 2^126;
-// infinities and what is not a number come out as in a division.
-__device__ __forceinline__ float over(float d) {
-  const float y = 0.25f * d;
+// elementary functions on the IBM RISC System/6000 processor", 1990). The approximation is asked for at an eighth of d, where neither it nor
+// its operand is subnormal; the steps are at d itself, so that a result which is subnormal is rounded once. `over` gives the division's bits for every d up to
+// 2^126 and for all but five beyond (which are a last place off); `divide` gives them for every z over 1 + exp(-z) (small z meet d = 2),
+// and for other z and d where z is at least 2^-100 and the result is normal.
+__device__ __forceinline__ float over_first(float d) {
   float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(y));
-  return 0.25f * (d < INFINITY ? fmaf(r, fmaf(-y, r, 1.0f), r) : r);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(0.125f * d));
+  return 0.125f * r;
+}
+__device__ __forceinline__ float over(float d) {
+  const float a = over_first(d);
+  return d < INFINITY ? fmaf(a, fmaf(-d, a, 1.0f), a) : a;
 }
 __device__ __forceinline__ float divide(float z, float d) {
-  const float y = 0.25f * d, x = 0.25f * z;
-  float a;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(a) : "f"(y));
-  const float r = fmaf(a, fmaf(-y, a, 1.0f), a), q = x * r;
-  const float better = fmaf(fmaf(-q, y, x), r, q);
-  return d < INFINITY && fabsf(better) < INFINITY ? better : x * a;
+  const float a = over_first(d), r = fmaf(a, fmaf(-d, a, 1.0f), a), q = z * r;
+  const float better = fmaf(fmaf(-q, d, z), r, q);
+  return copysignf(d < INFINITY && fabsf(better) < INFINITY ? better : z * a, z);      // (a zero's sign is lost on the way)
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

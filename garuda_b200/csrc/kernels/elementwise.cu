@@ -30,6 +30,14 @@ __global__ void embedding_kernel(const T* __restrict__ table, const int32_t* __r
   }
 }
 
+__global__ void divisions_kernel(const float* __restrict__ z, const float* __restrict__ d, float* __restrict__ quotient,
+                                 float* __restrict__ reciprocal, long long n) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  quotient[i] = gb::divide(z[i], d[i]);
+  reciprocal[i] = gb::over(d[i]);
+}
+
 // logits <- logits * scale, then (cap > 0) cap * tanh(logits / cap); in place, 32-bit
 __global__ void scale_softcap_kernel(float* __restrict__ x, long long n, float scale, float cap) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -450,6 +458,14 @@ GB_EXPORT int gb_embedding_copies(const void* table, int table_dtype, const int3
 GB_EXPORT int gb_embedding(const void* table, int table_dtype, const int32_t* ids, float* out, int T,
                            int d, int vocab, float scale, cudaStream_t stream) {
   return gb_embedding_copies(table, table_dtype, ids, out, T, d, vocab, scale, 1, stream);
+}
+
+// For tests of the divisions without a branch (common.cuh): quotient = z / d and reciprocal = 1 / d of n numbers, d from 1 on.
+GB_EXPORT int gb_selftest_divisions(const float* z, const float* d, float* quotient, float* reciprocal, long long n, cudaStream_t stream) {
+  if (n <= 0) return GB_OK;
+  if (n > 0x7fffffffLL) return gb::fail(GB_BAD_ARGUMENT, "selftest_divisions: %lld numbers", n);
+  divisions_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(z, d, quotient, reciprocal, n);
+  return gb::check_launch("selftest_divisions");
 }
 
 GB_EXPORT int gb_scale_softcap(float* x, long long n, float scale, float cap, cudaStream_t stream) {

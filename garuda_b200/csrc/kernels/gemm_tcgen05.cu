@@ -213,21 +213,11 @@ __device__ __forceinline__ void store_value<float>(float* p, float v) { *p = v; 
 template <>
 __device__ __forceinline__ void store_value<__nv_bfloat16>(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 
-// 1 / x, rounded, of an x from 1 to infinity, without a branch: one step of Newton's iteration from the hardware's
-// approximation (x a quarter of what it was meanwhile, so that no reciprocal of a finite number is subnormal): the bits of __frcp_rn for
-// every x up to 2^126 (all compared); beyond, where reciprocals are subnormal, one in five is a last place off. With __frcp_rn, whose
-// branch keeps 64 reciprocals a thread in a row, the gated epilogue of a 128 x 256 tile took 15,500 cycles, now 5,300.
-__device__ __forceinline__ float rounded_reciprocal(float x) {
-  const float y = 0.25f * x;
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(y));
-  return 0.25f * (x < INFINITY ? fmaf(r, fmaf(-y, r, 1.0f), r) : r);
-}
-
 // The SiLU-gate of the fused epilogues. The exponential is the hardware's fast one: its error
-// (about 2 ulp of a float) is far below the rounding of the bfloat16 result.
+// (about 2 ulp of a float) is far below the rounding of the bfloat16 result. gb::over has no branch: with __frcp_rn, whose
+// branch keeps 64 reciprocals a thread in a row, the gated epilogue of a 128 x 256 tile took 15,500 cycles, now 5,300.
 __device__ __forceinline__ float silu_gate_fast(float g, float u) {
-  return g * rounded_reciprocal(1.0f + __expf(-g)) * u;
+  return g * gb::over(1.0f + __expf(-g)) * u;
 }
 
 // The gated epilogues' activation, chosen at run time (uniform over the launch). tanh through the
@@ -236,12 +226,12 @@ __device__ __forceinline__ float gate_fast(const EpilogueArgs& ra, float g, floa
   if (ra.gate_act == GATE_SILU) return silu_gate_fast(g, u);
   if (ra.gate_act == GATE_GELU_TANH) {
     const float z = 0.7978845608028654f * (g + 0.044715f * g * g * g);
-    const float th = 1.0f - 2.0f * rounded_reciprocal(__expf(2.0f * z) + 1.0f);
+    const float th = 1.0f - 2.0f * gb::over(__expf(2.0f * z) + 1.0f);
     return 0.5f * g * (1.0f + th) * u;
   }
   g = fminf(g, ra.gate_limit);
   u = fminf(fmaxf(u, -ra.gate_limit), ra.gate_limit);
-  return g * rounded_reciprocal(1.0f + __expf(-1.702f * g)) * (u + 1.0f);
+  return g * gb::over(1.0f + __expf(-1.702f * g)) * (u + 1.0f);
 }
 
 // The exact gelu, z Phi(z). The complementary error function by formula 7.1.26 of Abramowitz and Stegun's "Handbook of
@@ -269,7 +259,7 @@ __device__ __forceinline__ float store_act_fast(const EpilogueArgs& ra, float z)
     return z > 0.f ? fmaf(ra.gate_limit * z, z, half) : fmaf(ra.act_second, __expf(z) - 1.0f - z, half);
   }
   if (ra.gate_act == STORE_GELU) return gelu_fast(z);
-  return 1.0f - 2.0f * rounded_reciprocal(__expf(2.0f * z) + 1.0f);
+  return 1.0f - 2.0f * gb::over(__expf(2.0f * z) + 1.0f);
 }
 
 // The same for a whole tile's 32 columns of a thread: the kind is looked at once, not per value.
@@ -286,7 +276,7 @@ __device__ __forceinline__ void store_act_32(const EpilogueArgs& ra, uint32_t (&
   } else if (ra.gate_act == STORE_XIELU) {
     GB_EACH(z > 0.f ? fmaf(ra.gate_limit * z, z, 0.5f * z) : fmaf(ra.act_second, __expf(z) - 1.0f - z, 0.5f * z))
   } else {
-    GB_EACH(1.0f - 2.0f * rounded_reciprocal(__expf(2.0f * z) + 1.0f))
+    GB_EACH(1.0f - 2.0f * gb::over(__expf(2.0f * z) + 1.0f))
   }
 #undef GB_EACH
 }

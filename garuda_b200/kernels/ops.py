@@ -131,6 +131,7 @@ class CudaOps:
         sig = {
             "gb_embedding": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p],
             "gb_embedding_copies": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int, c_void_p],
+            "gb_selftest_divisions": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p],
             "gb_scale_softcap": [c_void_p, c_longlong, c_float, c_float, c_void_p],
             "gb_layernorm": [c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p],
             "gb_dynamic_tanh": [c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p],
@@ -400,6 +401,15 @@ class CudaOps:
         self._check(self.core, self.core.gb_embedding_copies(
             table.data_ptr(), _tag(table, "embedding table"), ids.data_ptr(), out.data_ptr(), T,
             table.shape[1], table.shape[0], float(scale), int(copies), self._stream()), "embedding")
+
+    def selftest_divisions(self, z, d):
+        """``(z / d, 1 / d)`` as the kernels' sigmoid and SiLU take them (32-bit, ``d`` from 1 on)."""
+        self._on_device(z, d)
+        _need(z.dtype == d.dtype == torch.float32 and z.is_contiguous() and d.is_contiguous() and z.shape == d.shape, "selftest_divisions: operands")
+        quotient, reciprocal = torch.empty_like(z), torch.empty_like(z)
+        self._check(self.core, self.core.gb_selftest_divisions(z.data_ptr(), d.data_ptr(), quotient.data_ptr(), reciprocal.data_ptr(), z.numel(),
+                                                               self._stream()), "selftest_divisions")
+        return quotient, reciprocal
 
     def scale_softcap(self, x, scale: float = 1.0, cap: float = 0.0):
         """``x <- x * scale``, then with ``cap`` > 0 ``x <- cap * tanh(x / cap)``; in place, 32-bit."""
