@@ -36,6 +36,7 @@
 // Rows outside a matrix are zero-filled by TMA and masked in the epilogue; K
 // need not be a multiple of 64 (the tail is zero-filled) but must be a multiple
 // of 8, because a TMA row pitch is a multiple of 16 bytes.
+#include <atomic>
 #include <type_traits>
 
 #include "error_word.cuh"
@@ -2139,10 +2140,13 @@ int launch_tall(const CUtensorMap& mw, const CUtensorMap& mx, OT* out, int ldo, 
                               "gemm_tc (tall)");
 }
 
-// How many clusters of 2 s CTAs of the kernel above are resident at once (0: they cannot be). Asked once a size.
+// How many clusters of 2 s CTAs of the kernel above are resident at once (0: they cannot be). Asked once a size and device; an answer that
+// could not be had is not kept.
 int tall_clusters(int s) {
-  static int most[T_MAX_SPLIT + 1] = {};
-  if (most[s] == 0) {
+  static std::atomic<int> kept[gb::OncePerDevice::MAX_DEVICES][T_MAX_SPLIT + 1];      // one more than the answer (0: not asked)
+  const int device = gb::OncePerDevice::device();
+  const int known = device >= 0 ? kept[device][s].load(std::memory_order_relaxed) : 0;
+  if (known == 0) {
     auto kernel = gemm_tc_tall_kernel<EPI_STORE, float>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T_PIPE_BYTES + 1024);
     cudaLaunchConfig_t cfg = {};
@@ -2155,13 +2159,14 @@ int tall_clusters(int s) {
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
       cudaGetLastError();
-      n = -1;
+      return 0;
     }
-    most[s] = n;
+    if (device >= 0) kept[device][s].store(n + 1, std::memory_order_relaxed);
+    return n;
   }
-  return most[s] > 0 ? most[s] : 0;
+  return known - 1;
 }
 
 // Tile width for many tokens: the one that needs fewer rounds over the SMs (a 256-wide tile costs
@@ -2294,8 +2299,9 @@ GB_EXPORT int gb_tc_selftest_wait_runs_out(int limit_us, cudaStream_t stream) {
 
 // An RMS norm folded into the products around it (see EpilogueArgs). As the consumer: sums_in
 // [tiles_in, sums_ld] and eps, inv_width = 1 / features of the normed vector. As the producer
-// (accumulating products only): h_out [Mx, Nw] bfloat16, weight [Nw] 32-bit, sums_out
-// [gb_gemm_tc_norm_tiles(Mx, Nw), sums_ld]. Unused halves are null.
+// (accumulating products only): h_out [Mx, Nw] bfloat16, weight [Nw] 32-bit, sums_out [tiles_out, sums_ld] with
+// tiles_out = gb_gemm_tc_norm_tiles(Mx, Nw, K): all of its rows are written, and a product that would write
+// another number of them is refused. Unused halves are null.
 struct GbNormFold {
   const float* sums_in;
   int tiles_in;
@@ -2304,6 +2310,7 @@ struct GbNormFold {
   const float* weight;
   float* sums_out;
   int sums_ld;
+  int tiles_out;
 };
 
 namespace {
@@ -2333,13 +2340,19 @@ GB_EXPORT int gb_tc_hint_next_stream(const void* weights, long long bytes) {
   return GB_OK;
 }
 
-// Rows of sums_out that a product of Mx tokens and Nw output features writes when a norm is folded
+namespace {
+int norm_tiles(int Mx, int Nw, bool tall) {
+  if (Mx <= few_token_limit() || tall) return (Nw + BM - 1) / BM;      // a row per tile of 128 features
+  const int width = many_token_width(Mx, Nw);
+  return 2 * ((Nw + width - 1) / width);                      // a row per epilogue warp of a lane quarter
+}
+}  // namespace
+
+// Rows of sums_out that a product of Mx tokens, Nw output features and K channels writes when a norm is folded
 // in behind it; 0: this shape does not fold norms.
 GB_EXPORT int gb_gemm_tc_norm_tiles(int Mx, int Nw, int K) {
   TallShape tall;
-  if (Mx <= few_token_limit() || tall_plan(Mx, Nw, K, &tall)) return (Nw + BM - 1) / BM;      // a row per tile of 128 features
-  const int width = many_token_width(Mx, Nw);
-  return 2 * ((Nw + width - 1) / width);                      // a row per epilogue warp of a lane quarter
+  return norm_tiles(Mx, Nw, Mx > few_token_limit() && tall_plan(Mx, Nw, K, &tall));
 }
 
 // Whether gb_gemm_tc takes this problem (else the caller uses the plain kernel).
@@ -2349,12 +2362,6 @@ GB_EXPORT int gb_gemm_tc_supported(const void* x, const void* w, int Mx, int Nw,
   return 1;
 }
 
-// epi 0: out[Mx,Nw] = x w^T (out_dtype f32 or bf16); 1: out (f32) += x w^T;
-// 2: w holds gate and up rows packed in groups of 64 ([128 * ceil(Nw / 64), K], see the head of this
-// file); out[Mx,Nw] (bf16) = act(x gate^T, x up^T), act by gate_act: silu(g) u unless told otherwise.
-// alpha: the accumulating epilogue adds alpha * product. gate_act, gate_limit: the gated epilogue's
-// activation (GateAct), or with epi 0 and a bfloat16 output STORE_RELU2 / STORE_TANH / STORE_XIELU / STORE_GELU: out =
-// act(x w^T); act_second: the second number of an activation that has two (STORE_XIELU).
 // Whether a gated product of `tokens` rows takes the wide tiles.
 GB_EXPORT int gb_gemm_tc_wide(int tokens, int weight_rows, int K) { return wide_gated(tokens, weight_rows, K); }
 
@@ -2364,6 +2371,12 @@ GB_EXPORT int gb_gemm_tc_tall(int tokens, int features, int K) {
   return tall_plan(tokens, features, K, &sh) ? sh.split : 0;
 }
 
+// epi 0: out[Mx,Nw] = x w^T (out_dtype f32 or bf16); 1: out (f32) += x w^T;
+// 2: w holds gate and up rows packed in groups of 64 ([128 * ceil(Nw / 64), K], see the head of this
+// file); out[Mx,Nw] (bf16) = act(x gate^T, x up^T), act by gate_act: silu(g) u unless told otherwise.
+// alpha: the accumulating epilogue adds alpha * product. gate_act, gate_limit: the gated epilogue's
+// activation (GateAct), or with epi 0 and a bfloat16 output STORE_RELU2 / STORE_TANH / STORE_XIELU / STORE_GELU: out =
+// act(x w^T); act_second: the second number of an activation that has two (STORE_XIELU).
 GB_EXPORT int gb_gemm_tc(const void* x, const void* w, void* out, int Mx, int Nw, int K, int out_dtype, int epi,
                          const GbNormFold* norm, float alpha, int gate_act, float gate_limit, float act_second,
                          cudaStream_t stream) {
@@ -2387,6 +2400,11 @@ GB_EXPORT int gb_gemm_tc(const void* x, const void* w, void* out, int Mx, int Nw
   ra.act_second = act_second;
   if (ra.h_out != nullptr && (epi & 7) != EPI_ACCUMULATE)
     return gb::fail(GB_UNSUPPORTED, "gemm_tc: a norm is folded in behind accumulating products only (epilogue %d)", epi);
+  TallShape tall;
+  const bool takes_tall = (epi & 7) != EPI_SWIGLU && tall_plan(Mx, Nw, K, &tall);
+  if (ra.h_out != nullptr && norm->tiles_out != norm_tiles(Mx, Nw, takes_tall))
+    return gb::fail(GB_BAD_ARGUMENT, "gemm_tc: %d rows of sums for the norm behind, the product writes %d", norm->tiles_out,
+                    norm_tiles(Mx, Nw, takes_tall));
   CUtensorMap mm, mn;
   int rc;
   if (Mx <= few_token_limit()) {
@@ -2403,8 +2421,7 @@ GB_EXPORT int gb_gemm_tc(const void* x, const void* w, void* out, int Mx, int Nw
     if (ra.gate_act != GATE_SILU) return launch_wide<EPI_SWIGLU | EPI_GENERAL>(mm, mn, (__nv_bfloat16*)out, Nw, Mx, weight_rows, Nw, K, stream, ra);
     return launch_wide<EPI_SWIGLU>(mm, mn, (__nv_bfloat16*)out, Nw, Mx, weight_rows, Nw, K, stream, ra);
   }
-  TallShape tall;
-  if ((epi & 7) != EPI_SWIGLU && tall_plan(Mx, Nw, K, &tall)) {
+  if (takes_tall) {
     if ((rc = tensor_map_2d(w, Nw, K, BM, &mm))) return rc;
     if ((rc = tensor_map_2d(x, Mx, K, tall.part / 2, &mn))) return rc;
     if ((epi & 7) == EPI_ACCUMULATE && ra.h_out != nullptr)

@@ -22,7 +22,7 @@ _WAIT_NAMES = {1: "an operand tile never arrived (TMA)", 2: "a pipeline stage wa
 class NormFold(ctypes.Structure):
     """GbNormFold of gemm_tcgen05.cu: an RMS norm folded into the products around it."""
     _fields_ = [("sums_in", c_void_p), ("tiles_in", c_int), ("eps", c_float), ("inv_width", c_float),
-                ("h_out", c_void_p), ("weight", c_void_p), ("sums_out", c_void_p), ("sums_ld", c_int)]
+                ("h_out", c_void_p), ("weight", c_void_p), ("sums_out", c_void_p), ("sums_ld", c_int), ("tiles_out", c_int)]
 
 
 class TensorCoreKernels:
@@ -166,7 +166,7 @@ class TensorCoreKernels:
         fold = None
         if emit is not None:
             fold = NormFold(h_out=emit.values.data_ptr(), weight=emit.weight.data_ptr(),
-                            sums_out=emit.sums.data_ptr(), sums_ld=emit.sums.shape[1])
+                            sums_out=emit.sums.data_ptr(), sums_ld=emit.sums.shape[1], tiles_out=emit.sums.shape[0])
         return self._gemm(a, w, out, w.shape[0], 1 if accumulate else 0, fold, alpha=alpha)
 
     STORE_ACTS = {"relu2": 3, "tanh": 4, "gelu": 6}

@@ -113,3 +113,18 @@ def test_norm_folded_in(ops, M, d, K):
     g, u = h @ v[:2048].float().T, h @ v[2048:].float().T
     close(out, (torch.nn.functional.silu(g) * u).cpu(), torch.bfloat16, "gate/up behind it")
     ops.tc.check_errors()
+
+
+@pytest.mark.parametrize("M,N,K", [(333, 4096, 14336), (2048, 2048, 2048), (8, 2048, 2048)])
+def test_sums_of_another_size_are_refused(ops, M, N, K):
+    """The rows of the sums for the norm behind follow from the kernel that is chosen: room for another number is an error, not a write beyond it."""
+    from garuda_b200.kernels.ops import KernelError, PendingNorm
+    rows = ops.tc.norm_tiles(M, N, K)
+    a, w, _ = operands(M, N, K)
+    for n in (rows - 1, rows + 1):
+        out = torch.zeros(M, N, device="cuda")
+        pending = PendingNorm(torch.zeros(M, N, dtype=torch.bfloat16, device="cuda"), torch.zeros(rows + 1, M, device="cuda")[:n],
+                              torch.ones(N, device="cuda"), 1e-5, None, out)
+        with pytest.raises(KernelError, match="rows of sums"):
+            ops.tc.linear(a, w, out, True, emit=pending)
+        assert not out.any() and not pending.sums.any()
