@@ -1607,8 +1607,8 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 // --------------------------------------------------------------------------
 // Some hundreds of tokens: too few 128- and 256-row tiles of tokens for the SMs. As in the gated kernel above the weights are the
 // products' rows, 256 a pair of CTAs, and a block of up to 512 tokens their columns; where that makes few pairs, the K range is split
-// over the pairs of a cluster. A lane holds an output feature, so a warp's stores and the residual it adds to are whole 128-byte lines. With
-// a split every pair sends the columns (chunks of 16 tokens, dealt out in turn) that are not its own to their owner, four tokens of a
+// over the pairs of a cluster. A lane holds an output feature, so a warp's 32-bit stores and the residual it adds to are whole 128-byte lines (bfloat16
+// stores half lines). With a split every pair sends the columns (chunks of 16 tokens, dealt out in turn) that are not its own to their owner, four tokens of a
 // feature at a time, into the pipeline's memory, which is idle once all pairs have passed the cluster's barrier; the owner adds the pairs'
 // sums in their order. No scratch in global memory, no atomics, the same sums every time.
 // What bounds it: the products (a step of 64 channels takes 2 cycles a token and pair) until a token block is narrower than about 300,
@@ -2230,23 +2230,42 @@ bool wide_gated(int tokens, int weight_rows, int K) {
   return wide < steps * pair_cost && wide < steps * one128 && wide < steps * one256;
 }
 
+// Whether the rotating product's tiles of a pair of CTAs are 320 wide (two products a step, about 1.4 times a 256-wide tile's time): where that
+// saves a round over the pairs. 2,048 tokens times 2,560 features are 80 tiles of 256 columns for 74 pairs, but 64 of 320.
+bool rotates_320(int tokens, int features, int head_dim) {
+  const int most = sm_count() / 2, tiles_m = (tokens + 2 * BM - 1) / (2 * BM);
+  const int rounds256 = (tiles_m * ((features + 255) / 256) + most - 1) / most;
+  const int rounds320 = (tiles_m * ((features + 319) / 320) + most - 1) / most;
+  return 320 % head_dim == 0 && rounds320 * 14 < rounds256 * 10;
+}
+
 // Whether a product of some hundreds of tokens takes token blocks by 256 features, and how: cycles of a step of 64 channels times steps, and
 // what comes in front of and behind them, against those of the tiles that it would take otherwise; where it wins by less than a
 // tenth it stays with those. The numbers are fitted to back-to-back products of 257 to 2,048 tokens and 17 shapes (features x channels, us, other
 // tiles against these, 257 / 333 / 512 / 768 / 1,221 / 1,511 tokens): 4,096 x 14,336, 73 / 68 / 66 / 93 / 148 / 156 against 42 / 46 / 54 / 67 /
 // 100 / 118; 2,048 x 5,632, 28 / 28 / 28 / 29 / 34 / 35 against 17 / 18 / 22 / 23 / 27 / 31; where it says no: 6,160 x 2,048, 13.5 / 13.8 / 18.7 /
 // 23.3 against 14.9 / 16.3 / 19.6 / 22.9; 2,304 x 2,048, 13.3 at 768 and 17.2 at 1,221 against 15.0 and 19.4.
-bool tall_plan(int tokens, int features, int K, TallShape* best) {
+// head_dim above 0: the rotating product, whose epilogue weighs more in every kernel and which has tiles of 320 columns to go to. us, other
+// tiles against these: 2,560 x 2,048, 19.7 / 28.5 / 34.5 / 34.5 / 45.4 at 512 / 1,024 / 1,793 / 2,048 / 2,400 tokens against 15.9 / 24.2 / 30.3 /
+// 34.3 / 34.2 (2,048 stays with the 320-wide tiles, as does 2,300, 34.7 against 36.0); 6,144 x 4,096, 44 / 72 / 76 at 512 / 1,024 / 1,221
+// against 34 / 54 / 67, where it says no: 73 against 80 at 1,511; 1,536 x 2,048, 34.7 against 41.5 at 3,500, no either.
+bool tall_plan(int tokens, int features, int K, TallShape* best, int head_dim = 0) {
   if (tokens <= few_token_limit() || features < 2 * BM) return false;
   const int sms = sm_count(), pairs = sms / 2, kb = (K + BK - 1) / BK;
+  const bool rotates = head_dim > 0;
   auto rounds = [](int tiles, int places) { return (long long)((tiles + places - 1) / places); };
   const int tiles_m = (tokens + BM - 1) / BM;
   long long cost;
-  if (many_token_pairs(tokens, features)) cost = rounds((tokens + 255) / 256 * ((features + 255) / 256), pairs) * kb * 670 + 12500;
-  else if (pick_tile_width(tokens, features) == 128)
-    cost = rounds(tiles_m * ((features + 127) / 128), sms) * kb * (350 + 600 / tiles_m) + 7700;      // more rows of tiles share what L2 holds
-  else cost = rounds(tiles_m * ((features + 255) / 256), sms) * kb * 900 + 9000;
-  cost = cost * 10 / 11;
+  if (many_token_pairs(tokens, features)) {
+    if (rotates && rotates_320(tokens, features, head_dim)) cost = rounds((tokens + 255) / 256 * ((features + 319) / 320), pairs) * (kb * 940 + 23000) + 12500;
+    else cost = rounds((tokens + 255) / 256 * ((features + 255) / 256), pairs) * (kb * 670 + (rotates ? 20000 : 0)) + 12500;
+    if (rotates) cost = cost * 19 / 20;
+  } else if (pick_tile_width(tokens, features) == 128) {           // more rows of tiles share what L2 holds
+    cost = rounds(tiles_m * ((features + 127) / 128), sms) * (kb * (350 + 600 / tiles_m) + (rotates ? 10000 : 0)) + 7700;
+  } else {
+    cost = rounds(tiles_m * ((features + 255) / 256), sms) * (kb * 900 + (rotates ? 18000 : 0)) + 9000;
+  }
+  if (!rotates) cost = cost * 10 / 11;
   bool found = false;
   for (int blocks = (tokens + T_TOKENS - 1) / T_TOKENS, last = blocks + 2; blocks <= last; ++blocks) {
     TallShape sh;
@@ -2259,7 +2278,10 @@ bool tall_plan(int tokens, int features, int K, TallShape* best) {
     for (sh.split = 1; sh.split <= T_MAX_SPLIT; ++sh.split) {
       const int per = (kb + sh.split - 1) / sh.split;
       if ((sh.split - 1) * per >= kb || (sh.split > 1 && tiles > tall_clusters(sh.split))) break;
-      const long long c = (long long)per * step + 12 * cols + (sh.split > 1 ? 11000 + 40 * cols * (sh.split - 1) / sh.split : 12500);
+      const int sent = sh.split > 1 ? 40 * cols * (sh.split - 1) / sh.split : 0;
+      // (a rotating product's constants are fitted by themselves)
+      const long long c = rotates ? (long long)per * step * 6 / 5 + 12 * cols + 68 * cols / sh.split + (sh.split > 1 ? 6500 : 8000) + sent
+                                  : (long long)per * step + 12 * cols + (sh.split > 1 ? 11000 : 12500) + sent;
       if (c < cost) cost = c, *best = sh, found = true;
     }
   }
@@ -2365,10 +2387,15 @@ GB_EXPORT int gb_gemm_tc_supported(const void* x, const void* w, int Mx, int Nw,
 // Whether a gated product of `tokens` rows takes the wide tiles.
 GB_EXPORT int gb_gemm_tc_wide(int tokens, int weight_rows, int K) { return wide_gated(tokens, weight_rows, K); }
 
-// Whether another product of `tokens` rows takes token blocks by 256 features, and over how many pairs it splits K (0: it does not).
+// Whether another product of `tokens` rows takes token blocks by 256 features, and over how many pairs it splits K (0: it does not); the
+// same of the product that rotates heads of head_dim.
 GB_EXPORT int gb_gemm_tc_tall(int tokens, int features, int K) {
   TallShape sh;
   return tall_plan(tokens, features, K, &sh) ? sh.split : 0;
+}
+GB_EXPORT int gb_gemm_tc_tall_rotating(int tokens, int features, int K, int head_dim) {
+  TallShape sh;
+  return head_dim >= 16 && 128 % head_dim == 0 && tall_plan(tokens, features, K, &sh, head_dim) ? sh.split : 0;
 }
 
 // epi 0: out[Mx,Nw] = x w^T (out_dtype f32 or bf16); 1: out (f32) += x w^T;
@@ -2548,20 +2575,14 @@ GB_EXPORT int gb_gemm_tc_qkv(const void* x, const void* w, int Mx, int K, void* 
     return launch_cluster<64, EPI_ROPE, __nv_bfloat16>(mm, mn, none, 0, Nw, Nw, Mx, K, stream, ra);
   }
   TallShape tall;
-  if (tall_plan(Mx, Nw, K, &tall)) {
+  if (tall_plan(Mx, Nw, K, &tall, head_dim)) {
     if ((rc = tensor_map_2d(w, Nw, K, BM, &mm))) return rc;
     if ((rc = tensor_map_2d(x, Mx, K, tall.part / 2, &mn))) return rc;
     return launch_tall<EPI_ROPE>(mm, mn, none, 0, Mx, Nw, K, tall, stream, ra);
   }
   if ((rc = tensor_map_2d(x, Mx, K, BM, &mm))) return rc;
   if (many_token_pairs(Mx, Nw)) {
-    // 320-wide tiles (two products a step, about 1.4 times a 256-wide tile's time) where they save a
-    // round over the pairs: 2,048 tokens times 2,560 features are 80 tiles of 256 columns for 74 pairs,
-    // but 64 of 320
-    const int most = sm_count() / 2, tiles_m = (Mx + 2 * BM - 1) / (2 * BM);
-    const int rounds256 = (tiles_m * ((Nw + 255) / 256) + most - 1) / most;
-    const int rounds320 = (tiles_m * ((Nw + 319) / 320) + most - 1) / most;
-    if (320 % head_dim == 0 && rounds320 * 14 < rounds256 * 10) {
+    if (rotates_320(Mx, Nw, head_dim)) {
       if ((rc = tensor_map_2d(w, Nw, K, PairGeometry<320>::BOX_ROWS, &mn))) return rc;
       return launch_pair<320, EPI_ROPE, __nv_bfloat16>(mm, mn, none, 0, Mx, Nw, Nw, K, stream, ra);
     }

@@ -41,6 +41,8 @@ class TensorCoreKernels:
         L.gb_gemm_tc_wide.restype = c_int
         L.gb_gemm_tc_tall.argtypes = [c_int] * 3
         L.gb_gemm_tc_tall.restype = c_int
+        L.gb_gemm_tc_tall_rotating.argtypes = [c_int] * 4
+        L.gb_gemm_tc_tall_rotating.restype = c_int
         L.gb_gemm_tc_norm_tiles.argtypes = [c_int] * 3
         L.gb_gemm_tc_norm_tiles.restype = c_int
         L.gb_gemm_tc_supported.argtypes = [c_void_p, c_void_p, c_int, c_int, c_int]

@@ -32,6 +32,14 @@ def test_the_shapes_take_the_kernel(ops):
     assert ops.tc.lib.gb_gemm_tc_tall(256, 4096, 4096) == 0 and ops.tc.lib.gb_gemm_tc_tall(4096, 4096, 4096) == 0
 
 
+def test_the_rotating_product_goes_where_it_is_faster(ops):
+    """Its epilogue weighs more in these blocks than in the tiles that it would take otherwise, 320 wide ones among them."""
+    takes = lambda T, N, K, hd: ops.tc.lib.gb_gemm_tc_tall_rotating(T, N, K, hd) > 0
+    assert all(takes(*c) for c in [(257, 1536, 2048, 64), (1793, 2560, 2048, 64), (2400, 2560, 2048, 64), (1221, 6144, 4096, 128)])
+    others = [(2048, 2560, 2048, 64), (2300, 2560, 2048, 64), (1511, 6144, 4096, 128), (3500, 1536, 2048, 64)]
+    assert not any(takes(*c) for c in others) and all(ops.tc.lib.gb_gemm_tc_tall(*c[:3]) > 0 for c in others)
+
+
 # 32-bit sums of K products of either sign: the order moves them by some units of 2^-24 times sqrt(K)
 @pytest.mark.parametrize("M,N,K", SHAPES)
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
@@ -68,7 +76,7 @@ def test_rotated_into_pages(ops, T, Hq, Hkv, hd, d, interleaved):
     from garuda_b200.parts.rotary import RotaryParams
     from tests.plain.cpu_ops import CpuOps
     N, page = (Hq + 2 * Hkv) * hd, 8
-    assert ops.tc.lib.gb_gemm_tc_tall(T, N, d) > 0
+    assert ops.tc.lib.gb_gemm_tc_tall_rotating(T, N, d, hd) > 0
 
     class Ctx:
         ws = Workspace("cuda:0")
