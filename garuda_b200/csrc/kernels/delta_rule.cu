@@ -265,7 +265,8 @@ delta_recurrence_kernel(const float* __restrict__ prep, int W, const int32_t* __
 template <int DIM>
 struct FactorsSmem {
   delta_chunk::Lower L, B;
-  // [tokens][DIM + 8] each. k and q: then decayed on from their block's start; g: decays, keys decayed on to their block's end, values
+  // [tokens][DIM + 8] each. k and q: then decayed on from their block's start; g: decays (kept_decay), keys decayed on to their block's end,
+  // values
   float k[delta_chunk::C * (DIM + 8)], q[delta_chunk::C * (DIM + 8)], g[delta_chunk::C * (DIM + 8)];
   float2 through[delta_chunk::NB * DIM];         // whole blocks' decays (delta_chunk::Product)
   float beta[delta_chunk::C];
@@ -337,7 +338,7 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
   if (per_head) {
     // one decay for all key channels: every thread's warp makes one token's at a time
     for (int t = warp; t < C; t += 8) {
-      const float g = t < n ? expf(-rate * softplus(second[(size_t)(first + t) * P2 + h] + gb::to_float<WT>(dt_bias[h]))) : 1.f;
+      const float g = t < n ? kept_decay(-rate * softplus(second[(size_t)(first + t) * P2 + h] + gb::to_float<WT>(dt_bias[h]))) : 0.f;
       for (int d = lane; d < DIM; d += 32) sg[t * LD + d] = g;
     }
   } else {
@@ -347,7 +348,7 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
 #pragma unroll 4
     for (int t = tid / DIM; t < C; t += 256 / DIM) {
       float* a = sg + t * LD + tid % DIM;
-      *a = t < n ? expf(-rate * softplus(*a + bias)) : 1.f;
+      *a = t < n ? kept_decay(-rate * softplus(*a + bias)) : 0.f;
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -373,10 +374,12 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
 #pragma unroll
     for (int e = 0; e < VEC; ++e) x[e] = v[lane + 32 * e], ss = fmaf(x[e], x[e], ss);
     ss = gb::warp_sum(ss);
-    float inv = 1.0f / sqrtf(ss + 1e-6f);
-    if (row < C) inv *= 1.0f / sqrtf((float)DIM);
+    // queries over the root of DIM as well: of 64 an eighth, of 128 a sixteenth times the root of two
+    const bool query = row < C;
+    const float2 inv = one_over_root((ss + 1e-6f) * (query && DIM == 128 ? 0.5f : 1.f));
+    const float by = query ? (DIM == 128 ? 0.0625f : 0.125f) : 1.f;
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) v[lane + 32 * e] = x[e] * inv;
+    for (int e = 0; e < VEC; ++e) v[lane + 32 * e] = by * fmaf(x[e], inv.x, x[e] * inv.y);
   }
   __syncthreads();
   {
@@ -390,6 +393,11 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
       } else {
         x[0] = *reinterpret_cast<const pair_t*>(m + i * LD + d0);
       }
+    };
+    auto decays = [&](int i, pair_t (&x)[VEC / 2]) {
+      row(sg, i, x);
+#pragma unroll
+      for (int e = 0; e < VEC / 2; ++e) x[e] = make_pair(rounded_decay(both(x[e]).x), rounded_decay(both(x[e]).y));
     };
     auto dot = [](const pair_t (&a)[VEC / 2], const pair_t (&b)[VEC / 2]) {
       pair_t s = mul2(a[0], b[0]);
@@ -413,7 +421,7 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
     for (int ii = 0; ii < 4; ++ii) {       // the tokens of the four keys themselves
       const int i = j0 + ii;
       pair_t g[VEC / 2], k[VEC / 2], q[VEC / 2];
-      row(sg, i, g), row(sk, i, k), row(sq, i, q);
+      decays(i, g), row(sk, i, k), row(sq, i, q);
       float v[8];
 #pragma unroll
       for (int jj = 0; jj < 4; ++jj) {
@@ -427,7 +435,7 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
 #pragma unroll 2
     for (int i = j0 + 4; i < j1; ++i) {
       pair_t g[VEC / 2], k[VEC / 2], q[VEC / 2];
-      row(sg, i, g), row(sk, i, k), row(sq, i, q);
+      decays(i, g), row(sk, i, k), row(sq, i, q);
       float v[8];
 #pragma unroll
       for (int jj = 0; jj < 4; ++jj) {
@@ -449,7 +457,7 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
     Product on, behind;
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
-      on.by(g[t]);
+      on.by(whole_decay(g[t]));
       sq[at0 + t * LD] = on.of(sq[at0 + t * LD]);
       sk[at0 + t * LD] = on.of(k[t]);
     }
@@ -457,7 +465,7 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
 #pragma unroll
     for (int t = 7; t >= 0; --t) {
       sg[at0 + t * LD] = behind.of(k[t]);
-      behind.by(g[t]);
+      behind.by(whole_decay(g[t]));
     }
   }
   __syncthreads();

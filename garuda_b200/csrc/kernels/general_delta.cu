@@ -199,7 +199,7 @@ template <int DIM>
 struct FactorsSmem {
   delta_chunk::Lower E, F, G, H;
   // [tokens][DIM + 8] each: u and r, then decayed on from their block's start (u up to the token in front of it); alpha and k, then decayed on
-  // to their block's end; decays
+  // to their block's end; decays (kept_decay)
   float u[delta_chunk::C * (DIM + 8)], r[delta_chunk::C * (DIM + 8)], a[delta_chunk::C * (DIM + 8)], k[delta_chunk::C * (DIM + 8)],
       w[delta_chunk::C * (DIM + 8)];
   float2 through[delta_chunk::NB * DIM];         // whole blocks' decays (delta_chunk::Product)
@@ -255,7 +255,7 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
       const float u = k[e] * inv;
       su[d] = u;
       sa[d] = t < n ? sigmoid(sa[d] + rate[e]) * u : 0.f;
-      sw[d] = t < n ? expf(-decay_scale * sigmoid(sw[d] + decay[e])) : 1.f;
+      sw[d] = t < n ? kept_decay(-decay_scale * sigmoid(sw[d] + decay[e])) : 0.f;
       if (t >= n) sk[d] = sr[d] = 0.f;
     }
   }
@@ -271,6 +271,11 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
       } else {
         x[0] = *reinterpret_cast<const pair_t*>(m + i * LD + d0);
       }
+    };
+    auto decays = [&](int i, pair_t (&x)[VEC / 2]) {
+      row(sw, i, x);
+#pragma unroll
+      for (int e = 0; e < VEC / 2; ++e) x[e] = make_pair(rounded_decay(both(x[e]).x), rounded_decay(both(x[e]).y));
     };
     auto dot = [](const pair_t (&a)[VEC / 2], const pair_t (&b)[VEC / 2]) {
       pair_t s = mul2(a[0], b[0]);
@@ -291,7 +296,7 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
     for (int ii = 0; ii < 4; ++ii) {       // the tokens of the four keys themselves
       const int i = j0 + ii;
       pair_t w[VEC / 2], u[VEC / 2], x[VEC / 2];
-      row(sw, i, w), row(su, i, u), row(sr, i, x);
+      decays(i, w), row(su, i, u), row(sr, i, x);
       row(sa, i, pa[ii]), row(sk, i, pk[ii]);
       float before[8], after[8];
 #pragma unroll
@@ -307,7 +312,7 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
     }
     for (int i = j0 + 4; i < j1; ++i) {
       pair_t w[VEC / 2], u[VEC / 2], x[VEC / 2];
-      row(sw, i, w), row(su, i, u), row(sr, i, x);
+      decays(i, w), row(su, i, u), row(sr, i, x);
       float before[8], after[8];
 #pragma unroll
       for (int jj = 0; jj < 4; ++jj) {
@@ -330,14 +335,14 @@ gdelta_chunk_factors_kernel(const float* __restrict__ proj, int P, int col_r, in
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
       su[at0 + t * LD] = on.of(su[at0 + t * LD]);
-      on.by(w[t]);
+      on.by(whole_decay(w[t]));
       sr[at0 + t * LD] = on.of(sr[at0 + t * LD]);
     }
     sm.through[i] = on.both();
 #pragma unroll
     for (int t = 7; t >= 0; --t) {
       sa[at0 + t * LD] = behind.of(sa[at0 + t * LD]), sk[at0 + t * LD] = behind.of(sk[at0 + t * LD]);
-      behind.by(w[t]);
+      behind.by(whole_decay(w[t]));
     }
   }
   __syncthreads();

@@ -267,3 +267,56 @@ def test_as_near_64_bits_as_the_walk_token_by_token(ops, rule, dim, decay):
         o = ctx.ws._views["gdelta_o" if rule == "general" else "delta_o"][2]
         off.append([((x.double().flatten() - y.flatten()).norm() / y.norm()).item() for x, y in zip((o, state[:, :H * dim * vdim]), ref)])
     assert all(chunk <= 1.2 * token for token, chunk in zip(*off)), f"read-outs, state: token by token {off[0]}, by chunks {off[1]}"
+
+
+@pytest.mark.parametrize("rule,dim,decay,most", [
+    # decays that keep thousands of tokens: the chunks hold what a decay lacks of one, the walk the decay rounded to 24 bits
+    ("channel", 128, -8.0, 0.4), ("head", 64, -8.0, 0.4), ("general", 64, -8.0, 0.4), ("general", 128, -8.0, 0.4),
+    # decays that keep some tens of tokens: sums and triangular systems of 32 tokens may not be rounded further off than the walk's steps (the mean
+    # of six draws of 262,144 numbers: two kernels of one precision differ by a hundredth)
+    ("channel", 128, -3.0, 1.01), ("head", 128, -3.0, 1.01)])
+def test_readouts_no_further_from_64_bits_than_the_walk_token_by_token(ops, rule, dim, decay, most):
+    cuda, _ = ops
+    H, G, T, taps = 4, 2, 512, 4
+    off = torch.zeros(2)
+    for seed in range(6):
+        g = torch.Generator(device="cuda").manual_seed(100 * dim + seed)
+        draw = lambda *s, std=1.0, mean=0.0: torch.randn(*s, generator=g, device="cuda") * std + mean
+        if rule == "general":
+            HD = H * dim
+            cols = (0, HD, 2 * HD, 3 * HD, 4 * HD)
+            args, width = [draw(T, 5 * HD), cols, draw(T, HD), draw(HD, mean=decay), draw(HD), 0.6], HD * dim
+            ref = _general64(*args, H, dim, dim)[0]
+        else:
+            C, n_decay, width = (2 * G + H) * dim, H if rule == "head" else H * dim, H * dim * dim + (taps - 1) * (2 * G + H) * dim
+            args = [draw(T, C + H), draw(T, n_decay + H * dim), draw(C, taps, std=0.5), draw(H, std=0.3), draw(n_decay, std=0.3, mean=decay)]
+            ref = _gated64(*args, H, G, dim, dim, taps, rule == "head")[0]
+        for i, dt in enumerate((torch.float32, torch.bfloat16)):
+            ctx, _ = batches(step([T], [0]))
+            state, out = torch.zeros(1, width, device="cuda"), torch.zeros(T, H * dim, dtype=dt, device="cuda")
+            if rule == "general":
+                cuda.general_delta(ctx, *args, torch.ones(H * dim, device="cuda"), 1e-5, state, H, dim, dim, out)
+            else:
+                cuda.delta_rule(ctx, *args, torch.ones(dim, device="cuda"), 1e-5, state, H, G, dim, dim, taps, out, decay_per_head=rule == "head")
+            o = ctx.ws._views["gdelta_o" if rule == "general" else "delta_o"][2]
+            off[i] += ((o.double().flatten() - ref.flatten()).norm() / ref.norm()).item()
+    assert off[1] <= most * off[0], f"token by token {off[0] / 6:.3e}, by chunks {off[1] / 6:.3e}"
+
+
+def test_a_state_that_grows(ops):
+    """The generalized rule takes any scale: a negative one makes the state grow."""
+    cuda, cpu = ops
+    H, dim, vdim, T = 2, 64, 64, 150
+    HD = H * dim
+    cols = (0, HD, 2 * HD, 3 * HD, 4 * HD)
+    args = [rnd(T, 5 * HD, scale=0.5), cols, rnd(T, HD, seed=1), rnd(HD, seed=2) - 3.0, rnd(HD, seed=3), -0.2, rnd(HD, seed=4)]
+    to = lambda v: v.cuda() if torch.is_tensor(v) else v
+    state = rnd(1, HD * vdim, seed=6)
+    got, want = state.cuda(), state.clone()
+    out, ref = torch.zeros(T, HD, dtype=torch.bfloat16, device="cuda"), torch.zeros(T, HD, dtype=torch.bfloat16)
+    ctx_g, ctx_r = batches(step([T], [0]))
+    cuda.general_delta(ctx_g, *map(to, args), 1e-5, got, H, dim, vdim, out)
+    cpu.general_delta(ctx_r, *args, 1e-5, want, H, dim, vdim, ref)
+    assert "delta_blocks" in ctx_g.ws._bufs
+    close(out, ref, torch.bfloat16, "outputs")
+    close(got, want, torch.float32, "state", tol=2e-5)
