@@ -1,6 +1,7 @@
 """Products of some hundreds of tokens in token blocks by 256 features with K split over a cluster's pairs, against plain 32-bit
-products: one and two parts a block, one and several blocks, every split, features that fill no pair of CTAs, a K that is no multiple of
-a step, and each epilogue (stored, added, added with the next norm folded in, rotated into pages)."""
+products: one and two parts a block, one and several blocks, every split from one to four, features that fill no pair of CTAs, a K that is no
+multiple of a step, and each epilogue: stored, stored through each activation, added, added with the next norm folded in, rotated into
+pages, and rotated behind a folded norm."""
 import pytest
 import torch
 
@@ -10,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 # tokens, features, K
 SHAPES = [(257, 264, 2048), (333, 4096, 4104), (384, 1000, 2048), (511, 2048, 5632), (512, 18560, 4096), (513, 2048, 5632), (1030, 4096, 2048),
-          (1221, 4096, 2048), (300, 288, 2040)]
+          (1221, 4096, 2048), (300, 288, 2040), (270, 2500, 4104), (2262, 700, 4096)]
 
 
 @pytest.fixture(scope="module")
@@ -28,7 +29,7 @@ def operands(M, N, K, seed=0):
 
 def test_the_shapes_take_the_kernel(ops):
     splits = [ops.tc.lib.gb_gemm_tc_tall(*s) for s in SHAPES]
-    assert min(splits) > 0 and len(set(splits)) >= 3, splits
+    assert set(splits) == {1, 2, 3, 4}, splits
     assert ops.tc.lib.gb_gemm_tc_tall(256, 4096, 4096) == 0 and ops.tc.lib.gb_gemm_tc_tall(4096, 4096, 4096) == 0
 
 
@@ -67,6 +68,26 @@ def test_the_same_bits_every_time(ops):
     for o in outs:
         ops.linear(a, w, out=o)
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+# one part and two, each split
+@pytest.mark.parametrize("M,N,K", [(300, 288, 2040), (270, 2500, 4104), (511, 2048, 5632), (1221, 4096, 2048)])
+@pytest.mark.parametrize("kind", ["relu2", "tanh", "gelu", "xielu"])
+def test_stored_through_an_activation(ops, M, N, K, kind):
+    from tests.plain.cpu_ops import CpuOps
+    assert ops.tc.lib.gb_gemm_tc_tall(M, N, K) > 0
+    a, w, want = operands(M, N, K, seed=17)
+    out = torch.full((M + 1, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    want, ref = want.cpu(), torch.empty(M, N)
+    if kind == "xielu":
+        assert ops.tc.linear_xielu(a, w, out[:M], 0.8, 1.3)
+        CpuOps().xielu(want, ref, 0.8, 1.3)
+    else:
+        assert ops.tc.linear_act(a, w, out[:M], kind)
+        ref = {"relu2": torch.relu(want) ** 2, "tanh": torch.tanh(want), "gelu": torch.nn.functional.gelu(want)}[kind]
+    ops.tc.check_errors()
+    close(out[:M], ref, torch.bfloat16, kind)
+    assert out[M].isnan().all(), "a store beyond the tokens"
 
 
 @pytest.mark.parametrize("T,Hq,Hkv,hd,d", [(448, 32, 8, 128, 4096), (300, 4, 2, 64, 4096), (513, 6, 1, 32, 4096), (1030, 12, 2, 16, 4096)])
@@ -136,3 +157,36 @@ def test_sums_of_another_size_are_refused(ops, M, N, K):
         with pytest.raises(KernelError, match="rows of sums"):
             ops.tc.linear(a, w, out, True, emit=pending)
         assert not out.any() and not pending.sums.any()
+
+
+# split in one, two and four; one block of tokens and several
+@pytest.mark.parametrize("T,Hq,Hkv,hd,d", [(448, 32, 8, 128, 4096), (300, 4, 2, 64, 4096), (1030, 12, 2, 16, 4096), (900, 32, 8, 128, 4096)])
+def test_rotated_behind_a_folded_norm(ops, T, Hq, Hkv, hd, d):
+    """Each token at a scale of its own, which the norm takes out: the factors must be the tokens' own."""
+    from garuda_b200.engine.batch import StepContext, Workspace
+    from garuda_b200.parts.norm import RMSNorm
+    from garuda_b200.parts.rotary import RotaryParams
+    from tests.plain.cpu_ops import CpuOps
+    N, page = (Hq + 2 * Hkv) * hd, 8
+    assert ops.tc.lib.gb_gemm_tc_tall_rotating(T, N, d, hd) > 0
+    g = torch.Generator(device="cuda").manual_seed(T)
+    a, w_o = (torch.randn(T, 128, generator=g, device="cuda") * 0.5).bfloat16(), (torch.randn(d, 128, generator=g, device="cuda") * 0.1).bfloat16()
+    norm = RMSNorm(d, 1e-3)
+    norm.load({"weight": (1 + 0.3 * torch.randn(d, generator=g, device="cuda")).bfloat16()}, ops, torch.bfloat16)
+    ctx = StepContext(batch=None, ws=Workspace("cuda:0"), ops=ops, dtype=torch.bfloat16)
+    res = torch.randn(T, d, generator=g, device="cuda") * (1 + torch.arange(T, device="cuda") % 5)[:, None]
+    pending = ops.linear(a, w_o, res, accumulate=True, ctx=ctx, emit_norm=norm)
+    assert pending is not None
+    h = pending.values.float() * torch.rsqrt((res ** 2).mean(1, keepdim=True) + 1e-3)      # (32-bit rows in the reference)
+    w = (torch.randn(N, d, generator=g, device="cuda") * d ** -0.5).bfloat16()
+    req = torch.zeros(T, dtype=torch.int32)
+    positions, width = torch.arange(T, dtype=torch.int32) + 19, (T + 19) // page + 1
+    pages = torch.randperm(width, generator=torch.Generator().manual_seed(T)).int().view(1, width)
+    rotary = RotaryParams(10000.0, hd, False)
+    want = [torch.zeros(T, Hq, hd), torch.zeros(width, Hkv, page, hd), torch.zeros(width, Hkv, page, hd)]
+    CpuOps().qkv_rope_append(None, h.cpu(), w.float().cpu(), *want, positions, req, pages, Hq, Hkv, hd, rotary, page)
+    got = [torch.zeros_like(t, dtype=torch.bfloat16, device="cuda") for t in want]
+    ops.qkv_rope_append(ctx, pending, w, *got, positions.cuda(), req.cuda(), pages.cuda(), Hq, Hkv, hd, rotary, page)
+    ops.tc.check_errors()
+    for x, y, what in zip(got, want, "qkv"):
+        close(x, y, torch.bfloat16, what)
