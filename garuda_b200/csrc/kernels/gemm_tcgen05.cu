@@ -2323,7 +2323,7 @@ GB_EXPORT int gb_tc_selftest_wait_runs_out(int limit_us, cudaStream_t stream) {
 // [tiles_in, sums_ld] and eps, inv_width = 1 / features of the normed vector. As the producer
 // (accumulating products only): h_out [Mx, Nw] bfloat16, weight [Nw] 32-bit, sums_out [tiles_out, sums_ld] with
 // tiles_out = gb_gemm_tc_norm_tiles(Mx, Nw, K): all of its rows are written, and a product that would write
-// another number of them is refused. Unused halves are null.
+// another number of them is refused (0: the caller relies on that answer). Unused halves are null.
 struct GbNormFold {
   const float* sums_in;
   int tiles_in;
@@ -2429,7 +2429,7 @@ GB_EXPORT int gb_gemm_tc(const void* x, const void* w, void* out, int Mx, int Nw
     return gb::fail(GB_UNSUPPORTED, "gemm_tc: a norm is folded in behind accumulating products only (epilogue %d)", epi);
   TallShape tall;
   const bool takes_tall = (epi & 7) != EPI_SWIGLU && tall_plan(Mx, Nw, K, &tall);
-  if (ra.h_out != nullptr && norm->tiles_out != norm_tiles(Mx, Nw, takes_tall))
+  if (ra.h_out != nullptr && norm->tiles_out != 0 && norm->tiles_out != norm_tiles(Mx, Nw, takes_tall))
     return gb::fail(GB_BAD_ARGUMENT, "gemm_tc: %d rows of sums for the norm behind, the product writes %d", norm->tiles_out,
                     norm_tiles(Mx, Nw, takes_tall));
   CUtensorMap mm, mn;
