@@ -122,11 +122,6 @@ constexpr int CHUNK = 8;
 constexpr int SPLIT = 8;        // threads that share a column of S: thread `sub` holds the rows d with d % 8 == sub
 constexpr int REC_THREADS = 128, REC_COLS = REC_THREADS / SPLIT;
 
-__device__ __forceinline__ void cp_async_4(float* smem, const float* gmem) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s), "l"(gmem) : "memory");
-}
-
 // grid (H, R, ceil(vdim / 16)), 128 threads: 16 columns of S, eight threads a column. Each of the
 // eight sums its rows in ascending order and the eight are added as a tree, ((0 + 1) + (2 + 3)) +
 // ((4 + 5) + (6 + 7)): the same sums, in the same order, as the eight interleaved partial sums of
@@ -170,16 +165,16 @@ delta_recurrence_kernel(const float* __restrict__ prep, int W, const int32_t* __
       const int tt = i / dim, d = i % dim;
       const float* row = prep + (size_t)(c0 + tt) * W;
       float* to = dst + tt * tok_floats + (d % SPLIT) * per + d / SPLIT;
-      cp_async_4(to, row + off_q + d);
-      cp_async_4(to + SPLIT * per, row + off_k + d);
-      cp_async_4(to + 2 * SPLIT * per, row + off_g + d);
+      delta_chunk::copy_4(to, row + off_q + d);
+      delta_chunk::copy_4(to + SPLIT * per, row + off_k + d);
+      delta_chunk::copy_4(to + 2 * SPLIT * per, row + off_g + d);
     }
     for (int i = threadIdx.x; i < n * (ncols + 1); i += REC_THREADS) {
       const int tt = i / (ncols + 1), c = i % (ncols + 1);
       const float* row = prep + (size_t)(c0 + tt) * W;
       float* to = dst + tt * tok_floats + 3 * SPLIT * per;
-      if (c < ncols) cp_async_4(to + c, row + off_v + c);
-      else cp_async_4(to + REC_COLS, row + off_b);
+      if (c < ncols) delta_chunk::copy_4(to + c, row + off_v + c);
+      else delta_chunk::copy_4(to + REC_COLS, row + off_b);
     }
   };
   if (t0 < t1) fetch(t0, 0);
@@ -302,7 +297,7 @@ delta_chunk_factors_kernel(const float* __restrict__ proj, int P, const float* _
         for (int i = tid; i < n * (DIM / 4); i += 256)
           copy_16(to + i / (DIM / 4) * LD + i % (DIM / 4) * 4, from + (size_t)(i / (DIM / 4)) * pitch + i % (DIM / 4) * 4);
       } else {
-        for (int i = tid; i < n * DIM; i += 256) cp_async_4(to + i / DIM * LD + i % DIM, from + (size_t)(i / DIM) * pitch + i % DIM);
+        for (int i = tid; i < n * DIM; i += 256) delta_chunk::copy_4(to + i / DIM * LD + i % DIM, from + (size_t)(i / DIM) * pitch + i % DIM);
       }
     };
     const float* q0 = proj + (size_t)first * P + kvh * DIM;

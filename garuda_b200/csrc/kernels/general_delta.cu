@@ -67,11 +67,6 @@ constexpr int SPLIT = 8;        // threads that share a column of S: thread `sub
 constexpr int REC_THREADS = 128, REC_COLS = REC_THREADS / SPLIT;
 constexpr int VECS = 5;         // r, u, w, a*u, k
 
-__device__ __forceinline__ void cp_async_4(float* smem, const float* gmem) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s), "l"(gmem) : "memory");
-}
-
 // grid (H, R, ceil(vdim / 16)), 128 threads: 16 columns of S, eight threads a column. Each of the
 // eight sums its rows in ascending order and the eight are added as a tree, ((0 + 1) + (2 + 3)) +
 // ((4 + 5) + (6 + 7)): the same sums, in the same order, as the eight interleaved partial sums of
@@ -111,11 +106,11 @@ gdelta_recurrence_kernel(const float* __restrict__ prep, int W, const int32_t* _
       const float* row = prep + (size_t)(c0 + tt) * W + h * dim + d;
       float* to = dst + tt * tok_floats + (d % SPLIT) * per + d / SPLIT;
 #pragma unroll
-      for (int v = 0; v < VECS; ++v) cp_async_4(to + v * SPLIT * per, row + v * HD);
+      for (int v = 0; v < VECS; ++v) delta_chunk::copy_4(to + v * SPLIT * per, row + v * HD);
     }
     for (int i = threadIdx.x; i < n * ncols; i += REC_THREADS) {
       const int tt = i / ncols, c = i % ncols;
-      cp_async_4(dst + tt * tok_floats + VECS * SPLIT * per + c, prep + (size_t)(c0 + tt) * W + off_v + c);
+      delta_chunk::copy_4(dst + tt * tok_floats + VECS * SPLIT * per + c, prep + (size_t)(c0 + tt) * W + off_v + c);
     }
   };
   if (t0 < t1) fetch(t0, 0);
