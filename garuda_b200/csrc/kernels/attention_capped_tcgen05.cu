@@ -13,7 +13,7 @@
 //              bfloat16 over the scores read. The sink joins the denominator at the end.
 // What bounds it: instruction issue of the softmax warps. The cap's polynomial is nine operations a score, taken two scores an
 // instruction (f32x2); a score's exponential and sum are four more. A prompt of 2,048 tokens, 32 heads over 4 of 64, window 1,024, cap 30 and
-// sink: 126 us with mma.sync, 79 here, behind a flushed L2 (a branch a pair of scores for those beyond the cap, which the fetch of instructions waited for, cost 17
+// sink: 126 us with mma.sync, 79 here, behind a flushed L2 (72 in a row, since products are issued by an elected lane; a branch a pair of scores for those beyond the cap, which the fetch of instructions waited for, cost 17
 // more).
 // Every wait is bounded; a wait that runs out sets the error word and the CTA winds down.
 #include "attention_capped.cuh"

@@ -19,7 +19,7 @@
 // its last, and the tensor cores' sums, which are cut off and not rounded, are of eight products only: those pieces, and a
 // chunk's update of the state, are added by rounded 32-bit operations. With sums of 32 products in the tensor cores the read-outs and the
 // state of 2,048 tokens were 1.2 to 1.4 times as far from 64 bits as the token-by-token kernels' where decays forget within some tens of tokens;
-// now 0.7 to 1.1 times, at 237 us against 234 for the channel rule's kernels.
+// by pieces 0.7 to 1.1 times, at 237 us against 234 for the channel rule's kernels.
 //
 // Why this split: the token-by-token kernels are bound by a token's chain of dependent sums and shuffles (0.43 us a
 // token of 16 heads of 128 x 128, whatever the tokens do); a chunk's three products have no chain. On multiply-adds instead of the

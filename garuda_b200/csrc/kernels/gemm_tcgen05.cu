@@ -2189,7 +2189,11 @@ constexpr int few_token_limit() { return 256; }
 
 // More than 64 tokens: whether CTA pairs take the product, and the tile width over the weight's rows.
 // Pairs pay from about a thousand tokens (768: 3.9 ms a step with pairs, 3.4 without; 1,024: 4.4 against 4.5):
-// below that their 256 x 256 tiles are too few for the 74 pairs.
+// below that their 256 x 256 tiles are too few for the 74 pairs. That line is of whole steps and older than the kernel of token blocks
+// (tall_plan) and than issue by an elected lane, which gains the pairs more. What is left for this rule, stored in bfloat16, us with single CTAs against
+// pairs at 520 / 640 / 768 / 900 / 1,024 / 1,200 tokens: 2,048 features of 2,048 channels, 14 / 14 / 14 / 14 / 14 / 16 against 12 / 12 / 13 / 17 /
+// 16 / 18; 11,264 of 2,048, 45 / 44 / 40 / 68 / 62 / 53 against 36 / 35 / 35 / 44 / 43 / 44; 28,672 of 4,096, 127 / 131 / 186 / 351 / 306 /
+// 278 against 121 / 155 / 155 / 178 / 173 / 228.
 bool many_token_pairs(int tokens, int weight_rows, int epi = -1) {
   if (weight_rows < 256) return false;
   if (tokens >= 8 * BM) return true;
@@ -2212,12 +2216,13 @@ int many_token_width(int tokens, int weight_rows, int epi = -1) {
 // Whether a gated product takes the wide tiles: where their rounds over the pairs fetch fewer bytes a CTA than the other tiles' rounds
 // do (KB a step of 64 channels: a wide tile 16 of weights and an eighth of a part's tokens, the others 32 or, one CTA's 256 columns,
 // 48), a wide tile's epilogue, which its one accumulator stage leaves bare, counted at the 14 us in which a CTA fetches 1,050 KB.
-// In us, other tiles against wide ones, for 257 / 333 / 448 / 512 tokens: 2 x 14,336 rows of 4,096 channels, four rounds against
-// two, 115 / 117 / 118 / 118 against 96 / 102 / 109 / 119; 2 x 9,472 rows of 4,096, two against one, 68 / 68 / 70 / 70 against 56 /
-// 60 / 64 / -; 2 x 28,672 rows of 8,192, 370 / 377 / 387 / 413 against 319 / 344 / 375 / 399; where the line says no: 2 x 11,008 rows
-// of 4,096, three against two, 91 / 91 / 92 / 92 against 94 / 101 / 106 / -; 2 x 8,192 rows of 2,048, 41 / 41 / 42 / 43 against 37 /
-// 40 / 43 / 45. (Taken one call at a time behind a flushed L2. The activation's reciprocals have been rounded since: of calls that follow one another, 333
-// tokens of the first shape, SiLU 94 us then and 96 now, gelu 98 and 103.)
+// In us, other tiles against wide ones, for 257 / 333 / 448 / 512 tokens, one call at a time behind a flushed L2 (when the line was drawn): 2 x 14,336
+// rows of 4,096 channels, four rounds against two, 115 / 117 / 118 / 118 against 96 / 102 / 109 / 119; 2 x 9,472 rows of 4,096, two against
+// one, 68 / 68 / 70 / 70 against 56 / 60 / 64 / -; 2 x 28,672 rows of 8,192, 370 / 377 / 387 / 413 against 319 / 344 / 375 / 399. Since then the
+// other tiles' gated epilogue has lost its branch and both are issued by an elected lane. Calls that follow one another over weights that L2
+// does not hold: 90 / 93 / 101 / 103 against 74 / 92 / 116 / 129; 56 / 55 / 58 / 63 against 44 / 52 / 64 / 75; 341 / 348 / 373 / 364 against
+// 296 / 383 / 483 / 503: there the line, which has stayed, lies some 100 tokens high. Where it says no: 2 x 11,008 rows of 4,096, three
+// against two, 80 / 78 / 75 / 76 against 82 / 95 / 103 / 121; 2 x 8,192 rows of 2,048, 31 / 30 / 30 / 30 against 28 / 31 / 36 / 40.
 bool wide_gated(int tokens, int weight_rows, int K) {
   if (tokens <= few_token_limit() || tokens > W_TOKENS || weight_rows < 2 * BM) return false;
   const int sms = sm_count(), pairs = sms / 2;

@@ -18,7 +18,7 @@
 // What bounds it: the products (18 of 128 x 64 x 16 for the scores, each as long as one of 128 columns, and 4 of 128 x 256 x 16 a tile,
 // about 1,800 cycles), which the softmax of one group of 128 threads fits under; tiles of 128 keys would halve the scores' products but
 // not leave room for two of them. A prompt of 2,048 tokens,
-// 32 heads over rows of 256 + 32 channels: 350 us with mma.sync, 103 here (calls in a row).
+// 32 heads over rows of 256 + 32 channels: 350 us with mma.sync, 97 here (calls in a row; 103 before products were issued by an elected lane).
 // Every wait is bounded; a wait that runs out sets the error word and the CTA winds down.
 #include "error_word.cuh"
 #include "tc_common.cuh"

@@ -1224,9 +1224,11 @@ class CudaOps:
     DELTA_CHUNK_CUT = 48
     #: The same for the generalized rule of up to 64 channels and of more, whose tokens walked one by one cost less: (from how many tokens on,
     #: from how many the step's longest request must have where there are shorter ones beside it, in a step of fewer than 256 tokens). us
-    #: token by token / by chunks, 32 heads, one request: 64 channels, 48 tokens 29 / 47, 100 43 / 50, 128 52 / 51, 200 72 / 56; 128 channels, 48 50 /
-    #: 50, 64 60 / 51. Beside a single token: 64 channels, 128 tokens 60 / 65, 200 86 / 70; 128 channels, 64 tokens 69 / 72, 100 96 / 80;
-    #: beside 40 tokens: 64 channels, 200 tokens 88 / 84; 128 channels, 64 tokens 76 / 103, 100 103 / 110.
+    #: token by token / by chunks, 32 heads, one request: 64 channels, 48 tokens 24 / 25, 64 29 / 24, 100 40 / 26, 128 48 / 29, 200 69 / 34; 128
+    #: channels, 48 45 / 36, 64 55 / 37. Beside a single token: 64 channels, 64 tokens 34 / 34, 128 56 / 43, 200 82 / 53; 128 channels, 48
+    #: tokens 52 / 54, 64 65 / 54, 100 91 / 61; beside 40 single tokens: 64 channels, 64 tokens 53 / 54, 128 82 / 61; 128 channels, 48 125 / 135, 64 140 /
+    #: 136, 100 170 / 143. The lines were drawn when a chunk's factors took 1.5 times as long (64 channels, 128 tokens: 52 / 51) and have
+    #: stayed: by now the chunks are the faster ones from about 60 tokens on.
     GENERAL_CHUNK_CUTS = ((128, 160), (48, 100))
 
     def _delta_walked(self, b, out, cut: int, mixed: int = 0) -> int:
