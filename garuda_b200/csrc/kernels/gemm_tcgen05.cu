@@ -2253,7 +2253,8 @@ bool rotates_320(int tokens, int features, int head_dim) {
 // head_dim above 0: the rotating product, whose epilogue weighs more in every kernel and which has tiles of 320 columns to go to. us, other
 // tiles against these: 2,560 x 2,048, 19.7 / 28.5 / 34.5 / 34.5 / 45.4 at 512 / 1,024 / 1,793 / 2,048 / 2,400 tokens against 15.9 / 24.2 / 30.3 /
 // 34.3 / 34.2 (2,048 stays with the 320-wide tiles, as does 2,300, 34.7 against 36.0); 6,144 x 4,096, 44 / 72 / 76 at 512 / 1,024 / 1,221
-// against 34 / 54 / 67, where it says no: 73 against 80 at 1,511; 1,536 x 2,048, 34.7 against 41.5 at 3,500, no either.
+// against 34 / 54 / 67, where it says no: 73 against 80 at 1,511; 1,536 x 2,048, 34.7 against 41.5 at 3,500, no either (heads of 64; of 128, 6,144 x
+// 4,096, 43 / 61 / 61 against 35 / 52 / 60, no: 63 against 74 at 1,511; 3,072 x 3,072, 50 against 38 at 1,793, no: 51 against 53 at 2,600).
 bool tall_plan(int tokens, int features, int K, TallShape* best, int head_dim = 0) {
   if (tokens <= few_token_limit() || features < 2 * BM) return false;
   const int sms = sm_count(), pairs = sms / 2, kb = (K + BK - 1) / BK;
@@ -2262,8 +2263,10 @@ bool tall_plan(int tokens, int features, int K, TallShape* best, int head_dim = 
   const int tiles_m = (tokens + BM - 1) / BM;
   long long cost;
   if (many_token_pairs(tokens, features)) {
+    const long long n = rounds((tokens + 255) / 256 * ((features + 255) / 256), pairs);
+    cost = n * kb * 670 + 12500;
     if (rotates && rotates_320(tokens, features, head_dim)) cost = rounds((tokens + 255) / 256 * ((features + 319) / 320), pairs) * (kb * 940 + 23000) + 12500;
-    else cost = rounds((tokens + 255) / 256 * ((features + 255) / 256), pairs) * (kb * 670 + (rotates ? 20000 : 0)) + 12500;
+    else if (rotates) cost += head_dim == 128 ? 17000 + 10000 * (n - 1) : 20000 * n;       // (two heads a tile: half of a second round's hides)
     if (rotates) cost = cost * 19 / 20;
   } else if (pick_tile_width(tokens, features) == 128) {           // more rows of tiles share what L2 holds
     cost = rounds(tiles_m * ((features + 127) / 128), sms) * (kb * (350 + 600 / tiles_m) + (rotates ? 10000 : 0)) + 7700;

@@ -37,7 +37,8 @@ def test_the_rotating_product_goes_where_it_is_faster(ops):
     """Its epilogue weighs more in these blocks than in the tiles that it would take otherwise, 320 wide ones among them."""
     takes = lambda T, N, K, hd: ops.tc.lib.gb_gemm_tc_tall_rotating(T, N, K, hd) > 0
     assert all(takes(*c) for c in [(257, 1536, 2048, 64), (1793, 2560, 2048, 64), (2400, 2560, 2048, 64), (1221, 6144, 4096, 128)])
-    others = [(2048, 2560, 2048, 64), (2300, 2560, 2048, 64), (1511, 6144, 4096, 128), (3500, 1536, 2048, 64)]
+    others = [(2048, 2560, 2048, 64), (2300, 2560, 2048, 64), (1511, 6144, 4096, 128), (3500, 1536, 2048, 64), (3500, 1536, 2048, 128),
+              (2600, 3072, 3072, 128)]
     assert not any(takes(*c) for c in others) and all(ops.tc.lib.gb_gemm_tc_tall(*c[:3]) > 0 for c in others)
 
 
